@@ -6,7 +6,7 @@
 #include "common.cuh"
 
 template <typename T>
-__global__ void silu_mul_kernel(const T* __restrict__ gu, T* __restrict__ out, long long n_tokens, int inter) {
+__global__ void silu_mul_kernel(const T* gu, T* out, long long n_tokens, int inter) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -20,7 +20,7 @@ __global__ void silu_mul_kernel(const T* __restrict__ gu, T* __restrict__ out, l
 }
 
 // bfloat16, 8 elements per thread; inter % 8 == 0.
-__global__ void silu_mul_bf16x8_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out,
+__global__ void silu_mul_bf16x8_kernel(const __nv_bfloat16* gu, __nv_bfloat16* out,
                                        long long n_tokens, int inter) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
@@ -66,7 +66,7 @@ PB_API int pb_silu_mul(const void* gate_up, void* out, int dtype, int n_tokens, 
 //   a = min(gu[t, i], limit), b = clamp(gu[t, I + i], -limit, limit), out[t, i] = a * sigmoid(alpha * a) * (b + 1)
 // in float32, rounded once.
 template <typename T>
-__global__ void clamped_glu_kernel(const T* __restrict__ gu, T* __restrict__ out, long long n_tokens, int inter,
+__global__ void clamped_glu_kernel(const T* gu, T* out, long long n_tokens, int inter,
                                    float limit, float alpha) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
@@ -96,7 +96,7 @@ PB_API int pb_clamped_glu(const void* gate_up, void* out, int dtype, int n_token
 
 // tanh, element by element in float32 (the squashing between the two small products of a learned decay).
 template <typename T>
-__global__ void tanh_kernel(const T* __restrict__ x, T* __restrict__ out, long long n) {
+__global__ void tanh_kernel(const T* x, T* out, long long n) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -116,7 +116,7 @@ PB_API int pb_tanh(const void* x, void* out, int dtype, long long n, cudaStream_
 //   out[t, i] = gelu(gu[t, i]) * gu[t, I + i],  gelu(g) = 0.5 g (1 + tanh(sqrt(2 / pi) (g + 0.044715 g^3)))
 // in float32, rounded once.
 template <typename T>
-__global__ void gelu_tanh_mul_kernel(const T* __restrict__ gu, T* __restrict__ out, long long n_tokens, int inter) {
+__global__ void gelu_tanh_mul_kernel(const T* gu, T* out, long long n_tokens, int inter) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -129,7 +129,7 @@ __global__ void gelu_tanh_mul_kernel(const T* __restrict__ gu, T* __restrict__ o
 }
 
 // bfloat16, 8 elements per thread; inter % 8 == 0.
-__global__ void gelu_tanh_mul_bf16x8_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out,
+__global__ void gelu_tanh_mul_bf16x8_kernel(const __nv_bfloat16* gu, __nv_bfloat16* out,
                                             long long n_tokens, int inter) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
@@ -174,7 +174,7 @@ PB_API int pb_gelu_tanh_mul(const void* gate_up, void* out, int dtype, int n_tok
 
 // SiLU in place on the first `cols` columns of rows `ld` apart, float32 arithmetic, one rounding.
 template <typename T>
-__global__ void silu_cols_kernel(T* __restrict__ x, long long ld, long long n_tokens, int cols) {
+__global__ void silu_cols_kernel(T* x, long long ld, long long n_tokens, int cols) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -185,7 +185,7 @@ __global__ void silu_cols_kernel(T* __restrict__ x, long long ld, long long n_to
 }
 
 // bfloat16, 8 elements per thread; cols % 8 == 0, ld % 8 == 0, x 16-byte aligned.
-__global__ void silu_cols_bf16x8_kernel(__nv_bfloat16* __restrict__ x, long long ld, long long n_tokens, int cols) {
+__global__ void silu_cols_bf16x8_kernel(__nv_bfloat16* x, long long ld, long long n_tokens, int cols) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -224,7 +224,7 @@ PB_API int pb_silu_cols(void* x, long long ld, int dtype, int n_tokens, int cols
 // ReLU-gated product on a merged gate/up projection: out[t, i] = max(gu[t, i], 0) * gu[t, I + i], float32, one rounding.
 // V elements per thread (8 of bfloat16, 4 of float32 in 16-byte accesses; inter % V == 0).
 template <typename T, int V>
-__global__ void relu_mul_kernel(const T* __restrict__ gu, T* __restrict__ out, long long n_tokens, int inter) {
+__global__ void relu_mul_kernel(const T* gu, T* out, long long n_tokens, int inter) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -267,7 +267,7 @@ PB_API int pb_relu_mul(const void* gate_up, void* out, int dtype, int n_tokens, 
 
 // Squared ReLU in place on a dense array: x = max(x, 0)^2, float32, one rounding.
 template <typename T, int V>
-__global__ void relu2_kernel(T* __restrict__ x, long long n) {
+__global__ void relu2_kernel(T* x, long long n) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     const long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * V;
@@ -299,7 +299,7 @@ PB_API int pb_relu2_(void* x, int dtype, long long n, cudaStream_t stream) {
 
 // A gate per element, in place: y[t, i] *= sigmoid(gate[t, i]) for columns of two row-major arrays, float32, one rounding.
 template <typename T, int V>
-__global__ void __launch_bounds__(256) sigmoid_gate_kernel(T* __restrict__ y, long long ldy, const T* __restrict__ gate, long long ldg, int cols) {
+__global__ void __launch_bounds__(256) sigmoid_gate_kernel(T* y, long long ldy, const T* gate, long long ldg, int cols) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     const size_t t = blockIdx.x;

@@ -42,13 +42,13 @@ template <> struct Chunk<__nv_bfloat16> {
 };
 
 template <typename T, int VPL>
-__global__ void attention_paged_kernel(const T* __restrict__ q, const T* __restrict__ k_pages, const T* __restrict__ v_pages,
-                                       T* __restrict__ out, const float* __restrict__ sink, const int32_t* __restrict__ positions,
-                                       const int32_t* __restrict__ table_row, const int32_t* __restrict__ block_table,
+__global__ void attention_paged_kernel(const T* q, const T* k_pages, const T* v_pages,
+                                       T* out, const float* sink, const int32_t* positions,
+                                       const int32_t* table_row, const int32_t* block_table,
                                        int table_stride, int page_size, int num_pages, int n_tokens, int H, int G, int kd, int vd,
                                        int v_row, int Gv, float scale, int window, int keep_first, int chunk, float softcap,
-                                       const T* __restrict__ gate, long long ld_gate, int swizzle_k, int swizzle_v, int vec,
-                                       int* __restrict__ status) {
+                                       const T* gate, long long ld_gate, int swizzle_k, int swizzle_v, int vec,
+                                       int* status) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     extern __shared__ float q_all[];

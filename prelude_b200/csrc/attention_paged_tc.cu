@@ -315,10 +315,10 @@ __global__ void __launch_bounds__(256, 2) attention_paged_tc_kernel(TcParams p) 
 // exp(m_s - M) / L are made once, by the first warp; then every thread adds up its columns, the loads of all parts
 // in flight together.
 #define TC_MAX_SPLITS 64
-__global__ void __launch_bounds__(128) attention_paged_tc_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
-                                                                       const float* __restrict__ sink, const int32_t* __restrict__ table_row,
-                                                                       const bf16* __restrict__ gate, long long ld_gate,
-                                                                       bf16* __restrict__ out, int H, int vd, int splits) {
+__global__ void __launch_bounds__(128) attention_paged_tc_merge_kernel(const float* part_o, const float* part_ml,
+                                                                       const float* sink, const int32_t* table_row,
+                                                                       const bf16* gate, long long ld_gate,
+                                                                       bf16* out, int H, int vd, int splits) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     __shared__ float w_s[TC_MAX_SPLITS];

@@ -23,10 +23,10 @@
 
 template <typename T>
 __global__ void paged_attention_warp_kernel(
-    const T* __restrict__ q, const T* __restrict__ k_pages, const T* __restrict__ v_pages, T* __restrict__ out,
-    const int32_t* __restrict__ positions, const int32_t* __restrict__ token_seq,
-    const int32_t* __restrict__ block_table, int table_stride, int page_size, int num_pages, int n_tokens,
-    int n_heads, int n_kv_heads, int head_dim, float scale, int window, int swizzle, int* __restrict__ status) {
+    const T* q, const T* k_pages, const T* v_pages, T* out,
+    const int32_t* positions, const int32_t* token_seq,
+    const int32_t* block_table, int table_stride, int page_size, int num_pages, int n_tokens,
+    int n_heads, int n_kv_heads, int head_dim, float scale, int window, int swizzle, int* status) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     __shared__ float q_s[ATTN_REF_WARPS][ATTN_REF_MAX_D];

@@ -33,9 +33,9 @@ __device__ __forceinline__ float gd_softplus(float x) { return x > 20.0f ? x : l
 
 template <typename T, int NPL>
 __global__ void __launch_bounds__(256)
-gated_delta_scan_kernel(const T* __restrict__ u_in, long long ld_u, const T* __restrict__ b_in, long long ld_b, const T* __restrict__ a_in,
-                        long long ld_a, const float* __restrict__ a_log, const float* __restrict__ dt_bias, float* __restrict__ state,
-                        float* __restrict__ y, const int32_t* __restrict__ cu_q, const int32_t* __restrict__ slots, int H, int G, int D,
+gated_delta_scan_kernel(const T* u_in, long long ld_u, const T* b_in, long long ld_b, const T* a_in,
+                        long long ld_a, const float* a_log, const float* dt_bias, float* state,
+                        float* y, const int32_t* cu_q, const int32_t* slots, int H, int G, int D,
                         int E) {
     constexpr int NPAD = NPL * GD_LANES;
     constexpr int CHUNK = NPL == 32 ? 8 : 16;

@@ -26,11 +26,11 @@
 #define DA_WARPS 4
 
 template <typename T>
-__global__ void kv_write_pages_kernel(const T* __restrict__ k, long long k_stride, const T* __restrict__ v, long long v_stride,
-                                      T* __restrict__ k_pages, T* __restrict__ v_pages, const int32_t* __restrict__ positions,
-                                      const int32_t* __restrict__ token_row, const int32_t* __restrict__ block_table,
+__global__ void kv_write_pages_kernel(const T* k, long long k_stride, const T* v, long long v_stride,
+                                      T* k_pages, T* v_pages, const int32_t* positions,
+                                      const int32_t* token_row, const int32_t* block_table,
                                       int table_stride, int page_size, int num_pages, int n_k_heads, int dk, int n_v_heads,
-                                      int dv, int k_swizzle, int v_swizzle, int* __restrict__ status) {
+                                      int dv, int k_swizzle, int v_swizzle, int* status) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     const int t = blockIdx.x;
@@ -81,12 +81,12 @@ __host__ __device__ __forceinline__ float pb_query_temperature(int pos, float co
 
 template <typename T>
 __global__ void diff_attention_warp_kernel(
-    const T* __restrict__ q, long long q_stride, const T* __restrict__ gate, long long gate_stride,
-    const T* __restrict__ k_pages, const T* __restrict__ v_pages, T* __restrict__ out,
-    const int32_t* __restrict__ positions, const int32_t* __restrict__ token_row, const int32_t* __restrict__ block_table,
+    const T* q, long long q_stride, const T* gate, long long gate_stride,
+    const T* k_pages, const T* v_pages, T* out,
+    const int32_t* positions, const int32_t* token_row, const int32_t* block_table,
     int table_stride, int page_size, int num_pages, int n_tokens, int n_heads, int n_kv_heads, int dim, int vdim,
     float scale, float temp_coef, int temp_every, float lambda, float norm_eps, float out_scale, int window,
-    int k_swizzle, int v_swizzle, int* __restrict__ status) {
+    int k_swizzle, int v_swizzle, int* status) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     __shared__ float q_s[DA_WARPS][2][DA_MAX_D];

@@ -62,9 +62,9 @@ __device__ __forceinline__ void dt_st(__nv_bfloat16* p, const float (&v)[V]) {
 // x: n_parts arrays, part_stride elements apart, whose sum (in ascending order) is added; a block has blockDim.x * V columns
 // of one row
 template <typename TX, typename TY, int V>
-__global__ void __launch_bounds__(256) add_tanh_kernel(const TX* __restrict__ x, int n_parts, size_t part_stride, float* __restrict__ res,
-                                                       const int32_t* __restrict__ rows, int n_rows_total, float slope,
-                                                       const float* __restrict__ w, const float* __restrict__ b, TY* __restrict__ y, int width) {
+__global__ void __launch_bounds__(256) add_tanh_kernel(const TX* x, int n_parts, size_t part_stride, float* res,
+                                                       const int32_t* rows, int n_rows_total, float slope,
+                                                       const float* w, const float* b, TY* y, int width) {
     pb_grid_dep_launch();
     const int c = (blockIdx.y * blockDim.x + threadIdx.x) * V;
     if (c >= width) return;

@@ -6,8 +6,8 @@
 #include "common.cuh"
 
 template <typename T>
-__global__ void embed_gather_kernel(const int32_t* __restrict__ ids, const T* __restrict__ table,
-                                    float* __restrict__ out, int n_tokens, int width, int vocab) {
+__global__ void embed_gather_kernel(const int32_t* ids, const T* table,
+                                    float* out, int n_tokens, int width, int vocab) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     int t = blockIdx.x;
@@ -23,8 +23,8 @@ __global__ void embed_gather_kernel(const int32_t* __restrict__ ids, const T* __
 }
 
 // bfloat16 rows, 8 elements per thread and access; needs width % 8 == 0.
-__global__ void embed_gather_bf16x8_kernel(const int32_t* __restrict__ ids, const __nv_bfloat16* __restrict__ table,
-                                           float* __restrict__ out, int n_tokens, int width, int vocab) {
+__global__ void embed_gather_bf16x8_kernel(const int32_t* ids, const __nv_bfloat16* table,
+                                           float* out, int n_tokens, int width, int vocab) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     int t = blockIdx.x;
@@ -65,9 +65,9 @@ PB_API int pb_embed_gather(const int32_t* ids, const void* table, int table_dtyp
 // and a rate; it and its sine and cosine are taken in 64-bit, so that a position in the thousands loses nothing
 // to the rounding of the angle, and the sum is rounded once to the float32 residual stream.
 template <typename T>
-__global__ void embed_sinusoid_kernel(const int32_t* __restrict__ ids, const int32_t* __restrict__ positions,
-                                      const T* __restrict__ table, const double* __restrict__ rate,
-                                      float* __restrict__ out, int n_tokens, int width, int vocab) {
+__global__ void embed_sinusoid_kernel(const int32_t* ids, const int32_t* positions,
+                                      const T* table, const double* rate,
+                                      float* out, int n_tokens, int width, int vocab) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     int t = blockIdx.x;
@@ -101,8 +101,8 @@ PB_API int pb_embed_sinusoid(const int32_t* ids, const int32_t* positions, const
 
 // The same with every row multiplied by a constant: res[t, :] = table[ids[t], :] * scale (the product in float32).
 template <typename T>
-__global__ void embed_gather_scaled_kernel(const int32_t* __restrict__ ids, const T* __restrict__ table, float scale,
-                                           float* __restrict__ out, int n_tokens, int width, int vocab) {
+__global__ void embed_gather_scaled_kernel(const int32_t* ids, const T* table, float scale,
+                                           float* out, int n_tokens, int width, int vocab) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     const int t = blockIdx.x;

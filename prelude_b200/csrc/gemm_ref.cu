@@ -19,8 +19,8 @@
 #define GR_BK 16
 
 template <typename TA, typename TW, typename TC>
-__global__ void __launch_bounds__(256) gemm_ref_kernel(const TA* __restrict__ A, const TW* __restrict__ W,
-                                                       const float* __restrict__ bias, TC* __restrict__ C, int M,
+__global__ void __launch_bounds__(256) gemm_ref_kernel(const TA* A, const TW* W,
+                                                       const float* bias, TC* C, int M,
                                                        int N, int K, long long lda, long long ldw, long long ldc,
                                                        long long batch_a, long long batch_w, long long batch_c) {
     pb_grid_dep_launch();

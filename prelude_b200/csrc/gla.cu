@@ -63,8 +63,8 @@ __device__ __forceinline__ float gla_decay(float z, float inv_tau) {
 // over the rank runs in ascending order (as in gla_step_kernel).
 #define DECAY_TOKENS 8
 template <typename T>
-__global__ void __launch_bounds__(128) channel_decay_kernel(const T* __restrict__ x1, long long ld_x1, const T* __restrict__ w2,
-                                                            const float* __restrict__ bias, float inv_tau, float* __restrict__ out, int n_tokens,
+__global__ void __launch_bounds__(128) channel_decay_kernel(const T* x1, long long ld_x1, const T* w2,
+                                                            const float* bias, float inv_tau, float* out, int n_tokens,
                                                             int channels, int rank, int vec) {
     extern __shared__ __align__(16) float xs[];                // [DECAY_TOKENS][rank]
     pb_grid_dep_launch();
@@ -155,9 +155,9 @@ __device__ __forceinline__ int lanes_first(int j) {
 
 template <typename T, int RL, int R, int C, int CHUNK>
 __global__ void __launch_bounds__(256, 1)
-gla_scan_kernel(const T* __restrict__ q_in, const T* __restrict__ k_in, const T* __restrict__ v_in, long long ld, const float* __restrict__ decay,
-                float scale, float* __restrict__ state, float* __restrict__ y, const int32_t* __restrict__ cu_q,
-                const int32_t* __restrict__ slots, int H, int N, int P, int vec, int vec_state) {
+gla_scan_kernel(const T* q_in, const T* k_in, const T* v_in, long long ld, const float* decay,
+                float scale, float* state, float* y, const int32_t* cu_q,
+                const int32_t* slots, int H, int N, int P, int vec, int vec_state) {
     constexpr int NPAD = RL * R;
     constexpr int COLS = 4 * (32 / RL) * C;                    // of a block
     constexpr int BUF = CHUNK * (3 * NPAD + COLS);             // floats per half: k, q, decay, v
@@ -394,10 +394,10 @@ gla_scan_kernel(const T* __restrict__ q_in, const T* __restrict__ k_in, const T*
 #define STEP_ROWS 8
 template <typename T>
 __global__ void __launch_bounds__(STEP_THREADS)
-gla_step_kernel(const T* __restrict__ q_in, const T* __restrict__ k_in, const T* __restrict__ v_in, const T* __restrict__ x1,
-                const T* __restrict__ gate, long long ld, const T* __restrict__ w2, const float* __restrict__ bias, float inv_tau, float scale,
-                const float* __restrict__ norm_w, float eps, float* __restrict__ state, T* __restrict__ out, const int32_t* __restrict__ cu_q,
-                const int32_t* __restrict__ slots, int H, int N, int P, int rank, int vec) {
+gla_step_kernel(const T* q_in, const T* k_in, const T* v_in, const T* x1,
+                const T* gate, long long ld, const T* w2, const float* bias, float inv_tau, float scale,
+                const float* norm_w, float eps, float* state, T* out, const int32_t* cu_q,
+                const int32_t* slots, int H, int N, int P, int rank, int vec) {
     extern __shared__ __align__(16) float step_sm[];           // k, q, decay [N] each; outputs [row groups][P]; sums
     __shared__ float red[STEP_THREADS / 32];
     pb_grid_dep_launch();

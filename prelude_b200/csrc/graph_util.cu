@@ -9,8 +9,8 @@
 #include "common.cuh"
 
 // dst[idx[i]] = val[i]; an index outside [0, dst_len) is skipped and raises *status.
-__global__ void scatter_i32_kernel(int32_t* __restrict__ dst, long long dst_len, const int32_t* __restrict__ idx,
-                                   const int32_t* __restrict__ val, int n, int* __restrict__ status) {
+__global__ void scatter_i32_kernel(int32_t* dst, long long dst_len, const int32_t* idx,
+                                   const int32_t* val, int n, int* status) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -36,9 +36,9 @@ PB_API int pb_scatter_i32(int32_t* dst, long long dst_len, const int32_t* idx, c
 // After a decode step: the sampled token becomes the next input, positions and
 // sampling counters move on by one (and with them the count of tokens in the cache).  Lets a captured step run again and again
 // without the host in between.
-__global__ void decode_advance_kernel(int32_t* __restrict__ tokens, int32_t* __restrict__ positions,
-                                      int32_t* __restrict__ kv_len, long long* __restrict__ counters,
-                                      const int32_t* __restrict__ sampled, int n, int max_positions) {
+__global__ void decode_advance_kernel(int32_t* tokens, int32_t* positions,
+                                      int32_t* kv_len, long long* counters,
+                                      const int32_t* sampled, int n, int max_positions) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     int i = blockIdx.x * blockDim.x + threadIdx.x;

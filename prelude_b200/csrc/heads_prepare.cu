@@ -22,8 +22,8 @@ namespace {
 // norm: 0 none; 1 before the rotation (what is rotated is x / rms(x) * w); 2 after it (rotated(x) / rms(rotated(x)) * w).
 // A null w is a scale of ones.
 template <typename T>
-__device__ __forceinline__ void prepare_head(const T* __restrict__ in, T* __restrict__ out, int size, int norm, const float* __restrict__ w,
-                                             float eps, const float* __restrict__ cs, int rot_dims, int adjacent, int lane) {
+__device__ __forceinline__ void prepare_head(const T* in, T* out, int size, int norm, const float* w,
+                                             float eps, const float* cs, int rot_dims, int adjacent, int lane) {
     float inv = 1.0f;
     if (norm == 1) {
         float ss = 0.f;
@@ -56,15 +56,15 @@ __device__ __forceinline__ void prepare_head(const T* __restrict__ in, T* __rest
 }
 
 template <typename T>
-__global__ void heads_prepare_kernel(const T* __restrict__ q_in, long long ldq, const T* __restrict__ k_in, long long ldk,
-                                     const T* __restrict__ v_in, long long ldv, const float* __restrict__ q_w,
-                                     const float* __restrict__ k_w, int norm, float eps, const float* __restrict__ rates,
-                                     float amplitude, int rot_dims, int adjacent, const T* __restrict__ v_other, T* __restrict__ v_copy,
+__global__ void heads_prepare_kernel(const T* q_in, long long ldq, const T* k_in, long long ldk,
+                                     const T* v_in, long long ldv, const float* q_w,
+                                     const float* k_w, int norm, float eps, const float* rates,
+                                     float amplitude, int rot_dims, int adjacent, const T* v_other, T* v_copy,
                                      long long ld_other, float mix,
-                                     const int32_t* __restrict__ positions, const int32_t* __restrict__ table_row,
-                                     const int32_t* __restrict__ block_table, int table_stride, int page_size, int num_pages,
-                                     T* __restrict__ q_out, T* __restrict__ k_pages, T* __restrict__ v_pages, int H, int qd, int G,
-                                     int kd, int Gv, int vd, int* __restrict__ status) {
+                                     const int32_t* positions, const int32_t* table_row,
+                                     const int32_t* block_table, int table_stride, int page_size, int num_pages,
+                                     T* q_out, T* k_pages, T* v_pages, int H, int qd, int G,
+                                     int kd, int Gv, int vd, int* status) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     extern __shared__ float cs[];                          // cosine and sine of the token's angles

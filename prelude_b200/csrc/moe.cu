@@ -58,8 +58,8 @@ __device__ __forceinline__ void pb_ld16(const T* p, float (&out)[N]) { pb_unpack
 // float32, or bfloat16 whose products fit), float32 sums.  A warp takes a token and four experts; a lane sums every
 // 32nd element in ascending order and the lanes meet in a fixed tree, so the order depends on K alone.
 template <typename T>
-__global__ void __launch_bounds__(128) router_logits_kernel(const T* __restrict__ x, long long ldx, const T* __restrict__ W,
-                                                            float* __restrict__ out, int n_tokens, int n_experts, int K) {
+__global__ void __launch_bounds__(128) router_logits_kernel(const T* x, long long ldx, const T* W,
+                                                            float* out, int n_tokens, int n_experts, int K) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     const int lane = threadIdx.x & 31;
@@ -87,8 +87,8 @@ __global__ void __launch_bounds__(128) router_logits_kernel(const T* __restrict_
 // The same with 16 bytes per load: a lane takes runs of 16 bytes, every 32nd run, in ascending order, its elements one
 // after the other; the order of the sums still depends on K alone.  K a multiple of the run, rows 16-byte aligned.
 template <typename T>
-__global__ void __launch_bounds__(128) router_logits_vec_kernel(const T* __restrict__ x, long long ldx, const T* __restrict__ W,
-                                                                float* __restrict__ out, int n_tokens, int n_experts, int K) {
+__global__ void __launch_bounds__(128) router_logits_vec_kernel(const T* x, long long ldx, const T* W,
+                                                                float* out, int n_tokens, int n_experts, int K) {
     constexpr int VN = 16 / sizeof(T);
     pb_grid_dep_launch();
     const int lane = threadIdx.x & 31;
@@ -126,8 +126,8 @@ __global__ void __launch_bounds__(128) router_logits_vec_kernel(const T* __restr
 #define ROUTER_TT 4
 #define ROUTER_TE 8
 template <typename T>
-__global__ void __launch_bounds__(128) router_logits_tile_kernel(const T* __restrict__ x, long long ldx, const T* __restrict__ W,
-                                                                 float* __restrict__ out, int n_tokens, int n_experts, int K) {
+__global__ void __launch_bounds__(128) router_logits_tile_kernel(const T* x, long long ldx, const T* W,
+                                                                 float* out, int n_tokens, int n_experts, int K) {
     constexpr int VN = 16 / sizeof(T);
     pb_grid_dep_launch();
     const int lane = threadIdx.x & 31;
@@ -324,8 +324,8 @@ __device__ __forceinline__ void moe_route_token(const float* z, const MoeRouteAr
 }
 
 template <int SLOTS>
-__global__ void __launch_bounds__(128) moe_route_kernel(const float* __restrict__ logits, int n_tokens, MoeRouteArgs args, int32_t* __restrict__ ids,
-                                                        float* __restrict__ weights) {
+__global__ void __launch_bounds__(128) moe_route_kernel(const float* logits, int n_tokens, MoeRouteArgs args, int32_t* ids,
+                                                        float* weights) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -375,8 +375,8 @@ PB_API int pb_moe_route(const float* logits, const float* correction, const floa
 #define ROUTE_FEW_EXPERTS 256
 template <typename T, int SLOTS>
 __global__ void __cluster_dims__(ROUTE_CLUSTER, 1, 1) __launch_bounds__(32 * ROUTE_WARPS)
-moe_route_few_kernel(const T* __restrict__ x, long long ldx, const T* __restrict__ W, int K, MoeRouteArgs args, int32_t* __restrict__ ids,
-                     float* __restrict__ weights) {
+moe_route_few_kernel(const T* x, long long ldx, const T* W, int K, MoeRouteArgs args, int32_t* ids,
+                     float* weights) {
     constexpr int VN = 16 / sizeof(T);
     __shared__ float z[ROUTE_FEW_EXPERTS];
     pb_grid_dep_launch();
@@ -456,10 +456,10 @@ PB_API int pb_moe_route_few(const void* x, long long ldx, const void* W, int dty
 
 // One block.  ids [n_slots] in [0, n_experts); offsets [n_experts + 1]; order, place_of [n_slots];
 // tile_expert, tile_row0 [max_tiles], max_tiles >= ceil(n_slots / MOE_BM) + n_experts.
-__global__ void __launch_bounds__(1024) moe_sort_kernel(const int32_t* __restrict__ ids, int n_slots, int n_experts,
-                                                        int32_t* __restrict__ offsets, int32_t* __restrict__ order,
-                                                        int32_t* __restrict__ place_of, int32_t* __restrict__ tile_expert,
-                                                        int32_t* __restrict__ tile_row0, int max_tiles, int tile_rows) {
+__global__ void __launch_bounds__(1024) moe_sort_kernel(const int32_t* ids, int n_slots, int n_experts,
+                                                        int32_t* offsets, int32_t* order,
+                                                        int32_t* place_of, int32_t* tile_expert,
+                                                        int32_t* tile_row0, int max_tiles, int tile_rows) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     __shared__ int count[MOE_MAX_EXPERTS], start[MOE_MAX_EXPERTS + 1], tile0[MOE_MAX_EXPERTS + 1];
@@ -538,11 +538,11 @@ static bool moe_act_ok(int gated, const MoeAct& a) {
 }
 
 template <typename T, typename TC, bool GATED>
-__global__ void __launch_bounds__(256) moe_gemm_fma_kernel(const T* __restrict__ A, long long lda, const int32_t* __restrict__ order,
-                                                           int a_div, const T* __restrict__ W, long long w_expert_stride, int N,
-                                                           int K, const int32_t* __restrict__ tile_expert,
-                                                           const int32_t* __restrict__ tile_row0,
-                                                           const int32_t* __restrict__ offsets, TC* __restrict__ C, long long ldc, MoeAct act) {
+__global__ void __launch_bounds__(256) moe_gemm_fma_kernel(const T* A, long long lda, const int32_t* order,
+                                                           int a_div, const T* W, long long w_expert_stride, int N,
+                                                           int K, const int32_t* tile_expert,
+                                                           const int32_t* tile_row0,
+                                                           const int32_t* offsets, TC* C, long long ldc, MoeAct act) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     const int e = tile_expert[blockIdx.x];
@@ -622,12 +622,12 @@ __global__ void __launch_bounds__(256) moe_gemm_fma_kernel(const T* __restrict__
 #define MOE_LD (MOE_TK + 8)
 
 template <typename TC, bool GATED>
-__global__ void __launch_bounds__(256) moe_gemm_bf16_kernel(const __nv_bfloat16* __restrict__ A, long long lda,
-                                                            const int32_t* __restrict__ order, int a_div,
-                                                            const __nv_bfloat16* __restrict__ W, long long w_expert_stride, int N,
-                                                            int K, const int32_t* __restrict__ tile_expert,
-                                                            const int32_t* __restrict__ tile_row0,
-                                                            const int32_t* __restrict__ offsets, TC* __restrict__ C, long long ldc, MoeAct act) {
+__global__ void __launch_bounds__(256) moe_gemm_bf16_kernel(const __nv_bfloat16* A, long long lda,
+                                                            const int32_t* order, int a_div,
+                                                            const __nv_bfloat16* W, long long w_expert_stride, int N,
+                                                            int K, const int32_t* tile_expert,
+                                                            const int32_t* tile_row0,
+                                                            const int32_t* offsets, TC* C, long long ldc, MoeAct act) {
     using namespace nvcuda;
     pb_grid_dep_launch();
     pb_grid_dep_wait();
@@ -729,12 +729,12 @@ __device__ __forceinline__ void moe_mma(float* c, const unsigned* a, unsigned b0
 }
 
 template <typename TC, bool GATED>
-__global__ void __launch_bounds__(256) moe_gemm_large_kernel(const __nv_bfloat16* __restrict__ A, long long lda,
-                                                             const int32_t* __restrict__ order, int a_div,
-                                                             const __nv_bfloat16* __restrict__ W, long long w_expert_stride, int N,
-                                                             int K, const int32_t* __restrict__ tile_expert,
-                                                             const int32_t* __restrict__ tile_row0,
-                                                             const int32_t* __restrict__ offsets, TC* __restrict__ C, long long ldc, MoeAct act) {
+__global__ void __launch_bounds__(256) moe_gemm_large_kernel(const __nv_bfloat16* A, long long lda,
+                                                             const int32_t* order, int a_div,
+                                                             const __nv_bfloat16* W, long long w_expert_stride, int N,
+                                                             int K, const int32_t* tile_expert,
+                                                             const int32_t* tile_row0,
+                                                             const int32_t* offsets, TC* C, long long ldc, MoeAct act) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     const int e = tile_expert[blockIdx.x];
@@ -921,12 +921,12 @@ __device__ __forceinline__ void moe_unpack8(const uint4& raw, float (&f)[8]) {
 // slots that chose it, found by looking through them, and a slot's place is the slot itself.
 #define MOE_GEMV_SLOTS 512
 template <typename TC, bool GATED>
-__global__ void __launch_bounds__(256) moe_gemv_kernel(const __nv_bfloat16* __restrict__ A, long long lda,
-                                                       const int32_t* __restrict__ order, int a_div,
-                                                       const __nv_bfloat16* __restrict__ W, long long w_expert_stride, int N, int K,
-                                                       const int32_t* __restrict__ tile_expert, const int32_t* __restrict__ tile_row0,
-                                                       const int32_t* __restrict__ offsets, const int32_t* __restrict__ ids, int n_slots,
-                                                       TC* __restrict__ C, long long ldc, MoeAct act) {
+__global__ void __launch_bounds__(256) moe_gemv_kernel(const __nv_bfloat16* A, long long lda,
+                                                       const int32_t* order, int a_div,
+                                                       const __nv_bfloat16* W, long long w_expert_stride, int N, int K,
+                                                       const int32_t* tile_expert, const int32_t* tile_row0,
+                                                       const int32_t* offsets, const int32_t* ids, int n_slots,
+                                                       TC* C, long long ldc, MoeAct act) {
     __shared__ int slots_s[MOE_GEMV_SLOTS];
     __shared__ int count_s;
     pb_grid_dep_launch();
@@ -1054,8 +1054,8 @@ PB_API int pb_moe_gemv(const void* A, long long lda, const int32_t* order, int a
 // out[place, :] = x[order[place] / div, :]: the rows of a step's tokens in the order of their places (what a product
 // that reads its rows through tensor-map copies needs).
 template <typename T>
-__global__ void moe_gather_rows_kernel(const T* __restrict__ x, long long ldx, const int32_t* __restrict__ order, int div,
-                                       T* __restrict__ out, int width) {
+__global__ void moe_gather_rows_kernel(const T* x, long long ldx, const int32_t* order, int div,
+                                       T* out, int width) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     const size_t place = blockIdx.x;
@@ -1083,8 +1083,8 @@ PB_API int pb_moe_gather_rows(const void* x, long long ldx, const int32_t* order
 
 // out[t, :] = sum_c w[t, c] * y[place_of[t * top + c], :], choices in ascending order, float32 sums.
 template <typename T, typename TY>
-__global__ void moe_combine_kernel(const TY* __restrict__ y, const int32_t* __restrict__ place_of,
-                                   const float* __restrict__ weights, T* __restrict__ out, int top, int width) {
+__global__ void moe_combine_kernel(const TY* y, const int32_t* place_of,
+                                   const float* weights, T* out, int top, int width) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     const size_t t = blockIdx.x;
@@ -1175,7 +1175,7 @@ struct MoeSumArgs {
 };
 
 template <typename TY, typename TS, typename TO, int V>
-__global__ void __launch_bounds__(256) moe_sum_kernel(const TY* __restrict__ y, const TS* __restrict__ shared, TO* __restrict__ out, MoeSumArgs a) {
+__global__ void __launch_bounds__(256) moe_sum_kernel(const TY* y, const TS* shared, TO* out, MoeSumArgs a) {
     pb_grid_dep_launch();
     const int i = blockIdx.x, col = (blockIdx.y * blockDim.x + threadIdx.x) * V;
     if (col >= a.width) return;
@@ -1299,7 +1299,7 @@ __device__ __forceinline__ float moe_block_sum(float v, float* red) {
 // AHEAD (a few tokens): both scales, written by no kernel, are asked for before the wait; else (a prompt step) they come from
 // the cache when they are needed, which leaves registers for two blocks on a multiprocessor.
 template <typename TY, typename TS, typename TO, int V, int IT, bool AHEAD>
-__global__ void __launch_bounds__(512, AHEAD ? 1 : 2) moe_sum_normed_kernel(const TY* __restrict__ y, const TS* __restrict__ shared, TO* __restrict__ out,
+__global__ void __launch_bounds__(512, AHEAD ? 1 : 2) moe_sum_normed_kernel(const TY* y, const TS* shared, TO* out,
                                                                             MoeSumNormArgs a) {
     pb_grid_dep_launch();
     __shared__ float red[2][16];

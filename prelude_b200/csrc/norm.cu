@@ -29,8 +29,8 @@ __device__ __forceinline__ float block_sum(float v, float* smem) {
 }
 
 template <typename TX, typename TY>
-__global__ void add_rmsnorm_kernel(const TX* __restrict__ x, int n_parts, size_t part_stride, float* __restrict__ res,
-                                   const float* __restrict__ w, TY* __restrict__ y, int width, float eps) {
+__global__ void add_rmsnorm_kernel(const TX* x, int n_parts, size_t part_stride, float* res,
+                                   const float* w, TY* y, int width, float eps) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     __shared__ float red[32];
@@ -61,8 +61,8 @@ __global__ void add_rmsnorm_kernel(const TX* __restrict__ x, int n_parts, size_t
 // two passes.  width % 4 == 0, width <= 4 * blockDim * ITERS.
 // SCALED: what is added is xs times the parts' sum (taken on its own, in ascending order), as one fused multiply-add.
 template <typename TX, typename TY, int ITERS, bool SCALED = false>
-__global__ void add_rmsnorm_vec4_kernel(const TX* __restrict__ x, int n_parts, size_t part_stride, float* __restrict__ res,
-                                        const float* __restrict__ w, TY* __restrict__ y, int width, float eps, float xs) {
+__global__ void add_rmsnorm_vec4_kernel(const TX* x, int n_parts, size_t part_stride, float* res,
+                                        const float* w, TY* y, int width, float eps, float xs) {
     pb_grid_dep_launch();
     PB_TL(PB_TL_NORM, PB_TL_ENTRY);
     __shared__ float red[32];
@@ -219,9 +219,9 @@ PB_API int pb_add_rmsnorm(const void* x, int x_parts, long long part_stride, flo
 // final norm, crates/prelude-core/src/models/commons/mod.rs:227-243; the order
 // does not change the values).
 template <typename TX, typename TY>
-__global__ void gather_add_rmsnorm_kernel(const TX* __restrict__ x, int n_parts, size_t part_stride,
-                                          const float* __restrict__ res, const int32_t* __restrict__ rows,
-                                          const float* __restrict__ w, TY* __restrict__ y, int width, int n_rows_total,
+__global__ void gather_add_rmsnorm_kernel(const TX* x, int n_parts, size_t part_stride,
+                                          const float* res, const int32_t* rows,
+                                          const float* w, TY* y, int width, int n_rows_total,
                                           float eps) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
@@ -296,7 +296,7 @@ PB_API int pb_gather_add_rmsnorm(const void* x, int x_parts, long long part_stri
 // Plain norm of a tensor of the model's own type (used by parts that are not
 // on the residual stream, and by the per-kernel tests).
 template <typename T>
-__global__ void rmsnorm_kernel(const T* __restrict__ x, const float* __restrict__ w, T* __restrict__ y, int width,
+__global__ void rmsnorm_kernel(const T* x, const float* w, T* y, int width,
                                float eps) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
@@ -330,9 +330,9 @@ PB_API int pb_rmsnorm(const void* x, const float* w, void* y, int dtype, int row
 // sum is made.  plus: null, or what also joins the stream there (a loop of layers takes the embedding's output again).  With `rows` (the gather form) row i of y is made from row rows[i] of x and res, and res is left alone.
 // The row is kept in shared memory between the passes where it fits, else it is read again.
 template <typename TX, typename TY>
-__global__ void normed_add_rmsnorm_kernel(const TX* __restrict__ x, const float* __restrict__ wx, float eps_x,
-                                          float* __restrict__ res, const float* __restrict__ plus, const int32_t* __restrict__ rows,
-                                          int n_rows_total, const float* __restrict__ w, TY* __restrict__ y, int width, float eps, int keep) {
+__global__ void normed_add_rmsnorm_kernel(const TX* x, const float* wx, float eps_x,
+                                          float* res, const float* plus, const int32_t* rows,
+                                          int n_rows_total, const float* w, TY* y, int width, float eps, int keep) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     extern __shared__ float row_s[];
@@ -373,9 +373,9 @@ __global__ void normed_add_rmsnorm_kernel(const TX* __restrict__ x, const float*
 // registers between the passes; for every row of the stream, or (with `rows`) for the chosen rows, whose sum is not
 // stored.  width % 4 == 0, width <= 4 * blockDim * ITERS.
 template <typename TX, typename TY, int ITERS>
-__global__ void normed_add_rmsnorm_vec4_kernel(const TX* __restrict__ x, const float* __restrict__ wx, float eps_x,
-                                               float* __restrict__ res, const float* __restrict__ plus, const int32_t* __restrict__ rows,
-                                               int n_rows_total, const float* __restrict__ w, TY* __restrict__ y, int width, float eps) {
+__global__ void normed_add_rmsnorm_vec4_kernel(const TX* x, const float* wx, float eps_x,
+                                               float* res, const float* plus, const int32_t* rows,
+                                               int n_rows_total, const float* w, TY* y, int width, float eps) {
     pb_grid_dep_launch();
     __shared__ float red[32];
     const int n4 = width >> 2;
@@ -500,9 +500,9 @@ PB_API int pb_normed_add_rmsnorm(const void* x, const float* wx, float eps_x, fl
 // places whose logits are wanted).  x as for pb_add_rmsnorm: of type dtype, or x_parts float32 arrays whose sum,
 // taken in ascending order, is what is scaled and added.
 template <typename TX, typename TY>
-__global__ void scaled_add_rmsnorm_kernel(const TX* __restrict__ x, int n_parts, size_t part_stride, float scale, float* __restrict__ res,
-                                          const int32_t* __restrict__ rows, int n_rows_total, const float* __restrict__ w,
-                                          TY* __restrict__ y, int width, float eps) {
+__global__ void scaled_add_rmsnorm_kernel(const TX* x, int n_parts, size_t part_stride, float scale, float* res,
+                                          const int32_t* rows, int n_rows_total, const float* w,
+                                          TY* y, int width, float eps) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     __shared__ float red[32];
@@ -613,8 +613,8 @@ PB_API int pb_scaled_add_rmsnorm(const void* x, int x_parts, long long part_stri
 // out = sa * a / rms(a) * wa + sb * b / rms(b) * wb, computed and handed out in float32 (what the residual add takes as
 // a sum of one part).  One block per row.
 template <typename T>
-__global__ void normed_pair_sum_kernel(const T* __restrict__ a, const float* __restrict__ wa, float sa, const T* __restrict__ b,
-                                       const float* __restrict__ wb, float sb, float eps, float* __restrict__ out, int width) {
+__global__ void normed_pair_sum_kernel(const T* a, const float* wa, float sa, const T* b,
+                                       const float* wb, float sb, float eps, float* out, int width) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     __shared__ float red[32];

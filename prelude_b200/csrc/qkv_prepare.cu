@@ -73,14 +73,14 @@ __device__ __forceinline__ float rotated(const T* head, const float* w_head, flo
 }
 
 template <typename T>
-__global__ void qkv_prepare_kernel(const T* __restrict__ q_in, long long ldq, const T* __restrict__ k_in, long long ldk,
-                                   const T* __restrict__ v_in, long long ldv, const float* __restrict__ q_w,
-                                   const float* __restrict__ k_w, int k_norm_cols, float eps, RotArgs rot, int q_rot_off,
-                                   int k_rot_off, const int32_t* __restrict__ positions, const int32_t* __restrict__ table_row,
-                                   const int32_t* __restrict__ block_table, int table_stride, int page_size, int num_pages,
-                                   T* __restrict__ q_out, int q_split, T* __restrict__ q_out2, long long q2_head_stride,
-                                   long long q2_off, T* __restrict__ k_pages, T* __restrict__ v_pages, int H, int qd, int G,
-                                   int kd, int Gv, int vd, int swizzle_k, int swizzle_v, int* __restrict__ status) {
+__global__ void qkv_prepare_kernel(const T* q_in, long long ldq, const T* k_in, long long ldk,
+                                   const T* v_in, long long ldv, const float* q_w,
+                                   const float* k_w, int k_norm_cols, float eps, RotArgs rot, int q_rot_off,
+                                   int k_rot_off, const int32_t* positions, const int32_t* table_row,
+                                   const int32_t* block_table, int table_stride, int page_size, int num_pages,
+                                   T* q_out, int q_split, T* q_out2, long long q2_head_stride,
+                                   long long q2_off, T* k_pages, T* v_pages, int H, int qd, int G,
+                                   int kd, int Gv, int vd, int swizzle_k, int swizzle_v, int* status) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     __shared__ float red[32];
@@ -147,14 +147,14 @@ __global__ void qkv_prepare_kernel(const T* __restrict__ q_in, long long ldq, co
 // loads, sums and rotation partners from shared memory, 16-byte stores.  Takes rows whose q, k and v parts start on
 // 16-byte boundaries and have sizes in multiples of 8 (bfloat16) or 4 (float32) elements, heads and split points likewise.
 template <typename T>
-__global__ void qkv_prepare_staged_kernel(const T* __restrict__ q_in, long long ldq, const T* __restrict__ k_in, long long ldk,
-                                          const T* __restrict__ v_in, long long ldv, const float* __restrict__ q_w,
-                                          const float* __restrict__ k_w, int k_norm_cols, float eps, RotArgs rot, int q_rot_off,
-                                          int k_rot_off, const int32_t* __restrict__ positions, const int32_t* __restrict__ table_row,
-                                          const int32_t* __restrict__ block_table, int table_stride, int page_size, int num_pages,
-                                          T* __restrict__ q_out, int q_split, T* __restrict__ q_out2, long long q2_head_stride,
-                                          long long q2_off, T* __restrict__ k_pages, T* __restrict__ v_pages, int H, int qd, int G,
-                                          int kd, int Gv, int vd, int swizzle_k, int swizzle_v, int* __restrict__ status) {
+__global__ void qkv_prepare_staged_kernel(const T* q_in, long long ldq, const T* k_in, long long ldk,
+                                          const T* v_in, long long ldv, const float* q_w,
+                                          const float* k_w, int k_norm_cols, float eps, RotArgs rot, int q_rot_off,
+                                          int k_rot_off, const int32_t* positions, const int32_t* table_row,
+                                          const int32_t* block_table, int table_stride, int page_size, int num_pages,
+                                          T* q_out, int q_split, T* q_out2, long long q2_head_stride,
+                                          long long q2_off, T* k_pages, T* v_pages, int H, int qd, int G,
+                                          int kd, int Gv, int vd, int swizzle_k, int swizzle_v, int* status) {
     constexpr int VN = 16 / sizeof(T);
     pb_grid_dep_launch();
     pb_grid_dep_wait();

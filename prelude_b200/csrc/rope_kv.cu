@@ -27,13 +27,13 @@
 
 template <typename T>
 __global__ void qknorm_rope_kvwrite_kernel(
-    const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, long long token_stride,
-    T* __restrict__ q_out, T* __restrict__ k_pages, T* __restrict__ v_pages,
-    const float* __restrict__ q_weight, const float* __restrict__ k_weight, float eps,
-    const float* __restrict__ cos_table, const float* __restrict__ sin_table, int rotary_dim, int interleaved, int max_positions,
-    const int32_t* __restrict__ positions, const int32_t* __restrict__ token_seq,
-    const int32_t* __restrict__ block_table, int table_stride, int page_size, int num_pages,
-    int n_tokens, int n_heads, int n_kv_heads, int head_dim, int write_kv, int swizzle, int* __restrict__ status) {
+    const T* q, const T* k, const T* v, long long token_stride,
+    T* q_out, T* k_pages, T* v_pages,
+    const float* q_weight, const float* k_weight, float eps,
+    const float* cos_table, const float* sin_table, int rotary_dim, int interleaved, int max_positions,
+    const int32_t* positions, const int32_t* token_seq,
+    const int32_t* block_table, int table_stride, int page_size, int num_pages,
+    int n_tokens, int n_heads, int n_kv_heads, int head_dim, int write_kv, int swizzle, int* status) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     const int heads_per_token = n_heads + (write_kv ? 2 * n_kv_heads : 0);
@@ -113,13 +113,13 @@ PB_TIMELINE_UNIT(rope)
 // The vector kernel: LANES = head_dim / 8 lanes per (token, head), 8 elements each.
 template <int LANES>
 __global__ void __launch_bounds__(256) qknorm_rope_kvwrite_vec_kernel(
-    const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v,
-    long long token_stride, __nv_bfloat16* __restrict__ q_out, __nv_bfloat16* __restrict__ k_pages,
-    __nv_bfloat16* __restrict__ v_pages, const float* __restrict__ q_weight, const float* __restrict__ k_weight, float eps,
-    const float* __restrict__ cos_table, const float* __restrict__ sin_table, int rotary_dim, int interleaved, int max_positions,
-    const int32_t* __restrict__ positions, const int32_t* __restrict__ token_seq,
-    const int32_t* __restrict__ block_table, int table_stride, int page_size, int num_pages,
-    int n_tokens, int n_heads, int n_kv_heads, int write_kv, int swizzle, int* __restrict__ status) {
+    const __nv_bfloat16* q, const __nv_bfloat16* k, const __nv_bfloat16* v,
+    long long token_stride, __nv_bfloat16* q_out, __nv_bfloat16* k_pages,
+    __nv_bfloat16* v_pages, const float* q_weight, const float* k_weight, float eps,
+    const float* cos_table, const float* sin_table, int rotary_dim, int interleaved, int max_positions,
+    const int32_t* positions, const int32_t* token_seq,
+    const int32_t* block_table, int table_stride, int page_size, int num_pages,
+    int n_tokens, int n_heads, int n_kv_heads, int write_kv, int swizzle, int* status) {
     pb_grid_dep_launch();
     PB_TL(PB_TL_ROPE, PB_TL_ENTRY);
     constexpr int D = LANES * 8;
@@ -241,13 +241,13 @@ __global__ void __launch_bounds__(256) qknorm_rope_kvwrite_vec_kernel(
 // want but not this.
 template <int LANES, int G>
 __global__ void __launch_bounds__(256) qknorm_rope_kvwrite_heads_kernel(
-    const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v,
-    long long token_stride, __nv_bfloat16* __restrict__ q_out, __nv_bfloat16* __restrict__ k_pages,
-    __nv_bfloat16* __restrict__ v_pages, const float* __restrict__ q_weight, const float* __restrict__ k_weight, float eps,
-    const float* __restrict__ cos_table, const float* __restrict__ sin_table, int rotary_dim, int interleaved, int max_positions,
-    const int32_t* __restrict__ positions, const int32_t* __restrict__ token_seq,
-    const int32_t* __restrict__ block_table, int table_stride, int page_size, int num_pages,
-    int n_tokens, int n_heads, int n_kv_heads, int write_kv, int swizzle, int* __restrict__ status) {
+    const __nv_bfloat16* q, const __nv_bfloat16* k, const __nv_bfloat16* v,
+    long long token_stride, __nv_bfloat16* q_out, __nv_bfloat16* k_pages,
+    __nv_bfloat16* v_pages, const float* q_weight, const float* k_weight, float eps,
+    const float* cos_table, const float* sin_table, int rotary_dim, int interleaved, int max_positions,
+    const int32_t* positions, const int32_t* token_seq,
+    const int32_t* block_table, int table_stride, int page_size, int num_pages,
+    int n_tokens, int n_heads, int n_kv_heads, int write_kv, int swizzle, int* status) {
     pb_grid_dep_launch();
     PB_TL(PB_TL_ROPE, PB_TL_ENTRY);
     constexpr int D = LANES * 8;

@@ -11,12 +11,12 @@ namespace {
 #define RG_BLOCK 128
 #define RG_PART 16                                            // rows of a thread block
 
-__global__ void __launch_bounds__(256) rows_gather_kernel(const __nv_bfloat16* __restrict__ pages, __nv_bfloat16* __restrict__ out,
-                                                          const int32_t* __restrict__ block_seq, const int32_t* __restrict__ block_pos0,
-                                                          const int32_t* __restrict__ kv_len, const int32_t* __restrict__ cu_q,
-                                                          const int32_t* __restrict__ table_row, const int32_t* __restrict__ block_table,
+__global__ void __launch_bounds__(256) rows_gather_kernel(const __nv_bfloat16* pages, __nv_bfloat16* out,
+                                                          const int32_t* block_seq, const int32_t* block_pos0,
+                                                          const int32_t* kv_len, const int32_t* cu_q,
+                                                          const int32_t* table_row, const int32_t* block_table,
                                                           int table_stride, int page_size, int num_pages, int width,
-                                                          const int32_t* __restrict__ q_start, int window, int* __restrict__ status) {
+                                                          const int32_t* q_start, int window, int* status) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     const int seq = block_seq[blockIdx.x], pos0 = block_pos0[blockIdx.x] + blockIdx.y * RG_PART;

@@ -35,7 +35,7 @@ __device__ __forceinline__ ArgPair better(ArgPair a, ArgPair b) {
 }
 
 // Largest value and its first index over row[begin, end); every thread gets the result.
-__device__ ArgPair block_argmax(const float* __restrict__ row, int begin, int end, ArgPair* smem) {
+__device__ ArgPair block_argmax(const float* row, int begin, int end, ArgPair* smem) {
     ArgPair best{-INFINITY, 0x7fffffff};
     for (int i = begin + threadIdx.x; i < end; i += blockDim.x) {
         float v = row[i];
@@ -77,8 +77,8 @@ PB_API long long pb_sample_scratch_floats(int rows, int vocab) { return (long lo
 
 // pass 1: grid (chunks, rows).  part[row][chunk] = {max, first index (int bits), sum of exp((x - max) / T), unused}
 __global__ void __launch_bounds__(PART_THREADS) sample_partial_kernel(
-    const float* __restrict__ logits, long long row_stride, int vocab, const float* __restrict__ temperature,
-    float* __restrict__ part) {
+    const float* logits, long long row_stride, int vocab, const float* temperature,
+    float* part) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     __shared__ ArgPair smem[32];
@@ -131,9 +131,9 @@ PB_API float pb_philox_uniform(uint64_t seed, uint64_t counter) { return philox_
 
 // pass 2: one block per row
 __global__ void __launch_bounds__(PART_THREADS) sample_final_kernel(
-    const float* __restrict__ logits, long long row_stride, int vocab, const float* __restrict__ temperature,
-    const uint64_t* __restrict__ seeds, const uint64_t* __restrict__ counters, const float* __restrict__ part,
-    int nblk, int32_t* __restrict__ out) {
+    const float* logits, long long row_stride, int vocab, const float* temperature,
+    const uint64_t* seeds, const uint64_t* counters, const float* part,
+    int nblk, int32_t* out) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     __shared__ float sums[PART_THREADS];
@@ -240,8 +240,8 @@ PB_API int pb_sample(const float* logits, long long row_stride, int rows, int vo
 
 // probs[r, :] = softmax(logits[r, :] / T_r), for the host-side top-k / top-p draw.
 __global__ void __launch_bounds__(SAMP_THREADS) softmax_temperature_kernel(
-    const float* __restrict__ logits, long long row_stride, int vocab, const float* __restrict__ temperature,
-    float* __restrict__ probs) {
+    const float* logits, long long row_stride, int vocab, const float* temperature,
+    float* probs) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     __shared__ ArgPair smem[32];

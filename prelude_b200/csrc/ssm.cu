@@ -48,10 +48,10 @@ __device__ __forceinline__ float softplus_f(float x) { return x > 20.0f ? x : lo
 
 // ---------------------------------------------------------------------------------------------------------
 template <typename T>
-__global__ void causal_conv_silu_kernel(const T* __restrict__ in, long long ld_in, const float* __restrict__ w,
-                                        const float* __restrict__ bias, const T* __restrict__ carried, T* __restrict__ out,
-                                        const int32_t* __restrict__ token_seq, const int32_t* __restrict__ positions,
-                                        const int32_t* __restrict__ q_start, const int32_t* __restrict__ slots, int n_tokens,
+__global__ void causal_conv_silu_kernel(const T* in, long long ld_in, const float* w,
+                                        const float* bias, const T* carried, T* out,
+                                        const int32_t* token_seq, const int32_t* positions,
+                                        const int32_t* q_start, const int32_t* slots, int n_tokens,
                                         int channels, int taps) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
@@ -77,10 +77,10 @@ __global__ void causal_conv_silu_kernel(const T* __restrict__ in, long long ld_i
 // TAPS - 1 inputs in registers: while the run stays inside one sequence every input is read once.
 #define CONV_RUN 16                                          // a long step; a step of few tokens gives every token a block
 template <typename T, int TAPS>
-__global__ void causal_conv_silu_vec_kernel(const T* __restrict__ in, long long ld_in, const float* __restrict__ w,
-                                            const float* __restrict__ bias, const T* __restrict__ carried, T* __restrict__ out,
-                                            const int32_t* __restrict__ token_seq, const int32_t* __restrict__ positions,
-                                            const int32_t* __restrict__ q_start, const int32_t* __restrict__ slots, int n_tokens,
+__global__ void causal_conv_silu_vec_kernel(const T* in, long long ld_in, const float* w,
+                                            const float* bias, const T* carried, T* out,
+                                            const int32_t* token_seq, const int32_t* positions,
+                                            const int32_t* q_start, const int32_t* slots, int n_tokens,
                                             int channels, int run) {
     constexpr int VN = 16 / sizeof(T);
     pb_grid_dep_launch();
@@ -131,8 +131,8 @@ __global__ void causal_conv_silu_vec_kernel(const T* __restrict__ in, long long 
 // Row s of a sequence's carried inputs holds the input at in-step index s - (taps - 1) of its NEXT step.  One thread
 // owns a (sequence, channel): it reads rows above the one it writes, in ascending order, so nothing is lost.
 template <typename T>
-__global__ void conv_state_update_kernel(const T* __restrict__ in, long long ld_in, T* __restrict__ carried,
-                                         const int32_t* __restrict__ cu_q, const int32_t* __restrict__ slots, int channels, int taps) {
+__global__ void conv_state_update_kernel(const T* in, long long ld_in, T* carried,
+                                         const int32_t* cu_q, const int32_t* slots, int channels, int taps) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -168,9 +168,9 @@ __global__ void conv_state_update_kernel(const T* __restrict__ in, long long ld_
 // `a_log` holds the decays themselves.  With `activate` 0 the columns hold SiLU's values already.
 template <typename T, int NPL, bool FIXED>
 __global__ void __launch_bounds__(256)
-ssm_scan_kernel(const T* __restrict__ u, long long ld_u, const T* __restrict__ dt_in, long long ld_dt, const float* __restrict__ dt_bias,
-                const float* __restrict__ a_log, const float* __restrict__ d_skip, float* __restrict__ state,
-                float* __restrict__ y, const int32_t* __restrict__ cu_q, const int32_t* __restrict__ slots, int heads, int P,
+ssm_scan_kernel(const T* u, long long ld_u, const T* dt_in, long long ld_dt, const float* dt_bias,
+                const float* a_log, const float* d_skip, float* state,
+                float* y, const int32_t* cu_q, const int32_t* slots, int heads, int P,
                 int N, int groups, int activate) {
     constexpr int NPAD = NPL * SCAN_LANES;                     // state rows with padding: a power of two
     constexpr int CHUNK = NPL == 32 ? 8 : 16;                  // tokens per chunk
@@ -338,8 +338,8 @@ ssm_scan_kernel(const T* __restrict__ u, long long ld_u, const T* __restrict__ d
 
 // ---------------------------------------------------------------------------------------------------------
 template <typename T>
-__global__ void gated_group_rmsnorm_kernel(const float* __restrict__ y, const T* __restrict__ z, long long ld_z,
-                                           const float* __restrict__ w, T* __restrict__ out, int inner, int parts, float eps,
+__global__ void gated_group_rmsnorm_kernel(const float* y, const T* z, long long ld_z,
+                                           const float* w, T* out, int inner, int parts, float eps,
                                            int gate_after, int sigmoid_gate) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
@@ -365,8 +365,8 @@ __global__ void gated_group_rmsnorm_kernel(const float* __restrict__ y, const T*
 // The same for parts of up to 128 * ITERS elements (a norm per head): a warp per (token, part), four elements per access, the
 // part kept in registers between the sum and the store.  width, ld_z in multiples of 4, operands aligned.
 template <typename T, int ITERS>
-__global__ void __launch_bounds__(256) gated_part_rmsnorm_kernel(const float* __restrict__ y, const T* __restrict__ z, long long ld_z,
-                                                                 const float* __restrict__ w, T* __restrict__ out, int n_tokens, int inner, int parts,
+__global__ void __launch_bounds__(256) gated_part_rmsnorm_kernel(const float* y, const T* z, long long ld_z,
+                                                                 const float* w, T* out, int n_tokens, int inner, int parts,
                                                                  float eps, int gate_after, int sigmoid_gate) {
     pb_grid_dep_launch();
     const int lane = threadIdx.x & 31, width = inner / parts;
@@ -429,7 +429,7 @@ __global__ void __launch_bounds__(256) gated_part_rmsnorm_kernel(const float* __
 }
 
 template <typename TI, typename TO>
-__global__ void scaled_sum_kernel(const TI* __restrict__ a, float sa, const TI* __restrict__ b, float sb, TO* __restrict__ out, long long n) {
+__global__ void scaled_sum_kernel(const TI* a, float sa, const TI* b, float sb, TO* out, long long n) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;

@@ -29,9 +29,9 @@ namespace {
 #define WKV_LANES 8
 
 template <typename T>
-__global__ void token_shift_mix_kernel(const T* __restrict__ x, const T* __restrict__ carried, const float* __restrict__ mu,
-                                       T* __restrict__ out, const int32_t* __restrict__ token_seq, const int32_t* __restrict__ positions,
-                                       const int32_t* __restrict__ q_start, const int32_t* __restrict__ slots, int n_tokens, int width,
+__global__ void token_shift_mix_kernel(const T* x, const T* carried, const float* mu,
+                                       T* out, const int32_t* token_seq, const int32_t* positions,
+                                       const int32_t* q_start, const int32_t* slots, int n_tokens, int width,
                                        int n_mix) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
@@ -52,9 +52,9 @@ __global__ void token_shift_mix_kernel(const T* __restrict__ x, const T* __restr
 
 template <typename T, int NPL>
 __global__ void __launch_bounds__(256)
-wkv_scan_kernel(const T* __restrict__ r_in, long long ld_r, const T* __restrict__ k_in, long long ld_k, const T* __restrict__ v_in,
-                long long ld_v, const T* __restrict__ w_in, long long ld_w, const float* __restrict__ w0, const float* __restrict__ bonus,
-                float* __restrict__ state, float* __restrict__ y, const int32_t* __restrict__ cu_q, const int32_t* __restrict__ slots, int H,
+wkv_scan_kernel(const T* r_in, long long ld_r, const T* k_in, long long ld_k, const T* v_in,
+                long long ld_v, const T* w_in, long long ld_w, const float* w0, const float* bonus,
+                float* state, float* y, const int32_t* cu_q, const int32_t* slots, int H,
                 int D) {
     constexpr int NPAD = NPL * WKV_LANES;
     constexpr int CHUNK = NPL == 32 ? 4 : (NPL == 16 ? 8 : 16);

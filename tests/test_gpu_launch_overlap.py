@@ -1,0 +1,33 @@
+"""A kernel that is launched while the one before it is still running reads that one's results after its wait, never
+before: what the earlier kernel writes is poisoned first, so a number fetched too early shows."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("parts_width", [512, 256, 128, 1024])
+def test_the_gated_norm_waits_for_the_scan(parts_width):
+    """The state-space scan leaves multiprocessors free for the first blocks of the norm behind it.  Same arithmetic on
+    the same numbers: equal to the last bit to a norm that is launched long after the scan has ended."""
+    from prelude_b200.engine.batch import StepItem, build_step_batch
+    from prelude_b200.ops import kernels as K
+    T, H, P, N, groups = 2048, 64, 64, 128, 8
+    gen = torch.Generator(device=DEV).manual_seed(3)
+
+    def normal(*shape):
+        return torch.randn(shape, generator=gen, device=DEV)
+
+    u, z = normal(T, H * P + 2 * groups * N).bfloat16(), normal(T, H * P).bfloat16()
+    dt, head, weight = normal(T, H).bfloat16(), torch.zeros(H, device=DEV), normal(H * P)
+    state = torch.zeros(1, H, N, P, device=DEV)
+    batch = build_step_batch([StepItem("a", [0] * T, 0)], {}, [0], torch.device(DEV), 2, T)
+    for _ in range(4):
+        y = torch.full((T, H * P), float("nan"), device=DEV)
+        state.zero_()
+        K.ssm_scan(u, dt, head, head, head, state, batch, groups, out=y)
+        got = K.gated_group_rmsnorm(y, z, weight, H * P // parts_width, 1e-6)
+        torch.cuda.synchronize()
+        assert torch.isfinite(y).all()
+        assert torch.equal(got, K.gated_group_rmsnorm(y, z, weight, H * P // parts_width, 1e-6))
