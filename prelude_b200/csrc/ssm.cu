@@ -14,7 +14,7 @@
 // Decay, step size, softplus, exponentials, the state and the sums over it are float32 whatever the run's type;
 // the projections and the convolution's output are of the run's type.  A sequence's tokens are visited in order,
 // one after the other, by the same threads: the result does not depend on how a prompt was cut into steps or on
-// what else is in the batch.  All kernels find a step's sequences through device arrays (cumulative lengths,
+// what else is in the batch.  (A prompt step in bfloat16 runs the state-space recurrence by chunks: ssm_chunk.cu.)  All kernels find a step's sequences through device arrays (cumulative lengths,
 // state slots), with one block row per sequence the arrays have room for: a row whose length is not positive is
 // skipped, so the launches have the same shape whatever the step holds and can be recorded.
 #include "common.cuh"

@@ -1027,10 +1027,15 @@ def conv_state_update(x: torch.Tensor, carried: torch.Tensor, batch) -> None:
                                             _stream()), "conv_state_update")
 
 
+# tokens of a prompt step from which the recurrences run by chunks of tokens on the tensor cores (bfloat16 only)
+SCAN_CHUNKED_MIN_TOKENS = 32
+
+
 def ssm_scan(u: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: torch.Tensor, d_skip: torch.Tensor,
              state: torch.Tensor, batch, groups: int, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """The recurrence over the step's tokens, sequence by sequence; u [T, heads * P + 2 * groups * N] dense, dt [T, heads] a
-    view with dense rows, state float32 [slots, heads, N, P]; returns y float32 [T, heads * P]."""
+    view with dense rows, state float32 [slots, heads, N, P]; returns y float32 [T, heads * P].  A prompt step in bfloat16
+    runs by chunks of tokens (csrc/ssm_chunk.cu), in 32-bit and in a decode step token by token (csrc/ssm.cu)."""
     _need(u, "u")
     _need(dt, "dt", u.dtype, contiguous=False)
     for t, name in ((dt_bias, "dt_bias"), (a_log, "a_log"), (d_skip, "d_skip"), (state, "state")):
@@ -1041,7 +1046,14 @@ def ssm_scan(u: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: to
         raise KernelLibraryError(f"ssm_scan: u {tuple(u.shape)}, dt {tuple(dt.shape)}, state {tuple(state.shape)}, {groups} groups")
     if out is None:
         out = torch.empty((T, heads * P), dtype=torch.float32, device=u.device)
-    check(_l.library().pb_ssm_scan(u.data_ptr(), dt.data_ptr(), dt.stride(0), dtype_code(u.dtype), dt_bias.data_ptr(), a_log.data_ptr(),
+    lib = _l.library()
+    if (u.dtype == torch.bfloat16 and T >= SCAN_CHUNKED_MIN_TOKENS and not batch.decode_only
+            and lib.pb_ssm_scan_chunked_takes(u.data_ptr(), heads, P, N, groups)):
+        check(lib.pb_ssm_scan_chunked(u.data_ptr(), dt.data_ptr(), dt.stride(0), dt_bias.data_ptr(), a_log.data_ptr(), d_skip.data_ptr(),
+                                      state.data_ptr(), out.data_ptr(), batch.cu_q.data_ptr(), batch.state_slots.data_ptr(),
+                                      batch.cu_q.numel() - 1, heads, P, N, groups, _stream()), "ssm_scan_chunked")
+        return out
+    check(lib.pb_ssm_scan(u.data_ptr(), dt.data_ptr(), dt.stride(0), dtype_code(u.dtype), dt_bias.data_ptr(), a_log.data_ptr(),
                                    d_skip.data_ptr(), state.data_ptr(), out.data_ptr(), batch.cu_q.data_ptr(),
                                    batch.state_slots.data_ptr(), batch.cu_q.numel() - 1, heads, P, N, groups, _stream()), "ssm_scan")
     return out

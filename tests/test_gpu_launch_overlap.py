@@ -23,9 +23,12 @@ def test_the_gated_norm_waits_for_the_scan(parts_width):
     dt, head, weight = normal(T, H).bfloat16(), torch.zeros(H, device=DEV), normal(H * P)
     state = torch.zeros(1, H, N, P, device=DEV)
     batch = build_step_batch([StepItem("a", [0] * T, 0)], {}, [0], torch.device(DEV), 2, T)
+    busy = torch.randn(8192, 8192, device=DEV).bfloat16()
     for _ in range(4):
         y = torch.full((T, H * P), float("nan"), device=DEV)
         state.zero_()
+        for _ in range(3):
+            torch.mm(busy, busy)              # the host is ahead: the norm is queued before the scan begins
         K.ssm_scan(u, dt, head, head, head, state, batch, groups, out=y)
         got = K.gated_group_rmsnorm(y, z, weight, H * P // parts_width, 1e-6)
         torch.cuda.synchronize()

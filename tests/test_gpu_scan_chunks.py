@@ -1,0 +1,102 @@
+"""Recurrences of a prompt step by chunks of tokens on the tensor cores, alone, against a loop over the tokens in 64-bit
+and beside the kernels that visit the tokens one by one: at the chunks' edges, over several sequences of unequal length, with
+decays from none to all, and with numbers that are not finite."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _batch(lens):
+    from prelude_b200.engine.batch import StepItem, build_step_batch
+    return build_step_batch([StepItem(i, [0] * n, 0) for i, n in enumerate(lens)], {}, list(range(len(lens)))[::-1],
+                            torch.device(DEV), 2, 1 << 20)
+
+
+def _rel(a, b):
+    return float((a.double() - b).norm() / b.norm().clamp_min(1e-30))
+
+
+def _ssm_inputs(lens, H, P, N, groups, seed, step):
+    gen = torch.Generator(device=DEV).manual_seed(seed)
+    T = sum(lens)
+
+    def normal(*shape):
+        return torch.randn(shape, generator=gen, device=DEV)
+
+    u = normal(T, H * P + 2 * groups * N).bfloat16()
+    dt = normal(T, H + 3).bfloat16()[:, :H]
+    bias = torch.full((H,), math.log(math.expm1(step)), device=DEV) + 0.3 * normal(H)
+    a_log = torch.log(torch.rand(H, generator=gen, device=DEV) * 15 + 1)
+    return u, dt, bias, a_log, normal(H), normal(len(lens), H, N, P)
+
+
+def _ssm_exact(u, dt, bias, a_log, skip, state, lens, groups):
+    R, H, N, P = state.shape
+    u, S, inner, at = u.double(), state.double().clone(), H * P, 0
+    step = torch.nn.functional.softplus(dt.double() + bias.double(), threshold=50)
+    decay = torch.exp(-torch.exp(a_log.double()) * step)
+    y = torch.empty(u.shape[0], H, P, dtype=torch.float64, device=DEV)
+    for r, n in enumerate(lens):
+        slot = R - 1 - r
+        for t in range(at, at + n):
+            x = u[t, :inner].view(H, P)
+            B, C = (u[t, inner + k * groups * N:inner + (k + 1) * groups * N].view(groups, N).repeat_interleave(H // groups, 0) for k in (0, 1))
+            S[slot] = decay[t].view(H, 1, 1) * S[slot] + (step[t].view(H, 1) * B).unsqueeze(2) * x.unsqueeze(1)
+            y[t] = (S[slot] * C.unsqueeze(2)).sum(1) + skip.double().view(H, 1) * x
+        at += n
+    return y.view(-1, inner), S
+
+
+def _by_tokens(monkeypatch, K):
+    """The same call through the kernel that visits the tokens one by one."""
+    monkeypatch.setattr(K, "SCAN_CHUNKED_MIN_TOKENS", 1 << 30)
+
+
+@pytest.mark.parametrize("lens,H,P,N,groups", [
+    ([64], 8, 64, 128, 8), ([65, 1, 63], 4, 32, 128, 2), ([127, 40], 2, 16, 64, 1), ([33], 4, 64, 64, 4),
+    ([300, 17, 128], 64, 64, 128, 8), ([500], 128, 64, 128, 8), ([200], 3, 48, 128, 3), ([1000], 8, 128, 128, 1)])
+@pytest.mark.parametrize("step", [1e-3, 0.05, 1.0])
+def test_state_space_by_chunks(lens, H, P, N, groups, step, monkeypatch):
+    """No farther from 64-bit than token by token, or than the eight roundings of 6e-8 that the longest chain of products in a
+    chunk leaves (token by token the state is rounded once a token, so its error grows with the tokens that a decay leaves:
+    5e-6 over a thousand tokens that hardly decay)."""
+    from prelude_b200.ops import kernels as K
+    u, dt, bias, a_log, skip, state = _ssm_inputs(lens, H, P, N, groups, 1, step)
+    want_y, want_s = _ssm_exact(u, dt, bias, a_log, skip, state, lens, groups)
+    chunked, plain = state.clone(), state.clone()
+    y = K.ssm_scan(u, dt, bias, a_log, skip, chunked, _batch(lens), groups)
+    _by_tokens(monkeypatch, K)
+    y0 = K.ssm_scan(u, dt, bias, a_log, skip, plain, _batch(lens), groups)
+    errs = [_rel(y, want_y), _rel(chunked, want_s), _rel(y0, want_y), _rel(plain, want_s)]
+    print("chunks y %.2e state %.2e, tokens y %.2e state %.2e" % tuple(errs))
+    assert errs[0] <= max(errs[2], 8 * 6e-8) and errs[1] <= max(errs[3], 8 * 6e-8)
+    assert not torch.equal(y, y0)             # two kernels, not one twice
+
+
+def test_state_space_by_chunks_with_numbers_that_are_not_finite():
+    """An infinity in x spoils its own column from its token on; what lies before it, and other columns, stay as they are."""
+    from prelude_b200.ops import kernels as K
+    lens, H, P, N, groups = [150], 2, 32, 128, 1
+    u, dt, bias, a_log, skip, state = _ssm_inputs(lens, H, P, N, groups, 5, 0.05)
+    clean = K.ssm_scan(u, dt, bias, a_log, skip, state.clone(), _batch(lens), groups)
+    u[70, 3], u[100, P + 5] = float("inf"), float("nan")
+    y = K.ssm_scan(u, dt, bias, a_log, skip, state, _batch(lens), groups)
+    keep = torch.ones_like(y, dtype=torch.bool)
+    keep[70:, 3] = keep[100:, P + 5] = False
+    assert torch.equal(y[keep], clean[keep]) and not torch.isfinite(y[~keep]).any()
+    assert not torch.isfinite(state[0, 0, :, 3]).any() and torch.isfinite(state[0, 0, :, :3]).all()
+
+
+def test_state_space_by_chunks_with_decays_that_leave_nothing():
+    """Rates so large that a step forgets everything: the output is that of the current token alone."""
+    from prelude_b200.ops import kernels as K
+    lens, H, P, N, groups = [100], 2, 32, 64, 1
+    u, dt, bias, a_log, skip, state = _ssm_inputs(lens, H, P, N, groups, 6, 1.0)
+    a_log.fill_(30.0)
+    want_y, want_s = _ssm_exact(u, dt, bias, a_log, skip, state, lens, groups)
+    y = K.ssm_scan(u, dt, bias, a_log, skip, state, _batch(lens), groups)
+    assert _rel(y, want_y) < 1e-6 and _rel(state, want_s) < 1e-6
