@@ -26,16 +26,15 @@ namespace {
 __device__ __forceinline__ float silu_f(float x) { return x / (1.0f + expf(-x)); }
 __device__ __forceinline__ bool pb_aligned_dev(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
 // 16 bytes of a row as floats: 4 of float32, 8 of bfloat16
-__device__ __forceinline__ void pb_ld_vec(const float* p, float (&out)[4]) {
-    const float4 v = *reinterpret_cast<const float4*>(p);
-    out[0] = v.x; out[1] = v.y; out[2] = v.z; out[3] = v.w;
+__device__ __forceinline__ void pb_unpack_vec(const uint4& raw, float (&out)[4]) {
+    out[0] = __uint_as_float(raw.x); out[1] = __uint_as_float(raw.y); out[2] = __uint_as_float(raw.z); out[3] = __uint_as_float(raw.w);
 }
-__device__ __forceinline__ void pb_ld_vec(const __nv_bfloat16* p, float (&out)[8]) {
-    const uint4 raw = *reinterpret_cast<const uint4*>(p);
+__device__ __forceinline__ void pb_unpack_vec(const uint4& raw, float (&out)[8]) {
     const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
 #pragma unroll
     for (int i = 0; i < 4; ++i) { const float2 f = __bfloat1622float2(h[i]); out[2 * i] = f.x; out[2 * i + 1] = f.y; }
 }
+template <typename T, int VN> __device__ __forceinline__ void pb_ld_vec(const T* p, float (&out)[VN]) { pb_unpack_vec(*reinterpret_cast<const uint4*>(p), out); }
 __device__ __forceinline__ void pb_st_vec(float* p, const float (&v)[4]) { *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]); }
 __device__ __forceinline__ void pb_st_vec(__nv_bfloat16* p, const float (&v)[8]) {
     uint4 raw;
@@ -52,7 +51,7 @@ __global__ void causal_conv_silu_kernel(const T* in, long long ld_in, const floa
                                         const float* bias, const T* carried, T* out,
                                         const int32_t* token_seq, const int32_t* positions,
                                         const int32_t* q_start, const int32_t* slots, int n_tokens,
-                                        int channels, int taps) {
+                                        int channels, int taps, T* advance) {
     pb_grid_dep_launch();
     pb_grid_dep_wait();
     const int c = blockIdx.y * blockDim.x + threadIdx.x;
@@ -70,18 +69,23 @@ __global__ void causal_conv_silu_kernel(const T* in, long long ld_in, const floa
         acc = fmaf(w[(size_t)c * taps + j], x, acc);
     }
     pb_st(out + (size_t)t * channels + c, silu_f(acc));
+    if (advance != nullptr) {                              // the sequence's only token: the inputs move on by one
+        T* st = advance + (size_t)slots[seq] * (taps - 1) * channels + c;
+        for (int j = 0; j + 2 < taps; ++j) st[(size_t)j * channels] = st[(size_t)(j + 1) * channels];
+        if (taps > 1) st[(size_t)(taps - 2) * channels] = in[(size_t)t * ld_in + c];
+    }
 }
 
-// The same, 16 bytes of channels per thread and a run of consecutive tokens per block (channels, row stride and
-// pointers in multiples of 16 bytes; TAPS known at compile time).  A thread keeps its channels' taps and the last
-// TAPS - 1 inputs in registers: while the run stays inside one sequence every input is read once.
-#define CONV_RUN 16                                          // a long step; a step of few tokens gives every token a block
-template <typename T, int TAPS>
-__global__ void causal_conv_silu_vec_kernel(const T* in, long long ld_in, const float* w,
-                                            const float* bias, const T* carried, T* out,
-                                            const int32_t* token_seq, const int32_t* positions,
-                                            const int32_t* q_start, const int32_t* slots, int n_tokens,
-                                            int channels, int run) {
+// The same, 16 bytes of channels per thread and RUN consecutive tokens (channels, row stride and pointers in multiples of 16
+// bytes; TAPS known at compile time; a long step: CONV_RUN tokens a thread, a step of few tokens: one).  A run inside one
+// sequence asks for all its rows and the TAPS - 1 before it at once, so a thread waits for memory once; the rows that two
+// runs share come from the caches.  (One token after the other with the window kept in registers waited once a token: 2,048
+// tokens of 10,240 channels 87 us, now 48 and 5 of launching.)
+#define CONV_RUN 8
+template <typename T, int TAPS, int RUN>
+__global__ void __launch_bounds__(128) causal_conv_silu_vec_kernel(const T* in, long long ld_in, const float* w, const float* bias, const T* carried,
+                                                                   T* out, const int32_t* token_seq, const int32_t* positions, const int32_t* q_start,
+                                                                   const int32_t* slots, int n_tokens, int channels, T* advance) {
     constexpr int VN = 16 / sizeof(T);
     pb_grid_dep_launch();
     const int c = (blockIdx.y * blockDim.x + threadIdx.x) * VN;
@@ -90,41 +94,59 @@ __global__ void causal_conv_silu_vec_kernel(const T* in, long long ld_in, const 
 #pragma unroll
     for (int e = 0; e < VN; ++e) {
         bs[e] = bias ? bias[c + e] : 0.f;
+        if constexpr (TAPS == 4) {
+            const float4 v = *reinterpret_cast<const float4*>(w + (size_t)(c + e) * 4);
+            wt[e][0] = v.x; wt[e][1] = v.y; wt[e][2] = v.z; wt[e][3] = v.w;
+        } else {
 #pragma unroll
-        for (int j = 0; j < TAPS; ++j) wt[e][j] = w[(size_t)(c + e) * TAPS + j];
+            for (int j = 0; j < TAPS; ++j) wt[e][j] = w[(size_t)(c + e) * TAPS + j];
+        }
     }
     pb_grid_dep_wait();
-    float win[TAPS][VN];                                   // win[j]: the input under tap j
-    int prev_seq = -1;
-    const int t_end = min(n_tokens, (int)(blockIdx.x + 1) * run);
-    for (int t = blockIdx.x * run; t < t_end; ++t) {
-        const int seq = token_seq[t];
-        if (seq < 0) { prev_seq = -1; continue; }          // a padding row
-        const int i = positions[t] - q_start[seq];
-        if (seq == prev_seq) {                             // the token after the one before: shift, fetch one
-#pragma unroll
-            for (int j = 0; j + 1 < TAPS; ++j)
-#pragma unroll
-                for (int e = 0; e < VN; ++e) win[j][e] = win[j + 1][e];
-            pb_ld_vec(in + (size_t)t * ld_in + c, win[TAPS - 1]);
-        } else {
-            const T* old = carried + (size_t)slots[seq] * (TAPS - 1) * channels;
-#pragma unroll
-            for (int j = 0; j < TAPS; ++j) {
-                const int idx = i - (TAPS - 1 - j);
-                pb_ld_vec(idx >= 0 ? in + (size_t)(t - (TAPS - 1 - j)) * ld_in + c : old + (size_t)(TAPS - 1 + idx) * channels + c, win[j]);
-            }
-            prev_seq = seq;
-        }
+    const int t0 = blockIdx.x * RUN, t_end = min(n_tokens, t0 + RUN);
+    // row `idx` (below 0: before the step) of the sequence whose token `t` has in-step index `i`
+    auto row = [&](int t, int i, const T* old, int idx) {
+        return idx >= 0 ? in + (size_t)(t - i + idx) * ld_in + c : old + (size_t)(TAPS - 1 + idx) * channels + c;
+    };
+    auto token = [&](int t, const uint4* win) {            // win[j]: the input under tap j
         float acc[VN];
 #pragma unroll
-        for (int e = 0; e < VN; ++e) {
-            float a = bs[e];
+        for (int e = 0; e < VN; ++e) acc[e] = bs[e];
 #pragma unroll
-            for (int j = 0; j < TAPS; ++j) a = fmaf(wt[e][j], win[j][e], a);
-            acc[e] = silu_f(a);
+        for (int j = 0; j < TAPS; ++j) {
+            float x[VN];
+            pb_unpack_vec(win[j], x);
+#pragma unroll
+            for (int e = 0; e < VN; ++e) acc[e] = fmaf(wt[e][j], x[e], acc[e]);
         }
+#pragma unroll
+        for (int e = 0; e < VN; ++e) acc[e] = silu_f(acc[e]);
         pb_st_vec(out + (size_t)t * channels + c, acc);
+    };
+    const int seq0 = token_seq[t0];
+    if (RUN > 1 && t0 + RUN <= n_tokens && seq0 >= 0 && token_seq[t0 + RUN - 1] == seq0) {
+        const int i = positions[t0] - q_start[seq0];
+        const T* old = carried + (size_t)slots[seq0] * (TAPS - 1) * channels;
+        uint4 rows[RUN + TAPS - 1];
+#pragma unroll
+        for (int j = 0; j < RUN + TAPS - 1; ++j) rows[j] = *reinterpret_cast<const uint4*>(row(t0, i, old, i - (TAPS - 1) + j));
+#pragma unroll
+        for (int k = 0; k < RUN; ++k) token(t0 + k, rows + k);
+        return;
+    }
+    for (int t = t0; t < t_end; ++t) {                     // a run over the end of a sequence, and a step of few tokens
+        const int seq = token_seq[t];
+        if (seq < 0) continue;                             // a padding row
+        const int i = positions[t] - q_start[seq];
+        const T* old = carried + (size_t)slots[seq] * (TAPS - 1) * channels;
+        uint4 win[TAPS];
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) win[j] = *reinterpret_cast<const uint4*>(row(t, i, old, i - (TAPS - 1) + j));
+        token(t, win);
+        if (RUN == 1 && advance != nullptr) {              // the sequence's only token: the inputs move on by one
+#pragma unroll
+            for (int j = 1; j < TAPS; ++j) *reinterpret_cast<uint4*>(advance + ((size_t)slots[seq] * (TAPS - 1) + j - 1) * channels + c) = win[j];
+        }
     }
 }
 
@@ -362,50 +384,53 @@ __global__ void gated_group_rmsnorm_kernel(const float* y, const T* z, long long
         pb_st(o + i, yr[i] * gate(pb_ld(zr + i)) * inv * w[(size_t)part * width + i]);   // the same product either way
 }
 
-// The same for parts of up to 128 * ITERS elements (a norm per head): a warp per (token, part), four elements per access, the
-// part kept in registers between the sum and the store.  width, ld_z in multiples of 4, operands aligned.
+// The same for parts of up to 128 * ITERS elements: a warp per (token, part), four elements per access, the whole part asked for
+// at once and kept in registers between the sum and the store; the scales, which all tokens share, come from the caches when they
+// are needed.  width, ld_z in multiples of 4, operands aligned.  Parts of 1,024 (ITERS 8) on the kernel above, which reads a part
+// twice, an element an access: 2,048 x 8,192 in 80 us, here 51.
 template <typename T, int ITERS>
-__global__ void __launch_bounds__(256) gated_part_rmsnorm_kernel(const float* y, const T* z, long long ld_z,
-                                                                 const float* w, T* out, int n_tokens, int inner, int parts,
-                                                                 float eps, int gate_after, int sigmoid_gate) {
+__global__ void __launch_bounds__(256, ITERS >= 8 ? 3 : 4) gated_part_rmsnorm_kernel(const float* y, const T* z, long long ld_z, const float* w, T* out, int n_tokens,
+                                                                 int inner, int parts, float eps, int gate_after, int sigmoid_gate) {
     pb_grid_dep_launch();
     const int lane = threadIdx.x & 31, width = inner / parts;
     const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (item >= (long long)n_tokens * parts) return;
     const int t = (int)(item / parts), part = (int)(item % parts);
-    float4 wv[ITERS], yv[ITERS], gv[ITERS];
-#pragma unroll
-    for (int i = 0; i < ITERS; ++i) {
-        const int c = (lane + 32 * i) * 4;
-        wv[i] = c < width ? *reinterpret_cast<const float4*>(w + (size_t)part * width + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
+    float4 yv[ITERS];
+    uint2 zv[ITERS];
+    float4 zf[sizeof(T) == 4 ? ITERS : 1];
+    const float* wr = w + (size_t)part * width;
     pb_grid_dep_wait();
     const float* yr = y + (size_t)t * inner + (size_t)part * width;
     const T* zr = z + (size_t)t * ld_z + (size_t)part * width;
 #pragma unroll
     for (int i = 0; i < ITERS; ++i) {
         const int c = (lane + 32 * i) * 4;
-        yv[i] = gv[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        yv[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        zv[i] = make_uint2(0, 0);
+        if constexpr (sizeof(T) == 4) zf[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (c < width) {
             yv[i] = *reinterpret_cast<const float4*>(yr + c);
-            if constexpr (sizeof(T) == 2) {
-                const uint2 raw = *reinterpret_cast<const uint2*>(zr + c);
-                const __nv_bfloat162* hh = reinterpret_cast<const __nv_bfloat162*>(&raw);
-                const float2 a = __bfloat1622float2(hh[0]), b = __bfloat1622float2(hh[1]);
-                gv[i] = make_float4(a.x, a.y, b.x, b.y);
-            } else {
-                gv[i] = *reinterpret_cast<const float4*>(zr + c);
-            }
+            if constexpr (sizeof(T) == 2) zv[i] = *reinterpret_cast<const uint2*>(zr + c);
+            else zf[i] = *reinterpret_cast<const float4*>(zr + c);
         }
     }
     auto gate = [&](float v) { return sigmoid_gate ? 1.0f / (1.0f + expf(-v)) : silu_f(v); };
     float ss = 0.f;
 #pragma unroll
     for (int i = 0; i < ITERS; ++i) {
-        gv[i] = make_float4(gate(gv[i].x), gate(gv[i].y), gate(gv[i].z), gate(gv[i].w));
-        float4 v = yv[i];
-        if (!gate_after) { v.x *= gv[i].x; v.y *= gv[i].y; v.z *= gv[i].z; v.w *= gv[i].w; }
-        ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+        float4 g;
+        if constexpr (sizeof(T) == 2) {
+            const __nv_bfloat162* hh = reinterpret_cast<const __nv_bfloat162*>(&zv[i]);
+            const float2 a = __bfloat1622float2(hh[0]), b = __bfloat1622float2(hh[1]);
+            g = make_float4(a.x, a.y, b.x, b.y);
+        } else {
+            g = zf[i];
+        }
+        const float4 v = make_float4(yv[i].x * gate(g.x), yv[i].y * gate(g.y), yv[i].z * gate(g.z), yv[i].w * gate(g.w));
+        const float4 n = gate_after ? yv[i] : v;
+        ss += n.x * n.x + n.y * n.y + n.z * n.z + n.w * n.w;
+        yv[i] = v;                                             // the same product either way
     }
     const float inv = 1.0f / sqrtf(pb_warp_sum(ss) / (float)width + eps);
     T* o = out + (size_t)t * inner + (size_t)part * width;
@@ -413,8 +438,8 @@ __global__ void __launch_bounds__(256) gated_part_rmsnorm_kernel(const float* y,
     for (int i = 0; i < ITERS; ++i) {
         const int c = (lane + 32 * i) * 4;
         if (c < width) {
-            const float r[4] = {yv[i].x * gv[i].x * inv * wv[i].x, yv[i].y * gv[i].y * inv * wv[i].y, yv[i].z * gv[i].z * inv * wv[i].z,
-                                yv[i].w * gv[i].w * inv * wv[i].w};
+            const float4 wv = *reinterpret_cast<const float4*>(wr + c);
+            const float r[4] = {yv[i].x * inv * wv.x, yv[i].y * inv * wv.y, yv[i].z * inv * wv.z, yv[i].w * inv * wv.w};
             if constexpr (sizeof(T) == 2) {
                 const __nv_bfloat162 a = __floats2bfloat162_rn(r[0], r[1]), b = __floats2bfloat162_rn(r[2], r[3]);
                 uint2 raw;
@@ -440,7 +465,9 @@ __global__ void scaled_sum_kernel(const TI* a, float sa, const TI* b, float sb, 
 
 // in: the step's [x | B | C] columns of the input projection, [n_tokens, channels] with row stride ld_in; w float32
 // [channels, taps] (last column: the current token); carried [slots, taps - 1, channels]; out [n_tokens, channels] dense.
-PB_API int pb_causal_conv_silu(const void* in, long long ld_in, const float* w, const float* bias, const void* carried, void* out,
+// `advance`: every sequence has one token in this step, and the carried inputs are moved on as pb_conv_state_update would (the
+// thread that reads a sequence's inputs of a channel is then the only one that does: one launch less in a decode step).
+PB_API int pb_causal_conv_silu(const void* in, long long ld_in, const float* w, const float* bias, void* carried, void* out, int advance,
                                int dtype, const int32_t* token_seq, const int32_t* positions, const int32_t* q_start,
                                const int32_t* slots, int n_tokens, int channels, int taps, cudaStream_t stream) {
     PB_REQUIRE(n_tokens >= 0 && channels > 0 && taps >= 1 && ld_in >= channels, "causal_conv_silu: bad sizes");
@@ -448,22 +475,24 @@ PB_API int pb_causal_conv_silu(const void* in, long long ld_in, const float* w, 
     if (n_tokens == 0) return 0;
     PB_REQUIRE((channels + 127) / 128 < 65536, "causal_conv_silu: %d channels in one launch", channels);
     const int vn = dtype == PB_BF16 ? 8 : 4;
-    if (taps >= 2 && taps <= 4 && channels % vn == 0 && ld_in % vn == 0 && pb_aligned(in, 16) && pb_aligned(out, 16) && pb_aligned(carried, 16)) {
-        const int run = n_tokens <= 64 ? 1 : CONV_RUN;
-        const dim3 grid((n_tokens + run - 1) / run, (channels / vn + 63) / 64);
-#define CONV_LAUNCH(TAPS)                                                                                                     \
-    PB_DISPATCH_DTYPE(dtype, T, (pb_launch(causal_conv_silu_vec_kernel<T, TAPS>, grid, dim3(64), 0, stream, (const T*)in, ld_in, w, bias, \
-                                           (const T*)carried, (T*)out, token_seq, positions, q_start, slots, n_tokens, channels, run)))
-        if (taps == 2) CONV_LAUNCH(2);
-        else if (taps == 3) CONV_LAUNCH(3);
-        else CONV_LAUNCH(4);
+    if (taps >= 2 && taps <= 4 && channels % vn == 0 && ld_in % vn == 0 && pb_aligned(in, 16) && pb_aligned(out, 16) && pb_aligned(carried, 16) &&
+        (taps != 4 || pb_aligned(w, 16))) {
+        // up to 64 tokens a thread has one: a run's threads would leave most of the chip idle
+        const int run = n_tokens <= 64 || advance ? 1 : CONV_RUN, threads = run == 1 ? 64 : 128;
+        const dim3 grid((n_tokens + run - 1) / run, (channels / vn + threads - 1) / threads);
+#define CONV_LAUNCH(TAPS, RUN)                                                                                                \
+    PB_DISPATCH_DTYPE(dtype, T, (pb_launch(causal_conv_silu_vec_kernel<T, TAPS, RUN>, grid, dim3(threads), 0, stream, (const T*)in, ld_in, w, bias, \
+                                           (const T*)carried, (T*)out, token_seq, positions, q_start, slots, n_tokens, channels, advance ? (T*)carried : (T*)nullptr)))
+        if (taps == 2) { if (run == 1) CONV_LAUNCH(2, 1); else CONV_LAUNCH(2, CONV_RUN); }
+        else if (taps == 3) { if (run == 1) CONV_LAUNCH(3, 1); else CONV_LAUNCH(3, CONV_RUN); }
+        else { if (run == 1) CONV_LAUNCH(4, 1); else CONV_LAUNCH(4, CONV_RUN); }
 #undef CONV_LAUNCH
         PB_CHECK_LAUNCH("causal_conv_silu");
         return 0;
     }
     PB_DISPATCH_DTYPE(dtype, T,
         (pb_launch(causal_conv_silu_kernel<T>, dim3(n_tokens, (channels + 127) / 128), dim3(128), 0, stream, (const T*)in, ld_in, w, bias,
-                   (const T*)carried, (T*)out, token_seq, positions, q_start, slots, n_tokens, channels, taps)));
+                   (const T*)carried, (T*)out, token_seq, positions, q_start, slots, n_tokens, channels, taps, advance ? (T*)carried : (T*)nullptr)));
     PB_CHECK_LAUNCH("causal_conv_silu");
     return 0;
 }
@@ -546,7 +575,9 @@ PB_API int pb_gated_group_rmsnorm(const float* y, const void* z, long long ld_z,
     PB_REQUIRE(parts < 65536, "gated_group_rmsnorm: %d parts", parts);
     const int width = inner / parts;
     const size_t esz = dtype == PB_BF16 ? 2 : 4;
-    if (width <= 512 && width % 4 == 0 && ld_z % 4 == 0 && pb_aligned(y, 16) && pb_aligned(w, 16) && pb_aligned(z, 4 * esz) && pb_aligned(out, 4 * esz)) {
+    // parts of up to 1,024 in bfloat16 too where there are rows enough that a warp each fills the chip (2 x 8,192: 13 us against 11
+    // for a block each); in 32-bit a row's sum keeps one order whatever the step holds
+    if ((width <= 512 || (width <= 1024 && dtype == PB_BF16 && (long long)n_tokens * parts >= 4096)) && width % 4 == 0 && ld_z % 4 == 0 && pb_aligned(y, 16) && pb_aligned(w, 16) && pb_aligned(z, 4 * esz) && pb_aligned(out, 4 * esz)) {
         const long long items = (long long)n_tokens * parts;
         const int warps = items >= 4096 ? 8 : 1;
         const dim3 grid((unsigned)((items + warps - 1) / warps)), block(32 * warps);
@@ -556,7 +587,8 @@ PB_API int pb_gated_group_rmsnorm(const float* y, const void* z, long long ld_z,
                                            parts, eps, gate_after, sigmoid_gate)))
         if (width <= 128) PART_LAUNCH(1);
         else if (width <= 256) PART_LAUNCH(2);
-        else PART_LAUNCH(4);
+        else if (width <= 512) PART_LAUNCH(4);
+        else PART_LAUNCH(8);
 #undef PART_LAUNCH
         PB_CHECK_LAUNCH("gated_group_rmsnorm");
         return 0;

@@ -997,9 +997,10 @@ def attention_paged(q: torch.Tensor, k_pages: torch.Tensor, v_pages: Optional[to
 
 # -- the state-space mixer ------------------------------------------------------------------------------------------
 def causal_conv_silu(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], carried: torch.Tensor, batch,
-                     out: Optional[torch.Tensor] = None) -> torch.Tensor:
+                     out: Optional[torch.Tensor] = None, advance: bool = False) -> torch.Tensor:
     """silu(conv(x) + bias) per channel; x [T, C] a view with dense rows, weight float32 [C, taps], bias float32 [C] or
-    None, carried [slots, taps - 1, C] of x's type (the sequences' last inputs of earlier steps)."""
+    None, carried [slots, taps - 1, C] of x's type (the sequences' last inputs of earlier steps).  ``advance``: every sequence
+    has one token in this step, and ``carried`` is moved on as well (``conv_state_update`` does that for any step)."""
     _need(x, "x", contiguous=False)
     _need(weight, "weight", torch.float32)
     if bias is not None:
@@ -1012,7 +1013,7 @@ def causal_conv_silu(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch
     if out is None:
         out = torch.empty((T, C), dtype=x.dtype, device=x.device)
     check(_l.library().pb_causal_conv_silu(x.data_ptr(), x.stride(0), weight.data_ptr(), _ptr(bias), carried.data_ptr(),
-                                           out.data_ptr(), dtype_code(x.dtype), batch.token_seq.data_ptr(), batch.positions.data_ptr(),
+                                           out.data_ptr(), 1 if advance else 0, dtype_code(x.dtype), batch.token_seq.data_ptr(), batch.positions.data_ptr(),
                                            batch.q_start.data_ptr(), batch.state_slots.data_ptr(), T, C, taps, _stream()),
           "causal_conv_silu")
     return out

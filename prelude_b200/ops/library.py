@@ -97,7 +97,7 @@ _SIGNATURES = {
     "pb_attention_paged_tc_tile_tokens": ([I, I], I),
     "pb_attention_paged_tc_scratch_floats": ([I, I, I, I], L),
     "pb_attention_paged_tc_bf16": ([P, P, P, P, P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, I, I, F, I, I, I, F, P, L, I, P, P, P], I),
-    "pb_causal_conv_silu": ([P, L, P, P, P, P, I, P, P, P, P, I, I, I, P], I),
+    "pb_causal_conv_silu": ([P, L, P, P, P, P, I, I, P, P, P, P, I, I, I, P], I),
     "pb_conv_state_update": ([P, L, P, I, P, P, I, I, I, P], I),
     "pb_ssm_scan": ([P, P, L, I, P, P, P, P, P, P, P, I, I, I, I, I, P], I),
     "pb_ssm_scan_chunked_takes": ([P, I, I, I, I], I),

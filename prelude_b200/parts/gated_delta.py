@@ -91,8 +91,10 @@ class GatedDelta:
         g0 = self.channels
         b0 = g0 + self.inner
         qkv, gate, beta, a = proj[:, :g0], proj[:, g0:b0], proj[:, b0:b0 + H], proj[:, b0 + H:b0 + 2 * H]
-        u = K.causal_conv_silu(qkv, self.conv_w, None, carried, batch, out=batch.workspace("delta_conv", (T, self.channels), x.dtype))
-        K.conv_state_update(qkv, carried, batch)
+        u = K.causal_conv_silu(qkv, self.conv_w, None, carried, batch, out=batch.workspace("delta_conv", (T, self.channels), x.dtype),
+                               advance=batch.decode_only)
+        if not batch.decode_only:
+            K.conv_state_update(qkv, carried, batch)
         o = K.gated_delta_scan(u, beta, a, self.a_log, self.dt_bias, state, batch, s.num_kv_heads,
                                out=batch.workspace("delta_o", (T, self.inner), torch.float32))
         y = K.gated_group_rmsnorm(o, gate, self.norm_w, H, s.norm_eps, out=batch.workspace("delta_gated", (T, self.inner), x.dtype),

@@ -73,8 +73,10 @@ class StateSpace:
         proj = linear(x, self.w_in)
         z, xbc, dt = proj[:, :self.inner], proj[:, self.inner:self.inner + self.channels], proj[:, self.inner + self.channels:]
         u = K.causal_conv_silu(xbc, self.conv_w, self.conv_b, carried, batch,
-                               out=batch.workspace("ssm_conv", (T, self.channels), x.dtype))
-        K.conv_state_update(xbc, carried, batch)
+                               out=batch.workspace("ssm_conv", (T, self.channels), x.dtype),
+                               advance=batch.decode_only)
+        if not batch.decode_only:
+            K.conv_state_update(xbc, carried, batch)
         y = K.ssm_scan(u, dt, self.dt_bias, self.a_log, self.d_skip, state, batch, s.groups,
                        out=batch.workspace("ssm_y", (T, self.inner), torch.float32))
         g = K.gated_group_rmsnorm(y, z, self.norm_w, s.norm_groups, s.norm_eps,
