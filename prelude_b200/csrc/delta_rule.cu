@@ -12,7 +12,7 @@
 // cut into steps or on what else is in the batch.  The state of a sequence is read at the start of a step from its
 // slot and written back at the end.  Sequences are found through device arrays (cumulative lengths, state slots), one
 // block row per sequence the arrays have room for; a row whose length is not positive is skipped, so the launch has
-// the same shape whatever the step holds and can be recorded.
+// the same shape whatever the step holds and can be recorded.  (A prompt step in bfloat16 runs by chunks: delta_chunk.cu.)
 //
 // A block is eight warps on one head's state, 16 columns p of it.  Warps 0-3 compute: 16 columns x 8 lanes over the
 // state rows n, a lane keeping NPL rows in registers (rows 4 (8 i + j) .. + 3, so that the lanes of a column read

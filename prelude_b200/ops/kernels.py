@@ -1028,8 +1028,10 @@ def conv_state_update(x: torch.Tensor, carried: torch.Tensor, batch) -> None:
                                             _stream()), "conv_state_update")
 
 
-# tokens of a prompt step from which the recurrences run by chunks of tokens on the tensor cores (bfloat16 only)
+# tokens of a prompt step from which the recurrences run by chunks of tokens on the tensor cores (bfloat16 only).  State space:
+# 12 us either way at 32 tokens, 11.5 against 20 at 64; the gated delta rule, two kernels: 24 against 16 at 32, 24 against 28 at 64
 SCAN_CHUNKED_MIN_TOKENS = 32
+DELTA_CHUNKED_MIN_TOKENS = 64
 
 
 def ssm_scan(u: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: torch.Tensor, d_skip: torch.Tensor,
@@ -1268,7 +1270,8 @@ def gated_delta_scan(u: torch.Tensor, beta: torch.Tensor, a: torch.Tensor, a_log
                      state: torch.Tensor, batch, kv_heads: int, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """The gated delta rule over the step's tokens, sequence by sequence; u [T, 2 G D + H E] laid out [q | k | v] (the
     convolutions' outputs), beta and a [T, H] views with dense rows, state float32 [slots, H, D, E]; returns o float32
-    [T, H E].  See csrc/delta_rule.cu."""
+    [T, H E].  A prompt step in bfloat16 runs by chunks of tokens (csrc/delta_chunk.cu), in 32-bit and in a decode step token by
+    token (csrc/delta_rule.cu)."""
     T = u.shape[0]
     _rows_view(u, "u", T, None)
     _rows_view(beta, "beta", T, u.dtype)
@@ -1280,9 +1283,20 @@ def gated_delta_scan(u: torch.Tensor, beta: torch.Tensor, a: torch.Tensor, a_log
         raise KernelLibraryError(f"gated_delta_scan: u {tuple(u.shape)}, state {tuple(state.shape)}, {kv_heads} query/key heads")
     if out is None:
         out = torch.empty((T, H * E), dtype=torch.float32, device=u.device)
-    check(_l.library().pb_gated_delta_scan(u.data_ptr(), u.stride(0), beta.data_ptr(), beta.stride(0), a.data_ptr(), a.stride(0),
+    lib, n_seqs = _l.library(), batch.cu_q.numel() - 1
+    if (u.dtype == torch.bfloat16 and T >= DELTA_CHUNKED_MIN_TOKENS and not batch.decode_only
+            and lib.pb_gated_delta_chunked_takes(u.data_ptr(), u.stride(0), H, kv_heads, D, E)):
+        # what one kernel makes of every chunk for the other to read: dead when the call's kernels are done
+        n_chunks = lib.pb_gated_delta_chunks(T, n_seqs)
+        scratch = torch.empty((lib.pb_gated_delta_chunk_bytes(n_chunks, H),), dtype=torch.uint8, device=u.device)
+        check(lib.pb_gated_delta_scan_chunked(u.data_ptr(), u.stride(0), beta.data_ptr(), beta.stride(0), a.data_ptr(), a.stride(0),
+                                              a_log.data_ptr(), dt_bias.data_ptr(), state.data_ptr(), out.data_ptr(), batch.cu_q.data_ptr(),
+                                              batch.state_slots.data_ptr(), scratch.data_ptr(), n_chunks, n_seqs, H, kv_heads, D, E,
+                                              _stream()), "gated_delta_scan_chunked")
+        return out
+    check(lib.pb_gated_delta_scan(u.data_ptr(), u.stride(0), beta.data_ptr(), beta.stride(0), a.data_ptr(), a.stride(0),
                                            dtype_code(u.dtype), a_log.data_ptr(), dt_bias.data_ptr(), state.data_ptr(), out.data_ptr(),
-                                           batch.cu_q.data_ptr(), batch.state_slots.data_ptr(), batch.cu_q.numel() - 1, H, kv_heads, D, E,
+                                           batch.cu_q.data_ptr(), batch.state_slots.data_ptr(), n_seqs, H, kv_heads, D, E,
                                            _stream()), "gated_delta_scan")
     return out
 

@@ -125,6 +125,10 @@ _SIGNATURES = {
     "pb_tanh": ([P, P, I, L, P], I),
     "pb_heads_prepare": ([P, L, P, L, P, L, I, P, P, I, F, P, F, I, I, P, P, L, F, P, P, P, I, I, I, P, P, P, I, I, I, I, I, I, I, P, P], I),
     "pb_gated_delta_scan": ([P, L, P, L, P, L, I, P, P, P, P, P, P, I, I, I, I, I, P], I),
+    "pb_gated_delta_chunked_takes": ([P, L, I, I, I, I], I),
+    "pb_gated_delta_chunks": ([I, I], I),
+    "pb_gated_delta_chunk_bytes": ([I, I], L),
+    "pb_gated_delta_scan_chunked": ([P, L, P, L, P, L, P, P, P, P, P, P, P, I, I, I, I, I, I, P], I),
     "pb_token_shift_mix": ([P, P, P, P, I, P, P, P, P, I, I, I, P], I),
     "pb_wkv_scan": ([P, L, P, L, P, L, P, L, I, P, P, P, P, P, P, I, I, I, P], I),
 }

@@ -76,7 +76,8 @@ class GatedDelta:
         self.norm_w = vec(s.norm_name).repeat(s.num_heads).contiguous()     # one scale over value_dim, shared by the heads
 
     def activation_bytes_per_token(self, elem: int) -> int:
-        return (self.proj_cols + 8 + self.channels + self.inner) * elem + self.inner * 4 + self.spec.hidden_size * elem
+        # the scan by chunks of 64 tokens leaves 32 KB a chunk and head between its two kernels
+        return (self.proj_cols + 8 + self.channels + self.inner) * elem + self.inner * 4 + self.spec.hidden_size * elem + self.spec.num_heads * 512
 
     def cache_need(self) -> CombinedNeed:
         s = self.spec

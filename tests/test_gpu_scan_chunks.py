@@ -51,9 +51,17 @@ def _ssm_exact(u, dt, bias, a_log, skip, state, lens, groups):
     return y.view(-1, inner), S
 
 
+@pytest.fixture(autouse=True)
+def _chunks_whatever_the_length(monkeypatch):
+    from prelude_b200.ops import kernels as K
+    for name in ("SCAN_CHUNKED_MIN_TOKENS", "DELTA_CHUNKED_MIN_TOKENS"):
+        monkeypatch.setattr(K, name, 1)
+
+
 def _by_tokens(monkeypatch, K):
     """The same call through the kernel that visits the tokens one by one."""
-    monkeypatch.setattr(K, "SCAN_CHUNKED_MIN_TOKENS", 1 << 30)
+    for name in ("SCAN_CHUNKED_MIN_TOKENS", "DELTA_CHUNKED_MIN_TOKENS"):
+        monkeypatch.setattr(K, name, 1 << 30)
 
 
 @pytest.mark.parametrize("lens,H,P,N,groups", [
@@ -100,3 +108,72 @@ def test_state_space_by_chunks_with_decays_that_leave_nothing():
     want_y, want_s = _ssm_exact(u, dt, bias, a_log, skip, state, lens, groups)
     y = K.ssm_scan(u, dt, bias, a_log, skip, state, _batch(lens), groups)
     assert _rel(y, want_y) < 1e-6 and _rel(state, want_s) < 1e-6
+
+
+def _delta_inputs(lens, H, G, D, E, seed, step, key_noise=1.0):
+    """``key_noise`` below 1: keys that nearly repeat, so that what a token writes takes most of what the one before it wrote."""
+    gen = torch.Generator(device=DEV).manual_seed(seed)
+    T = sum(lens)
+
+    def normal(*shape):
+        return torch.randn(shape, generator=gen, device=DEV)
+
+    k = key_noise * normal(T, G * D) + (1 - key_noise) * normal(1, G * D)
+    u = torch.cat([normal(T, G * D), k, normal(T, H * E)], 1).bfloat16()
+    proj = normal(T, 2 * H + 8).bfloat16()
+    bias = torch.full((H,), math.log(math.expm1(step)), device=DEV) + 0.3 * normal(H)
+    a_log = torch.log(torch.rand(H, generator=gen, device=DEV) * 15 + 1)
+    return u, proj[:, :H], proj[:, H:2 * H], a_log, bias, normal(len(lens), H, D, E)
+
+
+def _delta_exact(u, b, a, a_log, bias, state, lens, G):
+    R, H, D, E = state.shape
+    u, S, at, T = u.double(), state.double().clone(), 0, u.shape[0]
+    q, k, v = u[:, :G * D].view(T, G, D), u[:, G * D:2 * G * D].view(T, G, D), u[:, 2 * G * D:].view(T, H, E)
+    q, k = ((x / torch.sqrt((x * x).sum(-1, keepdim=True) + 1e-6)).repeat_interleave(H // G, 1) for x in (q, k))
+    beta = torch.sigmoid(b.double())
+    decay = torch.exp(-torch.exp(a_log.double()) * torch.nn.functional.softplus(a.double() + bias.double(), threshold=50))
+    o = torch.empty(T, H, E, dtype=torch.float64, device=DEV)
+    for r, n in enumerate(lens):
+        slot = R - 1 - r
+        for t in range(at, at + n):
+            s = decay[t].view(H, 1, 1) * S[slot]
+            w = beta[t].view(H, 1) * (v[t] - (s * k[t].unsqueeze(2)).sum(1))
+            S[slot] = s + k[t].unsqueeze(2) * w.unsqueeze(1)
+            o[t] = (S[slot] * q[t].unsqueeze(2)).sum(1) * D ** -0.5
+        at += n
+    return o.view(T, H * E), S
+
+
+@pytest.mark.parametrize("lens,H,G,D,E", [
+    ([64], 4, 2, 128, 128), ([65, 1, 63], 4, 4, 64, 32), ([127, 40], 2, 1, 128, 16), ([33], 4, 2, 64, 64), ([1] * 40 + [70], 2, 2, 64, 16),
+    ([300, 17, 128], 16, 8, 128, 128), ([500], 32, 16, 128, 128), ([200], 3, 3, 128, 48), ([1000], 2, 1, 128, 32)])
+@pytest.mark.parametrize("step,key_noise", [(1e-3, 1.0), (0.05, 1.0), (1.0, 1.0), (1e-3, 0.1)])
+def test_gated_delta_rule_by_chunks(lens, H, G, D, E, step, key_noise, monkeypatch):
+    """No farther from 64-bit than token by token, or than a few roundings of 6e-8: eight products in the longest chain, and three
+    such products one behind the other (into the state, through the inverse, out of the state)."""
+    from prelude_b200.ops import kernels as K
+    u, b, a, a_log, bias, state = _delta_inputs(lens, H, G, D, E, 2, step, key_noise)
+    want_o, want_s = _delta_exact(u, b, a, a_log, bias, state, lens, G)
+    chunked, plain = state.clone(), state.clone()
+    o = K.gated_delta_scan(u, b, a, a_log, bias, chunked, _batch(lens), G)
+    _by_tokens(monkeypatch, K)
+    o0 = K.gated_delta_scan(u, b, a, a_log, bias, plain, _batch(lens), G)
+    errs = [_rel(o, want_o), _rel(chunked, want_s), _rel(o0, want_o), _rel(plain, want_s)]
+    print("chunks o %.2e state %.2e, tokens o %.2e state %.2e" % tuple(errs))
+    assert errs[0] <= max(errs[2], 3 * 8 * 6e-8) and errs[1] <= max(errs[3], 3 * 8 * 6e-8)
+    assert not torch.equal(o, o0)
+
+
+def test_gated_delta_rule_by_chunks_with_numbers_that_are_not_finite():
+    """An infinity in v spoils its own column from its token on, one in a key every column; what lies before stays as it is."""
+    from prelude_b200.ops import kernels as K
+    lens, H, G, D, E = [150], 2, 2, 64, 32
+    u, b, a, a_log, bias, state = _delta_inputs(lens, H, G, D, E, 5, 0.05)
+    clean = K.gated_delta_scan(u, b, a, a_log, bias, state.clone(), _batch(lens), G)
+    u[70, 2 * G * D + 3], u[100, G * D + D + 7] = float("inf"), float("nan")
+    o = K.gated_delta_scan(u, b, a, a_log, bias, state, _batch(lens), G)
+    keep = torch.ones_like(o, dtype=torch.bool)
+    keep[70:, 3] = keep[100:, E:] = False
+    assert torch.equal(o[keep], clean[keep]) and not torch.isfinite(o[~keep]).any()
+    assert not torch.isfinite(state[0, 0, :, 3]).any() and torch.isfinite(state[0, 0, :, :3]).all() and not torch.isfinite(state[0, 1]).any()
