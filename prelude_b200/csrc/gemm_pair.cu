@@ -26,7 +26,7 @@
 // from the float32 sums, without the merged projection ever being written or read.
 //
 // Work.  Persistent pairs: pair p of P takes tiles p, p + P, ...; tiles run down the rows of A first, so that the
-// pairs of a wave share a panel of B in the L2 cache.  (Dealing the last wave out in units of (tile, 64 of K), with
+// pairs of a wave share a panel of B in the L2 cache (the grouped form: along the columns first, see gp_tm).  (Dealing the last wave out in units of (tile, 64 of K), with
 // the parts of a split tile summed through the L2 cache, was measured: the products are bound by power here, not by
 // idle pairs - 64 pairs take as long as 74 - and the summing cost 10 us, so it did not pay.)
 //
@@ -89,6 +89,14 @@ struct GpParams {
     const int32_t* offsets;
     int expert_rows_b, map_rows_b;
 };
+
+// Which row tile and which column tile a pair's tile is.  Plain forms run down the rows of A first: the pairs of a wave share a
+// panel of B.  The grouped form runs along an expert's features first: the pairs of a wave then share a few experts' rows, which
+// stay in the L2 cache, and every panel of the experts' matrices is read once whichever way round.  (Rows first, all experts' rows
+// came from memory again for every column tile: 12,288 rows of 4,096 beside 2.1 GB of gate and up rows.  64 experts of
+// 2,048: gate and up 731 -> 455 us, down 346 -> 220.)
+__device__ __forceinline__ int gp_tm(const GpParams& p, int tile) { return p.tile_expert ? tile / p.tiles_n : tile % p.tiles_m; }
+__device__ __forceinline__ int gp_tn(const GpParams& p, int tile) { return p.tile_expert ? tile % p.tiles_n : tile / p.tiles_m; }
 
 // Where row tile tm lies: false when the grouped form has no such tile.
 __device__ __forceinline__ bool gp_tile(const GpParams& p, int tm, int& row_base, int& row_limit, int& b_off) {
@@ -322,7 +330,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             bool waited = false;
             if (!p.b_is_constant || p.tile_expert) { pb_grid_dep_wait(); waited = true; }   // the tile map is the kernel before's
             for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
-                const int tm = tile % p.tiles_m, tn = tile / p.tiles_m;
+                const int tm = gp_tm(p, tile), tn = gp_tn(p, tile);
                 int row_base, row_limit, b_off;
                 if (!gp_tile(p, tm, row_base, row_limit, b_off)) continue;
                 const int a_row = row_base + rank * GP_BM;
@@ -350,7 +358,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             bool ok = true;
             if (p.tile_expert) pb_grid_dep_wait();
             for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
-                if (p.tile_expert && p.tile_expert[tile % p.tiles_m] < 0) continue;       // seg counts the tiles that exist
+                if (p.tile_expert && p.tile_expert[gp_tm(p, tile)] < 0) continue;       // seg counts the tiles that exist
                 const int acc = seg & 1;
                 ok = __all_sync(0xffffffffu, tc_mbar_wait(&acc_empty[acc], ((seg >> 1) & 1) ^ 1));
                 if (!ok) break;
@@ -386,7 +394,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         int seg = 0;
         bool ok = true;
         for (int tile = pair; tile < n_tiles; tile += n_pairs) {
-            const int tm = tile % p.tiles_m, tn = tile / p.tiles_m;
+            const int tm = gp_tm(p, tile), tn = gp_tn(p, tile);
             int row_base, row_limit, b_off;
             if (!gp_tile(p, tm, row_base, row_limit, b_off)) continue;
             const int acc = seg & 1;
