@@ -1,0 +1,145 @@
+"""Kernels around the products, at the sizes where they change from one form to another, against the same in 64 bits."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+# one rounding to the type (bfloat16: eight bits), and a few roundings of 6e-8 before it
+UNIT = {torch.bfloat16: 2.0 ** -8 + 1e-6, torch.float32: 1.5e-6}
+
+
+def _gen(seed=1):
+    return torch.Generator(device=DEV).manual_seed(seed)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("width", [8, 12, 512, 516, 1536, 2048, 4104, 16384, 16392, 33000])
+@pytest.mark.parametrize("rows", [1, 5])
+def test_rmsnorm(dtype, width, rows):
+    from prelude_b200.ops import kernels as K
+    x = torch.randn(rows, width, generator=_gen(), device=DEV).to(dtype)
+    w = torch.rand(width, generator=_gen(2), device=DEV) + 0.5
+    y = x.double() / torch.sqrt((x.double() ** 2).mean(-1, keepdim=True) + 1e-6) * w.double()
+    got = K.rmsnorm(x, w, 1e-6).double()
+    assert bool(((got - y).abs() <= UNIT[dtype] * y.abs() + 1e-12).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("width", [64, 516, 2560, 8192, 8196, 9000])
+@pytest.mark.parametrize("parts", [0, 1, 4, 6, None])
+def test_final_norm_of_chosen_rows(dtype, width, parts):
+    """parts 0: nothing joins; None: one output of the run's type; else float32 parts of a product."""
+    from prelude_b200.ops import kernels as K
+    res = torch.randn(9, width, generator=_gen(), device=DEV)
+    w = torch.rand(width, generator=_gen(2), device=DEV) + 0.5
+    rows = torch.tensor([8, 0, 3, 3, -1, 9], dtype=torch.int32, device=DEV)
+    x, total = None, res.double()
+    if parts is None:
+        x = torch.randn(9, width, generator=_gen(3), device=DEV).to(dtype)
+        total = total + x.double()
+    elif parts:
+        p = torch.randn(parts, 9, width, generator=_gen(3), device=DEV)
+        x, total = K.PartialSums(p), total + p.double().sum(0)
+    y = total / torch.sqrt((total ** 2).mean(-1, keepdim=True) + 1e-6) * w.double()
+    before = res.clone()
+    got = K.gather_add_rmsnorm(x, res, rows, w, 1e-6, dtype).double()
+    assert torch.equal(res, before)
+    # the sum of up to seven terms is rounded at every step: 6e-8 of the terms, not of a sum that may cancel
+    assert bool(((got[:4] - y[rows[:4].long()]).abs() <= UNIT[dtype] * y[rows[:4].long()].abs() + 4e-6).all())
+    assert not got[4:].any()                               # no such row: zeros
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("T,inner,parts", [(2, 8192, 8), (2, 520, 1), (700, 8192, 8), (3, 4096, 1), (3, 4100, 1), (5, 96, 4), (3, 1026, 1)])
+@pytest.mark.parametrize("gate_after", [False, True])
+@pytest.mark.parametrize("sigmoid_gate", [False, True])
+def test_gated_norm(dtype, T, inner, parts, gate_after, sigmoid_gate):
+    from prelude_b200.ops import kernels as K
+    y = torch.randn(T, inner, generator=_gen(), device=DEV)
+    z = torch.randn(T, inner + 8, generator=_gen(2), device=DEV).to(dtype)[:, :inner]
+    w = torch.rand(inner, generator=_gen(3), device=DEV) + 0.5
+    g = torch.sigmoid(z.double()) * (1.0 if sigmoid_gate else z.double())
+    v = y.double() if gate_after else y.double() * g
+    v = v.view(T, parts, -1)
+    v = (v / torch.sqrt((v ** 2).mean(-1, keepdim=True) + 1e-6)).view(T, inner) * w.double() * (g if gate_after else 1.0)
+    got = K.gated_group_rmsnorm(y, z, w, parts, 1e-6, gate_after=gate_after, sigmoid_gate=sigmoid_gate).double()
+    assert bool(((got - v).abs() <= UNIT[dtype] * v.abs() + 1e-12).all())
+
+
+@pytest.mark.parametrize("requests", [1, 3])
+@pytest.mark.parametrize("H,P,N,groups", [(8, 64, 128, 8), (4, 32, 64, 2), (2, 4, 5, 1), (2, 256, 16, 2), (3, 48, 128, 3), (2, 128, 300 - 44, 1)])
+def test_state_space_step_of_single_tokens(requests, H, P, N, groups):
+    """float32: a sum over N products, rounded N times at most and by far not all the same way."""
+    from prelude_b200.engine.batch import StepItem, build_step_batch
+    from prelude_b200.ops import kernels as K
+    g = _gen(4)
+    u = torch.randn(requests, H * P + 2 * groups * N, generator=g, device=DEV).bfloat16()
+    dt = torch.randn(requests, H, generator=g, device=DEV).bfloat16()
+    bias, a_log, skip = (torch.randn(H, generator=g, device=DEV) for _ in range(3))
+    state = torch.randn(requests + 1, H, N, P, generator=g, device=DEV)
+    batch = build_step_batch([StepItem(i, [0], 5) for i in range(requests)], {}, list(range(requests, 0, -1)), torch.device(DEV), 2, 100)
+    S = state.double()[list(range(requests, 0, -1))]
+    x, step = u.double()[:, :H * P].view(-1, H, P), torch.nn.functional.softplus(dt.double() + bias.double())
+    B, C = (u.double()[:, H * P + k * groups * N:H * P + (k + 1) * groups * N].view(-1, groups, N).repeat_interleave(H // groups, 1) for k in (0, 1))
+    decay = torch.exp(-torch.exp(a_log.double()) * step)
+    S = decay[..., None, None] * S + (step.unsqueeze(-1) * B).unsqueeze(-1) * x.unsqueeze(2)
+    want = ((S * C.unsqueeze(-1)).sum(2) + skip.double().view(1, H, 1) * x).flatten(1)
+    before = state[0].clone()
+    got = K.ssm_scan(u, dt, bias, a_log, skip, state, batch, groups)
+    assert float((got.double() - want).norm() / want.norm()) < 1e-6
+    assert float((state.double()[list(range(requests, 0, -1))] - S).norm() / S.norm()) < 1e-6
+    assert torch.equal(state[0], before)                   # nobody's slot
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("H,d,rot,rank,dims", [(16, 128, 64, 512, 64), (32, 128, 64, 512, 32), (2, 32, 16, 64, 16), (5, 24, 8, 40, 8), (2, 16, 6, 24, 6),
+                                               (40, 192, 64, 512, 64)])
+@pytest.mark.parametrize("adjacent", [False, True])
+@pytest.mark.parametrize("split", [True, False])
+def test_queries_without_norm_beside_a_latent(dtype, H, d, rot, rank, dims, adjacent, split):
+    """Positions to 4,000: an angle in 32 bits is off by 2^-12 of a turn there at the fastest rate (4,000 x 6e-8)."""
+    from prelude_b200.ops import kernels as K
+    g = _gen(6)
+    T, pages, page = 7, 40, 4
+    q = torch.randn(T, H * (d + rot) + 8, generator=g, device=DEV).to(dtype)[:, :H * (d + rot)]
+    ckv = torch.randn(T, rank + rot, generator=g, device=DEV).to(dtype)
+    w, rates = torch.rand(rank, generator=g, device=DEV) + 0.5, torch.rand(dims // 2, generator=g, device=DEV)
+    pos = torch.tensor([0, 1, 2, 3, 4, 3999, 77], dtype=torch.int32, device=DEV)
+    table = torch.full((3, 1000), -1, dtype=torch.int32, device=DEV)
+    table[0, :2], table[2, 999], table[1, 19] = torch.tensor([5, 9], dtype=torch.int32, device=DEV), 30, 11
+    rows = torch.tensor([0, 0, 0, 0, 0, 2, -1], dtype=torch.int32, device=DEV)
+    k_pages = torch.zeros(pages, 1, page, rank + rot, dtype=dtype, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    cut = d if split else d + rot
+    out, out2 = torch.zeros(T, H, cut, dtype=dtype, device=DEV), torch.zeros(T, H, rank + rot, dtype=dtype, device=DEV)
+    K.qkv_prepare(q, ckv, None, n_heads=H, q_dim=d + rot, k_weight=w, k_norm_cols=rank, eps=1e-6, rates=rates, rot_dims=dims, adjacent=adjacent,
+                  amplitude=1.25, q_rot_off=d, k_rot_off=rank, positions=pos, table_row=rows, block_table=table, q_out=out, q_split=cut,
+                  q_out2=out2 if split else None, q2_off=rank, k_pages=k_pages, status=status)
+    ang = pos.double().view(-1, 1, 1) * rates.double().view(1, 1, -1)
+    c, s = ang.cos() * 1.25, ang.sin() * 1.25
+
+    def turn(x):
+        x = x.double().clone()
+        a, b = (x[..., 0:dims:2].clone(), x[..., 1:dims:2].clone()) if adjacent else (x[..., :dims // 2].clone(), x[..., dims // 2:dims].clone())
+        y = (a * c - b * s, b * c + a * s)
+        if adjacent:
+            x[..., 0:dims:2], x[..., 1:dims:2] = y
+        else:
+            x[..., :dims // 2], x[..., dims // 2:dims] = y
+        return x
+
+    live = rows >= 0
+    heads = q.double().view(T, H, d + rot)
+    turned = turn(heads[..., d:])
+    latent = ckv.double()[:, :rank]
+    latent = latent / torch.sqrt((latent ** 2).mean(-1, keepdim=True) + 1e-6) * w.double()
+    key = torch.cat([latent, turn(ckv[:, None, rank:])[:, 0]], -1)
+    tol = UNIT[dtype] + 2e-3 / (1 if dtype == torch.float32 else 1)     # 4,000 radians x 6e-8 x amplitude and size of the partner
+    got = torch.cat([out, out2[..., rank:]], -1) if split else out
+    want = torch.cat([heads[..., :d], turned], -1)
+    assert float((got.double() - want)[live].abs().max()) < tol * float(want.abs().max())
+    for t in range(T):
+        if live[t]:
+            have = k_pages[table[rows[t], int(pos[t]) // page].item(), 0, int(pos[t]) % page].double()
+            assert float((have - key[t]).abs().max()) < tol * float(key[t].abs().max())
+    assert int(status) == 0 and not out[6].any()
