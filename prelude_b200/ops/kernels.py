@@ -1038,7 +1038,8 @@ def ssm_scan(u: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: to
              state: torch.Tensor, batch, groups: int, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """The recurrence over the step's tokens, sequence by sequence; u [T, heads * P + 2 * groups * N] dense, dt [T, heads] a
     view with dense rows, state float32 [slots, heads, N, P]; returns y float32 [T, heads * P].  A prompt step in bfloat16
-    runs by chunks of tokens (csrc/ssm_chunk.cu), in 32-bit and in a decode step token by token (csrc/ssm.cu)."""
+    runs by chunks of tokens (csrc/ssm_chunk.cu), a decode step in bfloat16 on a kernel for single tokens, in 32-bit token
+    by token (csrc/ssm.cu)."""
     _need(u, "u")
     _need(dt, "dt", u.dtype, contiguous=False)
     for t, name in ((dt_bias, "dt_bias"), (a_log, "a_log"), (d_skip, "d_skip"), (state, "state")):
@@ -1055,6 +1056,11 @@ def ssm_scan(u: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: to
         check(lib.pb_ssm_scan_chunked(u.data_ptr(), dt.data_ptr(), dt.stride(0), dt_bias.data_ptr(), a_log.data_ptr(), d_skip.data_ptr(),
                                       state.data_ptr(), out.data_ptr(), batch.cu_q.data_ptr(), batch.state_slots.data_ptr(),
                                       batch.cu_q.numel() - 1, heads, P, N, groups, _stream()), "ssm_scan_chunked")
+        return out
+    if u.dtype == torch.bfloat16 and batch.decode_only and lib.pb_ssm_step_takes(u.data_ptr(), state.data_ptr(), heads, P, N, groups):
+        check(lib.pb_ssm_step(u.data_ptr(), dt.data_ptr(), dt.stride(0), dt_bias.data_ptr(), a_log.data_ptr(), d_skip.data_ptr(), state.data_ptr(),
+                              out.data_ptr(), batch.cu_q.data_ptr(), batch.state_slots.data_ptr(), batch.cu_q.numel() - 1, heads, P, N, groups,
+                              _stream()), "ssm_step")
         return out
     check(lib.pb_ssm_scan(u.data_ptr(), dt.data_ptr(), dt.stride(0), dtype_code(u.dtype), dt_bias.data_ptr(), a_log.data_ptr(),
                                    d_skip.data_ptr(), state.data_ptr(), out.data_ptr(), batch.cu_q.data_ptr(),

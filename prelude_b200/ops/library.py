@@ -100,6 +100,8 @@ _SIGNATURES = {
     "pb_causal_conv_silu": ([P, L, P, P, P, P, I, I, P, P, P, P, I, I, I, P], I),
     "pb_conv_state_update": ([P, L, P, I, P, P, I, I, I, P], I),
     "pb_ssm_scan": ([P, P, L, I, P, P, P, P, P, P, P, I, I, I, I, I, P], I),
+    "pb_ssm_step_takes": ([P, P, I, I, I, I], I),
+    "pb_ssm_step": ([P, P, L, P, P, P, P, P, P, P, I, I, I, I, I, P], I),
     "pb_ssm_scan_chunked_takes": ([P, I, I, I, I], I),
     "pb_ssm_scan_chunked": ([P, P, L, P, P, P, P, P, P, P, I, I, I, I, I, P], I),
     "pb_gated_group_rmsnorm": ([P, P, L, P, P, I, I, I, I, F, I, I, P], I),
