@@ -223,6 +223,123 @@ __global__ void qkv_prepare_staged_kernel(const T* q_in, long long ldq, const T*
     }
 }
 
+// The same where the queries take no norm (attention through a latent): nothing of a query depends on more than its own 16 bytes and
+// those of its rotation partners, so every thread asks for its QP pieces at once and keeps them in registers; the key row, its norm
+// included, is the last warp's, which reads it twice.  One barrier, for the token's angles.  Heads, split points and the rotated span
+// in whole pieces.  (Through shared memory as float32: 1,500 tokens of 16 x 192 queries and rows of 576 24.6 us, here 15.5; 16
+// tokens of 32 x 192 11.4, here 8.1.)
+#define QP_MOST 4                                          // pieces of queries a thread holds at most
+template <typename T>
+__device__ __forceinline__ void qp_turn(uint4& own, const uint4& other, int rel, const RotArgs& r, const float* cs) {
+    constexpr int VN = 16 / sizeof(T);
+    float a[VN], b[VN];
+    qp_ld_vec(reinterpret_cast<const T*>(&own), a);
+    if (r.adjacent) {
+#pragma unroll
+        for (int e = 0; e < VN; e += 2) {
+            const float c = cs[rel + e], s = cs[rel + e + 1], x = a[e], y = a[e + 1];
+            a[e] = x * c - y * s;
+            a[e + 1] = y * c + x * s;
+        }
+    } else {
+        qp_ld_vec(reinterpret_cast<const T*>(&other), b);
+        const int half = r.dims >> 1;
+        const bool first = rel < half;
+        const float* t = cs + 2 * (first ? rel : rel - half);
+#pragma unroll
+        for (int e = 0; e < VN; ++e) a[e] = first ? a[e] * t[2 * e] - b[e] * t[2 * e + 1] : a[e] * t[2 * e] + b[e] * t[2 * e + 1];
+    }
+    qp_st_vec(reinterpret_cast<T*>(&own), a);
+}
+
+template <typename T, int QP>
+__global__ void __launch_bounds__(256)
+qkv_prepare_direct_kernel(const T* q_in, long long ldq, const T* k_in, long long ldk, const T* v_in, long long ldv, const float* k_w, int k_norm_cols,
+                          float eps, RotArgs rot, int q_rot_off, int k_rot_off, const int32_t* positions, const int32_t* table_row, const int32_t* block_table,
+                          int table_stride, int page_size, int num_pages, T* q_out, int q_split, T* q_out2, long long q2_head_stride, long long q2_off,
+                          T* k_pages, T* v_pages, int H, int qd, int G, int kd, int Gv, int vd, int swizzle_k, int swizzle_v, int* status) {
+    constexpr int VN = 16 / sizeof(T);
+    extern __shared__ float cs[];                          // cosine and sine of the token's angles, times the amplitude
+    pb_grid_dep_launch();
+    pb_grid_dep_wait();
+    const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+    const int row = table_row[t];
+    if (row < 0) return;
+    const int p = positions[t], nq = H * qd, nk = k_pages ? G * kd : 0, half = rot.dims >> 1;
+    const bool keys = nk > 0 && tid >= (int)blockDim.x - 32;
+    const T* q = q_in + (size_t)t * ldq;
+    const T* k = k_in + (size_t)t * ldk;
+    // where a piece at element d of a head lies in the rotated span from `off` on, or -1
+    auto in_span = [&](int d, int off) { return rot.dims > 0 && d >= off && d < off + rot.dims ? d - off : -1; };
+    // the piece that the rotation pairs with the one at `at` (adjacent pairs lie in one piece)
+    auto partner = [&](const T* at, int rel) { return rot.adjacent ? make_uint4(0, 0, 0, 0) : *reinterpret_cast<const uint4*>(at + (rel < half ? half : -half)); };
+    uint4 mine[QP];
+#pragma unroll
+    for (int it = 0; it < QP; ++it) {
+        const int i = (tid + it * (int)blockDim.x) * VN;
+        mine[it] = i < nq ? *reinterpret_cast<const uint4*>(q + i) : make_uint4(0, 0, 0, 0);
+    }
+    int page = -1;
+    float ss = 0.f;
+    if (keys) {
+        page = block_table[(size_t)row * table_stride + p / page_size];
+        if (k_w != nullptr)
+            for (int i = lane * VN; i < k_norm_cols; i += 32 * VN) {
+                float v[VN];
+                qp_ld_vec(k + i, v);
+#pragma unroll
+                for (int e = 0; e < VN; ++e) ss += v[e] * v[e];
+            }
+    }
+    for (int i = tid; i < half; i += blockDim.x) {
+        float sn, c;
+        sincosf((float)p * rot.rates[i], &sn, &c);
+        cs[2 * i] = c * rot.amplitude;
+        cs[2 * i + 1] = sn * rot.amplitude;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int it = 0; it < QP; ++it) {
+        const int i = (tid + it * (int)blockDim.x) * VN;
+        if (i >= nq) break;
+        const int h = i / qd, d = i - h * qd, rel = in_span(d, q_rot_off);
+        if (rel >= 0) qp_turn<T>(mine[it], partner(q + i, rel), rel, rot, cs);
+        T* dst = d < q_split ? q_out + ((size_t)t * H + h) * q_split + d : q_out2 + ((size_t)t * H + h) * q2_head_stride + q2_off + (d - q_split);
+        *reinterpret_cast<uint4*>(dst) = mine[it];
+    }
+    if (keys) {
+        const float inv = k_w ? 1.0f / sqrtf(pb_warp_sum(ss) / (float)k_norm_cols + eps) : 1.0f;
+        if (page < 0 || page >= num_pages) {
+            if (lane == 0 && status) atomicExch(status, 2);
+        } else {
+            const int in_page = p % page_size;
+            for (int i = lane * VN; i < nk; i += 32 * VN) {
+                const int g = i / kd, d = i - g * kd, rel = in_span(d, k_rot_off);
+                uint4 own = *reinterpret_cast<const uint4*>(k + i);
+                if (k_w != nullptr && i < k_norm_cols) {       // (a rotated span that is normed is the general kernels' case)
+                    float v[VN];
+                    qp_ld_vec(reinterpret_cast<const T*>(&own), v);
+#pragma unroll
+                    for (int e = 0; e < VN; ++e) v[e] = v[e] * inv * k_w[i + e];
+                    qp_st_vec(reinterpret_cast<T*>(&own), v);
+                } else if (rel >= 0) {
+                    qp_turn<T>(own, partner(k + i, rel), rel, rot, cs);
+                }
+                *reinterpret_cast<uint4*>(k_pages + (((size_t)page * G + g) * page_size + in_page) * kd + pb_kv_elem_offset(d, in_page, swizzle_k)) = own;
+            }
+        }
+    }
+    if (nk == 0 || v_pages == nullptr || v_in == nullptr) return;
+    page = block_table[(size_t)row * table_stride + p / page_size];
+    if (page < 0 || page >= num_pages) return;                  // the key row's warp has raised the status
+    const int in_page = p % page_size;
+    for (int i = tid * VN; i < Gv * vd; i += blockDim.x * VN) {
+        const int g = i / vd, d0 = i - g * vd;
+        T* dst = v_pages + (((size_t)page * Gv + g) * page_size + in_page) * vd;
+        *reinterpret_cast<uint4*>(dst + pb_kv_elem_offset(d0, in_page, swizzle_v)) = *reinterpret_cast<const uint4*>(v_in + (size_t)t * ldv + i);
+    }
+}
+
 }  // namespace
 
 PB_API int pb_qkv_prepare(const void* q_in, long long ldq, const void* k_in, long long ldk, const void* v_in, long long ldv,
@@ -266,6 +383,30 @@ PB_API int pb_qkv_prepare(const void* q_in, long long ldq, const void* k_in, lon
     if (staged && k_pages != nullptr)
         staged = kd % vn == 0 && ldk % vn == 0 && pb_aligned(k_in, 16) && pb_aligned(k_pages, 16) && k_norm_cols % vn == 0 &&
                  (v_pages == nullptr || (vd % vn == 0 && ldv % vn == 0 && pb_aligned(v_in, 16) && pb_aligned(v_pages, 16)));
+    // the whole rotated span in pieces, and of the key row not among what the norm covers
+    auto whole = [&](int off) { return rates == nullptr || (off % vn == 0 && rot_dims % vn == 0 && (adjacent || (rot_dims / 2) % vn == 0)); };
+    const int nk = k_pages ? G * kd : 0;
+    bool direct = staged && q_w == nullptr && whole(q_rot_off) && H * qd <= QP_MOST * vn * 256 && (nk == 0 || whole(k_rot_off));
+    if (direct && nk > 0 && k_w != nullptr && rates != nullptr)
+        for (int g = 0; g < G; ++g) direct = direct && g * kd + k_rot_off >= k_norm_cols;
+    if (direct) {
+        const int pieces = H * qd / vn;
+        int block = 64;
+        while (block < 256 && block < pieces) block <<= 1;
+        const int each = (pieces + block - 1) / block;
+#define DIRECT_LAUNCH(QP)                                                                                                     \
+    PB_DISPATCH_DTYPE(dtype, T,                                                                                               \
+        (pb_launch(qkv_prepare_direct_kernel<T, QP>, dim3(n_tokens), dim3(block), (size_t)rot.dims * sizeof(float), stream, (const T*)q_in, ldq, \
+                   (const T*)k_in, ldk, (const T*)v_in, ldv, k_w, k_norm_cols, eps, rot, q_rot_off, k_rot_off, positions, table_row, block_table, table_stride, \
+                   page_size, num_pages, (T*)q_out, q_split, (T*)q_out2, q2_head_stride, q2_off, (T*)k_pages, (T*)v_pages, H, qd, G, kd, Gv, vd, swizzle_k, \
+                   swizzle_v, status)))
+        if (each <= 1) DIRECT_LAUNCH(1);
+        else if (each <= 2) DIRECT_LAUNCH(2);
+        else DIRECT_LAUNCH(QP_MOST);
+#undef DIRECT_LAUNCH
+        PB_CHECK_LAUNCH("qkv_prepare");
+        return 0;
+    }
     if (staged) {
         PB_DISPATCH_DTYPE(dtype, T,
             (pb_launch(qkv_prepare_staged_kernel<T>, dim3(n_tokens), dim3(threads >= 128 ? threads / 2 : threads), staged_bytes, stream, (const T*)q_in, ldq,
