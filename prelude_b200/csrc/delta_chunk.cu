@@ -73,12 +73,14 @@ __device__ __forceinline__ bool dc_find(const int32_t* cu_q, int n_seqs, int slo
 template <int D>
 struct DcPrep {
     static constexpr int LDK = D + 8, LDA = DC_L + 4, LDX = 36;
-    static constexpr int k = 0, q = k + DC_L * LDK * 2, a = q + DC_L * LDK * 2, t = a + DC_L * LDA * 4, x = t + DC_L * LDA * 4, num = x + 32 * LDX * 4;
-    static constexpr int bytes = num + (6 * DC_L + 4) * 4;
+    static constexpr int k = 0, q = k + DC_L * LDK * 2;
+    // the inverse is made where the keys and queries lay once their products are there: four blocks a multiprocessor
+    static constexpr int t = 0, x = t + DC_L * LDA * 4, rows = q + DC_L * LDK * 2, work = x + 32 * LDX * 4, a = rows > work ? rows : work;
+    static constexpr int num = a + DC_L * LDA * 4, bytes = num + (6 * DC_L + 4) * 4;
 };
 
 template <int D>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 4)
 delta_prepare_kernel(const bf16* u, long long ld_u, const bf16* b_in, long long ld_b, const bf16* a_in, long long ld_a, const float* a_log,
                      const float* dt_bias, const int32_t* cu_q, unsigned char* blobs, int n_seqs, int H, int G) {
     using Z = DcPrep<D>;
