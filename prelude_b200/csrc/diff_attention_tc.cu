@@ -19,7 +19,14 @@
 // Decoded tokens have a tile of their own (`tile_seq` null: tile i is token i).  Their keys can be cut into
 // `n_splits` ranges, one block each; the blocks then leave unnormalised sums with their maxima and the merge kernel
 // below adds them up and does the epilogue.
+//
+// A short prompt's tiles are few and unequal: the last ones walk sixteen times the keys of the first, and all are on the chip
+// at once, so the longest decides.  Their keys are then cut in two (`pair`): the two blocks of a tile are a cluster, the
+// second hands its sums over through its shared memory, and the first puts them together and does the epilogue.  1,024 tokens of 16
+// heads over 4 of 64: the layer 147.8 -> 142.7 us.
 #include "attention_common.cuh"
+
+#include <cooperative_groups.h>
 
 struct DiffAttnParams {
     const __nv_bfloat16* q; long long q_stride;          // [T, heads * 2 * dim]
@@ -32,6 +39,7 @@ struct DiffAttnParams {
     float* part_o;                                       // [T, heads, 2, n_splits, vdim]
     float* part_ml;                                      // [T, heads, 2, n_splits, 2]
     int n_splits, stages;
+    int pair;                                            // 1: the two key ranges of a prompt tile are put together inside a cluster
     int n_parts;                                         // partial sums per (token, head, map) that the merge kernel adds up
     int split_weights;                                   // the softmax weights enter O += P V as rounded part plus remainder
     int table_stride, page_size, num_pages, n_tokens, n_heads, n_kv_heads, dim, vdim, group, window;
@@ -273,7 +281,46 @@ __global__ void __launch_bounds__(256) diff_attention_mma_kernel(const DiffAttnP
         l[h] += __shfl_xor_sync(0xffffffffu, l[h], 2);
     }
 
-    if (DEC || p.n_splits > 1) {
+    if (!DEC && p.pair) {
+        // the second range's sums, maxima and sums of weights lie in its block's shared memory while the first one reads them
+        cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+        const int SA = vdim + 4;
+        float* part = reinterpret_cast<float*>(smem) + (size_t)map * 64 * SA;
+        float* ml = reinterpret_cast<float*>(smem) + (size_t)2 * 64 * SA + map * 128;
+        __syncthreads();                                     // everyone is done with the tiles
+        if (split == 1) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int r = row0 + gid + 8 * h;
+                if (t4 == 0) { ml[2 * r] = m[h]; ml[2 * r + 1] = l[h]; }
+#pragma unroll
+                for (int nt = 0; nt < 2 * NV; ++nt)
+                    if (nt * 8 < vdim) *reinterpret_cast<float2*>(part + (size_t)r * SA + nt * 8 + 2 * t4) = make_float2(o[nt][2 * h], o[nt][2 * h + 1]);
+            }
+        }
+        cluster.sync();
+        if (split == 0) {
+            const float* theirs = cluster.map_shared_rank(part, 1);
+            const float* their_ml = cluster.map_shared_rank(ml, 1);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int r = row0 + gid + 8 * h;
+                const float2 b = *reinterpret_cast<const float2*>(their_ml + 2 * r);
+                const float M = fmaxf(m[h], b.x);
+                const float wa = m[h] == -INFINITY ? 0.f : exp2f(m[h] - M), wb = b.x == -INFINITY ? 0.f : exp2f(b.x - M);
+                l[h] = l[h] * wa + b.y * wb;
+#pragma unroll
+                for (int nt = 0; nt < 2 * NV; ++nt)
+                    if (nt * 8 < vdim) {
+                        const float2 f = *reinterpret_cast<const float2*>(theirs + (size_t)r * SA + nt * 8 + 2 * t4);
+                        o[nt][2 * h] = o[nt][2 * h] * wa + f.x * wb;
+                        o[nt][2 * h + 1] = o[nt][2 * h + 1] * wa + f.y * wb;
+                    }
+            }
+        }
+        cluster.sync();
+        if (split == 1) return;
+    } else if (DEC || p.n_splits > 1) {
         // unnormalised sums with their maximum and sum, for the merge kernel
         const int n_parts = DEC ? 4 * p.n_splits : p.n_splits, part = DEC ? 4 * split + (warp & 3) : split;
 #pragma unroll
@@ -477,8 +524,22 @@ PB_API int pb_diff_attention_tc_bf16(const void* q, long long q_stride, const vo
     p.lambda = lambda; p.norm_eps = norm_eps; p.out_scale = out_scale; p.status = status;
     p.stages = diff_attention_smem(dim, vdim, 2) <= 200 * 1024 ? 2 : 1;
     const size_t smem = diff_attention_smem(dim, vdim, p.stages);
-    dim3 grid(n_tiles, n_kv_heads, n_splits);
+    // prompt tiles that four waves of two blocks a multiprocessor hold: in pairs (more of them even out by themselves)
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
+    const size_t handed = ((size_t)2 * 64 * (vdim + 4) + 256) * 4;
+    p.pair = !dec && tile_seq != nullptr && n_splits == 1 && handed <= smem && (long long)n_tiles * n_kv_heads <= 4ll * sms ? 1 : 0;
+    if (p.pair) p.n_splits = 2;
+    dim3 grid(n_tiles, n_kv_heads, p.n_splits);
     PB_REQUIRE(grid.y < 65536, "diff_attention_tc: too many key/value heads");
+    cudaLaunchConfig_t pairs = {};
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 2;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    pairs.gridDim = grid; pairs.blockDim = dim3(256); pairs.dynamicSmemBytes = smem; pairs.stream = stream;
+    pairs.attrs = attr; pairs.numAttrs = pb_pdl_enabled() ? 2 : 1;
 #define DA_LAUNCH_K(NVT, KST, DECT)                                                                                              \
     do {                                                                                                                         \
         static bool set_##NVT##_##KST##_##DECT = false;                                                                          \
@@ -486,7 +547,8 @@ PB_API int pb_diff_attention_tc_bf16(const void* q, long long q_stride, const vo
             cudaFuncSetAttribute(diff_attention_mma_kernel<NVT, KST, DECT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); \
             set_##NVT##_##KST##_##DECT = true;                                                                                   \
         }                                                                                                                        \
-        pb_launch(diff_attention_mma_kernel<NVT, KST, DECT>, grid, dim3(256), smem, stream, p);                                  \
+        if (p.pair) cudaLaunchKernelEx(&pairs, diff_attention_mma_kernel<NVT, KST, DECT>, (const DiffAttnParams)p);              \
+        else pb_launch(diff_attention_mma_kernel<NVT, KST, DECT>, grid, dim3(256), smem, stream, p);                             \
     } while (0)
 #define DA_LAUNCH(NVT)                                 \
     do {                                               \

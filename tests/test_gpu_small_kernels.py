@@ -143,3 +143,45 @@ def test_queries_without_norm_beside_a_latent(dtype, H, d, rot, rank, dims, adja
             have = k_pages[table[rows[t], int(pos[t]) // page].item(), 0, int(pos[t]) % page].double()
             assert float((have - key[t]).abs().max()) < tol * float(key[t].abs().max())
     assert int(status) == 0 and not out[6].any()
+
+
+@pytest.mark.parametrize("lens,H,G", [([700], 64, 4), ([700], 16, 4), ([65, 3, 64], 4, 2), ([2], 2, 1), ([1, 130], 6, 2), ([40], 64, 1)])
+@pytest.mark.parametrize("vdim,dim", [(128, 64), (32, 16), (256, 128)])
+@pytest.mark.parametrize("window", [None, 50])
+def test_differential_attention_of_prompts(lens, H, G, vdim, dim, window):
+    """Few tiles (their keys cut in two, put together inside a cluster) and many, against 64 bits: the weights enter the second
+    product as bfloat16 (2^-9 each, of sums that the difference of two maps and the norm behind it may double), the result is
+    rounded once more."""
+    from prelude_b200.cache.manager import CacheManager
+    from prelude_b200.config.spec import DiffAttentionSpec, QueryTemperatureSpec
+    from prelude_b200.engine.batch import StepItem, build_step_batch
+    from prelude_b200.ops import kernels as K
+    from prelude_b200.ops.diff_attention import diff_attention
+    from prelude_b200.parts.registry import KvPagesNeed
+    g, T, dev = _gen(8), sum(lens), torch.device(DEV)
+    spec = DiffAttentionSpec(hidden_size=64, num_heads=H, num_kv_heads=G, head_dim=dim, value_dim=vdim, softmax_scale=dim ** -0.5, lambda_init=0.5,
+                             norm_eps=1e-6, query_temperature=QueryTemperatureSpec(coef=0.1, every=32), window=window)
+    cache = CacheManager([KvPagesNeed(2 * G, dim, window, v_heads=G, v_head_dim=vdim)], 16, T // 16 + len(lens) + 1, len(lens), dev, torch.bfloat16)
+    for r, n in enumerate(lens):
+        cache.add_request(r)
+        cache.grow(r, n)
+    batch = build_step_batch([StepItem(r, [0] * n, 0) for r, n in enumerate(lens)], cache.block_tables(range(len(lens))),
+                             [cache.slot_of(r) for r in range(len(lens))], dev, 2, 1 << 20)
+    q, k, v, gate = (torch.randn(T, n, generator=g, device=DEV).bfloat16() for n in (H * 2 * dim, G * 2 * dim, G * vdim, H * vdim))
+    mine = cache.layer_cache(0)
+    K.kv_write_pages(k, v, mine.k_pages, mine.v_pages, batch.positions, batch.table_row_of_token, batch.block_tables[mine.group], batch.status)
+    got = diff_attention(q, gate, mine.k_pages, mine.v_pages, batch, mine.group, spec, 0.3).double()
+    at = 0
+    for n in lens:
+        i, j = torch.arange(n, device=DEV).view(-1, 1), torch.arange(n, device=DEV).view(1, -1)
+        hidden = (j > i) | ((i - j >= window) if window else (j > i))
+        tau = (1 + 0.1 * torch.log((torch.arange(1, n + 1, device=DEV) // 32 + 1).double())).view(1, n, 1)
+        qq, kk = q[at:at + n].double().view(n, H, 2, dim), k[at:at + n].double().view(n, G, 2, dim).repeat_interleave(H // G, 1)
+        vv = v[at:at + n].double().view(n, G, vdim).repeat_interleave(H // G, 1)
+        maps = [torch.einsum("hij,jhe->ihe", torch.softmax((torch.einsum("ihd,jhd->hij", qq[:, :, c], kk[:, :, c]) * dim ** -0.5 * tau).masked_fill(hidden, -1e300), -1), vv)
+                for c in (0, 1)]
+        o = maps[0] - 0.3 * maps[1]
+        o = o / torch.sqrt((o * o).mean(-1, keepdim=True) + 1e-6) * 0.5 * torch.sigmoid(gate[at:at + n].double().view(n, H, vdim))
+        assert float((got[at:at + n] - o).norm() / o.norm()) < 6e-3
+        at += n
+    assert int(batch.status) == 0
