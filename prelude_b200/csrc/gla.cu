@@ -11,7 +11,7 @@
 // (projections) are of the run's type.  A sequence's tokens are visited in order; a token's numbers do not depend on how a
 // prompt was cut into steps or on what else is in the batch.  Sequences are found through device arrays (cumulative
 // lengths, state slots), one block row per sequence the arrays have room for: a row whose length is not positive is
-// skipped, so the launches can be recorded.
+// skipped, so the launches can be recorded.  (A prompt step in bfloat16 runs the recurrence by sixteen tokens: gla_chunk.cu.)
 #include "common.cuh"
 
 #include <math.h>

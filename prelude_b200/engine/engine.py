@@ -63,13 +63,14 @@ class EngineStats:
 
 def _activation_reserve_bytes(model: DecoderModel, max_tokens: int, max_rows: int) -> int:
     """A generous bound on what one step allocates beside weights and cache.  A mixer or feed-forward says what it
-    allocates per token (``activation_bytes_per_token(element size)``); one that does not say is taken to use
-    sixteen rows of the hidden width in 32-bit, so that an unknown part never counts as nothing."""
+    allocates per token (``activation_bytes_per_token(element size)``), and per sequence beyond that where its workspace
+    rounds every sequence up (``activation_bytes_per_sequence``); one that does not say is taken to use sixteen rows of
+    the hidden width in 32-bit, so that an unknown part never counts as nothing."""
     spec = model.spec
     elem = 2 if model.ctx.dtype == torch.bfloat16 else 4
     widest = 0
     for b in model.blocks:
-        per_token = 4 * spec.hidden_size * 4              # residual, two normed copies, a delta
+        per_token, per_sequence = 4 * spec.hidden_size * 4, 0             # residual, two normed copies, a delta
         inner = b.parts() if callable(getattr(b, "parts", None)) else ()
         for part in inner:
             say = getattr(part, "activation_bytes_per_token", None)
@@ -77,8 +78,11 @@ def _activation_reserve_bytes(model: DecoderModel, max_tokens: int, max_rows: in
                 per_token += int(say(elem))
             elif callable(getattr(part, "forward", None)) and not hasattr(part, "add_forward"):
                 per_token += 16 * spec.hidden_size * 4
-        widest = max(widest, per_token)
-    return max_tokens * widest + 3 * max_rows * spec.vocab_size * 4 + (1 << 30)
+            say = getattr(part, "activation_bytes_per_sequence", None)
+            if callable(say):
+                per_sequence += int(say())
+        widest = max(widest, max_tokens * per_token + max_rows * per_sequence)
+    return widest + 3 * max_rows * spec.vocab_size * 4 + (1 << 30)
 
 
 class Engine:

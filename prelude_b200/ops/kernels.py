@@ -1029,9 +1029,11 @@ def conv_state_update(x: torch.Tensor, carried: torch.Tensor, batch) -> None:
 
 
 # tokens of a prompt step from which the recurrences run by chunks of tokens on the tensor cores (bfloat16 only).  State space:
-# 12 us either way at 32 tokens, 11.5 against 20 at 64; the gated delta rule, two kernels: 24 against 16 at 32, 24 against 28 at 64
+# 12 us either way at 32 tokens, 11.5 against 20 at 64; the gated delta rule, two kernels: 24 against 16 at 32, 24 against 28 at 64;
+# gated linear attention, two kernels over memory between them: 25 against 21 at 128 of 32 heads, 31 against 38 at 256
 SCAN_CHUNKED_MIN_TOKENS = 32
 DELTA_CHUNKED_MIN_TOKENS = 64
+GLA_CHUNKED_MIN_TOKENS = 256
 
 
 def ssm_scan(u: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: torch.Tensor, d_skip: torch.Tensor,
@@ -1381,15 +1383,26 @@ def gla_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Ten
              out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """S <- diag(decay) S + k v^T, o = scale * S^T q over the step's tokens, sequence by sequence; q, k [T, H N] and v
     [T, H P] columns of one projection, decay float32 [T, H N], state float32 [slots, H, N, P]; returns o float32
-    [T, H P].  See csrc/gla.cu."""
+    [T, H P].  A prompt step in bfloat16 runs by sixteen tokens at a time (csrc/gla_chunk.cu), in 32-bit token by token
+    (csrc/gla.cu)."""
     T, H, N, P = _gla_check(q, k, v, state, "gla_scan")
     _need(decay, "decay", torch.float32)
     if tuple(decay.shape) != (T, H * N):
         raise KernelLibraryError(f"gla_scan: decay {tuple(decay.shape)} for {T} tokens of {H * N} channels")
     if out is None:
         out = torch.empty((T, H * P), dtype=torch.float32, device=q.device)
-    check(_l.library().pb_gla_scan(q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), dtype_code(q.dtype), decay.data_ptr(), float(scale),
-                                   state.data_ptr(), out.data_ptr(), batch.cu_q.data_ptr(), batch.state_slots.data_ptr(), batch.cu_q.numel() - 1,
+    lib, n_seqs = _l.library(), batch.cu_q.numel() - 1
+    if (q.dtype == torch.bfloat16 and T >= GLA_CHUNKED_MIN_TOKENS and not batch.decode_only
+            and lib.pb_gla_chunked_takes(q.data_ptr(), k.data_ptr(), v.data_ptr(), decay.data_ptr(), q.stride(0), H, N, P)):
+        # what one kernel makes of every sixteen for the other to read: dead when the call's kernels are done
+        n_steps = lib.pb_gla_chunks(T, n_seqs)
+        scratch = torch.empty((lib.pb_gla_chunk_bytes(n_steps, H, N),), dtype=torch.uint8, device=q.device)
+        check(lib.pb_gla_scan_chunked(q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), decay.data_ptr(), float(scale), state.data_ptr(),
+                                      out.data_ptr(), batch.cu_q.data_ptr(), batch.state_slots.data_ptr(), scratch.data_ptr(), n_steps, n_seqs,
+                                      H, N, P, _stream()), "gla_scan_chunked")
+        return out
+    check(lib.pb_gla_scan(q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), dtype_code(q.dtype), decay.data_ptr(), float(scale),
+                                   state.data_ptr(), out.data_ptr(), batch.cu_q.data_ptr(), batch.state_slots.data_ptr(), n_seqs,
                                    H, N, P, _stream()), "gla_scan")
     return out
 

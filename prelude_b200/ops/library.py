@@ -119,6 +119,10 @@ _SIGNATURES = {
     "pb_sigmoid_gate_": ([P, L, P, L, I, I, I, P], I),
     "pb_channel_decay": ([P, L, P, P, F, P, I, I, I, I, P], I),
     "pb_gla_scan": ([P, P, P, L, I, P, F, P, P, P, P, I, I, I, I, P], I),
+    "pb_gla_chunked_takes": ([P, P, P, P, L, I, I, I], I),
+    "pb_gla_chunks": ([I, I], I),
+    "pb_gla_chunk_bytes": ([I, I, I], L),
+    "pb_gla_scan_chunked": ([P, P, P, L, P, F, P, P, P, P, P, I, I, I, I, I, P], I),
     "pb_gla_step_supported": ([I, I], I),
     "pb_gla_step": ([P, P, P, P, P, L, I, P, P, F, F, P, F, P, P, P, P, I, I, I, I, I, P], I),
     "pb_scaled_add_rmsnorm": ([P, I, L, F, P, P, I, I, P, P, I, I, F, P], I),

@@ -79,6 +79,9 @@ class GatedDelta:
         # the scan by chunks of 64 tokens leaves 32 KB a chunk and head between its two kernels
         return (self.proj_cols + 8 + self.channels + self.inner) * elem + self.inner * 4 + self.spec.hidden_size * elem + self.spec.num_heads * 512
 
+    def activation_bytes_per_sequence(self) -> int:
+        return self.spec.num_heads * 32768
+
     def cache_need(self) -> CombinedNeed:
         s = self.spec
         return CombinedNeed((StateNeed((s.num_heads, s.head_dim, s.value_dim), torch.float32),

@@ -69,7 +69,12 @@ class GatedLinearAttention:
         self.norm_heads = self.norm_w.repeat(s.num_heads).contiguous()     # one weight over value_dim, shared by the heads
 
     def activation_bytes_per_token(self, elem: int) -> int:
-        return (2 * self.qk_cols + 3 * self.v_cols + self.rank + 8) * elem + (self.qk_cols + self.v_cols) * 4 + self.spec.hidden_size * elem
+        # the scan by sixteen tokens leaves up to 26 KB a sixteen and head between its two kernels
+        return ((2 * self.qk_cols + 3 * self.v_cols + self.rank + 8) * elem + (self.qk_cols + self.v_cols) * 4 + self.spec.hidden_size * elem
+                + self.spec.num_heads * 1664)
+
+    def activation_bytes_per_sequence(self) -> int:
+        return self.spec.num_heads * 26624
 
     def cache_need(self) -> StateNeed:
         s = self.spec

@@ -46,6 +46,9 @@ class ParallelMixer:
     def activation_bytes_per_token(self, elem: int) -> int:
         return sum(getattr(m, "activation_bytes_per_token", lambda e: 0)(elem) for m in self.members)
 
+    def activation_bytes_per_sequence(self) -> int:
+        return sum(getattr(m, "activation_bytes_per_sequence", lambda: 0)() for m in self.members)
+
     def cache_need(self) -> CombinedNeed:
         return CombinedNeed(tuple(m.cache_need() for m in self.members))
 

@@ -54,13 +54,13 @@ def _ssm_exact(u, dt, bias, a_log, skip, state, lens, groups):
 @pytest.fixture(autouse=True)
 def _chunks_whatever_the_length(monkeypatch):
     from prelude_b200.ops import kernels as K
-    for name in ("SCAN_CHUNKED_MIN_TOKENS", "DELTA_CHUNKED_MIN_TOKENS"):
+    for name in ("SCAN_CHUNKED_MIN_TOKENS", "DELTA_CHUNKED_MIN_TOKENS", "GLA_CHUNKED_MIN_TOKENS"):
         monkeypatch.setattr(K, name, 1)
 
 
 def _by_tokens(monkeypatch, K):
     """The same call through the kernel that visits the tokens one by one."""
-    for name in ("SCAN_CHUNKED_MIN_TOKENS", "DELTA_CHUNKED_MIN_TOKENS"):
+    for name in ("SCAN_CHUNKED_MIN_TOKENS", "DELTA_CHUNKED_MIN_TOKENS", "GLA_CHUNKED_MIN_TOKENS"):
         monkeypatch.setattr(K, name, 1 << 30)
 
 
@@ -177,3 +177,63 @@ def test_gated_delta_rule_by_chunks_with_numbers_that_are_not_finite():
     keep[70:, 3] = keep[100:, E:] = False
     assert torch.equal(o[keep], clean[keep]) and not torch.isfinite(o[~keep]).any()
     assert not torch.isfinite(state[0, 0, :, 3]).any() and torch.isfinite(state[0, 0, :, :3]).all() and not torch.isfinite(state[0, 1]).any()
+
+
+def _gla_inputs(lens, H, N, P, seed, low, high):
+    """Decays between ``low`` and ``high``, spread over their logarithms."""
+    gen = torch.Generator(device=DEV).manual_seed(seed)
+    T = sum(lens)
+    proj = torch.randn(T, 2 * H * N + H * P + 8, generator=gen, device=DEV).bfloat16()
+    lo, hi = math.log(low), math.log(high)
+    decay = torch.exp(torch.rand(T, H * N, generator=gen, device=DEV) * (hi - lo) + lo)
+    state = torch.randn(len(lens), H, N, P, generator=gen, device=DEV)
+    return proj[:, :H * N], proj[:, H * N:2 * H * N], proj[:, 2 * H * N:2 * H * N + H * P], decay, state
+
+
+def _gla_exact(q, k, v, decay, scale, state, lens):
+    R, H, N, P = state.shape
+    T, S, at = q.shape[0], state.double().clone(), 0
+    q, k, v, a = q.double().view(T, H, N), k.double().view(T, H, N), v.double().view(T, H, P), decay.double().view(T, H, N)
+    o = torch.empty(T, H, P, dtype=torch.float64, device=DEV)
+    for r, n in enumerate(lens):
+        slot = R - 1 - r
+        for t in range(at, at + n):
+            S[slot] = a[t].unsqueeze(2) * S[slot] + k[t].unsqueeze(2) * v[t].unsqueeze(1)
+            o[t] = (S[slot] * q[t].unsqueeze(2)).sum(1) * scale
+        at += n
+    return o.view(T, H * P), S
+
+
+@pytest.mark.parametrize("lens,H,N,P", [
+    ([64], 4, 128, 128), ([17, 1, 15], 4, 64, 32), ([127, 40], 2, 128, 16), ([33], 4, 64, 64), ([1] * 40 + [70], 2, 64, 32),
+    ([300, 17, 128], 16, 128, 128), ([500], 32, 128, 128), ([200], 3, 128, 48), ([1000], 2, 64, 96), ([160], 64, 128, 128)])
+@pytest.mark.parametrize("low,high", [(0.99, 1.0), (0.9, 1.0), (1e-3, 1.0), (1e-38, 1e-3)])
+def test_gated_linear_attention_by_sixteens(lens, H, N, P, low, high, monkeypatch):
+    """No farther from 64-bit than token by token, or than the sixteen roundings of 6e-8 that a decay's product over sixteen
+    tokens collects."""
+    from prelude_b200.ops import kernels as K
+    q, k, v, decay, state = _gla_inputs(lens, H, N, P, 3, low, high)
+    want_o, want_s = _gla_exact(q, k, v, decay, 0.25, state, lens)
+    chunked, plain = state.clone(), state.clone()
+    o = K.gla_scan(q, k, v, decay, 0.25, chunked, _batch(lens))
+    _by_tokens(monkeypatch, K)
+    o0 = K.gla_scan(q, k, v, decay, 0.25, plain, _batch(lens))
+    errs = [_rel(o, want_o), _rel(chunked, want_s), _rel(o0, want_o), _rel(plain, want_s)]
+    print("sixteens o %.2e state %.2e, tokens o %.2e state %.2e" % tuple(errs))
+    assert errs[0] <= max(errs[2], 16 * 6e-8) and errs[1] <= max(errs[3], 16 * 6e-8)
+    assert not torch.equal(o, o0)
+
+
+def test_gated_linear_attention_by_sixteens_with_numbers_that_are_not_finite():
+    """An infinity in v spoils its own column from its token on; what lies before it, and other columns, stay as they are.  So
+    does one in a key, for every column of its head."""
+    from prelude_b200.ops import kernels as K
+    lens, H, N, P = [50], 2, 64, 32
+    q, k, v, decay, state = _gla_inputs(lens, H, N, P, 5, 0.9, 1.0)
+    clean = K.gla_scan(q, k, v, decay, 1.0, state.clone(), _batch(lens))
+    v[20, 3], k[37, N + 5] = float("inf"), float("nan")
+    o = K.gla_scan(q, k, v, decay, 1.0, state, _batch(lens))
+    keep = torch.ones_like(o, dtype=torch.bool)
+    keep[20:, 3] = keep[37:, P:] = False
+    assert torch.equal(o[keep], clean[keep]) and not torch.isfinite(o[~keep]).any()
+    assert not torch.isfinite(state[0, 0, :, 3]).any() and torch.isfinite(state[0, 0, :, :3]).all()
