@@ -786,6 +786,25 @@ def moe_gemm_pair(a_sorted: torch.Tensor, w: torch.Tensor, plan: MoePlan, gated:
     return out
 
 
+def moe_gemm_grouped(a_sorted: torch.Tensor, w: torch.Tensor, plan: MoePlan, gated: bool, status: torch.Tensor, out_dtype: Optional[torch.dtype] = None,
+                     max_pairs: int = 0, act: int = ACT_NONE, limit: float = 0.0, alpha: float = 0.0) -> torch.Tensor:
+    """``moe_gemm_pair`` for experts with fewer rows: the weights are the product's rows, the tokens its columns, 64 at a time; the
+    plain form's result is bfloat16 or float32."""
+    _need(a_sorted, "a_sorted", torch.bfloat16)
+    _need(w, "w", torch.bfloat16)
+    E, rows_w, Kdim = w.shape
+    out_dtype = out_dtype or torch.bfloat16
+    if plan.tile_rows != 256 or a_sorted.shape != (plan.order.numel(), Kdim) or (gated and (rows_w % 2 or out_dtype != torch.bfloat16)) \
+            or out_dtype not in (torch.bfloat16, torch.float32):
+        raise KernelLibraryError("moe_gemm_grouped: a plan of 256-row tiles, rows sorted by place and a bfloat16 or (plain) float32 result are needed")
+    out = torch.empty((a_sorted.shape[0], rows_w // 2 if gated else rows_w), dtype=out_dtype, device=a_sorted.device)
+    check(_l.library().pb_gemm_grouped_bf16(
+        a_sorted.data_ptr(), w.data_ptr(), out.data_ptr(), a_sorted.shape[0], rows_w, E, Kdim, a_sorted.stride(0), Kdim,
+        out.stride(0), 1 if gated else 0, 1 if out_dtype == torch.float32 else 0, act, float(limit), float(alpha), plan.tile_expert.data_ptr(),
+        plan.tile_row0.data_ptr(), plan.offsets.data_ptr(), plan.max_tiles, max_pairs, status.data_ptr(), _stream()), "gemm_grouped")
+    return out
+
+
 def moe_combine(y: torch.Tensor, plan: MoePlan, weights: torch.Tensor, out_dtype: torch.dtype) -> torch.Tensor:
     """out[t] = sum_c weights[t, c] * y[place of slot (t, c)], float32 sums; y [places, width] float32 or of out_dtype."""
     _need(y, "y")

@@ -109,6 +109,7 @@ _SIGNATURES = {
     "pb_silu_cols": ([P, L, I, I, I, P], I),
     "pb_gelu_tanh_mul": ([P, P, I, I, I, P], I),
     "pb_scaled_sum": ([P, F, P, F, P, I, I, L, P], I),
+    "pb_gemm_grouped_bf16": ([P, P, P, I, I, I, I, L, L, L, I, I, I, F, F, P, P, P, I, I, P, P], I),
     "pb_gemm_pair_grouped_bf16": ([P, P, P, I, I, I, I, L, L, L, I, I, F, F, P, P, P, I, I, P, P], I),
     "pb_gemm_pair_act_bf16": ([P, P, P, I, I, I, L, L, L, I, I, I, P, P], I),
     "pb_gemm_stream_act_bf16": ([P, P, P, I, I, I, L, L, L, I, I, I, P, P], I),

@@ -40,8 +40,13 @@ from .registry import RunContext, register_part
 MOE_FEW_ROWS = int(os.environ.get("PRELUDE_MOE_FEW_ROWS", "6"))
 # tokens up to which the router's product and choice run in one kernel
 ROUTE_FEW_TOKENS = int(os.environ.get("PRELUDE_MOE_ROUTE_FEW_TOKENS", "32"))
-# average rows per expert from which a step's products run on the paired-block tcgen05 kernel
+# average rows per expert from which a step's products run on the paired-block tcgen05 kernel with the tokens as rows (bfloat16
+# results throughout), and from which on the one with the weights as rows.  Against the 64- and 128-row tiles, both products and the
+# gather, us: 64 experts of 4,096 x 2,048 506 against 489 at 2 rows, 546 against 614 at 3, 584 against 751 at 4, 588 against 1,380
+# at 32, 598 against 1,135 at 64, 686 against 1,826 at 128; 32 experts of 2,048 x 2,048 163 against 154, 192 against 208, 190 against 253,
+# 182 against 390, 185 against 322, 195 against 485
 MOE_PAIR_MIN_ROWS = int(os.environ.get("PRELUDE_MOE_PAIR_MIN_ROWS", "192"))
+MOE_GROUPED_MIN_ROWS = int(os.environ.get("PRELUDE_MOE_GROUPED_MIN_ROWS", "3"))
 
 # an activation's name: (two matrices on the way up or one, its number in the products' epilogues)
 _ACTS = {"silu_gated": (True, K.ACT_NONE), "clamped_glu": (True, K.ACT_CLAMPED), "relu2": (False, K.ACT_RELU2)}
@@ -121,14 +126,18 @@ class RoutedExperts:
         shared = 0 if s.shared_size is None else 2 * s.shared_size * elem + s.hidden_size * 4
         return s.top_k * (s.expert_size * elem + s.hidden_size * 4) + s.n_experts * 4 + s.hidden_size * elem + shared
 
-    def pair_takes(self, x: torch.Tensor) -> bool:
-        """Whether a step's products run on the paired-block kernel: bfloat16, aligned sizes, and rows enough that an
-        expert's 256-row tiles are mostly full (PRELUDE_MOE_PAIR_MIN_ROWS rows per expert on average, default 192)."""
+    def _paired(self, x: torch.Tensor, rows: int) -> bool:
+        """Whether a step's products can run on the paired-block kernels, and has ``rows`` rows per expert on average."""
         s = self.spec
         return (x.dtype == torch.bfloat16 and L.PREFILL_GEMM != "cublas" and s.hidden_size % 8 == 0 and s.expert_size % 8 == 0
-                and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and x.shape[0] * s.top_k >= MOE_PAIR_MIN_ROWS * s.n_experts
+                and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and x.shape[0] * s.top_k >= rows * s.n_experts
                 # operands no smaller than one copy box of the kernel (128 rows of 64 elements)
                 and s.hidden_size >= 64 and s.expert_size >= 64 and s.n_experts * min(s.hidden_size, self.w_gate_up.shape[1]) >= 128)
+
+    def pair_takes(self, x: torch.Tensor) -> bool:
+        """Whether a step's products run on the paired-block kernel with the tokens as rows: bfloat16, aligned sizes, and rows enough that
+        an expert's 256-row tiles are mostly full (PRELUDE_MOE_PAIR_MIN_ROWS rows per expert on average, default 192)."""
+        return self._paired(x, MOE_PAIR_MIN_ROWS)
 
     def _router_args(self):
         s = self.spec
@@ -179,6 +188,12 @@ class RoutedExperts:
             h = K.moe_gemv(x, self.w_gate_up, ids, False, x.dtype, gated=self.gated, **self.act)
             y = K.moe_gemv(h, self.w_down, ids, True, torch.float32)
             return self._sum(y, None, weights, shared, x.dtype)
+        if self._paired(x, MOE_GROUPED_MIN_ROWS):
+            # fewer rows: the experts' weights are the rows of the paired-block products, the tokens their columns
+            plan = K.moe_sort(ids, s.n_experts, 256)
+            status = L.tc_status(x.device)
+            h = K.moe_gemm_grouped(K.moe_gather_rows(x, plan, s.top_k), self.w_gate_up, plan, self.gated, status, **self.act)
+            return self._sum(K.moe_gemm_grouped(h, self.w_down, plan, False, status, torch.float32), plan.place_of, weights, shared, x.dtype)
         plan = K.moe_sort(ids, s.n_experts, 64 if (small or few) else None)
         h = K.moe_gemm(x, self.w_gate_up, plan, gated=self.gated, gather_div=s.top_k, few_rows=few, **self.act)
         y = K.moe_gemm(h, self.w_down, plan, gated=False, out_dtype=torch.float32, few_rows=few)

@@ -185,3 +185,50 @@ def test_differential_attention_of_prompts(lens, H, G, vdim, dim, window):
         assert float((got[at:at + n] - o).norm() / o.norm()) < 6e-3
         at += n
     assert int(batch.status) == 0
+
+
+@pytest.mark.parametrize("counts", [[1], [0, 31, 32, 33, 0], [255, 256, 257, 64, 0, 300, 1], [0, 0, 130], [520, 16, 200] * 5])
+@pytest.mark.parametrize("K,N,act", [(64, 64, "silu"), (72, 136, "silu"), (200, 200, "clamped"), (328, 128, "silu"),
+                                     (64, 128, "none"), (136, 264, "relu2"), (520, 328, "none")])
+@pytest.mark.parametrize("max_pairs", [0, 3])
+def test_products_of_routed_experts_on_paired_blocks(counts, K, N, act, max_pairs):
+    """Experts with no rows, one, a step of columns more or less, and more than a tile, against 64 bits.  A float32 sum of products
+    is within 2^-20 of the sum of their magnitudes, the result rounded once (2^-8 with the last bit of the exponential;
+    2^-23 where it is float32)."""
+    from prelude_b200.ops import kernels as K_
+    from prelude_b200.ops.linear import tc_status
+    g, E, T = _gen(21), len(counts), sum(counts)
+    gated = act in ("silu", "clamped")
+    if E * (2 * N if gated else N) < 128:
+        pytest.skip("fewer rows than a block's")
+    ids = torch.cat([torch.full((n,), e, dtype=torch.int32, device=DEV) for e, n in enumerate(counts)])[torch.randperm(T, generator=g, device=DEV)].view(T, 1).contiguous()
+    x = torch.randn(T, K, generator=g, device=DEV).bfloat16()
+    w = (torch.randn(E, 2 * N if gated else N, K, generator=g, device=DEV) * K ** -0.5).bfloat16()
+    plan, status = K_.moe_sort(ids, E, 256), tc_status(torch.device(DEV))
+    code = {"silu": K_.ACT_NONE, "none": K_.ACT_NONE, "clamped": K_.ACT_CLAMPED, "relu2": K_.ACT_RELU2}[act]
+    rows = K_.moe_gather_rows(x, plan, 1)
+    outs = [(K_.moe_gemm_grouped(rows, w, plan, gated, status, None, max_pairs, act=code, limit=0.8, alpha=1.7), 2.0 ** -8),
+            (K_.moe_gemm_pair(rows, w, plan, gated, status, max_pairs, act=code, limit=0.8, alpha=1.7), 2.0 ** -8)]
+    if not gated:
+        outs.append((K_.moe_gemm_grouped(rows, w, plan, False, status, torch.float32, max_pairs, act=code), 2.0 ** -23))
+    wd, xd, e = w.double(), x.double(), ids.view(-1).long()
+    sums = torch.empty(T, w.shape[1], dtype=torch.float64, device=DEV)
+    mags = torch.empty_like(sums)
+    for i in range(E):
+        sums[e == i], mags[e == i] = xd[e == i] @ wd[i].T, xd[e == i].abs() @ wd[i].abs().T
+    err = mags * 2.0 ** -20
+    if gated:
+        a, b, ea, eb = sums[:, :N], sums[:, N:], err[:, :N], err[:, N:]
+        if act == "clamped":
+            a, b = a.clamp(max=0.8), b.clamp(-0.8, 0.8)
+            want, slope, rest = a * torch.sigmoid(1.7 * a) * (b + 1), 1.2 * (b + 1).abs(), (a * torch.sigmoid(1.7 * a)).abs()
+        else:
+            want, slope, rest = a * torch.sigmoid(a) * b, 1.2 * b.abs(), (a * torch.sigmoid(a)).abs()
+        bound = ea * slope + eb * rest
+    elif act == "relu2":
+        want, bound = sums.clamp(min=0) ** 2, 2 * err * (sums.abs() + err)
+    else:
+        want, bound = sums, err
+    for out, unit in outs:
+        assert ((out[plan.place_of.view(-1).long()].double() - want).abs() <= bound + want.abs() * unit + 1e-30).all()
+    assert int(status) == 0
