@@ -44,8 +44,10 @@ __device__ ArgPair block_argmax(const float* row, int begin, int end, ArgPair* s
 #pragma unroll
         for (int u = 0; u < 8; ++u) v[u] = row[i + u * blockDim.x];
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
-            if (v[u] > best.v) best = ArgPair{v[u], i + u * (int)blockDim.x};  // ascending indices: the first stays; NaN never wins
+        for (int u = 0; u < 8; ++u) {
+            const int at = i + u * (int)blockDim.x;
+            if (v[u] > best.v || (v[u] == best.v && at < best.i)) best = ArgPair{v[u], at};   // -inf beats no number at all; NaN never wins
+        }
     }
     for (; i < end; i += blockDim.x) {
         float v = row[i];

@@ -232,3 +232,21 @@ def test_products_of_routed_experts_on_paired_blocks(counts, K, N, act, max_pair
     for out, unit in outs:
         assert ((out[plan.place_of.view(-1).long()].double() - want).abs() <= bound + want.abs() * unit + 1e-30).all()
     assert int(status) == 0
+
+
+@pytest.mark.parametrize("width", [1, 255, 256, 257, 2047, 2048, 2049, 3000, 4096, 4097, 8192, 32000, 151936])
+def test_argmax_of_rows_that_hold_minus_infinity(width):
+    """Both loops over a chunk, eight loads at a time and the rest: a row of -inf alone gives its first index, one number among
+    -inf wins wherever it stands, NaN never does (a row of NaN gives 0)."""
+    from prelude_b200.ops import kernels as K
+    places = sorted({0, width // 3, width // 2, width - 1})
+    rows = torch.full((3 + len(places), width), float("-inf"), device=DEV)
+    rows[1] = float("nan")
+    rows[2, :(width + 1) // 2] = float("nan")               # then -inf, where there is more than one
+    for r, at in enumerate(places):
+        rows[3 + r, at] = -3.0e38
+    got = K.argmax(rows).tolist()
+    assert got == [0, 0, (width + 1) // 2 if width > 1 else 0] + places
+    zero = torch.zeros(len(got), device=DEV)
+    n = torch.zeros(len(got), dtype=torch.int64, device=DEV)
+    assert K.sample(rows, zero, n, n).tolist() == got
