@@ -158,7 +158,8 @@ delta_prepare_kernel(const bf16* u, long long ld_u, const bf16* b_in, long long 
             if (lane >= o) before += v;
         }
         const double last = __shfl_sync(0xffffffffu, before, 31);
-        before -= l[1];
+        before = __shfl_up_sync(0xffffffffu, before, 1);        // not before - l[1]: a NaN in l[1] would reach l[0]
+        if (lane == 0) before = 0.0;
         float* num = reinterpret_cast<float*>(blob + DC_NUM);
         int fb = bad[2 * lane] != 0.f ? 2 * lane : bad[2 * lane + 1] != 0.f ? 2 * lane + 1 : DC_L;
 #pragma unroll

@@ -108,7 +108,8 @@ ssm_chunk_kernel(const bf16* u, const bf16* dt_in, long long ld_dt, const float*
                 if (lane >= o) before += v;
             }
             const double last = __shfl_sync(0xffffffffu, before, 31);
-            before -= l[1];
+            before = __shfl_up_sync(0xffffffffu, before, 1);                      // not before - l[1]: a NaN in l[1] would reach l[0]
+            if (lane == 0) before = 0.0;
             float w[2];
             float* num = reinterpret_cast<float*>(buf + Z::num);
             int* bad = reinterpret_cast<int*>(buf + Z::bad);

@@ -237,3 +237,38 @@ def test_gated_linear_attention_by_sixteens_with_numbers_that_are_not_finite():
     keep[20:, 3] = keep[37:, P:] = False
     assert torch.equal(o[keep], clean[keep]) and not torch.isfinite(o[~keep]).any()
     assert not torch.isfinite(state[0, 0, :, 3]).any() and torch.isfinite(state[0, 0, :, :3]).all()
+
+
+@pytest.mark.parametrize("at", [0, 1, 62, 63, 64, 101])
+@pytest.mark.parametrize("kind", ["state space", "gated delta rule, decay", "gated delta rule, beta", "gated linear attention"])
+def test_a_step_size_or_decay_that_is_no_number_spoils_no_earlier_token(kind, at):
+    """The first or the second token of a pair, at a chunk's edges and inside one: every output of the head from that token on is NaN,
+    what lies before it and the other head stay as they are to the last bit."""
+    from prelude_b200.ops import kernels as K
+    lens = [150]
+    if kind == "state space":
+        P = 32
+        u, dt, bias, a_log, skip, state = _ssm_inputs(lens, 2, P, 64, 1, 5, 0.05)
+        poisoned, spoil = dt.clone(), (at, 1)
+        run = lambda d, s: K.ssm_scan(u, d, bias, a_log, skip, s, _batch(lens), 1)
+    elif kind.startswith("gated delta"):
+        P = 16
+        u, b, a, a_log, bias, state = _delta_inputs(lens, 2, 2, 64, P, 5, 0.05)
+        dt = a if kind.endswith("decay") else b
+        poisoned, spoil = dt.clone(), (at, 1)
+        run = lambda d, s: K.gated_delta_scan(u, *((b, d) if kind.endswith("decay") else (d, a)), a_log, bias, s, _batch(lens), 2)
+    else:
+        P = 32
+        q, k, v, dt, state = _gla_inputs(lens, 2, 64, P, 5, 0.9, 1.0)
+        poisoned, spoil = dt.clone(), (at, 64 + 9)
+        run = lambda d, s: K.gla_scan(q, k, v, d, 1.0, s, _batch(lens))
+    clean_state, state = state.clone(), state.clone()
+    clean = run(dt, clean_state)
+    poisoned[spoil] = float("nan")
+    y = run(poisoned, state)
+    keep = torch.ones_like(y, dtype=torch.bool)
+    keep[at:, P:] = False
+    assert torch.equal(y[keep], clean[keep]) and torch.isnan(y[~keep]).all()
+    assert torch.equal(state[0, 0], clean_state[0, 0])
+    gone = state[0, 1, 9] if kind == "gated linear attention" else state[0, 1]
+    assert torch.isnan(gone).all()
