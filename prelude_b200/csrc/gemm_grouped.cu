@@ -187,12 +187,9 @@ gemm_grouped_kernel(const __grid_constant__ GgMaps maps, GgParams p) {
                         const float theirs = swap[((up_row ? 0 : 16) + j) * 64];
                         float g = up_row ? theirs : v[j];
                         const float up = up_row ? v[16 + j] : theirs;
-                        if (p.act == PB_ACT_CLAMPED) {
-                            const float a = fminf(g, p.limit), b = fminf(fmaxf(up, -p.limit), p.limit);
-                            g = a / (1.0f + __expf(-p.alpha * a)) * (b + 1.0f);
-                        } else {
-                            g = g / (1.0f + __expf(-g)) * up;
-                        }
+                        // the exponential as in moe.cu's tiles, which take the same rows at other sizes
+                        if (p.act == PB_ACT_CLAMPED) g = pb_clamped_unit(g, up, p.limit, p.alpha);
+                        else g = g / (1.0f + expf(-g)) * up;
                         if (live && first + j < rows) dst[(size_t)(first + j) * p.ldo] = __float2bfloat16_rn(g);
                     }
                     asm volatile("bar.sync %0, 128;\n" ::"r"(2 + side) : "memory");        // the halves have been read

@@ -250,3 +250,27 @@ def test_argmax_of_rows_that_hold_minus_infinity(width):
     zero = torch.zeros(len(got), device=DEV)
     n = torch.zeros(len(got), dtype=torch.int64, device=DEV)
     assert K.sample(rows, zero, n, n).tolist() == got
+
+
+@pytest.mark.parametrize("act", ["silu", "clamped"])
+def test_gates_of_experts_with_few_rows_keep_32_bits(act):
+    """Gate and up sums of one exact product each: what is left of a gate's error before its rounding to bfloat16 is the
+    exponential's (two units in the last place at most) and three roundings, 4 x 2^-23 together."""
+    from prelude_b200.ops import kernels as K
+    from prelude_b200.ops.linear import tc_status
+    g, counts, N = _gen(31), [191, 64, 130], 512
+    T = sum(counts)
+    ids = torch.repeat_interleave(torch.arange(3, device=DEV), torch.tensor(counts, device=DEV)).int().view(T, 1)
+    x = torch.zeros(T, 64, device=DEV, dtype=torch.bfloat16)
+    x[:, 0], x[:, 1] = 24 * torch.rand(T, generator=g, device=DEV) - 12, 1
+    w = torch.zeros(3, 2 * N, 64, device=DEV, dtype=torch.bfloat16)
+    w[:, :N, 0], w[:, N:, 1] = 2 * torch.rand(3, N, generator=g, device=DEV), 1
+    plan = K.moe_sort(ids, 3, 256)
+    status = tc_status(torch.device(DEV))
+    out = K.moe_gemm_grouped(K.moe_gather_rows(x, plan, 1), w, plan, True, status, None, 0, act=K.ACT_NONE if act == "silu" else K.ACT_CLAMPED,
+                             limit=9.0, alpha=2.0)
+    z = x[:, 0].double().view(T, 1) * w[:, :N, 0].double()[ids.view(-1).long()]
+    want = z * torch.sigmoid(z) if act == "silu" else 2 * z.clamp(max=9.0) * torch.sigmoid(2 * z.clamp(max=9.0))
+    half_unit = torch.exp2(torch.floor(torch.log2(want.abs().clamp_min(1e-300))) - 8)
+    err = (out[plan.place_of.view(-1).long()].double() - want).abs()
+    assert bool((err <= half_unit + want.abs() * 4 * 2.0 ** -23).all()) and int(status) == 0
