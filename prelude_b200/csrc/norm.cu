@@ -69,16 +69,6 @@ __global__ void add_rmsnorm_vec4_kernel(const TX* x, int n_parts, size_t part_st
     PB_TL(PB_TL_NORM, PB_TL_ENTRY);
     __shared__ float red[32];
     size_t row = blockIdx.x;
-    if constexpr (GATHER) {
-        const int src = rows[row];                              // where the logits are wanted: the step's own input, written by no kernel
-        if (src < 0 || src >= n_rows_total) {
-            pb_grid_dep_wait();
-            for (int i = threadIdx.x; i < width; i += blockDim.x) pb_st(y + row * width + i, 0.f);
-            return;
-        }
-        row = src;
-    }
-    float4* r4 = reinterpret_cast<float4*>(res + row * width);
     const int n4 = width >> 2;
     // the scale is written by no kernel: it is fetched while the kernel before this one is still running
     const float4* w4 = reinterpret_cast<const float4*>(w);
@@ -90,6 +80,15 @@ __global__ void add_rmsnorm_vec4_kernel(const TX* x, int n_parts, size_t part_st
     }
     pb_grid_dep_wait();
     PB_TL(PB_TL_NORM, PB_TL_AFTER_WAIT);
+    if constexpr (GATHER) {
+        const int src = rows[row];                              // behind the wait: the kernel before may have chosen the rows
+        if (src < 0 || src >= n_rows_total) {
+            for (int i = threadIdx.x; i < width; i += blockDim.x) pb_st(y + row * width + i, 0.f);
+            return;
+        }
+        row = src;
+    }
+    float4* r4 = reinterpret_cast<float4*>(res + row * width);
     float4 keep[ITERS];
     float ss = 0.f;
     // Every load of the row is issued before the first sum (up to four parts): the kernel is one round trip to

@@ -34,3 +34,28 @@ def test_the_gated_norm_waits_for_the_scan(parts_width):
         torch.cuda.synchronize()
         assert torch.isfinite(y).all()
         assert torch.equal(got, K.gated_group_rmsnorm(y, z, weight, H * P // parts_width, 1e-6))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("width", [2048, 2050])
+def test_the_norm_of_chosen_rows_waits_for_the_choice(dtype, width):
+    """The rows are chosen by the kernel before: that of the largest of 60,000 numbers, on few multiprocessors.  Read too early
+    they are what lay there, -1, which gives zeros."""
+    from prelude_b200.ops import kernels as K
+    n, wide = 8, 60000
+    gen = torch.Generator(device=DEV).manual_seed(4)
+    res, weight = torch.randn(n, width, generator=gen, device=DEV), torch.rand(width, generator=gen, device=DEV) + 0.5
+    scores = torch.zeros(n, wide, device=DEV)
+    picks = torch.randperm(n, generator=gen, device=DEV)
+    scores[torch.arange(n, device=DEV), picks] = 1.0
+    zero, counts = torch.zeros(n, device=DEV), torch.zeros(n, dtype=torch.int64, device=DEV)
+    want = K.gather_add_rmsnorm(None, res, picks.int(), weight, 1e-6, dtype)
+    busy = torch.randn(8192, 8192, device=DEV).bfloat16()
+    for _ in range(4):
+        rows = torch.full((n,), -1, dtype=torch.int32, device=DEV)
+        for _ in range(3):
+            torch.mm(busy, busy)              # the host is ahead: the norm is queued before the choice begins
+        K.sample(scores, zero, counts, counts, out=rows)
+        got = K.gather_add_rmsnorm(None, res, rows, weight, 1e-6, dtype)
+        torch.cuda.synchronize()
+        assert rows.tolist() == picks.tolist() and torch.equal(got, want)
