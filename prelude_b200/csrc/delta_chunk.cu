@@ -621,9 +621,13 @@ int dc_run(const void* u, long long ld_u, const void* b_in, long long ld_b, cons
 
 }  // namespace
 
-// Whether pb_gated_delta_scan_chunked takes these sizes: rows and values in 16-byte pieces, keys of 64 or 128 elements.
-PB_API int pb_gated_delta_chunked_takes(const void* u, long long ld_u, int H, int G, int D, int E) {
-    return (D == 64 || D == 128) && E > 0 && E % 16 == 0 && H > 0 && H < 65536 && G > 0 && H % G == 0 && ld_u % 8 == 0 && pb_aligned(u, 16) ? 1 : 0;
+// Whether pb_gated_delta_scan_chunked takes these sizes and operands: rows and values in 16-byte pieces, keys of 64 or 128 elements,
+// state and result in 8-byte pieces (pb_gated_delta_scan takes any).
+PB_API int pb_gated_delta_chunked_takes(const void* u, long long ld_u, const float* state, const float* y, int H, int G, int D, int E) {
+    return (D == 64 || D == 128) && E > 0 && E % 16 == 0 && H > 0 && H < 65536 && G > 0 && H % G == 0 && ld_u % 8 == 0 && pb_aligned(u, 16) &&
+                   pb_aligned(state, 8) && pb_aligned(y, 8)
+               ? 1
+               : 0;
 }
 // Most chunks that n_tokens of n_seqs sequences can form, and the scratch memory (16-byte aligned) that the call needs for them.
 PB_API int pb_gated_delta_chunks(int n_tokens, int n_seqs) { return n_tokens / DC_L + (n_seqs < n_tokens ? n_seqs : n_tokens); }
@@ -634,10 +638,10 @@ PB_API long long pb_gated_delta_chunk_bytes(int n_chunks, int H) { return (long 
 PB_API int pb_gated_delta_scan_chunked(const void* u, long long ld_u, const void* b_in, long long ld_b, const void* a_in, long long ld_a, const float* a_log,
                                        const float* dt_bias, float* state, float* y, const int32_t* cu_q, const int32_t* slots, void* scratch, int n_chunks,
                                        int n_seqs, int H, int G, int D, int E, cudaStream_t stream) {
-    PB_REQUIRE(n_seqs >= 0 && n_chunks >= 0 && pb_gated_delta_chunked_takes(u, ld_u, H, G, D, E), "gated_delta_scan_chunked: %d over %d heads of %d, %d", H, G, D, E);
+    PB_REQUIRE(n_seqs >= 0 && n_chunks >= 0 && pb_gated_delta_chunked_takes(u, ld_u, state, y, H, G, D, E), "gated_delta_scan_chunked: %d over %d heads of %d, %d", H, G, D, E);
     PB_REQUIRE(u && b_in && a_in && a_log && dt_bias && state && y && cu_q && slots && scratch, "gated_delta_scan_chunked: null pointer");
     PB_REQUIRE(ld_u >= 2ll * G * D + (long long)H * E && ld_b >= H && ld_a >= H, "gated_delta_scan_chunked: rows too short");
-    PB_REQUIRE(pb_aligned(state, 8) && pb_aligned(y, 8) && pb_aligned(scratch, 16), "gated_delta_scan_chunked: misaligned operands");
+    PB_REQUIRE(pb_aligned(scratch, 16), "gated_delta_scan_chunked: misaligned operands");
     if (n_seqs == 0 || n_chunks == 0) return 0;
     PB_REQUIRE(n_seqs < 65536, "gated_delta_scan_chunked: %d sequences in one launch", n_seqs);
     int dev = 0, sms = 0;

@@ -493,11 +493,11 @@ int gc_run(const GcCall& c) {
 
 }  // namespace
 
-// Whether pb_gla_scan_chunked takes these sizes and operands: rows in 16-byte pieces, 64 or 128 channels, values in 16-column slices
+// Whether pb_gla_scan_chunked takes these sizes and operands: rows and results in 16-byte pieces, 64 or 128 channels, values in 16-column slices
 // (64 channels: 32, a column group for each half of the warps).
-PB_API int pb_gla_chunked_takes(const void* q, const void* k, const void* v, const void* decay, long long ld, int H, int N, int P) {
+PB_API int pb_gla_chunked_takes(const void* q, const void* k, const void* v, const void* decay, const float* y, long long ld, int H, int N, int P) {
     return (N == 64 || N == 128) && P > 0 && P % (N == 64 ? 32 : 16) == 0 && H > 0 && H < 65536 && ld % 8 == 0 && pb_aligned(q, 16) && pb_aligned(k, 16) &&
-                   pb_aligned(v, 16) && pb_aligned(decay, 16)
+                   pb_aligned(v, 16) && pb_aligned(decay, 16) && pb_aligned(y, 16)
                ? 1
                : 0;
 }
@@ -509,9 +509,9 @@ PB_API long long pb_gla_chunk_bytes(int n_steps, int H, int N) { return (long lo
 // head's state where that still gives four fifths of the multiprocessors a block (or the warps need two column groups), else 16.
 PB_API int pb_gla_scan_chunked(const void* q, const void* k, const void* v, long long ld, const float* decay, float scale, float* state, float* y,
                                const int32_t* cu_q, const int32_t* slots, void* scratch, int n_steps, int n_seqs, int H, int N, int P, cudaStream_t stream) {
-    PB_REQUIRE(n_seqs >= 0 && n_steps >= 0 && pb_gla_chunked_takes(q, k, v, decay, ld, H, N, P), "gla_scan_chunked: %d heads of %d x %d", H, N, P);
+    PB_REQUIRE(n_seqs >= 0 && n_steps >= 0 && pb_gla_chunked_takes(q, k, v, decay, y, ld, H, N, P), "gla_scan_chunked: %d heads of %d x %d", H, N, P);
     PB_REQUIRE(q && k && v && decay && state && y && cu_q && slots && scratch, "gla_scan_chunked: null pointer");
-    PB_REQUIRE(pb_aligned(y, 16) && pb_aligned(scratch, 16), "gla_scan_chunked: misaligned operands");
+    PB_REQUIRE(pb_aligned(scratch, 16), "gla_scan_chunked: misaligned operands");
     if (n_seqs == 0 || n_steps == 0) return 0;
     PB_REQUIRE(n_seqs < 65536, "gla_scan_chunked: %d sequences in one launch", n_seqs);
     int dev = 0, sms = 0;

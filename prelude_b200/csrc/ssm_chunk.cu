@@ -362,9 +362,13 @@ int sc_launch(const void* u, const void* dt_in, long long ld_dt, const float* dt
 
 }  // namespace
 
-// Whether pb_ssm_scan_chunked takes these sizes (and operands on 16-byte boundaries).
-PB_API int pb_ssm_scan_chunked_takes(const void* u, int heads, int P, int N, int groups) {
-    return (N == 64 || N == 128) && P > 0 && P % 16 == 0 && heads > 0 && groups > 0 && heads % groups == 0 && pb_aligned(u, 16) ? 1 : 0;
+// Whether pb_ssm_scan_chunked takes these sizes and operands: rows in 16-byte pieces, state and result in 8-byte ones (pb_ssm_scan
+// takes any).
+PB_API int pb_ssm_scan_chunked_takes(const void* u, const float* state, const float* y, int heads, int P, int N, int groups) {
+    return (N == 64 || N == 128) && P > 0 && P % 16 == 0 && heads > 0 && groups > 0 && heads % groups == 0 && pb_aligned(u, 16) && pb_aligned(state, 8) &&
+                   pb_aligned(y, 8)
+               ? 1
+               : 0;
 }
 
 // Operands as for pb_ssm_scan, bfloat16.  A block takes 64, 32 or 16 columns of a head's state, the most that still gives four
@@ -372,9 +376,8 @@ PB_API int pb_ssm_scan_chunked_takes(const void* u, int heads, int P, int N, int
 PB_API int pb_ssm_scan_chunked(const void* u, const void* dt_in, long long ld_dt, const float* dt_bias, const float* a_log, const float* d_skip,
                                float* state, float* y, const int32_t* cu_q, const int32_t* slots, int n_seqs, int heads, int P, int N, int groups,
                                cudaStream_t stream) {
-    PB_REQUIRE(n_seqs >= 0 && pb_ssm_scan_chunked_takes(u, heads, P, N, groups), "ssm_scan_chunked: %d heads of %d, state %d, %d groups", heads, P, N, groups);
+    PB_REQUIRE(n_seqs >= 0 && pb_ssm_scan_chunked_takes(u, state, y, heads, P, N, groups), "ssm_scan_chunked: %d heads of %d, state %d, %d groups", heads, P, N, groups);
     PB_REQUIRE(u && dt_in && dt_bias && a_log && d_skip && state && y && cu_q && slots && ld_dt >= heads, "ssm_scan_chunked: null pointer");
-    PB_REQUIRE(pb_aligned(state, 8) && pb_aligned(y, 8), "ssm_scan_chunked: state and result on 8-byte boundaries");
     if (n_seqs == 0) return 0;
     PB_REQUIRE(n_seqs < 65536, "ssm_scan_chunked: %d sequences in one launch", n_seqs);
     const long long states = (long long)heads * n_seqs;

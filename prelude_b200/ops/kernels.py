@@ -1073,7 +1073,7 @@ def ssm_scan(u: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: to
         out = torch.empty((T, heads * P), dtype=torch.float32, device=u.device)
     lib = _l.library()
     if (u.dtype == torch.bfloat16 and T >= SCAN_CHUNKED_MIN_TOKENS and not batch.decode_only
-            and lib.pb_ssm_scan_chunked_takes(u.data_ptr(), heads, P, N, groups)):
+            and lib.pb_ssm_scan_chunked_takes(u.data_ptr(), state.data_ptr(), out.data_ptr(), heads, P, N, groups)):
         check(lib.pb_ssm_scan_chunked(u.data_ptr(), dt.data_ptr(), dt.stride(0), dt_bias.data_ptr(), a_log.data_ptr(), d_skip.data_ptr(),
                                       state.data_ptr(), out.data_ptr(), batch.cu_q.data_ptr(), batch.state_slots.data_ptr(),
                                       batch.cu_q.numel() - 1, heads, P, N, groups, _stream()), "ssm_scan_chunked")
@@ -1312,7 +1312,7 @@ def gated_delta_scan(u: torch.Tensor, beta: torch.Tensor, a: torch.Tensor, a_log
         out = torch.empty((T, H * E), dtype=torch.float32, device=u.device)
     lib, n_seqs = _l.library(), batch.cu_q.numel() - 1
     if (u.dtype == torch.bfloat16 and T >= DELTA_CHUNKED_MIN_TOKENS and not batch.decode_only
-            and lib.pb_gated_delta_chunked_takes(u.data_ptr(), u.stride(0), H, kv_heads, D, E)):
+            and lib.pb_gated_delta_chunked_takes(u.data_ptr(), u.stride(0), state.data_ptr(), out.data_ptr(), H, kv_heads, D, E)):
         # what one kernel makes of every chunk for the other to read: dead when the call's kernels are done
         n_chunks = lib.pb_gated_delta_chunks(T, n_seqs)
         scratch = torch.empty((lib.pb_gated_delta_chunk_bytes(n_chunks, H),), dtype=torch.uint8, device=u.device)
@@ -1412,7 +1412,7 @@ def gla_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Ten
         out = torch.empty((T, H * P), dtype=torch.float32, device=q.device)
     lib, n_seqs = _l.library(), batch.cu_q.numel() - 1
     if (q.dtype == torch.bfloat16 and T >= GLA_CHUNKED_MIN_TOKENS and not batch.decode_only
-            and lib.pb_gla_chunked_takes(q.data_ptr(), k.data_ptr(), v.data_ptr(), decay.data_ptr(), q.stride(0), H, N, P)):
+            and lib.pb_gla_chunked_takes(q.data_ptr(), k.data_ptr(), v.data_ptr(), decay.data_ptr(), out.data_ptr(), q.stride(0), H, N, P)):
         # what one kernel makes of every sixteen for the other to read: dead when the call's kernels are done
         n_steps = lib.pb_gla_chunks(T, n_seqs)
         scratch = torch.empty((lib.pb_gla_chunk_bytes(n_steps, H, N),), dtype=torch.uint8, device=q.device)

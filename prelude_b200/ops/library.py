@@ -102,7 +102,7 @@ _SIGNATURES = {
     "pb_ssm_scan": ([P, P, L, I, P, P, P, P, P, P, P, I, I, I, I, I, P], I),
     "pb_ssm_step_takes": ([P, P, I, I, I, I], I),
     "pb_ssm_step": ([P, P, L, P, P, P, P, P, P, P, I, I, I, I, I, P], I),
-    "pb_ssm_scan_chunked_takes": ([P, I, I, I, I], I),
+    "pb_ssm_scan_chunked_takes": ([P, P, P, I, I, I, I], I),
     "pb_ssm_scan_chunked": ([P, P, L, P, P, P, P, P, P, P, I, I, I, I, I, P], I),
     "pb_gated_group_rmsnorm": ([P, P, L, P, P, I, I, I, I, F, I, I, P], I),
     "pb_decay_scan": ([P, L, I, P, P, P, P, P, I, I, I, I, I, P], I),
@@ -120,7 +120,7 @@ _SIGNATURES = {
     "pb_sigmoid_gate_": ([P, L, P, L, I, I, I, P], I),
     "pb_channel_decay": ([P, L, P, P, F, P, I, I, I, I, P], I),
     "pb_gla_scan": ([P, P, P, L, I, P, F, P, P, P, P, I, I, I, I, P], I),
-    "pb_gla_chunked_takes": ([P, P, P, P, L, I, I, I], I),
+    "pb_gla_chunked_takes": ([P, P, P, P, P, L, I, I, I], I),
     "pb_gla_chunks": ([I, I], I),
     "pb_gla_chunk_bytes": ([I, I, I], L),
     "pb_gla_scan_chunked": ([P, P, P, L, P, F, P, P, P, P, P, I, I, I, I, I, P], I),
@@ -132,7 +132,7 @@ _SIGNATURES = {
     "pb_tanh": ([P, P, I, L, P], I),
     "pb_heads_prepare": ([P, L, P, L, P, L, I, P, P, I, F, P, F, I, I, P, P, L, F, P, P, P, I, I, I, P, P, P, I, I, I, I, I, I, I, P, P], I),
     "pb_gated_delta_scan": ([P, L, P, L, P, L, I, P, P, P, P, P, P, I, I, I, I, I, P], I),
-    "pb_gated_delta_chunked_takes": ([P, L, I, I, I, I], I),
+    "pb_gated_delta_chunked_takes": ([P, L, P, P, I, I, I, I], I),
     "pb_gated_delta_chunks": ([I, I], I),
     "pb_gated_delta_chunk_bytes": ([I, I], L),
     "pb_gated_delta_scan_chunked": ([P, L, P, L, P, L, P, P, P, P, P, P, P, I, I, I, I, I, I, P], I),

@@ -272,3 +272,31 @@ def test_a_step_size_or_decay_that_is_no_number_spoils_no_earlier_token(kind, at
     assert torch.equal(state[0, 0], clean_state[0, 0])
     gone = state[0, 1, 9] if kind == "gated linear attention" else state[0, 1]
     assert torch.isnan(gone).all()
+
+
+@pytest.mark.parametrize("odd_state,odd_result", [(False, True), (True, False), (True, True)])
+@pytest.mark.parametrize("kind", ["state space", "gated delta rule", "gated linear attention"])
+def test_state_and_result_anywhere(kind, odd_state, odd_result):
+    """A result or a state that begins four bytes past a boundary is taken as before there were chunks (by tokens, where the
+    chunks' wider accesses do not fit)."""
+    from prelude_b200.ops import kernels as K
+    lens, H = [40, 70], 2
+    if kind == "state space":
+        u, dt, bias, a_log, skip, state = _ssm_inputs(lens, H, 32, 64, 1, 5, 0.05)
+        width, run = H * 32, lambda s, o: K.ssm_scan(u, dt, bias, a_log, skip, s, _batch(lens), 1, out=o)
+    elif kind == "gated delta rule":
+        u, b, a, a_log, bias, state = _delta_inputs(lens, H, 2, 64, 16, 5, 0.05)
+        width, run = H * 16, lambda s, o: K.gated_delta_scan(u, b, a, a_log, bias, s, _batch(lens), 2, out=o)
+    else:
+        q, k, v, decay, state = _gla_inputs(lens, H, 64, 32, 5, 0.9, 1.0)
+        width, run = H * 32, lambda s, o: K.gla_scan(q, k, v, decay, 1.0, s, _batch(lens), out=o)
+
+    def at(shape, odd):
+        n = math.prod(shape)
+        return torch.zeros(n + 1, device=DEV)[odd:n + odd].view(shape)
+
+    want_s = state.clone()
+    want = run(want_s, at((sum(lens), width), False))
+    got_s = at(tuple(state.shape), odd_state).copy_(state)
+    got = run(got_s, at((sum(lens), width), odd_result))
+    assert _rel(got, want.double()) < 1e-6 and _rel(got_s, want_s.double()) < 1e-6
