@@ -387,6 +387,18 @@ PB_API int pb_qkv_prepare(const void* q_in, long long ldq, const void* k_in, lon
     auto whole = [&](int off) { return rates == nullptr || (off % vn == 0 && rot_dims % vn == 0 && (adjacent || (rot_dims / 2) % vn == 0)); };
     const int nk = k_pages ? G * kd : 0;
     bool direct = staged && q_w == nullptr && whole(q_rot_off) && H * qd <= QP_MOST * vn * 256 && (nk == 0 || whole(k_rot_off));
+    // queries written over what is read: a thread reads its pieces' rotation partners, and the last warp its key row, after others have
+    // stored; the staged kernel has read both rows by then
+    const size_t esz = dtype == PB_BF16 ? 2 : 4;
+    auto meets = [&](const void* a, size_t a_elems, const void* b, size_t b_elems) {
+        const char *p = (const char*)a, *q = (const char*)b;
+        return p != nullptr && q != nullptr && p < q + b_elems * esz && q < p + a_elems * esz;
+    };
+    const size_t last = (size_t)n_tokens - 1, q_elems = last * ldq + (size_t)H * qd, k_elems = nk ? last * ldk + nk : 0;
+    const void* outs[2] = {q_out, q_split < qd ? q_out2 : nullptr};
+    const size_t out_elems[2] = {(size_t)n_tokens * H * q_split, (size_t)n_tokens * H * q2_head_stride};
+    for (int i = 0; i < 2; ++i)
+        direct = direct && !meets(q_in, q_elems, outs[i], out_elems[i]) && !(k_elems && meets(k_in, k_elems, outs[i], out_elems[i]));
     if (direct && nk > 0 && k_w != nullptr && rates != nullptr)
         for (int g = 0; g < G; ++g) direct = direct && g * kd + k_rot_off >= k_norm_cols;
     if (direct) {

@@ -274,3 +274,26 @@ def test_gates_of_experts_with_few_rows_keep_32_bits(act):
     half_unit = torch.exp2(torch.floor(torch.log2(want.abs().clamp_min(1e-300))) - 8)
     err = (out[plan.place_of.view(-1).long()].double() - want).abs()
     assert bool((err <= half_unit + want.abs() * 4 * 2.0 ** -23).all()) and int(status) == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("adjacent", [False, True])
+@pytest.mark.parametrize("H,d,dims", [(16, 128, 128), (64, 64, 64), (2, 32, 16)])
+def test_queries_turned_where_they_lie(dtype, adjacent, H, d, dims):
+    """``q_out`` the memory of ``q_in``: the same numbers as into memory of its own, but for the last bit (two kernels; a
+    difference of two products of numbers below 6 may be off by 6 x 2^-23 in either)."""
+    from prelude_b200.ops import kernels as K
+    g, T = _gen(9), 300
+    q = torch.randn(T, H * d, generator=g, device=DEV).to(dtype)
+    rates = torch.rand(dims // 2, generator=g, device=DEV)
+    pos, rows = torch.arange(T, dtype=torch.int32, device=DEV), torch.zeros(T, dtype=torch.int32, device=DEV)
+
+    def turn(x, out):
+        return K.qkv_prepare(x, None, None, n_heads=H, q_dim=d, rates=rates, rot_dims=dims, adjacent=adjacent, amplitude=1.0, positions=pos,
+                             table_row=rows, q_out=out).clone()
+
+    want = turn(q, torch.empty_like(q))
+    for _ in range(3):
+        mine = q.clone()
+        got = turn(mine, mine)
+        assert bool(((got.double() - want.double()).abs() <= 2 * UNIT[dtype] * want.double().abs() + 2 * 6 * 2.0 ** -23).all())
