@@ -21,6 +21,7 @@
 // sequences of 592 and 1,185 tokens, 16 heads, 118 against 432; 64 tokens 24 against 28, 32 tokens 24 against 16.  Against 64-bit:
 // output 0.9 to 2.1e-7 (token by token 1.1e-7 to 3.2e-6), state 0.4 to 2.9e-7 (0.5e-7 to 9e-6: the slower the decay the larger).
 #include "mma_sync.cuh"
+#include "sequences.cuh"
 
 #include <math.h>
 
@@ -38,38 +39,6 @@ constexpr int DC_TILE = 3 * 32 * 16, DC_TRI = 10 * DC_TILE, DC_NUM = 2 * DC_TRI,
 __device__ __forceinline__ float dc_softplus(float x) { return x > 20.0f ? x : log1pf(expf(x)); }
 __device__ __forceinline__ int dc_tri(int i) { return i * (i + 1) / 2; }
 
-// Chunks of the sequences before `seq`; a warp together.
-__device__ __forceinline__ int dc_chunks_before(const int32_t* cu_q, int seq, int lane) {
-    int n = 0;
-    for (int r = lane; r < seq; r += 32) n += max(0, (cu_q[r + 1] - cu_q[r] + DC_L - 1) / DC_L);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
-    return n;
-}
-// The sequence and the chunk in it that number `slot` of all chunks is, or false; a warp together.
-__device__ __forceinline__ bool dc_find(const int32_t* cu_q, int n_seqs, int slot, int lane, int& seq, int& chunk) {
-    int base = 0;
-    for (int r0 = 0; r0 < n_seqs; r0 += 32) {
-        const int r = r0 + lane;
-        const int n = r < n_seqs ? max(0, (cu_q[r + 1] - cu_q[r] + DC_L - 1) / DC_L) : 0;
-        int upto = n;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, upto, o);
-            if (lane >= o) upto += v;
-        }
-        const unsigned hit = __ballot_sync(0xffffffffu, base + upto > slot);
-        if (hit) {
-            const int at = __ffs(hit) - 1;
-            seq = r0 + at;
-            chunk = slot - base - (__shfl_sync(0xffffffffu, upto, at) - __shfl_sync(0xffffffffu, n, at));
-            return true;
-        }
-        base += __shfl_sync(0xffffffffu, upto, 31);
-    }
-    return false;
-}
-
 template <int D>
 struct DcPrep {
     static constexpr int LDK = D + 8, LDA = DC_L + 4, LDX = 36;
@@ -82,16 +51,17 @@ struct DcPrep {
 template <int D>
 __global__ void __launch_bounds__(256, 4)
 delta_prepare_kernel(const bf16* u, long long ld_u, const bf16* b_in, long long ld_b, const bf16* a_in, long long ld_a, const float* a_log,
-                     const float* dt_bias, const int32_t* cu_q, unsigned char* blobs, int n_seqs, int H, int G) {
+                     const float* dt_bias, const int32_t* cu_q, unsigned char* blobs, int n_seqs, int least, int few, int beside, int H, int G) {
     using Z = DcPrep<D>;
     extern __shared__ __align__(16) unsigned char dp_sm[];
     pb_grid_dep_launch();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.y, g = h / (H / G);
     const float rate = expf(a_log[h]), bias = dt_bias[h];       // written by no kernel: before the wait
     pb_grid_dep_wait();
-    int seq, chunk;
-    if (!dc_find(cu_q, n_seqs, blockIdx.x, lane, seq, chunk)) return;
-    const int t_first = cu_q[seq] + chunk * DC_L, cnt = min(DC_L, cu_q[seq + 1] - t_first);
+    int t_first = 0;
+    if (beside > 0) least = pb_length_limit(cu_q, n_seqs, least, few, beside, lane);
+    const int cnt = pb_find_chunk<DC_L>(cu_q, n_seqs, least, blockIdx.x, lane, t_first);
+    if (cnt <= 0) return;
     bf16* ks = reinterpret_cast<bf16*>(dp_sm + Z::k);
     bf16* qs = reinterpret_cast<bf16*>(dp_sm + Z::q);
     float* A = reinterpret_cast<float*>(dp_sm + Z::a);
@@ -323,23 +293,17 @@ __device__ __forceinline__ void dc_mma6(float (&big)[4], float (&small)[4], cons
 // eight make U (a row tile and half of the columns each); then warps 4-7 finish the outputs and warps 0-3 the state, which lives in
 // their registers from chunk to chunk.
 template <int D, int PB>
-__global__ void __launch_bounds__(DC_ALL, 1)
-delta_walk_kernel(const bf16* u, long long ld_u, const unsigned char* blobs, float* state, float* y, const int32_t* cu_q, const int32_t* slots, int H,
-                  int G, int E) {
+__device__ __forceinline__ void dc_sequence(unsigned char* dw_sm, const bf16* u, long long ld_u, const unsigned char* blobs, float* state, float* y, const int32_t* cu_q,
+                                            int seq, int least, int slot, int h, int p_first, int H, int G, int E) {
     using Z = DcLayout<D, PB>;
-    extern __shared__ __align__(16) unsigned char dw_sm[];
-    pb_grid_dep_launch();
-    const int slices = E / PB;
-    const int h = blockIdx.x / slices, p_first = (blockIdx.x % slices) * PB, g = h / (H / G);
+    const int g = h / (H / G);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    pb_grid_dep_wait();
-    const int first = cu_q[blockIdx.y], n_tok = cu_q[blockIdx.y + 1] - first;
-    if (n_tok <= 0) return;
+    const int first = cu_q[seq], n_tok = cu_q[seq + 1] - first;
     const int n_chunks = (n_tok + DC_L - 1) / DC_L;
 
     if (tid >= DC_MUL) {
         const int pt = tid - DC_MUL;
-        const unsigned char* blob = blobs + ((size_t)dc_chunks_before(cu_q, blockIdx.y, lane) * H + h) * DC_BLOB;
+        const unsigned char* blob = blobs + ((size_t)pb_chunks_before<DC_L>(cu_q, seq, least, lane) * H + h) * DC_BLOB;
         auto fetch = [&](int ch) {
             unsigned char* buf = dw_sm + (ch & 1) * Z::half;
             const int t0 = ch * DC_L, cnt = min(DC_L, n_tok - t0);
@@ -385,7 +349,7 @@ delta_walk_kernel(const bf16* u, long long ld_u, const unsigned char* blobs, flo
     bf16* ws = reinterpret_cast<bf16*>(dw_sm + Z::w);
     int* bads = reinterpret_cast<int*>(dw_sm + Z::bad);
     const int n0 = ST * 16 * warp;                              // warps 0-3: first row of the state
-    float* S = state + (((size_t)slots[blockIdx.y] * H + h) * D + n0 + r0) * E + p_first + c0;
+    float* S = state + (((size_t)slot * H + h) * D + n0 + r0) * E + p_first + c0;
     float st[ST][PT][4];
 #pragma unroll
     for (int a = 0; a < ST; ++a)
@@ -593,30 +557,55 @@ delta_walk_kernel(const bf16* u, long long ld_u, const unsigned char* blobs, flo
     }
 }
 
-template <int D, int PB>
-int dc_walk(const void* u, long long ld_u, const void* scratch, float* state, float* y, const int32_t* cu_q, const int32_t* slots, int n_seqs, int H, int G,
-            int E, cudaStream_t stream) {
+template <int D, int PB, bool RECORDED>
+__global__ void __launch_bounds__(DC_ALL, 1)
+delta_walk_kernel(const bf16* u, long long ld_u, const unsigned char* blobs, float* state, float* y, const int32_t* cu_q, const int32_t* slots, PbSequences which,
+                  int H, int G, int E) {
+    extern __shared__ __align__(16) unsigned char dw_sm[];
+    pb_grid_dep_launch();
+    const int slices = E / PB;
+    const int h = blockIdx.x / slices, p_first = (blockIdx.x % slices) * PB;
+    pb_grid_dep_wait();
+    pb_for_sequences<RECORDED>(cu_q, which, [&](int seq, int least) {
+        dc_sequence<D, PB>(dw_sm, u, ld_u, blobs, state, y, cu_q, seq, least, slots[seq], h, p_first, H, G, E);
+    });
+}
+
+struct DcCall {
+    const void *u, *b, *a;
+    long long ld_u, ld_b, ld_a;
+    const float *a_log, *dt_bias;
+    float *state, *y;
+    const int32_t *cu_q, *slots;
+    void* scratch;
+    int n_chunks, n_long, counted, H, G, E;
+    PbSequences all;
+    cudaStream_t stream;
+};
+
+template <int D, int PB, bool RECORDED>
+int dc_walk(const DcCall& c, int rows, const PbSequences& which) {
     constexpr int bytes = DcLayout<D, PB>::bytes;
-    static const cudaError_t set = cudaFuncSetAttribute(delta_walk_kernel<D, PB>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    static const cudaError_t set = cudaFuncSetAttribute(delta_walk_kernel<D, PB, RECORDED>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     PB_REQUIRE(set == cudaSuccess, "gated_delta_scan_chunked: %s", cudaGetErrorString(set));
-    pb_launch(delta_walk_kernel<D, PB>, dim3(H * (E / PB), n_seqs), dim3(DC_ALL), bytes, stream, (const bf16*)u, ld_u, (const unsigned char*)scratch, state, y,
-              cu_q, slots, H, G, E);
+    pb_launch(delta_walk_kernel<D, PB, RECORDED>, dim3(c.H * (c.E / PB), rows), dim3(DC_ALL), bytes, c.stream, (const bf16*)c.u, c.ld_u, (const unsigned char*)c.scratch,
+              c.state, c.y, c.cu_q, c.slots, which, c.H, c.G, c.E);
     PB_CHECK_LAUNCH("gated_delta_scan_chunked");
     return 0;
 }
 
 template <int D>
-int dc_run(const void* u, long long ld_u, const void* b_in, long long ld_b, const void* a_in, long long ld_a, const float* a_log, const float* dt_bias,
-           float* state, float* y, const int32_t* cu_q, const int32_t* slots, void* scratch, int n_chunks, int n_seqs, int H, int G, int E, int pb,
-           cudaStream_t stream) {
+int dc_run(const DcCall& c) {
     constexpr int bytes = DcPrep<D>::bytes;
     static const cudaError_t set = cudaFuncSetAttribute(delta_prepare_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     PB_REQUIRE(set == cudaSuccess, "gated_delta_scan_chunked: %s", cudaGetErrorString(set));
-    pb_launch(delta_prepare_kernel<D>, dim3(n_chunks, H), dim3(256), bytes, stream, (const bf16*)u, ld_u, (const bf16*)b_in, ld_b, (const bf16*)a_in, ld_a,
-              a_log, dt_bias, cu_q, (unsigned char*)scratch, n_seqs, H, G);
+    pb_launch(delta_prepare_kernel<D>, dim3(c.n_chunks, c.H), dim3(256), bytes, c.stream, (const bf16*)c.u, c.ld_u, (const bf16*)c.b, c.ld_b, (const bf16*)c.a,
+              c.ld_a, c.a_log, c.dt_bias, c.cu_q, (unsigned char*)c.scratch, c.all.n_seqs, c.all.from, c.all.few, c.all.beside, c.H, c.G);
     PB_CHECK_LAUNCH("gated_delta_scan_chunked");
-    if (pb == 32) return dc_walk<D, 32>(u, ld_u, scratch, state, y, cu_q, slots, n_seqs, H, G, E, stream);
-    return dc_walk<D, 16>(u, ld_u, scratch, state, y, cu_q, slots, n_seqs, H, G, E, stream);
+    return pb_for_widths(c.H, c.E, 16, 32, c.all, c.n_long, c.counted, [&](int width, int rows, const PbSequences& which) {
+        if (which.recorded) return width == 32 ? dc_walk<D, 32, true>(c, rows, which) : dc_walk<D, 16, true>(c, rows, which);
+        return width == 32 ? dc_walk<D, 32, false>(c, rows, which) : dc_walk<D, 16, false>(c, rows, which);
+    });
 }
 
 }  // namespace
@@ -629,24 +618,23 @@ PB_API int pb_gated_delta_chunked_takes(const void* u, long long ld_u, const flo
                ? 1
                : 0;
 }
-// Most chunks that n_tokens of n_seqs sequences can form, and the scratch memory (16-byte aligned) that the call needs for them.
-PB_API int pb_gated_delta_chunks(int n_tokens, int n_seqs) { return n_tokens / DC_L + (n_seqs < n_tokens ? n_seqs : n_tokens); }
+// Most chunks that n_tokens of n_long sequences can form, and the scratch memory (16-byte aligned) that the call needs for them.
+PB_API int pb_gated_delta_chunks(int n_tokens, int n_long) { return n_tokens / DC_L + (n_long < n_tokens ? n_long : n_tokens); }
 PB_API long long pb_gated_delta_chunk_bytes(int n_chunks, int H) { return (long long)n_chunks * H * DC_BLOB; }
 
-// Operands as for pb_gated_delta_scan, bfloat16; n_chunks and scratch as the two functions above say.  A block of the walk takes
-// 32 columns of a head's state where that still gives four fifths of the multiprocessors a block, else 16.
+// Operands as for pb_gated_delta_scan, bfloat16, for the sequences of at least `least` tokens; pb_gated_delta_scan with `below` = least
+// does the others.  n_chunks and scratch as the two functions above say; n_long: how many such sequences there are (`counted`), or the
+// most there can be, for a step that is being recorded (few, beside: sequences.cuh).
 PB_API int pb_gated_delta_scan_chunked(const void* u, long long ld_u, const void* b_in, long long ld_b, const void* a_in, long long ld_a, const float* a_log,
                                        const float* dt_bias, float* state, float* y, const int32_t* cu_q, const int32_t* slots, void* scratch, int n_chunks,
-                                       int n_seqs, int H, int G, int D, int E, cudaStream_t stream) {
+                                       int n_seqs, int least, int few, int beside, int n_long, int counted, int H, int G, int D, int E, cudaStream_t stream) {
     PB_REQUIRE(n_seqs >= 0 && n_chunks >= 0 && pb_gated_delta_chunked_takes(u, ld_u, state, y, H, G, D, E), "gated_delta_scan_chunked: %d over %d heads of %d, %d", H, G, D, E);
     PB_REQUIRE(u && b_in && a_in && a_log && dt_bias && state && y && cu_q && slots && scratch, "gated_delta_scan_chunked: null pointer");
     PB_REQUIRE(ld_u >= 2ll * G * D + (long long)H * E && ld_b >= H && ld_a >= H, "gated_delta_scan_chunked: rows too short");
     PB_REQUIRE(pb_aligned(scratch, 16), "gated_delta_scan_chunked: misaligned operands");
-    if (n_seqs == 0 || n_chunks == 0) return 0;
-    PB_REQUIRE(n_seqs < 65536, "gated_delta_scan_chunked: %d sequences in one launch", n_seqs);
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
-    const int pb = E % 32 == 0 && (long long)H * n_seqs * (E / 32) >= sms - sms / 5 ? 32 : 16;
-    if (D == 128) return dc_run<128>(u, ld_u, b_in, ld_b, a_in, ld_a, a_log, dt_bias, state, y, cu_q, slots, scratch, n_chunks, n_seqs, H, G, E, pb, stream);
-    return dc_run<64>(u, ld_u, b_in, ld_b, a_in, ld_a, a_log, dt_bias, state, y, cu_q, slots, scratch, n_chunks, n_seqs, H, G, E, pb, stream);
+    PB_REQUIRE(least > 0 && n_long >= 0 && n_long <= n_seqs && n_long < 65536, "gated_delta_scan_chunked: %d of %d sequences in one launch", n_long, n_seqs);
+    if (n_long == 0 || n_chunks == 0) return 0;
+    const DcCall c{u, b_in, a_in, ld_u, ld_b, ld_a, a_log, dt_bias, state, y, cu_q, slots, scratch, n_chunks, n_long, counted, H, G, E,
+                   PbSequences{n_seqs, least, INT_MAX, few, beside, 0, 0, 0, 0}, stream};
+    return D == 128 ? dc_run<128>(c) : dc_run<64>(c);
 }

@@ -23,6 +23,7 @@
 // 0.01 - 2.0e-7 in the state (token by token 0.6 - 2.5e-7 and 0.01 - 2.6e-7).  The walk issues in 46 % of the cycles, the tensor units work in
 // 30 %: the rest is the fixed latencies of its chain.
 #include "mma_sync.cuh"
+#include "sequences.cuh"
 
 namespace {
 
@@ -38,38 +39,6 @@ template <int N>
 struct GcBlob {
     static constexpr int q = 0, k = N / 16 * 3 * 512, w = 2 * k, d = w + 3 * 512, bytes = d + N * 4;
 };
-
-// Sixteens of the sequences before `seq`; a warp together.
-__device__ __forceinline__ int gc_before(const int32_t* cu_q, int seq, int lane) {
-    int n = 0;
-    for (int r = lane; r < seq; r += 32) n += max(0, (cu_q[r + 1] - cu_q[r] + GC_L - 1) / GC_L);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
-    return n;
-}
-// First token of the sixteen that number `slot` of all is, and how many tokens it has (0: there is none); a warp together.
-__device__ __forceinline__ int gc_find(const int32_t* cu_q, int n_seqs, int slot, int lane, int& first) {
-    int base = 0;
-    for (int r0 = 0; r0 < n_seqs; r0 += 32) {
-        const int r = r0 + lane;
-        const int n = r < n_seqs ? max(0, (cu_q[r + 1] - cu_q[r] + GC_L - 1) / GC_L) : 0;
-        int upto = n;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, upto, o);
-            if (lane >= o) upto += v;
-        }
-        const unsigned hit = __ballot_sync(0xffffffffu, base + upto > slot);
-        if (hit) {
-            const int at = __ffs(hit) - 1, seq = r0 + at;
-            const int step = slot - base - (__shfl_sync(0xffffffffu, upto, at) - __shfl_sync(0xffffffffu, n, at));
-            first = cu_q[seq] + step * GC_L;
-            return min(GC_L, cu_q[seq + 1] - first);
-        }
-        base += __shfl_sync(0xffffffffu, upto, 31);
-    }
-    return 0;
-}
 
 // Sum over the lanes of sixteen numbers a lane: every exchange halves the numbers a lane still holds.  Lane l ends with number
 // (bit 4, bit 3, bit 2, bit 1 of l).
@@ -104,7 +73,7 @@ gla_prepare_kernel(const bf16* q_in, const bf16* k_in, long long ld, const float
     const bool operands = warp & 1;
     pb_grid_dep_wait();
     int first = 0;
-    const int cnt = slot < n_steps ? gc_find(cu_q, n_seqs, slot, lane, first) : 0;      // the same for both warps
+    const int cnt = slot < n_steps ? pb_find_chunk<GC_L>(cu_q, n_seqs, 1, slot, lane, first) : 0;      // the same for both warps
     unsigned char* rows = gw_sm + at * Z::slot;
     // all rows at once by way of shared memory: as loads into registers they are put off until a token wants its own, one trip to
     // memory each.  The two warps fetch half of them each.
@@ -261,25 +230,18 @@ __device__ __forceinline__ void gc_mma6(float (&big)[4], float (&small)[4], cons
 // before and bring what the first kernel left of the next one, and its v, and what is three sixteens ahead on its way, into shared memory.  One barrier a
 // sixteen.
 template <int N, int PB>
-__global__ void __launch_bounds__(GC_ALL, 1)
-gla_walk_kernel(const bf16* v_in, long long ld, float scale, const unsigned char* blobs,
-                float* state, float* y, const int32_t* cu_q, const int32_t* slots, int H, int P) {
+__device__ __forceinline__ void gc_sequence(unsigned char* gc_sm, const bf16* v_in, long long ld, float scale, const unsigned char* blobs, float* state, float* y,
+                                            const int32_t* cu_q, int seq, int slot, int h, int p_first, int H, int P) {
     using Z = GcLayout<N, PB>;
-    extern __shared__ __align__(16) unsigned char gc_sm[];
-    pb_grid_dep_launch();
-    const int slices = P / PB;
-    const int h = blockIdx.x / slices, p_first = (blockIdx.x % slices) * PB;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    pb_grid_dep_wait();
-    const int first = cu_q[blockIdx.y], n_tok = cu_q[blockIdx.y + 1] - first;
-    if (n_tok <= 0) return;
+    const int first = cu_q[seq], n_tok = cu_q[seq + 1] - first;
     const int n_steps = (n_tok + GC_L - 1) / GC_L;
     int* bads = reinterpret_cast<int*>(gc_sm + Z::bad);         // of four sixteens: the first token whose v is not finite, per column
 
     if (tid >= GC_MUL) {
         constexpr int FETCH = GC_ALL - GC_MUL;
         const int pt = tid - GC_MUL;
-        const unsigned char* blob = blobs + ((size_t)gc_before(cu_q, blockIdx.y, lane) * H + h) * GcBlob<N>::bytes;
+        const unsigned char* blob = blobs + ((size_t)pb_chunks_before<GC_L>(cu_q, seq, 1, lane) * H + h) * GcBlob<N>::bytes;
         constexpr int VP = PB / 8, V_IT = (GC_L * VP + FETCH - 1) / FETCH;
         uint4 vr[V_IT];
         auto ask = [&](int s) {                                 // v two sixteens ahead, in registers: nothing here may wait for it
@@ -364,7 +326,7 @@ gla_walk_kernel(const bf16* v_in, long long ld, float scale, const unsigned char
     static_assert(PT >= 1, "16 columns a warp at least");
     const int nw = warp % NW, pg = warp / NW;
     const int r0 = lane >> 2, c0 = (lane & 3) * 2;
-    float* S = state + (((size_t)slots[blockIdx.y] * H + h) * N + nw * 16 + c0) * P + p_first + pg * PW + r0;
+    float* S = state + (((size_t)slot * H + h) * N + nw * 16 + c0) * P + p_first + pg * PW + r0;
     float st[PT][2][4];                                         // [16 columns p][8 channels]: rows p = r0, r0 + 8, channels c0, c0 + 1
 #pragma unroll
     for (int a = 0; a < PT; ++a)
@@ -465,6 +427,20 @@ gla_walk_kernel(const bf16* v_in, long long ld, float scale, const unsigned char
             for (int e = 0; e < 4; ++e) S[(size_t)(8 * v + (e & 1)) * P + 16 * a + (e >> 1) * 8] = st[a][v][e];
 }
 
+template <int N, int PB, bool RECORDED>
+__global__ void __launch_bounds__(GC_ALL, 1)
+gla_walk_kernel(const bf16* v_in, long long ld, float scale, const unsigned char* blobs, float* state, float* y, const int32_t* cu_q, const int32_t* slots,
+                PbSequences which, int H, int P) {
+    extern __shared__ __align__(16) unsigned char gc_sm[];
+    pb_grid_dep_launch();
+    const int slices = P / PB;
+    const int h = blockIdx.x / slices, p_first = (blockIdx.x % slices) * PB;
+    pb_grid_dep_wait();
+    pb_for_sequences<RECORDED>(cu_q, which, [&](int seq, int) {
+        gc_sequence<N, PB>(gc_sm, v_in, ld, scale, blobs, state, y, cu_q, seq, slots[seq], h, p_first, H, P);
+    });
+}
+
 struct GcCall {
     const bf16 *q, *k, *v;
     long long ld;
@@ -473,22 +449,35 @@ struct GcCall {
     float *state, *y;
     const int32_t *cu_q, *slots;
     unsigned char* scratch;
-    int n_steps, n_seqs, H, P;
+    int n_steps, n_seqs, most, counted, H, P;
     cudaStream_t stream;
 };
 
-template <int N, int PB>
-int gc_run(const GcCall& c) {
+template <int N, int PB, bool RECORDED>
+int gc_walk(const GcCall& c, int rows, const PbSequences& which) {
     constexpr int bytes = GcLayout<N, PB>::bytes;
-    static const cudaError_t set = cudaFuncSetAttribute(gla_walk_kernel<N, PB>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    static const cudaError_t set = cudaFuncSetAttribute(gla_walk_kernel<N, PB, RECORDED>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     PB_REQUIRE(set == cudaSuccess, "gla_scan_chunked: %s", cudaGetErrorString(set));
-    static const cudaError_t set_w = cudaFuncSetAttribute(gla_prepare_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, GcRows<N>::bytes);
-    PB_REQUIRE(set_w == cudaSuccess, "gla_scan_chunked: %s", cudaGetErrorString(set_w));
-    pb_launch(gla_prepare_kernel<N>, dim3((c.n_steps + GP_SLOTS - 1) / GP_SLOTS, c.H), dim3(64 * GP_SLOTS), GcRows<N>::bytes, c.stream, c.q, c.k, c.ld, c.decay, c.cu_q, c.scratch, c.n_steps, c.n_seqs, c.H);
-    PB_CHECK_LAUNCH("gla_scan_chunked");
-    pb_launch(gla_walk_kernel<N, PB>, dim3(c.H * (c.P / PB), c.n_seqs), dim3(GC_ALL), bytes, c.stream, c.v, c.ld, c.scale, (const unsigned char*)c.scratch, c.state, c.y, c.cu_q, c.slots, c.H, c.P);
+    pb_launch(gla_walk_kernel<N, PB, RECORDED>, dim3(c.H * (c.P / PB), rows), dim3(GC_ALL), bytes, c.stream, c.v, c.ld, c.scale, (const unsigned char*)c.scratch, c.state, c.y,
+              c.cu_q, c.slots, which, c.H, c.P);
     PB_CHECK_LAUNCH("gla_scan_chunked");
     return 0;
+}
+
+template <int N>
+int gc_run(const GcCall& c) {
+    static const cudaError_t set = cudaFuncSetAttribute(gla_prepare_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, GcRows<N>::bytes);
+    PB_REQUIRE(set == cudaSuccess, "gla_scan_chunked: %s", cudaGetErrorString(set));
+    pb_launch(gla_prepare_kernel<N>, dim3((c.n_steps + GP_SLOTS - 1) / GP_SLOTS, c.H), dim3(64 * GP_SLOTS), GcRows<N>::bytes, c.stream, c.q, c.k, c.ld, c.decay, c.cu_q,
+              c.scratch, c.n_steps, c.n_seqs, c.H);
+    PB_CHECK_LAUNCH("gla_scan_chunked");
+    // 64 channels: always two column groups of 16
+    const PbSequences all{c.n_seqs, 1, INT_MAX, 0, 0, 0, 0, 0, 0};
+    return pb_for_widths(c.H, c.P, N == 64 ? 32 : 16, 32, all, c.most, c.counted, [&](int width, int rows, const PbSequences& which) {
+        if constexpr (N == 64) return which.recorded ? gc_walk<64, 32, true>(c, rows, which) : gc_walk<64, 32, false>(c, rows, which);
+        else if (which.recorded) return width == 32 ? gc_walk<128, 32, true>(c, rows, which) : gc_walk<128, 16, true>(c, rows, which);
+        else return width == 32 ? gc_walk<128, 32, false>(c, rows, which) : gc_walk<128, 16, false>(c, rows, which);
+    });
 }
 
 }  // namespace
@@ -505,21 +494,17 @@ PB_API int pb_gla_chunked_takes(const void* q, const void* k, const void* v, con
 PB_API int pb_gla_chunks(int n_tokens, int n_seqs) { return n_tokens / GC_L + (n_seqs < n_tokens ? n_seqs : n_tokens); }
 PB_API long long pb_gla_chunk_bytes(int n_steps, int H, int N) { return (long long)n_steps * H * (N == 64 ? GcBlob<64>::bytes : GcBlob<128>::bytes); }
 
-// Operands as for pb_gla_scan, bfloat16; n_steps and scratch as the two functions above say.  A block of the walk takes 32 columns of a
-// head's state where that still gives four fifths of the multiprocessors a block (or the warps need two column groups), else 16.
+// Operands as for pb_gla_scan, bfloat16; n_steps and scratch as the two functions above say.  most: how many sequences there are
+// (`counted`), or can be, for a step that is being recorded.
 PB_API int pb_gla_scan_chunked(const void* q, const void* k, const void* v, long long ld, const float* decay, float scale, float* state, float* y,
-                               const int32_t* cu_q, const int32_t* slots, void* scratch, int n_steps, int n_seqs, int H, int N, int P, cudaStream_t stream) {
+                               const int32_t* cu_q, const int32_t* slots, void* scratch, int n_steps, int n_seqs, int most, int counted, int H, int N, int P,
+                               cudaStream_t stream) {
     PB_REQUIRE(n_seqs >= 0 && n_steps >= 0 && pb_gla_chunked_takes(q, k, v, decay, y, ld, H, N, P), "gla_scan_chunked: %d heads of %d x %d", H, N, P);
     PB_REQUIRE(q && k && v && decay && state && y && cu_q && slots && scratch, "gla_scan_chunked: null pointer");
     PB_REQUIRE(pb_aligned(scratch, 16), "gla_scan_chunked: misaligned operands");
-    if (n_seqs == 0 || n_steps == 0) return 0;
-    PB_REQUIRE(n_seqs < 65536, "gla_scan_chunked: %d sequences in one launch", n_seqs);
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
-    const long long states = (long long)H * n_seqs;
-    const int fill = sms - sms / 5;
-    const int pb = N == 64 || (P % 32 == 0 && states * (P / 32) >= fill) ? 32 : 16;
-    const GcCall c{(const bf16*)q, (const bf16*)k, (const bf16*)v, ld, decay, scale, state, y, cu_q, slots, (unsigned char*)scratch, n_steps, n_seqs, H, P, stream};
-    if (N == 128) return pb == 32 ? gc_run<128, 32>(c) : gc_run<128, 16>(c);
-    return gc_run<64, 32>(c);
+    PB_REQUIRE(most >= 0 && most <= n_seqs && most < 65536, "gla_scan_chunked: %d of %d sequences in one launch", most, n_seqs);
+    if (most == 0 || n_steps == 0) return 0;
+    const GcCall c{(const bf16*)q, (const bf16*)k, (const bf16*)v, ld, decay, scale, state, y, cu_q, slots, (unsigned char*)scratch, n_steps, n_seqs, most,
+                   counted, H, P, stream};
+    return N == 128 ? gc_run<128>(c) : gc_run<64>(c);
 }

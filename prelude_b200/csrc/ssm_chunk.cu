@@ -23,6 +23,7 @@
 // f and f + 2 of x (what lies above the diagonal is skipped; tiles i are dealt to the schedulers long with short); the two halves
 // are added through shared memory.  For the state warp w owns rows 16 w .. 16 w + 15, in registers from chunk to chunk.
 #include "mma_sync.cuh"
+#include "sequences.cuh"
 
 #include <math.h>
 
@@ -44,20 +45,12 @@ struct ScLayout {
 
 __device__ __forceinline__ float sc_softplus(float v) { return v > 20.0f ? v : log1pf(expf(v)); }
 
+// One sequence's tokens through one head's columns p_first ..; all threads of the block.
 template <int N, int PB>
-__global__ void __launch_bounds__(SC_ALL, 1)
-ssm_chunk_kernel(const bf16* u, const bf16* dt_in, long long ld_dt, const float* dt_bias, const float* a_log, const float* d_skip, float* state,
-                 float* y, const int32_t* cu_q, const int32_t* slots, int heads, int P, int groups) {
+__device__ __forceinline__ void sc_sequence(unsigned char* sc_sm, const bf16* u, const bf16* dt_in, long long ld_dt, float neg_a, float bias, float skip, float* state,
+                                            float* y, int first, int n_tok, int slot, int h, int p_first, int heads, int P, int groups) {
     using Z = ScLayout<N, PB>;
-    extern __shared__ __align__(16) unsigned char sc_sm[];
-    pb_grid_dep_launch();
-    const int slices = P / PB;
-    const int h = blockIdx.x / slices, p_first = (blockIdx.x % slices) * PB;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const float neg_a = -expf(a_log[h]), bias = dt_bias[h], skip = d_skip[h];     // written by no kernel: before the wait
-    pb_grid_dep_wait();
-    const int first = cu_q[blockIdx.y], n_tok = cu_q[blockIdx.y + 1] - first;
-    if (n_tok <= 0) return;
     const int inner = heads * P, channels = inner + 2 * groups * N;
     const int g = h / (heads / groups);
     const int n_chunks = (n_tok + SC_L - 1) / SC_L;
@@ -170,7 +163,7 @@ ssm_chunk_kernel(const bf16* u, const bf16* dt_in, long long ld_dt, const float*
     const bool owns = warp < NK;                                                   // rows 16 warp .. + 15 of the state
     bf16* ss = reinterpret_cast<bf16*>(sc_sm + Z::s);
     float* yx = reinterpret_cast<float*>(sc_sm + Z::yx);
-    float* S = state + (((size_t)slots[blockIdx.y] * heads + h) * N + warp * 16 + r0) * P + p_first + c0;
+    float* S = state + (((size_t)slot * heads + h) * N + warp * 16 + r0) * P + p_first + c0;
     float st[PT][4];
 #pragma unroll
     for (int q = 0; q < PT; ++q) {
@@ -348,14 +341,30 @@ ssm_chunk_kernel(const bf16* u, const bf16* dt_in, long long ld_dt, const float*
     }
 }
 
-template <int N, int PB>
+template <int N, int PB, bool RECORDED>
+__global__ void __launch_bounds__(SC_ALL, 1)
+ssm_chunk_kernel(const bf16* u, const bf16* dt_in, long long ld_dt, const float* dt_bias, const float* a_log, const float* d_skip, float* state,
+                 float* y, const int32_t* cu_q, const int32_t* slots, PbSequences which, int heads, int P, int groups) {
+    extern __shared__ __align__(16) unsigned char sc_sm[];
+    pb_grid_dep_launch();
+    const int slices = P / PB;
+    const int h = blockIdx.x / slices, p_first = (blockIdx.x % slices) * PB;
+    const float neg_a = -expf(a_log[h]), bias = dt_bias[h], skip = d_skip[h];     // written by no kernel: before the wait
+    pb_grid_dep_wait();
+    pb_for_sequences<RECORDED>(cu_q, which, [&](int seq, int) {
+        const int first = cu_q[seq];
+        sc_sequence<N, PB>(sc_sm, u, dt_in, ld_dt, neg_a, bias, skip, state, y, first, cu_q[seq + 1] - first, slots[seq], h, p_first, heads, P, groups);
+    });
+}
+
+template <int N, int PB, bool RECORDED>
 int sc_launch(const void* u, const void* dt_in, long long ld_dt, const float* dt_bias, const float* a_log, const float* d_skip, float* state, float* y,
-              const int32_t* cu_q, const int32_t* slots, int n_seqs, int heads, int P, int groups, cudaStream_t stream) {
+              const int32_t* cu_q, const int32_t* slots, const PbSequences& which, int rows, int heads, int P, int groups, cudaStream_t stream) {
     constexpr int bytes = ScLayout<N, PB>::bytes;
-    static const cudaError_t set = cudaFuncSetAttribute(ssm_chunk_kernel<N, PB>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    static const cudaError_t set = cudaFuncSetAttribute(ssm_chunk_kernel<N, PB, RECORDED>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     PB_REQUIRE(set == cudaSuccess, "ssm_scan_chunked: %s", cudaGetErrorString(set));
-    pb_launch(ssm_chunk_kernel<N, PB>, dim3(heads * (P / PB), n_seqs), dim3(SC_ALL), bytes, stream, (const bf16*)u, (const bf16*)dt_in, ld_dt, dt_bias,
-              a_log, d_skip, state, y, cu_q, slots, heads, P, groups);
+    pb_launch(ssm_chunk_kernel<N, PB, RECORDED>, dim3(heads * (P / PB), rows), dim3(SC_ALL), bytes, stream, (const bf16*)u, (const bf16*)dt_in, ld_dt, dt_bias,
+              a_log, d_skip, state, y, cu_q, slots, which, heads, P, groups);
     PB_CHECK_LAUNCH("ssm_scan_chunked");
     return 0;
 }
@@ -371,27 +380,37 @@ PB_API int pb_ssm_scan_chunked_takes(const void* u, const float* state, const fl
                : 0;
 }
 
-// Operands as for pb_ssm_scan, bfloat16.  A block takes 64, 32 or 16 columns of a head's state, the most that still gives four
-// fifths of the multiprocessors a block: more columns share C B^T and the operand loads, fewer leave a shorter chunk.
+// Operands as for pb_ssm_scan, bfloat16, for the sequences of at least `least` tokens; pb_ssm_step does those of one.  n_long: how many
+// there are (`counted`), or the most there can be, for a step that is being recorded (few, beside: sequences.cuh).
 PB_API int pb_ssm_scan_chunked(const void* u, const void* dt_in, long long ld_dt, const float* dt_bias, const float* a_log, const float* d_skip,
-                               float* state, float* y, const int32_t* cu_q, const int32_t* slots, int n_seqs, int heads, int P, int N, int groups,
-                               cudaStream_t stream) {
+                               float* state, float* y, const int32_t* cu_q, const int32_t* slots, int n_seqs, int least, int few, int beside, int n_long, int counted,
+                               int heads, int P, int N, int groups, cudaStream_t stream) {
     PB_REQUIRE(n_seqs >= 0 && pb_ssm_scan_chunked_takes(u, state, y, heads, P, N, groups), "ssm_scan_chunked: %d heads of %d, state %d, %d groups", heads, P, N, groups);
     PB_REQUIRE(u && dt_in && dt_bias && a_log && d_skip && state && y && cu_q && slots && ld_dt >= heads, "ssm_scan_chunked: null pointer");
-    if (n_seqs == 0) return 0;
-    PB_REQUIRE(n_seqs < 65536, "ssm_scan_chunked: %d sequences in one launch", n_seqs);
-    const long long states = (long long)heads * n_seqs;
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
-    const int fill = sms - sms / 5;
-    const int pb = P % 64 == 0 && states * (P / 64) >= fill ? 64 : P % 32 == 0 && states * (P / 32) >= fill ? 32 : 16;
-#define SC_CASE(NN, PP) if (N == NN && pb == PP) return sc_launch<NN, PP>(u, dt_in, ld_dt, dt_bias, a_log, d_skip, state, y, cu_q, slots, n_seqs, heads, P, groups, stream)
-    SC_CASE(128, 64);
-    SC_CASE(128, 32);
-    SC_CASE(128, 16);
-    SC_CASE(64, 64);
-    SC_CASE(64, 32);
-    SC_CASE(64, 16);
+    PB_REQUIRE(least > 0 && n_long >= 0 && n_long <= n_seqs && n_long < 65536, "ssm_scan_chunked: %d of %d sequences in one launch", n_long, n_seqs);
+    const PbSequences all{n_seqs, least, INT_MAX, few, beside, 0, 0, 0, 0};
+    return pb_for_widths(heads, P, 16, 64, all, n_long, counted, [&](int width, int rows, const PbSequences& which) {
+#define SC_ARGS u, dt_in, ld_dt, dt_bias, a_log, d_skip, state, y, cu_q, slots, which, rows, heads, P, groups, stream
+#define SC_CASE(NN, PP) if (N == NN && width == PP) return which.recorded ? sc_launch<NN, PP, true>(SC_ARGS) : sc_launch<NN, PP, false>(SC_ARGS)
+        SC_CASE(128, 64);
+        SC_CASE(128, 32);
+        SC_CASE(128, 16);
+        SC_CASE(64, 64);
+        SC_CASE(64, 32);
+        SC_CASE(64, 16);
 #undef SC_CASE
-    return pb_fail("ssm_scan_chunked: state %d", N);
+#undef SC_ARGS
+        return pb_fail("ssm_scan_chunked: state %d", N);
+    });
+}
+
+// For tests: the launches that pb_for_widths makes of a walk, four numbers each - width, rows, lo, hi; how many there are.
+PB_API int pb_walk_launches(int heads, int cols, int narrowest, int widest, int n_long, int counted, int* out) {
+    int n = 0;
+    pb_for_widths(heads, cols, narrowest, widest, PbSequences{n_long, 1, INT_MAX, 0, 0, 0, 0, 0, 0}, n_long, counted, [&](int width, int rows, const PbSequences& which) {
+        int* o = out + 4 * n++;
+        o[0] = width; o[1] = rows; o[2] = which.lo; o[3] = which.hi;
+        return 0;
+    });
+    return n;
 }

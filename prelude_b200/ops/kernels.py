@@ -7,7 +7,7 @@ is missing the call raises.
 """
 from __future__ import annotations
 
-from typing import Optional
+from typing import NamedTuple, Optional
 
 import torch
 
@@ -1055,6 +1055,21 @@ DELTA_CHUNKED_MIN_TOKENS = 64
 GLA_CHUNKED_MIN_TOKENS = 256
 
 
+class _Split(NamedTuple):
+    """A step whose sequences run by chunks."""
+    n_long: int       # how many there are (``counted``), or can be
+    counted: bool     # False: a step that is being recorded, which is replayed for other lengths
+
+
+def _split(batch, T: int, min_tokens: int) -> Optional[_Split]:
+    """The sequences of a step of T tokens, which run by chunks from ``min_tokens`` on.  None: nothing runs by chunks."""
+    if batch.decode_only or T < min_tokens:
+        return None
+    n_seqs = batch.cu_q.numel() - 1
+    counted = batch.extras.get("recorder") is None and batch.q_lens.shape[0] == n_seqs
+    return _Split(n_seqs if counted else min(n_seqs, T), counted)
+
+
 def ssm_scan(u: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: torch.Tensor, d_skip: torch.Tensor,
              state: torch.Tensor, batch, groups: int, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """The recurrence over the step's tokens, sequence by sequence; u [T, heads * P + 2 * groups * N] dense, dt [T, heads] a
@@ -1072,20 +1087,23 @@ def ssm_scan(u: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: to
     if out is None:
         out = torch.empty((T, heads * P), dtype=torch.float32, device=u.device)
     lib = _l.library()
-    if (u.dtype == torch.bfloat16 and T >= SCAN_CHUNKED_MIN_TOKENS and not batch.decode_only
-            and lib.pb_ssm_scan_chunked_takes(u.data_ptr(), state.data_ptr(), out.data_ptr(), heads, P, N, groups)):
+    n_seqs = batch.cu_q.numel() - 1
+    part = None
+    if u.dtype == torch.bfloat16 and lib.pb_ssm_scan_chunked_takes(u.data_ptr(), state.data_ptr(), out.data_ptr(), heads, P, N, groups):
+        part = _split(batch, T, SCAN_CHUNKED_MIN_TOKENS)
+    if part is not None:
         check(lib.pb_ssm_scan_chunked(u.data_ptr(), dt.data_ptr(), dt.stride(0), dt_bias.data_ptr(), a_log.data_ptr(), d_skip.data_ptr(),
-                                      state.data_ptr(), out.data_ptr(), batch.cu_q.data_ptr(), batch.state_slots.data_ptr(),
-                                      batch.cu_q.numel() - 1, heads, P, N, groups, _stream()), "ssm_scan_chunked")
+                                      state.data_ptr(), out.data_ptr(), batch.cu_q.data_ptr(), batch.state_slots.data_ptr(), n_seqs, 1, 0, 0,
+                                      part.n_long, part.counted, heads, P, N, groups, _stream()), "ssm_scan_chunked")
         return out
     if u.dtype == torch.bfloat16 and batch.decode_only and lib.pb_ssm_step_takes(u.data_ptr(), state.data_ptr(), heads, P, N, groups):
         check(lib.pb_ssm_step(u.data_ptr(), dt.data_ptr(), dt.stride(0), dt_bias.data_ptr(), a_log.data_ptr(), d_skip.data_ptr(), state.data_ptr(),
-                              out.data_ptr(), batch.cu_q.data_ptr(), batch.state_slots.data_ptr(), batch.cu_q.numel() - 1, heads, P, N, groups,
+                              out.data_ptr(), batch.cu_q.data_ptr(), batch.state_slots.data_ptr(), n_seqs, heads, P, N, groups,
                               _stream()), "ssm_step")
         return out
     check(lib.pb_ssm_scan(u.data_ptr(), dt.data_ptr(), dt.stride(0), dtype_code(u.dtype), dt_bias.data_ptr(), a_log.data_ptr(),
                                    d_skip.data_ptr(), state.data_ptr(), out.data_ptr(), batch.cu_q.data_ptr(),
-                                   batch.state_slots.data_ptr(), batch.cu_q.numel() - 1, heads, P, N, groups, _stream()), "ssm_scan")
+                                   batch.state_slots.data_ptr(), n_seqs, heads, P, N, groups, _stream()), "ssm_scan")
     return out
 
 
@@ -1310,16 +1328,17 @@ def gated_delta_scan(u: torch.Tensor, beta: torch.Tensor, a: torch.Tensor, a_log
         raise KernelLibraryError(f"gated_delta_scan: u {tuple(u.shape)}, state {tuple(state.shape)}, {kv_heads} query/key heads")
     if out is None:
         out = torch.empty((T, H * E), dtype=torch.float32, device=u.device)
-    lib, n_seqs = _l.library(), batch.cu_q.numel() - 1
-    if (u.dtype == torch.bfloat16 and T >= DELTA_CHUNKED_MIN_TOKENS and not batch.decode_only
-            and lib.pb_gated_delta_chunked_takes(u.data_ptr(), u.stride(0), state.data_ptr(), out.data_ptr(), H, kv_heads, D, E)):
+    lib, n_seqs, part = _l.library(), batch.cu_q.numel() - 1, None
+    if u.dtype == torch.bfloat16 and lib.pb_gated_delta_chunked_takes(u.data_ptr(), u.stride(0), state.data_ptr(), out.data_ptr(), H, kv_heads, D, E):
+        part = _split(batch, T, DELTA_CHUNKED_MIN_TOKENS)
+    if part is not None:
         # what one kernel makes of every chunk for the other to read: dead when the call's kernels are done
-        n_chunks = lib.pb_gated_delta_chunks(T, n_seqs)
+        n_chunks = lib.pb_gated_delta_chunks(T, part.n_long)
         scratch = torch.empty((lib.pb_gated_delta_chunk_bytes(n_chunks, H),), dtype=torch.uint8, device=u.device)
         check(lib.pb_gated_delta_scan_chunked(u.data_ptr(), u.stride(0), beta.data_ptr(), beta.stride(0), a.data_ptr(), a.stride(0),
                                               a_log.data_ptr(), dt_bias.data_ptr(), state.data_ptr(), out.data_ptr(), batch.cu_q.data_ptr(),
-                                              batch.state_slots.data_ptr(), scratch.data_ptr(), n_chunks, n_seqs, H, kv_heads, D, E,
-                                              _stream()), "gated_delta_scan_chunked")
+                                              batch.state_slots.data_ptr(), scratch.data_ptr(), n_chunks, n_seqs, 1, 0,
+                                              0, part.n_long, part.counted, H, kv_heads, D, E, _stream()), "gated_delta_scan_chunked")
         return out
     check(lib.pb_gated_delta_scan(u.data_ptr(), u.stride(0), beta.data_ptr(), beta.stride(0), a.data_ptr(), a.stride(0),
                                            dtype_code(u.dtype), a_log.data_ptr(), dt_bias.data_ptr(), state.data_ptr(), out.data_ptr(),
@@ -1410,15 +1429,16 @@ def gla_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Ten
         raise KernelLibraryError(f"gla_scan: decay {tuple(decay.shape)} for {T} tokens of {H * N} channels")
     if out is None:
         out = torch.empty((T, H * P), dtype=torch.float32, device=q.device)
-    lib, n_seqs = _l.library(), batch.cu_q.numel() - 1
-    if (q.dtype == torch.bfloat16 and T >= GLA_CHUNKED_MIN_TOKENS and not batch.decode_only
-            and lib.pb_gla_chunked_takes(q.data_ptr(), k.data_ptr(), v.data_ptr(), decay.data_ptr(), out.data_ptr(), q.stride(0), H, N, P)):
+    lib, n_seqs, part = _l.library(), batch.cu_q.numel() - 1, None
+    if q.dtype == torch.bfloat16 and lib.pb_gla_chunked_takes(q.data_ptr(), k.data_ptr(), v.data_ptr(), decay.data_ptr(), out.data_ptr(), q.stride(0), H, N, P):
+        part = _split(batch, T, GLA_CHUNKED_MIN_TOKENS)
+    if part is not None:
         # what one kernel makes of every sixteen for the other to read: dead when the call's kernels are done
-        n_steps = lib.pb_gla_chunks(T, n_seqs)
+        n_steps = lib.pb_gla_chunks(T, part.n_long)
         scratch = torch.empty((lib.pb_gla_chunk_bytes(n_steps, H, N),), dtype=torch.uint8, device=q.device)
         check(lib.pb_gla_scan_chunked(q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), decay.data_ptr(), float(scale), state.data_ptr(),
                                       out.data_ptr(), batch.cu_q.data_ptr(), batch.state_slots.data_ptr(), scratch.data_ptr(), n_steps, n_seqs,
-                                      H, N, P, _stream()), "gla_scan_chunked")
+                                      part.n_long, part.counted, H, N, P, _stream()), "gla_scan_chunked")
         return out
     check(lib.pb_gla_scan(q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), dtype_code(q.dtype), decay.data_ptr(), float(scale),
                                    state.data_ptr(), out.data_ptr(), batch.cu_q.data_ptr(), batch.state_slots.data_ptr(), n_seqs,

@@ -300,3 +300,44 @@ def test_state_and_result_anywhere(kind, odd_state, odd_result):
     got_s = at(tuple(state.shape), odd_state).copy_(state)
     got = run(got_s, at((sum(lens), width), odd_result))
     assert _rel(got, want.double()) < 1e-6 and _rel(got_s, want_s.double()) < 1e-6
+
+
+def _scan(kind, lens, H, seed=5):
+    """(A call (state, batch) -> result, the state it starts from) over sequences of these lengths."""
+    from prelude_b200.ops import kernels as K
+    if kind == "state space":
+        u, dt, bias, a_log, skip, state = _ssm_inputs(lens, H, 64, 64, 1, seed, 0.05)
+        return lambda s, b: K.ssm_scan(u, dt, bias, a_log, skip, s, b, 1), state
+    if kind == "gated delta rule":
+        u, b_, a, a_log, bias, state = _delta_inputs(lens, H, H, 64, 128, seed, 0.05)
+        return lambda s, b: K.gated_delta_scan(u, b_, a, a_log, bias, s, b, H), state
+    q, k, v, decay, state = _gla_inputs(lens, H, 128, 128, seed, 0.9, 1.0)
+    return lambda s, b: K.gla_scan(q, k, v, decay, 1.0, s, b), state
+
+
+KINDS = ["state space", "gated delta rule", "gated linear attention"]
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("H", [2, 16, 64])
+@pytest.mark.parametrize("lens", [[70], [30, 40], [1] * 20 + [64], [1, 24, 1, 70, 23, 24, 50], [3, 5], [24] * 9, [2] * 60, [1, 1, 70], [1, 1, 1, 70, 80]])
+@pytest.mark.parametrize("room", [16, 256])
+def test_a_recorded_step_runs_what_a_launched_one_does(kind, H, lens, room):
+    """Room for more requests than there are and lengths that are known on the device alone: the same routes and slices, to the last
+    bit; rows behind the last request, whose lengths are not positive, are nobody's."""
+    if len(lens) > room:
+        pytest.skip("more requests than rows")
+    pad = 13
+    run, state = _scan(kind, lens + [pad], H)              # the last sequence's tokens are the recorded step's padding
+    plain, launched, full = state.clone(), _batch(lens + [pad]), _batch(lens + [pad])
+    launched.cu_q, launched.state_slots, launched.q_lens = launched.cu_q[:-1].clone(), launched.state_slots[:-1].clone(), launched.q_lens[:-1]
+    y = run(plain, launched)
+
+    def with_room(t, n):
+        return torch.cat([t, torch.zeros(n - t.numel(), dtype=t.dtype, device=DEV)])
+
+    full.cu_q, full.state_slots = with_room(launched.cu_q, room + 1), with_room(launched.state_slots, room)
+    full.extras["recorder"] = object()
+    again = state.clone()
+    got = run(again, full)
+    assert torch.equal(got[:sum(lens)], y[:sum(lens)]) and torch.equal(again, plain)
