@@ -18,7 +18,7 @@
 // state rows n, a lane keeping NPL rows in registers (rows 4 (8 i + j) .. + 3, so that the lanes of a column read
 // consecutive 16-byte pieces of k and q).  Warps 4-7 load: while the others work on one chunk of tokens they put the
 // next chunk's unit q and k, its v, beta and g into the other half of shared memory.
-#include "common.cuh"
+#include "sequences.cuh"
 
 #include <math.h>
 
@@ -31,28 +31,23 @@ namespace {
 
 __device__ __forceinline__ float gd_softplus(float x) { return x > 20.0f ? x : log1pf(expf(x)); }
 
+template <int NPL>
+struct GdLayout {
+    static constexpr int NPAD = NPL * GD_LANES, CHUNK = NPL == 32 ? 8 : 16;
+    static constexpr int TOK = 2 * NPAD + GD_COLS + 4;            // floats per token: k, q, v, beta, g (+ padding to 16 bytes)
+    static constexpr int BUF = CHUNK * TOK;
+};
+
+// Sequence r's tokens through columns p_first .. of one head's state; all threads of the block.
 template <typename T, int NPL>
-__global__ void __launch_bounds__(256)
-gated_delta_scan_kernel(const T* u_in, long long ld_u, const T* b_in, long long ld_b, const T* a_in,
-                        long long ld_a, const float* a_log, const float* dt_bias, float* state,
-                        float* y, const int32_t* cu_q, const int32_t* slots, int H, int G, int D,
-                        int E) {
-    constexpr int NPAD = NPL * GD_LANES;
-    constexpr int CHUNK = NPL == 32 ? 8 : 16;
-    constexpr int TOK = 2 * NPAD + GD_COLS + 4;                   // floats per token: k, q, v, beta, g (+ padding to 16 bytes)
-    constexpr int BUF = CHUNK * TOK;
-    __shared__ __align__(16) float sm[2 * BUF];
-    pb_grid_dep_launch();
-    const int col_blocks = (E + GD_COLS - 1) / GD_COLS;
-    const int h = blockIdx.x / col_blocks, p_first = (blockIdx.x % col_blocks) * GD_COLS;
-    const int r = blockIdx.y;
+__device__ __forceinline__ void gd_sequence(float* sm, const T* u_in, long long ld_u, const T* b_in, long long ld_b, const T* a_in, long long ld_a, float rate,
+                                            float bias, float* state, float* y, const int32_t* cu_q, const int32_t* slots, int r, int h, int p_first, int H, int G,
+                                            int D, int E) {
+    constexpr int NPAD = GdLayout<NPL>::NPAD, CHUNK = GdLayout<NPL>::CHUNK, TOK = GdLayout<NPL>::TOK, BUF = GdLayout<NPL>::BUF;
     const int tid = threadIdx.x;
     const bool computes = tid < GD_COLS * GD_LANES;
-    const float rate = expf(a_log[h]), bias = dt_bias[h];        // written by no kernel: before the wait
     const float q_scale = 1.0f / sqrtf((float)D);
-    pb_grid_dep_wait();
     const int first = cu_q[r], n_tok = cu_q[r + 1] - first;
-    if (n_tok <= 0) return;
     const int g = h / (H / G);
     const int n_chunks = (n_tok + CHUNK - 1) / CHUNK;
 
@@ -176,14 +171,41 @@ gated_delta_scan_kernel(const T* u_in, long long ld_u, const T* b_in, long long 
     }
 }
 
+// A launched step: a row of blocks a sequence; one of no tokens, or of which.below and more, has nothing to do.  RECORDED: the sequences
+// are looked up.
+template <typename T, int NPL, bool RECORDED>
+__global__ void __launch_bounds__(256)
+gated_delta_scan_kernel(const T* u_in, long long ld_u, const T* b_in, long long ld_b, const T* a_in,
+                        long long ld_a, const float* a_log, const float* dt_bias, float* state,
+                        float* y, const int32_t* cu_q, const int32_t* slots, PbSequences which, int H, int G, int D,
+                        int E) {
+    __shared__ __align__(16) float sm[2 * GdLayout<NPL>::BUF];
+    pb_grid_dep_launch();
+    const int col_blocks = (E + GD_COLS - 1) / GD_COLS;
+    const int h = blockIdx.x / col_blocks, p_first = (blockIdx.x % col_blocks) * GD_COLS;
+    const float rate = expf(a_log[h]), bias = dt_bias[h];        // written by no kernel: before the wait
+    pb_grid_dep_wait();
+    auto work = [&](int r, int) {
+        gd_sequence<T, NPL>(sm, u_in, ld_u, b_in, ld_b, a_in, ld_a, rate, bias, state, y, cu_q, slots, r, h, p_first, H, G, D, E);
+    };
+    if constexpr (RECORDED) {
+        pb_for_sequences<true>(cu_q, which, work);
+    } else {
+        const int n_tok = cu_q[blockIdx.y + 1] - cu_q[blockIdx.y];
+        if (n_tok > 0 && n_tok < which.below) work(blockIdx.y, 0);
+    }
+}
+
 }  // namespace
 
 // u: the convolutions' outputs [n_tokens, 2 * G * D + H * E] laid out [q | k | v], rows ld_u apart; b_in, a_in: the
 // [n_tokens, H] columns of a projection (rows ld_b, ld_a apart); a_log, dt_bias float32 [H]; state float32
-// [slots, H, D, E]; y float32 [n_tokens, H * E] dense.  cu_q [n_seqs + 1], slots [n_seqs].
+// [slots, H, D, E]; y float32 [n_tokens, H * E] dense.  cu_q [n_seqs + 1], slots [n_seqs].  below > 0: only the sequences of fewer tokens
+// than that; n_short: how many there are (`counted`), or the most there can be, for a step that is being recorded (few, beside:
+// sequences.cuh).
 PB_API int pb_gated_delta_scan(const void* u, long long ld_u, const void* b_in, long long ld_b, const void* a_in, long long ld_a, int dtype,
                                const float* a_log, const float* dt_bias, float* state, float* y, const int32_t* cu_q, const int32_t* slots,
-                               int n_seqs, int H, int G, int D, int E, cudaStream_t stream) {
+                               int n_seqs, int H, int G, int D, int E, int below, int few, int beside, int n_short, int counted, cudaStream_t stream) {
     PB_REQUIRE(n_seqs >= 0 && H > 0 && G > 0 && H % G == 0 && D > 0 && E > 0, "gated_delta_scan: bad sizes");
     PB_REQUIRE(D <= 32 * GD_LANES, "gated_delta_scan: keys of %d elements (at most %d)", D, 32 * GD_LANES);
     PB_REQUIRE(u && b_in && a_in && a_log && dt_bias && state && y && cu_q && slots, "gated_delta_scan: null pointer");
@@ -191,15 +213,21 @@ PB_API int pb_gated_delta_scan(const void* u, long long ld_u, const void* b_in, 
     if (n_seqs == 0) return 0;
     PB_REQUIRE(n_seqs < 65536, "gated_delta_scan: %d sequences in one launch", n_seqs);
     const int col_blocks = (E + GD_COLS - 1) / GD_COLS;
-    const dim3 grid(H * col_blocks, n_seqs), block(2 * GD_COLS * GD_LANES);
-    const int npl = (D + GD_LANES - 1) / GD_LANES;
-#define GD_LAUNCH(NPL)                                                                                                             \
-    PB_DISPATCH_DTYPE(dtype, T, (pb_launch(gated_delta_scan_kernel<T, NPL>, grid, block, 0, stream, (const T*)u, ld_u, (const T*)b_in, ld_b, \
-                                           (const T*)a_in, ld_a, a_log, dt_bias, state, y, cu_q, slots, H, G, D, E)))
-    if (npl <= 4) GD_LAUNCH(4);
-    else if (npl <= 8) GD_LAUNCH(8);
-    else if (npl <= 16) GD_LAUNCH(16);
-    else GD_LAUNCH(32);
+    const int npl = (D + GD_LANES - 1) / GD_LANES, recorded = below > 0 && !counted;
+    const PbSequences which{n_seqs, 1, below > 0 ? below : INT_MAX, few, beside, 0, recorded, 0, 0};
+    if (recorded) PB_REQUIRE(dtype == PB_BF16 && npl <= 16, "gated_delta_scan: by length in a recorded step: bfloat16, keys of at most %d", 16 * GD_LANES);
+    if (below > 0 && n_short <= 0) return 0;
+    const dim3 grid(H * col_blocks, recorded ? pb_recorded_rows(n_short, (long long)H * col_blocks, 6) : n_seqs), block(2 * GD_COLS * GD_LANES);
+#define GD_LAUNCH(T, NPL, R)                                                                                                       \
+    pb_launch(gated_delta_scan_kernel<T, NPL, R>, grid, block, 0, stream, (const T*)u, ld_u, (const T*)b_in, ld_b, (const T*)a_in, ld_a, a_log, dt_bias, \
+              state, y, cu_q, slots, which, H, G, D, E)
+    if (recorded) {
+        if (npl <= 8) GD_LAUNCH(__nv_bfloat16, 8, true);
+        else GD_LAUNCH(__nv_bfloat16, 16, true);
+    } else if (npl <= 4) PB_DISPATCH_DTYPE(dtype, T, (GD_LAUNCH(T, 4, false)));
+    else if (npl <= 8) PB_DISPATCH_DTYPE(dtype, T, (GD_LAUNCH(T, 8, false)));
+    else if (npl <= 16) PB_DISPATCH_DTYPE(dtype, T, (GD_LAUNCH(T, 16, false)));
+    else PB_DISPATCH_DTYPE(dtype, T, (GD_LAUNCH(T, 32, false)));
 #undef GD_LAUNCH
     PB_CHECK_LAUNCH("gated_delta_scan");
     return 0;

@@ -17,7 +17,7 @@
 // what else is in the batch.  (A prompt step in bfloat16 runs the state-space recurrence by chunks: ssm_chunk.cu.)  All kernels find a step's sequences through device arrays (cumulative lengths,
 // state slots), with one block row per sequence the arrays have room for: a row whose length is not positive is
 // skipped, so the launches have the same shape whatever the step holds and can be recorded.
-#include "common.cuh"
+#include "sequences.cuh"
 
 #include <math.h>
 
@@ -358,66 +358,75 @@ ssm_scan_kernel(const T* u, long long ld_u, const T* dt_in, long long ld_dt, con
     }
 }
 
-// One token per sequence (a decode step) in bfloat16: a block owns a head's state, a thread four columns and every 16th (or so) row of
+// One token per sequence (a decode step, or those sequences of any step: `which`) in bfloat16: a block owns a head's state, a thread four columns and every 16th (or so) row of
 // it, eight rows' pieces under way at a time; the rows' shares of the output meet in shared memory in their order.  What bounds it is
 // the state, read and written once.  (The scan above reads it 16 bytes of a row at a time, and makes ready for a chunk of
 // sixteen tokens: 2 sequences, 128 heads of 128 x 64, 16.3 us, here 6.7.)
 #define SSM_STEP_THREADS 256
 #define SSM_STEP_ROWS 8
+// RECORDED as in delta_rule.cu.
+template <bool RECORDED>
 __global__ void __launch_bounds__(SSM_STEP_THREADS)
 ssm_step_kernel(const __nv_bfloat16* u, const __nv_bfloat16* dt_in, long long ld_dt, const float* dt_bias, const float* a_log, const float* d_skip,
-                float* state, float* y, const int32_t* cu_q, const int32_t* slots, int heads, int P, int N, int groups) {
+                float* state, float* y, const int32_t* cu_q, const int32_t* slots, PbSequences which, int heads, int P, int N, int groups) {
     __shared__ __align__(16) float part[SSM_STEP_THREADS * 4];
     pb_grid_dep_launch();
-    const int h = blockIdx.x, r = blockIdx.y, tid = threadIdx.x;
+    const int h = blockIdx.x, tid = threadIdx.x;
     const float neg_a = -expf(a_log[h]), bias = dt_bias[h], skip = d_skip[h];     // written by no kernel: before the wait
     const int cg = P >> 2, rg = SSM_STEP_THREADS / cg, c = tid % cg, row0 = tid / cg;
     pb_grid_dep_wait();
-    const int t = cu_q[r];
-    if (cu_q[r + 1] - t <= 0) return;
-    const int inner = heads * P, g = h / (heads / groups);
-    const __nv_bfloat16* row = u + (size_t)t * (inner + 2 * groups * N);
-    float4* S = reinterpret_cast<float4*>(state + ((size_t)slots[r] * heads + h) * N * (size_t)P) + c;
-    const bool works = row0 < rg;
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (works) {
-        const uint2 xr = *reinterpret_cast<const uint2*>(row + h * P + 4 * c);
-        const float dt = softplus_f(pb_ld(dt_in + (size_t)t * ld_dt + h) + bias), decay = expf(neg_a * dt);
-        const float2 x0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&xr.x)), x1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&xr.y));
-        const float4 dx = make_float4(dt * x0.x, dt * x0.y, dt * x1.x, dt * x1.y);
-        const __nv_bfloat16* B = row + inner + g * N;
-        const __nv_bfloat16* C = B + groups * N;
-        for (int n0 = row0; n0 < N; n0 += rg * SSM_STEP_ROWS) {
-            float4 s[SSM_STEP_ROWS];
-            float b[SSM_STEP_ROWS], cc[SSM_STEP_ROWS];
+    auto work = [&](int r, int) {
+        const int t = cu_q[r];
+        const int inner = heads * P, g = h / (heads / groups);
+        const __nv_bfloat16* row = u + (size_t)t * (inner + 2 * groups * N);
+        float4* S = reinterpret_cast<float4*>(state + ((size_t)slots[r] * heads + h) * N * (size_t)P) + c;
+        const bool works = row0 < rg;
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (works) {
+            const uint2 xr = *reinterpret_cast<const uint2*>(row + h * P + 4 * c);
+            const float dt = softplus_f(pb_ld(dt_in + (size_t)t * ld_dt + h) + bias), decay = expf(neg_a * dt);
+            const float2 x0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&xr.x)), x1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&xr.y));
+            const float4 dx = make_float4(dt * x0.x, dt * x0.y, dt * x1.x, dt * x1.y);
+            const __nv_bfloat16* B = row + inner + g * N;
+            const __nv_bfloat16* C = B + groups * N;
+            for (int n0 = row0; n0 < N; n0 += rg * SSM_STEP_ROWS) {
+                float4 s[SSM_STEP_ROWS];
+                float b[SSM_STEP_ROWS], cc[SSM_STEP_ROWS];
 #pragma unroll
-            for (int i = 0; i < SSM_STEP_ROWS; ++i) {
-                const int n = min(n0 + i * rg, N - 1);
-                s[i] = S[(size_t)n * cg];
-                b[i] = pb_ld(B + n);
-                cc[i] = pb_ld(C + n);
-            }
+                for (int i = 0; i < SSM_STEP_ROWS; ++i) {
+                    const int n = min(n0 + i * rg, N - 1);
+                    s[i] = S[(size_t)n * cg];
+                    b[i] = pb_ld(B + n);
+                    cc[i] = pb_ld(C + n);
+                }
 #pragma unroll
-            for (int i = 0; i < SSM_STEP_ROWS; ++i) {
-                const int n = n0 + i * rg;
-                if (n < N) {
-                    s[i] = make_float4(fmaf(decay, s[i].x, dx.x * b[i]), fmaf(decay, s[i].y, dx.y * b[i]), fmaf(decay, s[i].z, dx.z * b[i]), fmaf(decay, s[i].w, dx.w * b[i]));
-                    S[(size_t)n * cg] = s[i];
-                    acc.x = fmaf(s[i].x, cc[i], acc.x); acc.y = fmaf(s[i].y, cc[i], acc.y);
-                    acc.z = fmaf(s[i].z, cc[i], acc.z); acc.w = fmaf(s[i].w, cc[i], acc.w);
+                for (int i = 0; i < SSM_STEP_ROWS; ++i) {
+                    const int n = n0 + i * rg;
+                    if (n < N) {
+                        s[i] = make_float4(fmaf(decay, s[i].x, dx.x * b[i]), fmaf(decay, s[i].y, dx.y * b[i]), fmaf(decay, s[i].z, dx.z * b[i]), fmaf(decay, s[i].w, dx.w * b[i]));
+                        S[(size_t)n * cg] = s[i];
+                        acc.x = fmaf(s[i].x, cc[i], acc.x); acc.y = fmaf(s[i].y, cc[i], acc.y);
+                        acc.z = fmaf(s[i].z, cc[i], acc.z); acc.w = fmaf(s[i].w, cc[i], acc.w);
+                    }
                 }
             }
+            if (row0 == 0) {
+                acc.x = fmaf(skip, x0.x, acc.x); acc.y = fmaf(skip, x0.y, acc.y); acc.z = fmaf(skip, x1.x, acc.z); acc.w = fmaf(skip, x1.y, acc.w);
+            }
+            *reinterpret_cast<float4*>(part + tid * 4) = acc;
         }
-        if (row0 == 0) {
-            acc.x = fmaf(skip, x0.x, acc.x); acc.y = fmaf(skip, x0.y, acc.y); acc.z = fmaf(skip, x1.x, acc.z); acc.w = fmaf(skip, x1.y, acc.w);
+        __syncthreads();
+        if (tid < P) {
+            float v = part[tid];
+            for (int k = 1; k < rg; ++k) v += part[k * P + tid];
+            y[(size_t)t * inner + h * P + tid] = v;
         }
-        *reinterpret_cast<float4*>(part + tid * 4) = acc;
-    }
-    __syncthreads();
-    if (tid < P) {
-        float v = part[tid];
-        for (int k = 1; k < rg; ++k) v += part[k * P + tid];
-        y[(size_t)t * inner + h * P + tid] = v;
+    };
+    if constexpr (RECORDED) {
+        pb_for_sequences<true>(cu_q, which, work);
+    } else {
+        const int n_tok = cu_q[blockIdx.y + 1] - cu_q[blockIdx.y];
+        if (n_tok > 0 && n_tok < which.below) work(blockIdx.y, 0);
     }
 }
 
@@ -642,7 +651,9 @@ PB_API int pb_ssm_scan(const void* u, const void* dt_in, long long ld_dt, int dt
     return 0;
 }
 
-// The same for a step of one token per sequence, bfloat16: whether it takes the sizes, and the call.
+// The same for a step of one token per sequence, bfloat16: whether it takes the sizes, and the call.  `single`: a step of any lengths, of
+// which only the sequences of one token are visited; n_short: how many there are (`counted`), or the most there can be, for a step that is
+// being recorded (few, beside: sequences.cuh).
 PB_API int pb_ssm_step_takes(const void* u, const float* state, int heads, int P, int N, int groups) {
     return heads > 0 && groups > 0 && heads % groups == 0 && P >= 4 && P % 4 == 0 && P <= SSM_STEP_THREADS && N > 0 && (heads * P + 2 * groups * N) % 4 == 0 &&
                    pb_aligned(u, 8) && pb_aligned(state, 16)
@@ -650,13 +661,22 @@ PB_API int pb_ssm_step_takes(const void* u, const float* state, int heads, int P
                : 0;
 }
 PB_API int pb_ssm_step(const void* u, const void* dt_in, long long ld_dt, const float* dt_bias, const float* a_log, const float* d_skip, float* state, float* y,
-                       const int32_t* cu_q, const int32_t* slots, int n_seqs, int heads, int P, int N, int groups, cudaStream_t stream) {
+                       const int32_t* cu_q, const int32_t* slots, int n_seqs, int heads, int P, int N, int groups, int single, int few, int beside, int n_short, int counted,
+                       cudaStream_t stream) {
     PB_REQUIRE(n_seqs >= 0 && pb_ssm_step_takes(u, state, heads, P, N, groups), "ssm_step: %d heads of %d, state %d, %d groups", heads, P, N, groups);
     PB_REQUIRE(u && dt_in && dt_bias && a_log && d_skip && state && y && cu_q && slots && ld_dt >= heads, "ssm_step: null pointer");
     if (n_seqs == 0) return 0;
     PB_REQUIRE(n_seqs < 65536, "ssm_step: %d sequences in one launch", n_seqs);
-    pb_launch(ssm_step_kernel, dim3(heads, n_seqs), dim3(SSM_STEP_THREADS), 0, stream, (const __nv_bfloat16*)u, (const __nv_bfloat16*)dt_in, ld_dt, dt_bias, a_log, d_skip,
-              state, y, cu_q, slots, heads, P, N, groups);
+    if (single && n_short <= 0) return 0;
+    const int recorded = single && !counted;
+    const PbSequences which{n_seqs, 1, single ? 2 : INT_MAX, few, beside, 0, recorded, 0, 0};
+    const dim3 grid(heads, recorded ? pb_recorded_rows(n_short, heads, 8) : n_seqs);
+#define STEP_LAUNCH(R)                                                                                                             \
+    pb_launch(ssm_step_kernel<R>, grid, dim3(SSM_STEP_THREADS), 0, stream, (const __nv_bfloat16*)u, (const __nv_bfloat16*)dt_in, ld_dt, dt_bias, a_log, \
+              d_skip, state, y, cu_q, slots, which, heads, P, N, groups)
+    if (recorded) STEP_LAUNCH(true);
+    else STEP_LAUNCH(false);
+#undef STEP_LAUNCH
     PB_CHECK_LAUNCH("ssm_step");
     return 0;
 }

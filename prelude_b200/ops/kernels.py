@@ -1047,35 +1047,53 @@ def conv_state_update(x: torch.Tensor, carried: torch.Tensor, batch) -> None:
                                             _stream()), "conv_state_update")
 
 
-# tokens of a prompt step from which the recurrences run by chunks of tokens on the tensor cores (bfloat16 only).  State space:
-# 12 us either way at 32 tokens, 11.5 against 20 at 64; the gated delta rule, two kernels: 24 against 16 at 32, 24 against 28 at 64;
-# gated linear attention, two kernels over memory between them: 25 against 21 at 128 of 32 heads, 31 against 38 at 256
+# Tokens of a prompt step from which the recurrences run by chunks of tokens on the tensor cores (bfloat16 only), and which of its
+# sequences then do: (length, few, beside) as in _split.  us, token by token against chunks, read from memory:
+# state space, 64 heads of 128 x 64: one sequence of 8 tokens 12 / 12, of 32 18 / 12; 16 of 2 57 / 61, of 8 84 / 61; 60 of one token and one
+#   of 64 193 / 211, and 68 with the single tokens on the kernel that a decode step takes;
+# gated delta rule, 16 heads of 128 x 128: one of 32 21 / 25, of 64 31 / 25; 16 of 8 53 / 72, of 16 80 / 78, of 32 121 / 78; 60 of one token
+#   and one of 64 113 / 236, of 128 137 / 238, and 117 with the short ones token by token, of 512 277 / 270, and 131;
+# gated linear attention, 16 heads of 128 x 128: one of 128 23 / 23, of 256 35 / 31; 16 of 16 45 / 37; 60 of one token and one of 512
+#   178 / 131: a sequence of one token costs little in sixteens, and none is taken out.
 SCAN_CHUNKED_MIN_TOKENS = 32
 DELTA_CHUNKED_MIN_TOKENS = 64
 GLA_CHUNKED_MIN_TOKENS = 256
+SCAN_CHUNKED_LENGTHS = (2, 2, 2)
+DELTA_CHUNKED_LENGTHS = (16, 4, 128)
 
 
 class _Split(NamedTuple):
-    """A step whose sequences run by chunks."""
-    n_long: int       # how many there are (``counted``), or can be
+    """How a step's sequences part: those of at least ``least`` tokens run by chunks, the others token by token."""
+    least: int
+    few: int          # with ``beside`` > 0 the limit is looked up on the device, as ``_split`` says
+    beside: int
+    n_long: int       # how many there are of either (``counted``), or can be
+    n_short: int
     counted: bool     # False: a step that is being recorded, which is replayed for other lengths
 
 
-def _split(batch, T: int, min_tokens: int) -> Optional[_Split]:
-    """The sequences of a step of T tokens, which run by chunks from ``min_tokens`` on.  None: nothing runs by chunks."""
+def _split(batch, T: int, min_tokens: int, length: int = 1, few: int = 0, beside: int = 1) -> Optional[_Split]:
+    """The parts of a step of T tokens, by chunks from ``min_tokens`` on: all sequences where no more than ``few`` have fewer than
+    ``length`` tokens, else those of ``beside`` tokens (which is no less).  None: nothing runs by chunks."""
     if batch.decode_only or T < min_tokens:
         return None
-    n_seqs = batch.cu_q.numel() - 1
-    counted = batch.extras.get("recorder") is None and batch.q_lens.shape[0] == n_seqs
-    return _Split(n_seqs if counted else min(n_seqs, T), counted)
+    n_seqs, length = batch.cu_q.numel() - 1, min(length, min_tokens)
+    if batch.extras.get("recorder") is not None or batch.q_lens.shape[0] != n_seqs:
+        if length == 1:
+            return _Split(1, 0, 0, min(n_seqs, T), 0, False)
+        return _Split(length, few, beside, min(n_seqs, T // length + few), min(n_seqs, T), False)
+    if length == 1 or int((batch.q_lens < length).sum()) <= few:
+        return _Split(1, 0, 0, n_seqs, 0, True)
+    n_short = int((batch.q_lens < beside).sum())
+    return _Split(beside, 0, 0, n_seqs - n_short, n_short, True) if n_short < n_seqs else None
 
 
 def ssm_scan(u: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: torch.Tensor, d_skip: torch.Tensor,
              state: torch.Tensor, batch, groups: int, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """The recurrence over the step's tokens, sequence by sequence; u [T, heads * P + 2 * groups * N] dense, dt [T, heads] a
     view with dense rows, state float32 [slots, heads, N, P]; returns y float32 [T, heads * P].  A prompt step in bfloat16
-    runs by chunks of tokens (csrc/ssm_chunk.cu), a decode step in bfloat16 on a kernel for single tokens, in 32-bit token
-    by token (csrc/ssm.cu)."""
+    runs by chunks of tokens (csrc/ssm_chunk.cu), but for its sequences of one token, which run as a decode step's do on a kernel for
+    single tokens; in 32-bit token by token (csrc/ssm.cu)."""
     _need(u, "u")
     _need(dt, "dt", u.dtype, contiguous=False)
     for t, name in ((dt_bias, "dt_bias"), (a_log, "a_log"), (d_skip, "d_skip"), (state, "state")):
@@ -1088,18 +1106,21 @@ def ssm_scan(u: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: to
         out = torch.empty((T, heads * P), dtype=torch.float32, device=u.device)
     lib = _l.library()
     n_seqs = batch.cu_q.numel() - 1
+    steps = u.dtype == torch.bfloat16 and lib.pb_ssm_step_takes(u.data_ptr(), state.data_ptr(), heads, P, N, groups)
     part = None
     if u.dtype == torch.bfloat16 and lib.pb_ssm_scan_chunked_takes(u.data_ptr(), state.data_ptr(), out.data_ptr(), heads, P, N, groups):
-        part = _split(batch, T, SCAN_CHUNKED_MIN_TOKENS)
+        part = _split(batch, T, SCAN_CHUNKED_MIN_TOKENS, *(SCAN_CHUNKED_LENGTHS if steps else ()))
     if part is not None:
         check(lib.pb_ssm_scan_chunked(u.data_ptr(), dt.data_ptr(), dt.stride(0), dt_bias.data_ptr(), a_log.data_ptr(), d_skip.data_ptr(),
-                                      state.data_ptr(), out.data_ptr(), batch.cu_q.data_ptr(), batch.state_slots.data_ptr(), n_seqs, 1, 0, 0,
-                                      part.n_long, part.counted, heads, P, N, groups, _stream()), "ssm_scan_chunked")
-        return out
-    if u.dtype == torch.bfloat16 and batch.decode_only and lib.pb_ssm_step_takes(u.data_ptr(), state.data_ptr(), heads, P, N, groups):
+                                      state.data_ptr(), out.data_ptr(), batch.cu_q.data_ptr(), batch.state_slots.data_ptr(), n_seqs, part.least,
+                                      part.few, part.beside, part.n_long, part.counted, heads, P, N, groups, _stream()), "ssm_scan_chunked")
+    if steps and (batch.decode_only or (part is not None and part.n_short)):
+        which = (0, 0, 0, 0, 1) if part is None else (1, part.few, part.beside, part.n_short, part.counted)
         check(lib.pb_ssm_step(u.data_ptr(), dt.data_ptr(), dt.stride(0), dt_bias.data_ptr(), a_log.data_ptr(), d_skip.data_ptr(), state.data_ptr(),
-                              out.data_ptr(), batch.cu_q.data_ptr(), batch.state_slots.data_ptr(), n_seqs, heads, P, N, groups,
+                              out.data_ptr(), batch.cu_q.data_ptr(), batch.state_slots.data_ptr(), n_seqs, heads, P, N, groups, *which,
                               _stream()), "ssm_step")
+        return out
+    if part is not None:
         return out
     check(lib.pb_ssm_scan(u.data_ptr(), dt.data_ptr(), dt.stride(0), dtype_code(u.dtype), dt_bias.data_ptr(), a_log.data_ptr(),
                                    d_skip.data_ptr(), state.data_ptr(), out.data_ptr(), batch.cu_q.data_ptr(),
@@ -1315,7 +1336,7 @@ def gated_delta_scan(u: torch.Tensor, beta: torch.Tensor, a: torch.Tensor, a_log
                      state: torch.Tensor, batch, kv_heads: int, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """The gated delta rule over the step's tokens, sequence by sequence; u [T, 2 G D + H E] laid out [q | k | v] (the
     convolutions' outputs), beta and a [T, H] views with dense rows, state float32 [slots, H, D, E]; returns o float32
-    [T, H E].  A prompt step in bfloat16 runs by chunks of tokens (csrc/delta_chunk.cu), in 32-bit and in a decode step token by
+    [T, H E].  The longer sequences of a prompt step in bfloat16 run by chunks of tokens (csrc/delta_chunk.cu), all else token by
     token (csrc/delta_rule.cu)."""
     T = u.shape[0]
     _rows_view(u, "u", T, None)
@@ -1330,19 +1351,21 @@ def gated_delta_scan(u: torch.Tensor, beta: torch.Tensor, a: torch.Tensor, a_log
         out = torch.empty((T, H * E), dtype=torch.float32, device=u.device)
     lib, n_seqs, part = _l.library(), batch.cu_q.numel() - 1, None
     if u.dtype == torch.bfloat16 and lib.pb_gated_delta_chunked_takes(u.data_ptr(), u.stride(0), state.data_ptr(), out.data_ptr(), H, kv_heads, D, E):
-        part = _split(batch, T, DELTA_CHUNKED_MIN_TOKENS)
+        part = _split(batch, T, DELTA_CHUNKED_MIN_TOKENS, *DELTA_CHUNKED_LENGTHS)
     if part is not None:
         # what one kernel makes of every chunk for the other to read: dead when the call's kernels are done
         n_chunks = lib.pb_gated_delta_chunks(T, part.n_long)
         scratch = torch.empty((lib.pb_gated_delta_chunk_bytes(n_chunks, H),), dtype=torch.uint8, device=u.device)
         check(lib.pb_gated_delta_scan_chunked(u.data_ptr(), u.stride(0), beta.data_ptr(), beta.stride(0), a.data_ptr(), a.stride(0),
                                               a_log.data_ptr(), dt_bias.data_ptr(), state.data_ptr(), out.data_ptr(), batch.cu_q.data_ptr(),
-                                              batch.state_slots.data_ptr(), scratch.data_ptr(), n_chunks, n_seqs, 1, 0,
-                                              0, part.n_long, part.counted, H, kv_heads, D, E, _stream()), "gated_delta_scan_chunked")
-        return out
+                                              batch.state_slots.data_ptr(), scratch.data_ptr(), n_chunks, n_seqs, part.least, part.few,
+                                              part.beside, part.n_long, part.counted, H, kv_heads, D, E, _stream()), "gated_delta_scan_chunked")
+        if not part.n_short:
+            return out
+    which = (0, 0, 0, 0, 1) if part is None else (part.least, part.few, part.beside, part.n_short, part.counted)
     check(lib.pb_gated_delta_scan(u.data_ptr(), u.stride(0), beta.data_ptr(), beta.stride(0), a.data_ptr(), a.stride(0),
                                            dtype_code(u.dtype), a_log.data_ptr(), dt_bias.data_ptr(), state.data_ptr(), out.data_ptr(),
-                                           batch.cu_q.data_ptr(), batch.state_slots.data_ptr(), n_seqs, H, kv_heads, D, E,
+                                           batch.cu_q.data_ptr(), batch.state_slots.data_ptr(), n_seqs, H, kv_heads, D, E, *which,
                                            _stream()), "gated_delta_scan")
     return out
 

@@ -101,7 +101,7 @@ _SIGNATURES = {
     "pb_conv_state_update": ([P, L, P, I, P, P, I, I, I, P], I),
     "pb_ssm_scan": ([P, P, L, I, P, P, P, P, P, P, P, I, I, I, I, I, P], I),
     "pb_ssm_step_takes": ([P, P, I, I, I, I], I),
-    "pb_ssm_step": ([P, P, L, P, P, P, P, P, P, P, I, I, I, I, I, P], I),
+    "pb_ssm_step": ([P, P, L, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, P], I),
     "pb_ssm_scan_chunked_takes": ([P, P, P, I, I, I, I], I),
     "pb_ssm_scan_chunked": ([P, P, L, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, P], I),
     "pb_walk_launches": ([I, I, I, I, I, I, P], I),
@@ -132,7 +132,7 @@ _SIGNATURES = {
     "pb_embed_gather_scaled": ([P, P, I, F, P, I, I, I, P], I),
     "pb_tanh": ([P, P, I, L, P], I),
     "pb_heads_prepare": ([P, L, P, L, P, L, I, P, P, I, F, P, F, I, I, P, P, L, F, P, P, P, I, I, I, P, P, P, I, I, I, I, I, I, I, P, P], I),
-    "pb_gated_delta_scan": ([P, L, P, L, P, L, I, P, P, P, P, P, P, I, I, I, I, I, P], I),
+    "pb_gated_delta_scan": ([P, L, P, L, P, L, I, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, P], I),
     "pb_gated_delta_chunked_takes": ([P, L, P, P, I, I, I, I], I),
     "pb_gated_delta_chunks": ([I, I], I),
     "pb_gated_delta_chunk_bytes": ([I, I], L),

@@ -318,15 +318,59 @@ def _scan(kind, lens, H, seed=5):
 KINDS = ["state space", "gated delta rule", "gated linear attention"]
 
 
+def _thresholds(monkeypatch, tokens, lengths=(1, 0, 1)):
+    from prelude_b200.ops import kernels as K
+    for name in ("SCAN_CHUNKED_MIN_TOKENS", "DELTA_CHUNKED_MIN_TOKENS", "GLA_CHUNKED_MIN_TOKENS"):
+        monkeypatch.setattr(K, name, tokens)
+    monkeypatch.setattr(K, "DELTA_CHUNKED_LENGTHS", lengths)
+
+
+@pytest.mark.parametrize("lens,limit", [([1] * 60 + [30], 70), ([1, 24, 1, 70, 23, 24], 70), ([1, 24, 70, 23, 24], 1), ([23] * 5, 70), ([24, 100], 1),
+                                        ([1] * 130 + [90] + [1] * 130, 70)])
+def test_every_sequence_of_the_delta_rule_runs_as_its_own_length_asks(lens, limit, monkeypatch):
+    """Sequences of one token beside portions: where more than two have fewer than 24, those of 70 run by chunks, the others
+    token by token - to the last bit what each gives where all run one way."""
+    run, state = _scan("gated delta rule", lens, 2)
+    results = []
+    for tokens, lengths in ((1 << 30, (1, 0, 1)), (1, (1, 0, 1)), (24, (24, 2, 70))):
+        _thresholds(monkeypatch, tokens, lengths)
+        s = state.clone()
+        results.append((run(s, _batch(lens)), s))
+    (y_tok, s_tok), (y_chunk, s_chunk), (y, s) = results
+    at = 0
+    for r, n in enumerate(lens):
+        want_y, want_s = (y_chunk, s_chunk) if n >= limit else (y_tok, s_tok)
+        slot = len(lens) - 1 - r
+        assert torch.equal(y[at:at + n], want_y[at:at + n]) and torch.equal(s[slot], want_s[slot])
+        at += n
+
+
+@pytest.mark.parametrize("lens", [[1] * 60 + [30], [1, 24, 1, 70, 2, 24, 1], [1] * 130 + [90] + [1] * 130])
+def test_single_tokens_of_a_state_space_step_run_as_a_decode_step_does(lens, monkeypatch):
+    """Sequences of one token beside portions: to the last bit what a step of single tokens alone gives them."""
+    from prelude_b200.ops import kernels as K
+    _thresholds(monkeypatch, 24)
+    H = 2
+    u, dt, bias, a_log, skip, state = _ssm_inputs(lens, H, 64, 64, 1, 5, 0.05)
+    alone, at = state.clone(), [sum(lens[:r]) for r, n in enumerate(lens) if n == 1]
+    b = _batch([1] * len(at))
+    b.state_slots = torch.tensor([len(lens) - 1 - r for r, n in enumerate(lens) if n == 1], dtype=torch.int32, device=DEV)
+    want = K.ssm_scan(u[at].contiguous(), dt[at].contiguous(), bias, a_log, skip, alone, b, 1)
+    got = K.ssm_scan(u, dt, bias, a_log, skip, state, _batch(lens), 1)
+    slots = b.state_slots.long()
+    assert torch.equal(got[at], want) and torch.equal(state[slots], alone[slots])
+
+
 @pytest.mark.parametrize("kind", KINDS)
 @pytest.mark.parametrize("H", [2, 16, 64])
 @pytest.mark.parametrize("lens", [[70], [30, 40], [1] * 20 + [64], [1, 24, 1, 70, 23, 24, 50], [3, 5], [24] * 9, [2] * 60, [1, 1, 70], [1, 1, 1, 70, 80]])
 @pytest.mark.parametrize("room", [16, 256])
-def test_a_recorded_step_runs_what_a_launched_one_does(kind, H, lens, room):
+def test_a_recorded_step_runs_what_a_launched_one_does(kind, H, lens, room, monkeypatch):
     """Room for more requests than there are and lengths that are known on the device alone: the same routes and slices, to the last
     bit; rows behind the last request, whose lengths are not positive, are nobody's."""
     if len(lens) > room:
         pytest.skip("more requests than rows")
+    _thresholds(monkeypatch, 24, (24, 2, 60))
     pad = 13
     run, state = _scan(kind, lens + [pad], H)              # the last sequence's tokens are the recorded step's padding
     plain, launched, full = state.clone(), _batch(lens + [pad]), _batch(lens + [pad])

@@ -1,4 +1,4 @@
-"""In how wide slices of a head's state the sequences of a step run by chunks of tokens: the rules, on the CPU."""
+"""Which sequences of a step run by chunks of tokens, and in how wide slices of a head's state: the rules, on the CPU."""
 import ctypes
 
 import numpy as np
@@ -18,12 +18,34 @@ def _batch(lens, room=None, **more):
                      q_lens=np.asarray(lens, np.int32), **more)
 
 
-@pytest.mark.parametrize("tokens,least,most", [(32, 32, 32), (1024, 64, 256), (4096, 1, 256)])
-def test_a_recorded_step_allows_for_every_spread_of_its_tokens(tokens, least, most):
+RULES = {"state space": (32, 2, 2, 2), "gated delta rule": (64, 16, 4, 128), "gated linear attention": (256,)}
+
+
+@pytest.mark.parametrize("kind,lens,want", [
+    ("gated delta rule", [500], (1, 0, 0, 1, 0, True)), ("gated delta rule", [1, 15, 15, 15, 700], (1, 0, 0, 5, 0, True)),
+    ("gated delta rule", [63], None), ("gated delta rule", [1] * 60 + [8], None), ("gated delta rule", [1] * 60 + [127], None),
+    ("gated delta rule", [1] * 60 + [128, 127], (128, 0, 0, 1, 61, True)), ("gated delta rule", [15] * 5 + [128], (128, 0, 0, 1, 5, True)),
+    ("gated delta rule", [16] * 5, (1, 0, 0, 5, 0, True)), ("state space", [1] * 60 + [8], (2, 0, 0, 1, 60, True)),
+    ("state space", [1, 1, 30], (1, 0, 0, 3, 0, True)), ("state space", [1] * 40, None), ("state space", [2] * 16, (1, 0, 0, 16, 0, True)),
+    ("state space", [31], None), ("gated linear attention", [1] * 60 + [196], (1, 0, 0, 61, 0, True)), ("gated linear attention", [255], None)])
+def test_sequences_go_by_their_own_length(kind, lens, want):
+    """One token each beside a portion: however many tokens the step has, only a sequence that is long itself goes by chunks, where
+    chunks do not pay for many short ones."""
+    assert K._split(_batch(lens), sum(lens), *RULES[kind]) == want
+
+
+@pytest.mark.parametrize("kind,tokens,want", [
+    ("state space", 32, (2, 2, 2, 18, 32, False)), ("state space", 1024, (2, 2, 2, 256, 256, False)), ("state space", 31, None),
+    ("gated delta rule", 64, (16, 4, 128, 8, 64, False)), ("gated delta rule", 1024, (16, 4, 128, 68, 256, False)), ("gated delta rule", 32, None),
+    ("gated linear attention", 256, (1, 0, 0, 256, 0, False)), ("gated linear attention", 224, None)])
+def test_a_recorded_step_allows_for_every_spread_of_its_tokens(kind, tokens, want):
     """It has room for 256 requests and is replayed with other lengths: neither its rows nor the lengths at hand count."""
-    assert K._split(_batch([tokens], room=256, extras={"recorder": object()}), tokens, least) == (most, False)
-    assert K._split(_batch([tokens - 1, 1]), tokens, least) == (2, True)
-    assert K._split(_batch([tokens]), tokens, tokens + 1) is None
+    assert K._split(_batch([tokens], room=256, extras={"recorder": object()}), tokens, *RULES[kind]) == want
+
+
+def test_the_rules_are_those_of_the_kernels():
+    assert RULES == {"state space": (K.SCAN_CHUNKED_MIN_TOKENS, *K.SCAN_CHUNKED_LENGTHS), "gated linear attention": (K.GLA_CHUNKED_MIN_TOKENS,),
+                     "gated delta rule": (K.DELTA_CHUNKED_MIN_TOKENS, *K.DELTA_CHUNKED_LENGTHS)}
 
 
 def test_a_decode_step_has_no_chunks():
