@@ -18,8 +18,10 @@
 // What bounds it: the chain of chunks, with three barriers in each.  A block therefore takes few columns of a head's state (16
 // or 32), and whatever does not depend on the state is taken out of the chain.  2,048 tokens of one sequence, heads of 128 x 128:
 // 16 heads (128 blocks of 16 columns) 111 us against 733 token by token (pb_gated_delta_scan), 32 heads (128 of 32) 196 against 750;
-// sequences of 592 and 1,185 tokens, 16 heads, 118 against 432; 64 tokens 24 against 28, 32 tokens 24 against 16.  Against 64-bit:
-// output 0.9 to 2.1e-7 (token by token 1.1e-7 to 3.2e-6), state 0.4 to 2.9e-7 (0.5e-7 to 9e-6: the slower the decay the larger).
+// sequences of 592 and 1,185 tokens, 16 heads, 118 against 432; 64 tokens from memory 25 against 31, 32 tokens 25 against 21.  Error against
+// 64-bit where decays are slow (a step of 1e-3): output 1.0 to 2.1e-7 (token by token 2.1e-7 to 3.2e-6), state 0.4 to 2.9e-7 (0.7e-7 to
+// 9e-6); where they are fast (0.05 and more) it is up to 1.7 times the tokens' in their place: 0.9 to 1.9e-7 (1.1 to 1.6e-7), state 0.4
+// to 1.3e-7 (0.5 to 1.4e-7).
 #include "mma_sync.cuh"
 #include "sequences.cuh"
 
@@ -36,7 +38,6 @@ constexpr int DC_MUL = 256, DC_ALL = 384;                   // multiplying threa
 // beta, exp(l) / (|q| sqrt(D)), exp(l_last - l) / |k| - exp(l_last), and the first token whose key, beta or decay is not finite
 constexpr int DC_TILE = 3 * 32 * 16, DC_TRI = 10 * DC_TILE, DC_NUM = 2 * DC_TRI, DC_BLOB = DC_NUM + 4 * DC_L * 4 + 16;
 
-__device__ __forceinline__ float dc_softplus(float x) { return x > 20.0f ? x : log1pf(expf(x)); }
 __device__ __forceinline__ int dc_tri(int i) { return i * (i + 1) / 2; }
 
 template <int D>
@@ -107,7 +108,7 @@ delta_prepare_kernel(const bf16* u, long long ld_u, const bf16* b_in, long long 
         finite = __all_sync(0xffffffffu, finite);
         if (lane == e) {
             const float bt = tt < cnt ? 1.0f / (1.0f + expf(-braw)) : 0.f;
-            const float lg = tt < cnt ? -rate * dc_softplus(araw + bias) : 0.f;      // a token past the end: decay 1, nothing written
+            const float lg = tt < cnt ? -rate * pb_softplus(araw + bias) : 0.f;      // a token past the end: decay 1, nothing written
             ik[tt] = 1.0f / sqrtf(sk + 1e-6f);
             iq[tt] = q_scale / sqrtf(sq + 1e-6f);
             beta[tt] = bt;
@@ -277,17 +278,6 @@ struct DcLayout {
     static_assert(half % 16 == 0 && blob % 16 == 0 && s % 16 == 0 && bytes <= 227 * 1024, "shared memory");
 };
 
-// acc[0] += the products of A's and B's largest parts, acc[1] += the other five of the six that count.  a: three parts of an A
-// operand; b[p]: the two registers of an n8 tile of B's part p.
-__device__ __forceinline__ void dc_mma6(float (&big)[4], float (&small)[4], const unsigned (&a)[3][4], const unsigned (&b)[3][2]) {
-    pb_mma(small, a[2], b[0][0], b[0][1]);
-    pb_mma(small, a[1], b[1][0], b[1][1]);
-    pb_mma(small, a[0], b[2][0], b[2][1]);
-    pb_mma(small, a[1], b[0][0], b[0][1]);
-    pb_mma(small, a[0], b[1][0], b[1][1]);
-    pb_mma(big, a[0], b[0][0], b[0][1]);
-}
-
 // The walk over a head's chunks.  A block is one head's state [D, PB columns] and twelve warps.  Warps 8-11 fetch the next
 // chunk's K, Q, V and what the first kernel left while the others work.  Warps 0-3 make K S and from it R, warps 4-7 Q S; all
 // eight make U (a row tile and half of the columns each); then warps 4-7 finish the outputs and warps 0-3 the state, which lives in
@@ -454,7 +444,7 @@ __device__ __forceinline__ void dc_sequence(unsigned char* dw_sm, const bf16* u,
 #pragma unroll
                 for (int q = 0; q < HT; ++q) {
                     const unsigned bq[3][2] = {{b[0][2 * q], b[0][2 * q + 1]}, {b[1][2 * q], b[1][2 * q + 1]}, {b[2][2 * q], b[2][2 * q + 1]}};
-                    dc_mma6(big[q], small[q], a, bq);
+                    pb_mma6(big[q], small[q], a, bq);
                 }
             }
             const float wa = num[3 * DC_L + ta], wb = num[3 * DC_L + tb];
@@ -492,7 +482,7 @@ __device__ __forceinline__ void dc_sequence(unsigned char* dw_sm, const bf16* u,
 #pragma unroll
                         for (int e = 0; e < 2; ++e) {
                             const unsigned bq[3][2] = {{b[0][2 * e], b[0][2 * e + 1]}, {b[1][2 * e], b[1][2 * e + 1]}, {b[2][2 * e], b[2][2 * e + 1]}};
-                            dc_mma6(big[q + e], small[q + e], a, bq);
+                            pb_mma6(big[q + e], small[q + e], a, bq);
                         }
                     }
                 }

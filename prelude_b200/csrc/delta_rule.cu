@@ -8,11 +8,12 @@
 //
 // Unit norms, sigmoid, softplus, exponentials, the state and every sum over it are float32 whatever the run's type;
 // q, k, v (the convolutions' outputs) and the projections b and a are of the run's type.  A sequence's tokens are
-// visited in order by the same threads with the same operations, so the result does not depend on how a prompt was
-// cut into steps or on what else is in the batch.  The state of a sequence is read at the start of a step from its
+// visited in order by the same threads with the same operations, so here the result does not depend on how a prompt was
+// cut into steps or on what else is in the batch.  (In bfloat16 the longer sequences of a prompt step run by chunks, delta_chunk.cu,
+// which changes the last bits.)  The state of a sequence is read at the start of a step from its
 // slot and written back at the end.  Sequences are found through device arrays (cumulative lengths, state slots), one
 // block row per sequence the arrays have room for; a row whose length is not positive is skipped, so the launch has
-// the same shape whatever the step holds and can be recorded.  (A prompt step in bfloat16 runs by chunks: delta_chunk.cu.)
+// the same shape whatever the step holds and can be recorded.
 //
 // A block is eight warps on one head's state, 16 columns p of it.  Warps 0-3 compute: 16 columns x 8 lanes over the
 // state rows n, a lane keeping NPL rows in registers (rows 4 (8 i + j) .. + 3, so that the lanes of a column read
@@ -28,8 +29,6 @@ namespace {
 
 #define GD_COLS 16
 #define GD_LANES 8
-
-__device__ __forceinline__ float gd_softplus(float x) { return x > 20.0f ? x : log1pf(expf(x)); }
 
 template <int NPL>
 struct GdLayout {
@@ -112,7 +111,7 @@ __device__ __forceinline__ void gd_sequence(float* sm, const T* u_in, long long 
             if (lane < GD_COLS) dst[2 * NPAD + lane] = vv[u];
             if (lane == 0) {
                 dst[2 * NPAD + GD_COLS] = 1.0f / (1.0f + expf(-braw[u]));
-                dst[2 * NPAD + GD_COLS + 1] = expf(-rate * gd_softplus(araw[u] + bias));
+                dst[2 * NPAD + GD_COLS + 1] = expf(-rate * pb_softplus(araw[u] + bias));
             }
         }
     };

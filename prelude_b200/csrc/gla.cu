@@ -8,10 +8,11 @@
 //   pb_gla_step         one token per sequence (a decode step): decay, recurrence, norm per head and gate in one kernel
 //
 // Decays and their logarithms, the state and every sum over it are float32 whatever the run's type; q, k, v and x1
-// (projections) are of the run's type.  A sequence's tokens are visited in order; a token's numbers do not depend on how a
+// (projections) are of the run's type.  A sequence's tokens are visited in order; a token's numbers do not depend here on how a
 // prompt was cut into steps or on what else is in the batch.  Sequences are found through device arrays (cumulative
 // lengths, state slots), one block row per sequence the arrays have room for: a row whose length is not positive is
-// skipped, so the launches can be recorded.  (A prompt step in bfloat16 runs the recurrence by sixteen tokens: gla_chunk.cu.)
+// skipped, so the launches can be recorded.  (A prompt step in bfloat16 runs the recurrence by sixteen tokens,
+// which changes the last bits: gla_chunk.cu.)
 #include "common.cuh"
 
 #include <math.h>

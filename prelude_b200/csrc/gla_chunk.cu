@@ -20,7 +20,7 @@
 //
 // Measured against token by token (gla.cu), both kernels, heads of 128 x 128: 2,048 tokens 276 -> 177 us of 32 heads, 298 -> 148 of 16;
 // 1,777 tokens of two sequences, 16 heads: 160 -> 100; 256 tokens of 32: 38 -> 31.  Error against 64 bits 0.6 - 1.9e-7 in the outputs and
-// 0.01 - 2.0e-7 in the state (token by token 0.6 - 2.5e-7 and 0.01 - 2.6e-7).  The walk issues in 46 % of the cycles, the tensor units work in
+// 0.01 - 2.0e-7 in the state (token by token 0.6 - 2.5e-7 and 0.01 - 2.6e-7; decays of 0.9 to 1 a tenth farther than they, of 0.99 to 1 a fifth nearer).  The walk issues in 46 % of the cycles, the tensor units work in
 // 30 %: the rest is the fixed latencies of its chain.
 #include "mma_sync.cuh"
 #include "sequences.cuh"
@@ -215,16 +215,6 @@ struct GcLayout {
     static_assert(v % 16 == 0 && half % 16 == 0 && o % 16 == 0 && bytes <= 227 * 1024, "shared memory");
 };
 
-// Products of two operands in three parts each: the largest into `big`, the other five that count into `small`.
-__device__ __forceinline__ void gc_mma6(float (&big)[4], float (&small)[4], const unsigned (&a)[3][4], const unsigned (&b0)[3], const unsigned (&b1)[3]) {
-    pb_mma(small, a[2], b0[0], b1[0]);
-    pb_mma(small, a[1], b0[1], b1[1]);
-    pb_mma(small, a[0], b0[2], b1[2]);
-    pb_mma(small, a[1], b0[0], b1[0]);
-    pb_mma(small, a[0], b0[1], b1[1]);
-    pb_mma(big, a[0], b0[0], b1[0]);
-}
-
 // The walk.  A block is one head's state [N, PB columns] and twelve warps.  Warps 0-7 multiply: warp (n, g) owns channels 16 n ..
 // 16 n + 15 of column group g.  Warps 8-11: while the others work on one sixteen they add up the shares of the outputs of the one
 // before and bring what the first kernel left of the next one, and its v, and what is three sixteens ahead on its way, into shared memory.  One barrier a
@@ -360,7 +350,8 @@ __device__ __forceinline__ void gc_sequence(unsigned char* gc_sm, const bf16* v_
                 unsigned b0[3], b1[3];
                 pb_split3(st[a][0][2 * b], st[a][0][2 * b + 1], b0);
                 pb_split3(st[a][1][2 * b], st[a][1][2 * b + 1], b1);
-                gc_mma6(big[a][b], small[a][b], qf, b0, b1);
+                const unsigned sb[3][2] = {{b0[0], b1[0]}, {b0[1], b1[1]}, {b0[2], b1[2]}};
+                pb_mma6(big[a][b], small[a][b], qf, sb);
             }
         // the weights times v: 8 columns each from some of the warps
         constexpr int TILES = PW / 8;

@@ -38,6 +38,17 @@ __device__ __forceinline__ void pb_split3(float a, float b, unsigned (&out)[3]) 
     }
 }
 
+// A product of two operands in three parts each, of whose nine products the six that reach float32's last bit are taken: the largest
+// into `big`, the other five into `small`.  a: three parts of an A operand; b[p]: the two registers of an n8 tile of B's part p.
+__device__ __forceinline__ void pb_mma6(float (&big)[4], float (&small)[4], const unsigned (&a)[3][4], const unsigned (&b)[3][2]) {
+    pb_mma(small, a[2], b[0][0], b[0][1]);
+    pb_mma(small, a[1], b[1][0], b[1][1]);
+    pb_mma(small, a[0], b[2][0], b[2][1]);
+    pb_mma(small, a[1], b[0][0], b[0][1]);
+    pb_mma(small, a[0], b[1][0], b[1][1]);
+    pb_mma(big, a[0], b[0][0], b[0][1]);
+}
+
 // Addresses for ldmatrix.x4 of a lane, in elements of a row-major tile with row stride `ld`:
 //   an A operand [16 rows m][16 columns k]; and two n8 tiles of a B operand stored [k][n], read transposed (n 0-7: r0, r1;
 //   n 8-15: r2, r3)

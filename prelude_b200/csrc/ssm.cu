@@ -12,11 +12,12 @@
 //                           after the norm, y brought to unit root mean square in equal parts, times a scale, times silu(z)
 //
 // Decay, step size, softplus, exponentials, the state and the sums over it are float32 whatever the run's type;
-// the projections and the convolution's output are of the run's type.  A sequence's tokens are visited in order,
-// one after the other, by the same threads: the result does not depend on how a prompt was cut into steps or on
-// what else is in the batch.  (A prompt step in bfloat16 runs the state-space recurrence by chunks: ssm_chunk.cu.)  All kernels find a step's sequences through device arrays (cumulative lengths,
-// state slots), with one block row per sequence the arrays have room for: a row whose length is not positive is
-// skipped, so the launches have the same shape whatever the step holds and can be recorded.
+// the projections and the convolution's output are of the run's type.  A scan here visits a sequence's tokens in order,
+// one after the other, by the same threads.  In 32-bit all results are therefore the same however a prompt was cut into steps and
+// whatever else is in the batch.  In bfloat16 the state-space recurrence is not, in the last bits: a prompt step runs it by chunks
+// (ssm_chunk.cu), but for sequences of one token, which pb_ssm_step visits; and the gated norm's order of sums follows the number of
+// rows.  All kernels find a step's sequences through device arrays (cumulative lengths, state slots): a row whose length is not positive
+// is skipped, so the launches have the same shape whatever the step holds and can be recorded.
 #include "sequences.cuh"
 
 #include <math.h>
@@ -43,8 +44,6 @@ __device__ __forceinline__ void pb_st_vec(__nv_bfloat16* p, const float (&v)[8])
     for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
     *reinterpret_cast<uint4*>(p) = raw;
 }
-__device__ __forceinline__ float softplus_f(float x) { return x > 20.0f ? x : log1pf(expf(x)); }
-
 // ---------------------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void causal_conv_silu_kernel(const T* in, long long ld_in, const float* w,
@@ -305,7 +304,7 @@ ssm_scan_kernel(const T* u, long long ld_u, const T* dt_in, long long ld_dt, con
             if (idx < cnt * SCAN_COLS) buf[2 * CHUNK * NPAD + idx] = xv[it];
         }
         if (!FIXED && lt < cnt) {
-            const float dt = softplus_f(dt_raw + bias);
+            const float dt = pb_softplus(dt_raw + bias);
             buf[2 * CHUNK * NPAD + CHUNK * SCAN_COLS + lt] = dt;
             buf[2 * CHUNK * NPAD + CHUNK * SCAN_COLS + CHUNK + lt] = expf(neg_a * dt);
         }
@@ -361,7 +360,8 @@ ssm_scan_kernel(const T* u, long long ld_u, const T* dt_in, long long ld_dt, con
 // One token per sequence (a decode step, or those sequences of any step: `which`) in bfloat16: a block owns a head's state, a thread four columns and every 16th (or so) row of
 // it, eight rows' pieces under way at a time; the rows' shares of the output meet in shared memory in their order.  What bounds it is
 // the state, read and written once.  (The scan above reads it 16 bytes of a row at a time, and makes ready for a chunk of
-// sixteen tokens: 2 sequences, 128 heads of 128 x 64, 16.3 us, here 6.7.)
+// sixteen tokens: 2 sequences, 128 heads of 128 x 64, 16.3 us, here 6.7.)  Beside a prompt portion it takes the sequences of one token:
+// 60 of them and a portion of 64, 64 heads of 128 x 64, 68 us against 211 by chunks and 193 token by token.
 #define SSM_STEP_THREADS 256
 #define SSM_STEP_ROWS 8
 // RECORDED as in delta_rule.cu.
@@ -384,7 +384,7 @@ ssm_step_kernel(const __nv_bfloat16* u, const __nv_bfloat16* dt_in, long long ld
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
         if (works) {
             const uint2 xr = *reinterpret_cast<const uint2*>(row + h * P + 4 * c);
-            const float dt = softplus_f(pb_ld(dt_in + (size_t)t * ld_dt + h) + bias), decay = expf(neg_a * dt);
+            const float dt = pb_softplus(pb_ld(dt_in + (size_t)t * ld_dt + h) + bias), decay = expf(neg_a * dt);
             const float2 x0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&xr.x)), x1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&xr.y));
             const float4 dx = make_float4(dt * x0.x, dt * x0.y, dt * x1.x, dt * x1.y);
             const __nv_bfloat16* B = row + inner + g * N;

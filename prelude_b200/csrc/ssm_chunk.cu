@@ -14,8 +14,10 @@
 // What bounds it: the chain of chunks (a block owns a head's state and cannot start a chunk before the one ahead is done) and, in
 // a chunk, the warp products and the operand loads from shared memory that feed them.  2,048 tokens, state 128 x 64: 64 heads
 // (128 blocks of 32 columns) 114 us against 481 token by token on the float32 units (pb_ssm_scan), 128 heads (128 blocks of 64)
-// 164 against 962; 64 tokens 11.5 against 20, 32 tokens 12 each.  Against 64-bit: output 1.4 to 1.8e-7 (token by token 0.9e-7 to
-// 1.3e-6), state 0.5 to 2.6e-7 (0.5e-7 to 5.6e-6: the slower the decay, the more roundings pile up there).
+// 164 against 962; 64 heads, 64 tokens from memory 14 against 27, 32 tokens 12 against 18.  Error against 64-bit where decays are slow (a
+// step of 1e-3): output 1.4 to 1.8e-7 (token by token 1.6e-7 to 1.3e-6: the more tokens a decay leaves, the more roundings pile up
+// there), state 0.3 to 2.6e-7 (2.2e-7 to 5.6e-6); where they are fast (0.05 and more) it is up to twice the tokens' in their place:
+// 0.9 to 1.7e-7 (0.9 to 1.1e-7), state 0.5 to 1.3e-7 (0.5 to 1.2e-7).
 //
 // A block is one head's state [N, PB columns] and twelve warps.  Warps 8-11 fetch: while the others work on one chunk they
 // bring the next chunk's B, C and x into the other half of shared memory and make its sums of logarithms and its weighted x.
@@ -42,8 +44,6 @@ struct ScLayout {
     static constexpr int s = 2 * half, yx = s + 3 * N * LDP * 2, bytes = yx + SC_L * LDY * 4;
     static_assert(half % 16 == 0 && bytes <= 227 * 1024, "shared memory");
 };
-
-__device__ __forceinline__ float sc_softplus(float v) { return v > 20.0f ? v : log1pf(expf(v)); }
 
 // One sequence's tokens through one head's columns p_first ..; all threads of the block.
 template <int N, int PB>
@@ -89,7 +89,7 @@ __device__ __forceinline__ void sc_sequence(unsigned char* sc_sm, const bf16* u,
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
                 const int tt = 2 * lane + e;
-                dt[e] = tt < cnt ? sc_softplus(pb_ld(dt_in + (size_t)(first + t0 + tt) * ld_dt + h) + bias) : 0.f;
+                dt[e] = tt < cnt ? pb_softplus(pb_ld(dt_in + (size_t)(first + t0 + tt) * ld_dt + h) + bias) : 0.f;
                 const float a = neg_a * dt[e];
                 l[e] = a < -110.0f ? -110.0 : (double)a;                          // a token past the end: decay 1
             }

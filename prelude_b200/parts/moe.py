@@ -181,7 +181,6 @@ class RoutedExperts:
             status = L.tc_status(x.device)
             h = K.moe_gemm_pair(K.moe_gather_rows(x, plan, s.top_k), self.w_gate_up, plan, self.gated, status, **self.act)
             return self._sum(K.moe_gemm_pair(h, self.w_down, plan, False, status), plan.place_of, weights, shared, x.dtype)
-        # tiles of 128 rows where the experts have many rows each and the tensor-core kernel takes the shapes, else of 64
         small = x.dtype != torch.bfloat16 or s.hidden_size % 8 or s.expert_size % 8
         few = not small and x.shape[0] * s.top_k <= MOE_FEW_ROWS * s.n_experts       # a decode step: stream the weights
         if few and K.moe_gemv_takes(x, self.w_gate_up, ids.numel()):
@@ -194,6 +193,8 @@ class RoutedExperts:
             status = L.tc_status(x.device)
             h = K.moe_gemm_grouped(K.moe_gather_rows(x, plan, s.top_k), self.w_gate_up, plan, self.gated, status, **self.act)
             return self._sum(K.moe_gemm_grouped(h, self.w_down, plan, False, status, torch.float32), plan.place_of, weights, shared, x.dtype)
+        # what the paired blocks do not take: tiles of 128 rows where the experts have many rows each and the mma.sync kernel takes the
+        # shapes, else of 64
         plan = K.moe_sort(ids, s.n_experts, 64 if (small or few) else None)
         h = K.moe_gemm(x, self.w_gate_up, plan, gated=self.gated, gather_div=s.top_k, few_rows=few, **self.act)
         y = K.moe_gemm(h, self.w_down, plan, gated=False, out_dtype=torch.float32, few_rows=few)
