@@ -1074,18 +1074,23 @@ class _Split(NamedTuple):
 
 def _split(batch, T: int, min_tokens: int, length: int = 1, few: int = 0, beside: int = 1) -> Optional[_Split]:
     """The parts of a step of T tokens, by chunks from ``min_tokens`` on: all sequences where no more than ``few`` have fewer than
-    ``length`` tokens, else those of ``beside`` tokens (which is no less).  None: nothing runs by chunks."""
+    ``length`` tokens, else those of ``beside`` tokens (which is no less).  None: nothing runs by chunks.  Where all run one way the
+    launches serve other lengths too; where they part, a capture by whoever it is takes the form that a recorded step does."""
     if batch.decode_only or T < min_tokens:
         return None
     n_seqs, length = batch.cu_q.numel() - 1, min(length, min_tokens)
-    if batch.extras.get("recorder") is not None or batch.q_lens.shape[0] != n_seqs:
-        if length == 1:
-            return _Split(1, 0, 0, min(n_seqs, T), 0, False)
-        return _Split(length, few, beside, min(n_seqs, T // length + few), min(n_seqs, T), False)
-    if length == 1 or int((batch.q_lens < length).sum()) <= few:
-        return _Split(1, 0, 0, n_seqs, 0, True)
-    n_short = int((batch.q_lens < beside).sum())
-    return _Split(beside, 0, 0, n_seqs - n_short, n_short, True) if n_short < n_seqs else None
+    recorded = batch.extras.get("recorder") is not None or batch.q_lens.shape[0] != n_seqs
+    if length == 1:
+        return _Split(1, 0, 0, min(n_seqs, T), 0, False) if recorded else _Split(1, 0, 0, n_seqs, 0, True)
+    if not recorded:
+        if int((batch.q_lens < length).sum()) <= few:
+            return _Split(1, 0, 0, n_seqs, 0, True)
+        n_short = int((batch.q_lens < beside).sum())
+        if n_short == n_seqs:
+            return None
+        if not (batch.cu_q.is_cuda and torch.cuda.is_current_stream_capturing()):
+            return _Split(beside, 0, 0, n_seqs - n_short, n_short, True)
+    return _Split(length, few, beside, min(n_seqs, T // length + few), min(n_seqs, T), False)
 
 
 def ssm_scan(u: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: torch.Tensor, d_skip: torch.Tensor,

@@ -3,6 +3,7 @@ and beside the kernels that visit the tokens one by one: at the chunks' edges, o
 decays from none to all, and with numbers that are not finite."""
 import math
 
+import numpy as np
 import pytest
 import torch
 
@@ -385,3 +386,29 @@ def test_a_recorded_step_runs_what_a_launched_one_does(kind, H, lens, room, monk
     again = state.clone()
     got = run(again, full)
     assert torch.equal(got[:sum(lens)], y[:sum(lens)]) and torch.equal(again, plain)
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("first", [[1] * 20 + [100, 80], [10] * 2 + [9] * 20, [180] + [0] * 20 + [20], [9] * 21 + [11]])
+def test_a_captured_call_serves_other_lengths(kind, first, monkeypatch):
+    """A graph of the call, replayed after the cumulative lengths have been filled anew: the same as a call of its own."""
+    _thresholds(monkeypatch, 24, (24, 2, 60))
+    others = [[1] * 20 + [90, 90], [60, 61, 2, 20, 24, 33] + [0] * 16, [200] + [0] * 21, [9] * 20 + [10, 10]]
+    run, state = _scan(kind, first, 16)
+    held = _batch([max(n, 1) for n in first])
+    held.cu_q = torch.tensor([sum(first[:r]) for r in range(len(first) + 1)], dtype=torch.int32, device=DEV)
+    held.q_lens = np.asarray(first, np.int32)
+    mine = state.clone()
+    run(mine, held)                                         # the library's attributes, the allocator's memory
+    mine.copy_(state)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = run(mine, held)
+    for lens in others:
+        held.cu_q.copy_(torch.tensor([sum(lens[:r]) for r in range(len(lens) + 1)], dtype=torch.int32))
+        mine.copy_(state)
+        graph.replay()
+        want_s, b = state.clone(), _batch([max(n, 1) for n in lens])
+        b.cu_q, b.q_lens = held.cu_q, np.asarray(lens, np.int32)
+        want = run(want_s, b)
+        assert _rel(y, want.double()) < 2e-6 and _rel(mine, want_s.double()) < 2e-6
