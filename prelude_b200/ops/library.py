@@ -40,6 +40,8 @@ _SIGNATURES = {
     "pb_sample": ([P, L, I, I, P, P, P, P, P, P], I),
     "pb_softmax_temperature": ([P, L, I, I, P, P, P], I),
     "pb_philox_uniform": ([c_uint64, c_uint64], F),
+    "pb_attention_latent_supported": ([I, I, I, I, I], I),
+    "pb_attention_latent_bf16": ([P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, F, I, P, L, I, I, P, P], I),
     "pb_attention_prefill_bf16": ([P, P, P, P, P, I, P, P, P, P, P, P, I, I, I, I, I, I, I, F, I, I, P, P], I),
     "pb_attention_prefill_tc_supported": ([I, I, I, I, I], I),
     "pb_attention_prefill_tc_tile_tokens": ([I, I], I),

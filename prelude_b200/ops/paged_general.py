@@ -2,6 +2,9 @@
 cached key rows, a window, a sink.  Picks the kernel for the type and shape; which one ran changes the rounding,
 never what is computed.
 
+A decode step over a latent that is key and value at once, with rows enough, goes to the tcgen05 kernel for such steps
+(``latent_takes``); all else as follows.
+
 float32 always runs the plain warp-per-row kernel.  bfloat16 runs the tensor-core kernel where it takes the shape
 (key size in multiples of 16, value size in multiples of 32 up to 512), prompt portions and single tokens alike; a
 step of few rows has its keys dealt to several blocks per row (PRELUDE_GENERAL_ATTN=plain turns it off).  Prompt
@@ -25,6 +28,10 @@ from .library import check
 KERNEL = os.environ.get("PRELUDE_GENERAL_ATTN", "auto")
 PROMPT_KERNEL = os.environ.get("PRELUDE_GENERAL_PROMPT_ATTN", "auto")
 MAX_SPLITS = 32
+# rows that a token sees, at most, from which a decode step over a latent goes to the tcgen05 kernel, of few tokens and of more (32
+# heads, us there / on the general kernel: 512 rows, 2 tokens 11.6 / 10.7, 8 tokens 11.8 / 12.2, 16 tokens 13.7 / 17.3; 3,000 rows, 1 token
+# 15.7 / 20.5, 16 tokens 22.2 / 42.7; 64 rows, 16 tokens 12.2 / 9.5)
+LATENT_MIN_ROWS, LATENT_FEW_TOKENS, LATENT_MIN_ROWS_FEW = 512, 8, 1024
 
 
 def tc_takes(q: torch.Tensor, k_pages: torch.Tensor, v_pages: Optional[torch.Tensor], value_dim: int) -> bool:
@@ -34,6 +41,30 @@ def tc_takes(q: torch.Tensor, k_pages: torch.Tensor, v_pages: Optional[torch.Ten
     if v_pages is not None and v_pages.shape[1] != G:
         return False
     return bool(_l.library().pb_attention_paged_tc_supported(H, G, kd, value_dim, 1 if v_pages is None else 0))
+
+
+def latent_takes(q: torch.Tensor, k_pages: torch.Tensor, v_pages: Optional[torch.Tensor], value_dim: int, batch, keep_first: int,
+                 chunk: Optional[int], softcap: Optional[float], context: int = LATENT_MIN_ROWS_FEW) -> bool:
+    """Whether the tcgen05 kernel for single tokens over a shared latent takes the call: values inside the key rows, no mask but the
+    causal one and a window, no cap, and rows enough (``LATENT_MIN_ROWS``; ``context``: those that a token sees at most)."""
+    if (KERNEL == "plain" or q.dtype != torch.bfloat16 or not batch.decode_only or v_pages is not None or keep_first or chunk or softcap
+            or context < (LATENT_MIN_ROWS if q.shape[0] >= LATENT_FEW_TOKENS else LATENT_MIN_ROWS_FEW)):
+        return False
+    return bool(_l.library().pb_attention_latent_supported(q.shape[1], k_pages.shape[1], q.shape[2], value_dim, k_pages.shape[2]))
+
+
+def attention_latent(q: torch.Tensor, k_pages: torch.Tensor, value_dim: int, batch, group: int, scale: float, window: Optional[int],
+                     sink: Optional[torch.Tensor], gate: Optional[torch.Tensor], out: torch.Tensor, parts: int = 0) -> torch.Tensor:
+    """``attention_general`` on that kernel.  ``parts`` (tests): blocks that share a token's rows."""
+    table = batch.block_tables[group]
+    num_pages, G, page_size, kd = k_pages.shape
+    T, H, _ = q.shape
+    check(_l.library().pb_attention_latent_bf16(
+        q.data_ptr(), k_pages.data_ptr(), out.data_ptr(), K._ptr(sink), batch.positions.data_ptr(), batch.table_row_of_token.data_ptr(),
+        table.data_ptr(), table.shape[1], page_size, num_pages, T, H, G, kd, value_dim, float(scale), int(window or 0), K._ptr(gate),
+        0 if gate is None else gate.stride(0), batch.max_kv_len if batch.max_kv_len else table.shape[1] * page_size, parts,
+        batch.status.data_ptr(), _l.current_stream_ptr(q.device)), "attention_latent")
+    return out
 
 
 def attention_general(q: torch.Tensor, k_pages: torch.Tensor, v_pages: Optional[torch.Tensor], value_dim: int, batch, group: int,
@@ -58,6 +89,9 @@ def attention_general(q: torch.Tensor, k_pages: torch.Tensor, v_pages: Optional[
         recorder.run_between_pieces(lambda: attention_general(q, k_pages, v_pages, value_dim, batch, group, scale, window, sink, out,
                                                               keep_first, chunk, softcap, gate, below))
         return out
+    seen = batch.max_kv_len if batch.max_kv_len else batch.block_tables[group].shape[1] * k_pages.shape[2]
+    if latent_takes(q, k_pages, v_pages, value_dim, batch, keep_first, chunk, softcap, min(seen, window) if window else seen):
+        return attention_latent(q, k_pages, value_dim, batch, group, scale, window, sink, gate, out)
     lib = _l.library()
     table = batch.block_tables[group]
     num_pages, G, page_size, _ = k_pages.shape
