@@ -68,6 +68,22 @@ __device__ __forceinline__ float pb_clamped_unit(float g, float u, float limit, 
     const float a = fminf(g, limit), b = fminf(fmaxf(u, -limit), limit);
     return a / (1.0f + expf(-alpha * a)) * (b + 1.0f);
 }
+// 1 / v in one instruction, within a unit of the last place.  The rounded division takes a branch of its own every time, so that a thread's
+// divisions wait for one another, 100 cycles each: where eight or more stand side by side they are most of a kernel's time.
+__device__ __forceinline__ float pb_rcp(float v) {
+    float r;
+    asm("rcp.approx.f32 %0, %1;\n" : "=f"(r) : "f"(v));
+    return r;
+}
+// sigmoid and SiLU for a result of type T, in float32: what is rounded to bfloat16 behind it takes the reciprocal above, float32 the division
+template <typename T> __device__ __forceinline__ float pb_sigmoid_for(float v) {
+    if constexpr (sizeof(T) == 2) return pb_rcp(1.0f + expf(-v));
+    else return 1.0f / (1.0f + expf(-v));
+}
+template <typename T> __device__ __forceinline__ float pb_silu_for(float v) {
+    if constexpr (sizeof(T) == 2) return v * pb_rcp(1.0f + expf(-v));
+    else return v / (1.0f + expf(-v));
+}
 __device__ __forceinline__ float pb_softplus(float v) { return v > 20.0f ? v : log1pf(expf(v)); }
 __device__ __forceinline__ float pb_relu2(float v) { v = fmaxf(v, 0.f); return v * v; }
 __device__ __forceinline__ float pb_warp_max(float v) {

@@ -1,9 +1,11 @@
 """Differential attention over a step's batch: picks the kernel for the type and shape.
 
 float32 always runs the plain warp-per-row kernel.  bfloat16 runs the
-tensor-core kernel where it takes the shape (key and value sizes in multiples
+mma.sync kernel where it takes the shape (key and value sizes in multiples
 of 16 up to 256, at most 64 query heads per key/value head) and the plain
-kernel otherwise.  Which one ran changes the rounding, never what is computed.
+kernel otherwise; a step with prompt portions runs the tcgen05 kernel where that
+takes the shape (keys of 64, values of 64 or 128, a power of two of at most 16 query
+heads per key/value head).  Which one ran changes the rounding, never what is computed.
 
 A step of single tokens (a decode step) gives every token a tile of its own
 and cuts its keys into ranges, one block each, so that a few long requests
@@ -23,13 +25,13 @@ from . import library as _l
 from .attention import _prefill_plan, _sm_count
 from .library import check
 
-# PRELUDE_DIFF_ATTN=ref sends bfloat16 to the plain kernel as well
+# PRELUDE_DIFF_ATTN=ref sends bfloat16 to the plain kernel as well, =mma all of it to the mma.sync kernel
 KERNEL = os.environ.get("PRELUDE_DIFF_ATTN", "auto")
 # Whether the softmax weights (computed in float32) enter the second product as one bfloat16 number, as in the
 # framework's other attention kernels, or as a rounded part plus what the rounding lost (PRELUDE_DIFF_ATTN_SPLIT=1:
 # two bfloat16 numbers, 16 bits of the weight, twice the tensor-core work of that product).  Measured against
 # 64-bit logits the two differ by less than a twentieth of the error that the bfloat16 queries, keys and values
-# cause, so the single number is the default.
+# cause, so the single number is the default.  (The tcgen05 kernel always takes two.)
 SPLIT_WEIGHTS = os.environ.get("PRELUDE_DIFF_ATTN_SPLIT", "0") == "1"
 
 
@@ -83,6 +85,21 @@ def diff_attention(q: torch.Tensor, gate: Optional[torch.Tensor], k_pages: torch
             if scratch is None:
                 scratch = batch.extras[key] = torch.empty(floats, dtype=torch.float32, device=q.device)
     else:
+        # every portion, single tokens among them, on the tcgen05 kernel where it takes the shape, else on the mma.sync kernel (16 heads over 4,
+        # us there / here: 16 tokens 13.3 / 22.9, 1,024 tokens 34 / 106, 64 behind 2,000 57 / 90; 512 beside 16 single tokens behind 2,000 57 / 129)
+        gate_at = (0, None) if gate is None else (gate.stride(0), gate.data_ptr())
+        if (coef >= 0.0 and KERNEL != "mma" and lib.pb_diff_attention_tcgen05_supported(
+                spec.num_heads, spec.num_kv_heads, dim, vdim, page_size, q.stride(0), q.data_ptr(), *gate_at)):
+            tile_seq, tile_tok0, n_tiles = _prefill_plan(
+                batch, lib.pb_diff_attention_tcgen05_tile_tokens(spec.num_heads, spec.num_kv_heads), 0, None)
+            check(lib.pb_diff_attention_tcgen05_bf16(
+                q.data_ptr(), q.stride(0), K._ptr(gate), gate_at[0], k_pages.data_ptr(), v_pages.data_ptr(), out.data_ptr(),
+                table.data_ptr(), table.shape[1], batch.table_row_of_token.data_ptr(), batch.cu_q.data_ptr(), batch.q_start.data_ptr(),
+                K._ptr(tile_seq), K._ptr(tile_tok0), n_tiles, page_size, num_pages, T, spec.num_heads, spec.num_kv_heads, dim, vdim,
+                float(spec.softmax_scale), float(coef), int(every), float(lam), float(spec.norm_eps), float(1.0 - spec.lambda_init),
+                int(spec.window) if spec.window else 0, 1 if K.kv_swizzled(q.dtype, dim) else 0, 1 if K.kv_swizzled(q.dtype, vdim) else 0,
+                batch.status.data_ptr(), _l.current_stream_ptr(q.device)), "diff_attention_tcgen05")
+            return out
         tile_seq, tile_tok0, n_tiles = _prefill_plan(batch, 64 // (spec.num_heads // spec.num_kv_heads), 0, None)
     check(lib.pb_diff_attention_tc_bf16(
         q.data_ptr(), q.stride(0), K._ptr(gate), gate.stride(0) if gate is not None else 0, k_pages.data_ptr(), v_pages.data_ptr(),

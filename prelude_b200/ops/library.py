@@ -40,6 +40,9 @@ _SIGNATURES = {
     "pb_sample": ([P, L, I, I, P, P, P, P, P, P], I),
     "pb_softmax_temperature": ([P, L, I, I, P, P, P], I),
     "pb_philox_uniform": ([c_uint64, c_uint64], F),
+    "pb_diff_attention_tcgen05_supported": ([I, I, I, I, I, L, P, L, P], I),
+    "pb_diff_attention_tcgen05_tile_tokens": ([I, I], I),
+    "pb_diff_attention_tcgen05_bf16": ([P, L, P, L, P, P, P, P, I, P, P, P, P, P, I, I, I, I, I, I, I, I, F, F, I, F, F, F, I, I, I, P, P], I),
     "pb_attention_latent_supported": ([I, I, I, I, I], I),
     "pb_attention_latent_bf16": ([P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, F, I, P, L, I, I, P, P], I),
     "pb_attention_prefill_bf16": ([P, P, P, P, P, I, P, P, P, P, P, P, I, I, I, I, I, I, I, F, I, I, P, P], I),
