@@ -38,7 +38,7 @@ __global__ void silu_mul_bf16x8_kernel(const __nv_bfloat16* gu, __nv_bfloat16* o
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         float2 g = __bfloat1622float2(g2[k]), u = __bfloat1622float2(u2[k]);
-        o2[k] = __floats2bfloat162_rn(g.x / (1.0f + expf(-g.x)) * u.x, g.y / (1.0f + expf(-g.y)) * u.y);
+        o2[k] = __floats2bfloat162_rn(pb_silu_for<__nv_bfloat16>(g.x) * u.x, pb_silu_for<__nv_bfloat16>(g.y) * u.y);
     }
     *reinterpret_cast<uint4*>(out + t * inter + c) = oraw;
 }
@@ -197,7 +197,7 @@ __global__ void silu_cols_bf16x8_kernel(__nv_bfloat16* x, long long ld, long lon
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         const float2 f = __bfloat1622float2(h[k]);
-        h[k] = __floats2bfloat162_rn(f.x / (1.0f + expf(-f.x)), f.y / (1.0f + expf(-f.y)));
+        h[k] = __floats2bfloat162_rn(pb_silu_for<__nv_bfloat16>(f.x), pb_silu_for<__nv_bfloat16>(f.y));
     }
     *reinterpret_cast<uint4*>(p) = raw;
 }
@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(256) sigmoid_gate_kernel(T* y, long long ldy, 
         g[0] = gr[0];
     }
 #pragma unroll
-    for (int e = 0; e < V; ++e) pb_st(v + e, pb_ld(v + e) / (1.0f + expf(-pb_ld(g + e))));
+    for (int e = 0; e < V; ++e) pb_st(v + e, pb_ld(v + e) * pb_sigmoid_for<T>(pb_ld(g + e)));
     if constexpr (V > 1) *reinterpret_cast<uint4*>(yr) = *reinterpret_cast<const uint4*>(v);
     else yr[0] = v[0];
 }

@@ -67,7 +67,7 @@ __global__ void causal_conv_silu_kernel(const T* in, long long ld_in, const floa
                                  : pb_ld(old + (size_t)(taps - 1 + idx) * channels + c);
         acc = fmaf(w[(size_t)c * taps + j], x, acc);
     }
-    pb_st(out + (size_t)t * channels + c, silu_f(acc));
+    pb_st(out + (size_t)t * channels + c, pb_silu_for<T>(acc));
     if (advance != nullptr) {                              // the sequence's only token: the inputs move on by one
         T* st = advance + (size_t)slots[seq] * (taps - 1) * channels + c;
         for (int j = 0; j + 2 < taps; ++j) st[(size_t)j * channels] = st[(size_t)(j + 1) * channels];
@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(128) causal_conv_silu_vec_kernel(const T* in, 
             for (int e = 0; e < VN; ++e) acc[e] = fmaf(wt[e][j], x[e], acc[e]);
         }
 #pragma unroll
-        for (int e = 0; e < VN; ++e) acc[e] = silu_f(acc[e]);
+        for (int e = 0; e < VN; ++e) acc[e] = pb_silu_for<T>(acc[e]);
         pb_st_vec(out + (size_t)t * channels + c, acc);
     };
     const int seq0 = token_seq[t0];
@@ -442,7 +442,7 @@ __global__ void gated_group_rmsnorm_kernel(const float* y, const T* z, long long
     const float* yr = y + (size_t)t * inner + (size_t)part * width;
     const T* zr = z + (size_t)t * ld_z + (size_t)part * width;
     float ss = 0.f;
-    auto gate = [&](float z) { return sigmoid_gate ? 1.0f / (1.0f + expf(-z)) : silu_f(z); };
+    auto gate = [&](float z) { return sigmoid_gate ? pb_sigmoid_for<T>(z) : pb_silu_for<T>(z); };
     for (int i = threadIdx.x; i < width; i += blockDim.x) { const float v = gate_after ? yr[i] : yr[i] * gate(pb_ld(zr + i)); ss += v * v; }
     ss = pb_warp_sum(ss);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
@@ -487,7 +487,7 @@ __global__ void __launch_bounds__(256, ITERS >= 8 ? 3 : 4) gated_part_rmsnorm_ke
             else zf[i] = *reinterpret_cast<const float4*>(zr + c);
         }
     }
-    auto gate = [&](float v) { return sigmoid_gate ? 1.0f / (1.0f + expf(-v)) : silu_f(v); };
+    auto gate = [&](float v) { return sigmoid_gate ? pb_sigmoid_for<T>(v) : pb_silu_for<T>(v); };
     float ss = 0.f;
 #pragma unroll
     for (int i = 0; i < ITERS; ++i) {
@@ -548,7 +548,7 @@ __global__ void gated_block_rmsnorm_kernel(const float* y, const T* z, long long
             gv = *reinterpret_cast<const float4*>(zr);
         }
     }
-    auto gate = [&](float v) { return sigmoid_gate ? 1.0f / (1.0f + expf(-v)) : silu_f(v); };
+    auto gate = [&](float v) { return sigmoid_gate ? pb_sigmoid_for<T>(v) : pb_silu_for<T>(v); };
     const float4 v = make_float4(yv.x * gate(gv.x), yv.y * gate(gv.y), yv.z * gate(gv.z), yv.w * gate(gv.w));
     const float4 n = gate_after ? yv : v;
     const float ss = pb_warp_sum(n.x * n.x + n.y * n.y + n.z * n.z + n.w * n.w);
