@@ -5,16 +5,16 @@
 //
 // For experts with fewer rows than fill the tiles of gemm_pair.cu's grouped form: the weights are the product's 256 rows, the tokens its
 // columns, 64 to 256 of them, and the down projection's result is float32.  What bounds it are the weights, each of which is read once:
-// 64 experts of 4,096 x 2,048 with 32 rows each, both products, 577 us for 3.2 GB (5.6 TB/s) against 1,380 on the 64-row tiles of
-// moe.cu; with 128 rows 671 against 1,826.  (From 192 rows on the form with the tokens as rows is ahead, 690 against 740: a product of 128
-// or 192 columns reads as much shared memory for its rows as one of 256.)
+// 64 experts of 4,096 x 2,048 with 16 rows each, both products, 511 us for 3.2 GB (6.3 TB/s) against 1,380 on the 64-row tiles of
+// moe.cu; with 128 rows 592 against 1,826.  (From 192 rows on the form with the tokens as rows takes them, 637 against 659 with the float32
+// result here.)
 //
 // A pair's tile is 256 rows of an expert's matrix (gated: 128 gate rows and the 128 up rows of the same features, 64 of each in each
 // block) by at most 256 of its tokens.  Each block holds its 128 weight rows and half of the tokens; its tensor memory receives its rows'
 // sums for all tokens.  Tiles run along an expert's features first: the pairs of a wave share a few experts' tokens, which stay in the
 // L2 cache.
 //
-// In each block: warp 8 issues the tensor-map copies (six stages), warp 9 of the leading block the products for both, warps 0..7
+// In each block: warp 8 issues the tensor-map copies (three stages), warp 9 of the leading block the products for both, warps 0..7
 // read the sums out of tensor memory (two accumulators: one's stores overlap the next one's products).  A thread has one row, that is
 // one feature: 32 lanes write 64 bytes of a token's row.  In the gated form gate and up sums of a feature lie in
 // lanes 64 apart; the warps swap halves of every 32 columns through shared memory.  Every wait is bounded in time; a
@@ -24,6 +24,10 @@
 namespace {
 
 constexpr int GG_STEP = 64;                                 // tokens come in steps of this many, half of them in each block
+// A stage holds two copies of 64 of K: what it costs the warp that issues the products - wait, vote, election, commit - is 500 to 600 cycles,
+// longer than four products of fewer than 256 columns take.  (Stages of one copy, six of them, both products, us: 64 experts of 4,096 x 2,048
+// with 4 rows each 571, now 504; with 64 rows 584, now 536; with 160 rows 773, now 645.  gemm_pair.cu's products have 256 columns, and gained nothing.)
+constexpr int GG_STAGES = 3, GG_SUB = 2, GG_STAGE_BYTES = GG_SUB * GP_STAGE_BYTES;
 constexpr int GG_SWAP = 2 * 2 * 16 * 64 * 4;                // two sets of epilogue warps, two halves of 32 columns, 64 features
 
 // Copy boxes: a block's 128 weight rows, or 64 gate rows and 64 up rows; its tokens, 128, 64 or 32 of them.  (In copies of 16 rows, with
@@ -59,7 +63,7 @@ gemm_grouped_kernel(const __grid_constant__ GgMaps maps, GgParams p) {
     pb_grid_dep_launch();
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    __shared__ __align__(8) uint64_t full_bar[GP_STAGES], empty_bar[GP_STAGES], acc_full[2], acc_empty[2];
+    __shared__ __align__(8) uint64_t full_bar[GG_STAGES], empty_bar[GG_STAGES], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_holder;
     __shared__ int s_ok;
 
@@ -71,7 +75,7 @@ gemm_grouped_kernel(const __grid_constant__ GgMaps maps, GgParams p) {
 
     if (threadIdx.x == 0) {
         s_ok = 1;
-        for (int s = 0; s < GP_STAGES; ++s) { tc_mbar_init(&full_bar[s], 1); tc_mbar_init(&empty_bar[s], 1); }
+        for (int s = 0; s < GG_STAGES; ++s) { tc_mbar_init(&full_bar[s], 1); tc_mbar_init(&empty_bar[s], 1); }
         for (int a = 0; a < 2; ++a) { tc_mbar_init(&acc_full[a], 1); tc_mbar_init(&acc_empty[a], 2 * GP_EPI_WARPS); }   // the epilogue warps of both blocks
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
@@ -94,21 +98,25 @@ gemm_grouped_kernel(const __grid_constant__ GgMaps maps, GgParams p) {
                 const int half = columns / 2, x_row = row0 + rank * half;
                 const int w_row = expert * p.expert_rows + (p.gated ? tn * 128 + rank * 64 : tn * 256 + rank * 128);
                 for (int kb = 0; kb < p.kblocks; ++kb, ++fill) {
-                    const int stage = fill % GP_STAGES;
-                    ok = tc_mbar_wait(&empty_bar[stage], ((fill / GP_STAGES) & 1) ^ 1);
+                    const int stage = fill % GG_STAGES;
+                    ok = tc_mbar_wait(&empty_bar[stage], ((fill / GG_STAGES) & 1) ^ 1);
                     if (!ok) break;
-                    unsigned char* sw = smem + stage * GP_STAGE_BYTES;
                     const uint32_t leader_full = gp_map_to_rank(tc_smem(&full_bar[stage]), 0);
-                    if (rank == 0) tc_mbar_expect_tx(&full_bar[stage], 2 * GP_A_BYTES + columns * GP_BK * 2);   // both blocks' copies land on this barrier
-                    gp_tma_load_2d(sw, &maps.w, kb * GP_BK, w_row, leader_full);
-                    if (p.gated) gp_tma_load_2d(sw + 64 * GP_BK * 2, &maps.w, kb * GP_BK, w_row + p.out_cols, leader_full);
-                    int r = 0;
+                    if (rank == 0) tc_mbar_expect_tx(&full_bar[stage], GG_SUB * (2 * GP_A_BYTES + columns * GP_BK * 2));   // both blocks' copies land on this barrier
 #pragma unroll
-                    for (int i = 0; i < 3; ++i)
-                        if (half & (128 >> i)) {
-                            gp_tma_load_2d(sw + GP_A_BYTES + r * GP_BK * 2, &maps.x[i], kb * GP_BK, x_row + r, leader_full);
-                            r += 128 >> i;
-                        }
+                    for (int sub = 0; sub < GG_SUB; ++sub) {
+                        unsigned char* sw = smem + stage * GG_STAGE_BYTES + sub * GP_STAGE_BYTES;
+                        const int k = (kb * GG_SUB + sub) * GP_BK;
+                        gp_tma_load_2d(sw, &maps.w, k, w_row, leader_full);
+                        if (p.gated) gp_tma_load_2d(sw + 64 * GP_BK * 2, &maps.w, k, w_row + p.out_cols, leader_full);
+                        int r = 0;
+#pragma unroll
+                        for (int i = 0; i < 3; ++i)
+                            if (half & (128 >> i)) {
+                                gp_tma_load_2d(sw + GP_A_BYTES + r * GP_BK * 2, &maps.x[i], k, x_row + r, leader_full);
+                                r += 128 >> i;
+                            }
+                    }
                 }
             }
             if (!ok && p.status) atomicExch(p.status, 8);
@@ -128,16 +136,19 @@ gemm_grouped_kernel(const __grid_constant__ GgMaps maps, GgParams p) {
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + acc * 256;
                 for (int kb = 0; kb < p.kblocks; ++kb, ++fill) {
-                    const int stage = fill % GP_STAGES;
-                    ok = __all_sync(0xffffffffu, tc_mbar_wait(&full_bar[stage], (fill / GP_STAGES) & 1));
+                    const int stage = fill % GG_STAGES;
+                    ok = __all_sync(0xffffffffu, tc_mbar_wait(&full_bar[stage], (fill / GG_STAGES) & 1));
                     if (!ok) break;
                     tc_fence_after();
                     if (tc_elect_one()) {
-                        const unsigned char* sw = smem + stage * GP_STAGE_BYTES;
-                        const uint64_t dw = tc_smem_desc(sw), dx = tc_smem_desc(sw + GP_A_BYTES);
 #pragma unroll
-                        for (int k = 0; k < GP_BK / 16; ++k)
-                            gp_mma2(d_tmem, dw + 2 * k, dx + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                        for (int sub = 0; sub < GG_SUB; ++sub) {
+                            const unsigned char* sw = smem + stage * GG_STAGE_BYTES + sub * GP_STAGE_BYTES;
+                            const uint64_t dw = tc_smem_desc(sw), dx = tc_smem_desc(sw + GP_A_BYTES);
+#pragma unroll
+                            for (int k = 0; k < GP_BK / 16; ++k)
+                                gp_mma2(d_tmem, dw + 2 * k, dx + 2 * k, idesc, (kb > 0 || sub > 0 || k > 0) ? 1u : 0u);
+                        }
                         gp_commit_both(&empty_bar[stage]);               // the stage is free in both blocks when these finish
                         if (kb + 1 == p.kblocks) gp_commit_both(&acc_full[acc]);
                     }
@@ -153,7 +164,7 @@ gemm_grouped_kernel(const __grid_constant__ GgMaps maps, GgParams p) {
         const int quarter = warp & 3, side = warp >> 2;
         const int row = quarter * 32 + lane;                // row of the block's half = tensor-memory lane
         const bool up_row = p.gated && quarter >= 2;
-        float* swap = reinterpret_cast<float*>(smem + GP_STAGES * GP_STAGE_BYTES) + side * (2 * 16 * 64) + (row & 63);
+        float* swap = reinterpret_cast<float*>(smem + GG_STAGES * GG_STAGE_BYTES) + side * (2 * 16 * 64) + (row & 63);
         int seg = 0;
         bool ok = true;
         for (int tile = pair; tile < n_tiles; tile += n_pairs) {
@@ -248,7 +259,7 @@ PB_API int pb_gemm_grouped_bf16(const void* A, const void* B, void* out, int pla
     p.expert_rows = expert_rows_b; p.gated = gated ? 1 : 0; p.act = act; p.limit = limit; p.alpha = alpha;
     p.tiles_m = max_m_tiles;
     p.tiles_n = gated ? (p.out_cols + 127) / 128 : (p.out_cols + 255) / 256;
-    p.kblocks = (K + GP_BK - 1) / GP_BK;
+    p.kblocks = (K + GG_SUB * GP_BK - 1) / (GG_SUB * GP_BK);          // (a copy that starts behind K brings zeros)
     p.tile_expert = tile_expert; p.tile_row0 = tile_row0; p.offsets = offsets;
     const long long tiles = (long long)p.tiles_m * p.tiles_n;
     PB_REQUIRE(tiles < (1ll << 30), "gemm_grouped: %lld tiles are too many", tiles);
@@ -259,7 +270,7 @@ PB_API int pb_gemm_grouped_bf16(const void* A, const void* B, void* out, int pla
     if (int e = gp_make_map(&maps.w, B, n_experts * expert_rows_b, K, ldb, gated ? 64 : 128)) return e;
     for (int i = 0; i < 3; ++i)
         if (int e = gp_make_map(&maps.x[i], A, places, K, lda, 128 >> i)) return e;
-    const size_t smem = (size_t)GP_STAGES * GP_STAGE_BYTES + GG_SWAP + 1024;
+    const size_t smem = (size_t)GG_STAGES * GG_STAGE_BYTES + GG_SWAP + 1024;
     static const cudaError_t set = cudaFuncSetAttribute(gemm_grouped_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     PB_REQUIRE(set == cudaSuccess, "gemm_grouped: cannot get %zu bytes of shared memory: %s", smem, cudaGetErrorString(set));
     pb_launch(gemm_grouped_kernel, dim3((unsigned)(2 * pairs)), dim3(GP_THREADS), smem, stream, maps, p);
