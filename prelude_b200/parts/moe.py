@@ -24,6 +24,7 @@ first tensor.
 """
 from __future__ import annotations
 
+import math
 import os
 from typing import Dict
 
@@ -47,6 +48,18 @@ ROUTE_FEW_TOKENS = int(os.environ.get("PRELUDE_MOE_ROUTE_FEW_TOKENS", "32"))
 # 182 against 390, 185 against 322, 195 against 485
 MOE_PAIR_MIN_ROWS = int(os.environ.get("PRELUDE_MOE_PAIR_MIN_ROWS", "192"))
 MOE_GROUPED_MIN_ROWS = int(os.environ.get("PRELUDE_MOE_GROUPED_MIN_ROWS", "3"))
+
+
+def grouped_min_rows(matrix: int, gated: bool) -> float:
+    """Average rows per expert from which the product with the weights as rows, its sort and its gather are ahead of the kernel that only streams
+    the weights, once for every (token, expert) pair; ``matrix``: elements of one of an expert's matrices.  The whole feed-forward, us, streamed
+    / there: gated, 4,096 x 2,048 1.1 rows 401 / 410, 1.5 457 / 442, 3 686 / 551, 6 1,131 / 565; 2,048 x 2,048 1.5 154 / 154, 2 180 / 172,
+    4 250 / 176; 2,048 x 768 0.5 139 / 149, 1.5 244 / 207, 4 440 / 260; without a gate, 4,096 x 2,048 0.2 135 / 137, 0.4 199 / 186, 1.5 420 / 340;
+    2,048 x 2,048 0.5 86 / 88, 1 117 / 115, 2 154 / 137; 2,048 x 768 0.25 90 / 96, 1 170 / 150; 1,024 x 512, either, 3 37 / 39, 5 41 / 39."""
+    if matrix < 3 << 19:
+        return math.inf
+    return min(1.5 if gated else 0.375 if matrix >= 8 << 20 else 1.0, MOE_GROUPED_MIN_ROWS)
+
 
 # an activation's name: (two matrices on the way up or one, its number in the products' epilogues)
 _ACTS = {"silu_gated": (True, K.ACT_NONE), "clamped_glu": (True, K.ACT_CLAMPED), "relu2": (False, K.ACT_RELU2)}
@@ -126,7 +139,7 @@ class RoutedExperts:
         shared = 0 if s.shared_size is None else 2 * s.shared_size * elem + s.hidden_size * 4
         return s.top_k * (s.expert_size * elem + s.hidden_size * 4) + s.n_experts * 4 + s.hidden_size * elem + shared
 
-    def _paired(self, x: torch.Tensor, rows: int) -> bool:
+    def _paired(self, x: torch.Tensor, rows: float) -> bool:
         """Whether a step's products can run on the paired-block kernels, and has ``rows`` rows per expert on average."""
         s = self.spec
         return (x.dtype == torch.bfloat16 and L.PREFILL_GEMM != "cublas" and s.hidden_size % 8 == 0 and s.expert_size % 8 == 0
@@ -183,11 +196,12 @@ class RoutedExperts:
             return self._sum(K.moe_gemm_pair(h, self.w_down, plan, False, status), plan.place_of, weights, shared, x.dtype)
         small = x.dtype != torch.bfloat16 or s.hidden_size % 8 or s.expert_size % 8
         few = not small and x.shape[0] * s.top_k <= MOE_FEW_ROWS * s.n_experts       # a decode step: stream the weights
-        if few and K.moe_gemv_takes(x, self.w_gate_up, ids.numel()):
+        streamed = few and K.moe_gemv_takes(x, self.w_gate_up, ids.numel())
+        if streamed and not self._paired(x, grouped_min_rows(s.hidden_size * s.expert_size, self.gated)):
             h = K.moe_gemv(x, self.w_gate_up, ids, False, x.dtype, gated=self.gated, **self.act)
             y = K.moe_gemv(h, self.w_down, ids, True, torch.float32)
             return self._sum(y, None, weights, shared, x.dtype)
-        if self._paired(x, MOE_GROUPED_MIN_ROWS):
+        if streamed or self._paired(x, MOE_GROUPED_MIN_ROWS):
             # fewer rows: the experts' weights are the rows of the paired-block products, the tokens their columns
             plan = K.moe_sort(ids, s.n_experts, 256)
             status = L.tc_status(x.device)
