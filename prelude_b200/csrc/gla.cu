@@ -60,6 +60,61 @@ __device__ __forceinline__ float gla_decay(float z, float inv_tau) {
 }
 
 // ---------------------------------------------------------------------------------------------------------
+// For ranks of 16 or 32 in bfloat16: a thread owns one channel, its row of the matrix in registers, and walks the block's tokens eight at a
+// time, two in one instruction; their narrow rows lie in shared memory turned, so that one access brings four tokens.  Sums over the rank
+// in ascending order, as below, and the same bits.  (2,048 tokens of 4,096 channels, rank 32: 58 us below, where a block has eight tokens and
+// a thread fetches its row of the matrix for them alone; 36 here.)
+template <int RANK>
+__global__ void __launch_bounds__(128) channel_decay_rows_kernel(const __nv_bfloat16* x1, long long ld_x1, const __nv_bfloat16* w2, const float* bias,
+                                                                 float inv_tau, float* out, int n_tokens, int channels, int block_tokens) {
+    extern __shared__ __align__(16) float xs[];                // [RANK][block_tokens + 4]
+    pb_grid_dep_launch();
+    const int c = blockIdx.y * blockDim.x + threadIdx.x, ld = block_tokens + 4;
+    const int t0 = blockIdx.x * block_tokens, cnt = min(block_tokens, n_tokens - t0);
+    const int cc = min(c, channels - 1);
+    const float b = bias[cc];                                  // matrix and bias are written by no kernel: before the wait
+    u64 w[RANK];
+#pragma unroll
+    for (int r = 0; r < RANK; r += 8) {
+        float f[8];
+        gla_unpack(*reinterpret_cast<const uint4*>(w2 + (size_t)cc * RANK + r), f);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) w[r + e] = pk2(f[e], f[e]);
+    }
+    pb_grid_dep_wait();
+    for (int i = threadIdx.x; i < block_tokens * (RANK / 8); i += blockDim.x) {
+        const int u = i / (RANK / 8), r = i % (RANK / 8) * 8;
+        float f[8];
+        gla_unpack(u < cnt ? *reinterpret_cast<const uint4*>(x1 + (size_t)(t0 + u) * ld_x1 + r) : make_uint4(0, 0, 0, 0), f);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) xs[(r + e) * ld + u] = f[e];
+    }
+    __syncthreads();
+    if (c >= channels) return;
+#pragma unroll 1
+    for (int u0 = 0; u0 < cnt; u0 += 8) {
+        u64 acc[4];
+#pragma unroll
+        for (int p = 0; p < 4; ++p) acc[p] = pk2(0.f, 0.f);
+#pragma unroll
+        for (int r = 0; r < RANK; ++r) {
+            const ulonglong2 lo = *reinterpret_cast<const ulonglong2*>(xs + r * ld + u0), hi = *reinterpret_cast<const ulonglong2*>(xs + r * ld + u0 + 4);
+            acc[0] = fma2(lo.x, w[r], acc[0]);
+            acc[1] = fma2(lo.y, w[r], acc[1]);
+            acc[2] = fma2(hi.x, w[r], acc[2]);
+            acc[3] = fma2(hi.y, w[r], acc[3]);
+        }
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+            const float2 z = up2(acc[p]);
+            float* o = out + (size_t)(t0 + u0 + 2 * p) * channels + c;
+            const float d0 = gla_decay(z.x + b, inv_tau), d1 = gla_decay(z.y + b, inv_tau);
+            if (u0 + 2 * p < cnt) o[0] = d0;
+            if (u0 + 2 * p + 1 < cnt) o[channels] = d1;
+        }
+    }
+}
+
 // A thread owns one channel and DECAY_TOKENS tokens, whose narrow rows the block keeps in shared memory as float32; the sum
 // over the rank runs in ascending order (as in gla_step_kernel).
 #define DECAY_TOKENS 8
@@ -500,6 +555,18 @@ PB_API int pb_channel_decay(const void* x1, long long ld_x1, const void* w2, con
     PB_REQUIRE(smem <= 48 * 1024, "channel_decay: a rank of %d (at most %d)", rank, 48 * 1024 / DECAY_TOKENS / 4);
     PB_REQUIRE((channels + 127) / 128 < 65536, "channel_decay: %d channels", channels);
     if (n_tokens == 0) return 0;
+    if (dtype == PB_BF16 && (rank == 16 || rank == 32) && n_tokens >= 64 && pb_aligned(w2, 16) && pb_aligned(x1, 16) && ld_x1 % 8 == 0) {
+        // as many tokens a block as leave the chip twice full
+        const int cols = (channels + 127) / 128, tokens = (long long)((n_tokens + 63) / 64) * cols >= 296 ? 64 : 16;
+        const dim3 grid((n_tokens + tokens - 1) / tokens, cols);
+        const size_t bytes = (size_t)rank * (tokens + 4) * sizeof(float);
+        if (rank == 16) pb_launch(channel_decay_rows_kernel<16>, grid, dim3(128), bytes, stream, (const __nv_bfloat16*)x1, ld_x1, (const __nv_bfloat16*)w2, bias, 1.0f / tau,
+                                  out, n_tokens, channels, tokens);
+        else pb_launch(channel_decay_rows_kernel<32>, grid, dim3(128), bytes, stream, (const __nv_bfloat16*)x1, ld_x1, (const __nv_bfloat16*)w2, bias, 1.0f / tau, out,
+                       n_tokens, channels, tokens);
+        PB_CHECK_LAUNCH("channel_decay");
+        return 0;
+    }
     const int vec = rank % (dtype == PB_BF16 ? 8 : 4) == 0 && pb_aligned(w2, 16) ? 1 : 0;
     PB_DISPATCH_DTYPE(dtype, T, (pb_launch(channel_decay_kernel<T>, dim3((n_tokens + DECAY_TOKENS - 1) / DECAY_TOKENS, (channels + 127) / 128), dim3(128),
                                            smem, stream, (const T*)x1, ld_x1, (const T*)w2, bias, 1.0f / tau, out, n_tokens, channels, rank, vec)));

@@ -22,6 +22,8 @@
 
 #include <math.h>
 
+#include <type_traits>
+
 namespace {
 
 __device__ __forceinline__ float silu_f(float x) { return x / (1.0f + expf(-x)); }
@@ -34,6 +36,19 @@ __device__ __forceinline__ void pb_unpack_vec(const uint4& raw, float (&out)[8])
     const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
 #pragma unroll
     for (int i = 0; i < 4; ++i) { const float2 f = __bfloat1622float2(h[i]); out[2 * i] = f.x; out[2 * i + 1] = f.y; }
+}
+// 8 bytes of a bfloat16 row as floats
+__device__ __forceinline__ void pb_unpack_vec(const uint2& raw, float (&out)[4]) {
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) { const float2 f = __bfloat1622float2(h[i]); out[2 * i] = f.x; out[2 * i + 1] = f.y; }
+}
+__device__ __forceinline__ void pb_st_vec(__nv_bfloat16* p, const float (&v)[4]) {
+    uint2 raw;
+    __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&raw);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) h[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+    *reinterpret_cast<uint2*>(p) = raw;
 }
 template <typename T, int VN> __device__ __forceinline__ void pb_ld_vec(const T* p, float (&out)[VN]) { pb_unpack_vec(*reinterpret_cast<const uint4*>(p), out); }
 __device__ __forceinline__ void pb_st_vec(float* p, const float (&v)[4]) { *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]); }
@@ -79,13 +94,15 @@ __global__ void causal_conv_silu_kernel(const T* in, long long ld_in, const floa
 // bytes; TAPS known at compile time; a long step: CONV_RUN tokens a thread, a step of few tokens: one).  A run inside one
 // sequence asks for all its rows and the TAPS - 1 before it at once, so a thread waits for memory once; the rows that two
 // runs share come from the caches.  (One token after the other with the window kept in registers waited once a token: 2,048
-// tokens of 10,240 channels 87 us, now 48 and 5 of launching.)
+// tokens of 10,240 channels 87 us, 48 in runs, 43 with the one-instruction reciprocal, now 33, with twice the warps and half the registers.)
 #define CONV_RUN 8
 template <typename T, int TAPS, int RUN>
 __global__ void __launch_bounds__(128) causal_conv_silu_vec_kernel(const T* in, long long ld_in, const float* w, const float* bias, const T* carried,
                                                                    T* out, const int32_t* token_seq, const int32_t* positions, const int32_t* q_start,
                                                                    const int32_t* slots, int n_tokens, int channels, T* advance) {
-    constexpr int VN = 16 / sizeof(T);
+    // a run's thread has 4 channels whatever the type: with 8 it takes 161 registers, and 12 warps a multiprocessor wait for memory
+    constexpr int VN = RUN > 1 ? 4 : 16 / sizeof(T);
+    using Raw = std::conditional_t<VN * sizeof(T) == 16, uint4, uint2>;
     pb_grid_dep_launch();
     const int c = (blockIdx.y * blockDim.x + threadIdx.x) * VN;
     if (c >= channels) return;
@@ -107,7 +124,7 @@ __global__ void __launch_bounds__(128) causal_conv_silu_vec_kernel(const T* in, 
     auto row = [&](int t, int i, const T* old, int idx) {
         return idx >= 0 ? in + (size_t)(t - i + idx) * ld_in + c : old + (size_t)(TAPS - 1 + idx) * channels + c;
     };
-    auto token = [&](int t, const uint4* win) {            // win[j]: the input under tap j
+    auto token = [&](int t, const Raw* win) {            // win[j]: the input under tap j
         float acc[VN];
 #pragma unroll
         for (int e = 0; e < VN; ++e) acc[e] = bs[e];
@@ -126,9 +143,9 @@ __global__ void __launch_bounds__(128) causal_conv_silu_vec_kernel(const T* in, 
     if (RUN > 1 && t0 + RUN <= n_tokens && seq0 >= 0 && token_seq[t0 + RUN - 1] == seq0) {
         const int i = positions[t0] - q_start[seq0];
         const T* old = carried + (size_t)slots[seq0] * (TAPS - 1) * channels;
-        uint4 rows[RUN + TAPS - 1];
+        Raw rows[RUN + TAPS - 1];
 #pragma unroll
-        for (int j = 0; j < RUN + TAPS - 1; ++j) rows[j] = *reinterpret_cast<const uint4*>(row(t0, i, old, i - (TAPS - 1) + j));
+        for (int j = 0; j < RUN + TAPS - 1; ++j) rows[j] = *reinterpret_cast<const Raw*>(row(t0, i, old, i - (TAPS - 1) + j));
 #pragma unroll
         for (int k = 0; k < RUN; ++k) token(t0 + k, rows + k);
         return;
@@ -138,13 +155,13 @@ __global__ void __launch_bounds__(128) causal_conv_silu_vec_kernel(const T* in, 
         if (seq < 0) continue;                             // a padding row
         const int i = positions[t] - q_start[seq];
         const T* old = carried + (size_t)slots[seq] * (TAPS - 1) * channels;
-        uint4 win[TAPS];
+        Raw win[TAPS];
 #pragma unroll
-        for (int j = 0; j < TAPS; ++j) win[j] = *reinterpret_cast<const uint4*>(row(t, i, old, i - (TAPS - 1) + j));
+        for (int j = 0; j < TAPS; ++j) win[j] = *reinterpret_cast<const Raw*>(row(t, i, old, i - (TAPS - 1) + j));
         token(t, win);
         if (RUN == 1 && advance != nullptr) {              // the sequence's only token: the inputs move on by one
 #pragma unroll
-            for (int j = 1; j < TAPS; ++j) *reinterpret_cast<uint4*>(advance + ((size_t)slots[seq] * (TAPS - 1) + j - 1) * channels + c) = win[j];
+            for (int j = 1; j < TAPS; ++j) *reinterpret_cast<Raw*>(advance + ((size_t)slots[seq] * (TAPS - 1) + j - 1) * channels + c) = win[j];
         }
     }
 }
@@ -456,32 +473,33 @@ __global__ void gated_group_rmsnorm_kernel(const float* y, const T* z, long long
         pb_st(o + i, yr[i] * gate(pb_ld(zr + i)) * inv * w[(size_t)part * width + i]);   // the same product either way
 }
 
-// The same for parts of up to 128 * ITERS elements: a warp per (token, part), four elements per access, the whole part asked for
-// at once and kept in registers between the sum and the store; the scales, which all tokens share, come from the caches when they
-// are needed.  width, ld_z in multiples of 4, operands aligned.  Parts of 1,024 (ITERS 8) on the kernel above, which reads a part
-// twice, an element an access: 2,048 x 8,192 in 80 us, here 51.
-template <typename T, int ITERS>
-__global__ void __launch_bounds__(256, ITERS >= 8 ? 3 : 4) gated_part_rmsnorm_kernel(const float* y, const T* z, long long ld_z, const float* w, T* out, int n_tokens,
+// The same for parts of up to 128 * ITERS * WARPS elements: WARPS warps per (token, part), four elements per access, the whole part asked
+// for at once and kept in registers between the sum and the store; the scales, which all tokens share, come from the caches when they
+// are needed.  width, ld_z in multiples of 4, operands aligned, fewer than 2^31 parts.  What bounds it is how much is under way: parts of
+// 1,024, 2,048 x 8,192, 80 us on the kernel above, which reads a part twice, an element an access, 33 with a warp a part (80 registers), 29 with
+// two.  (Four parts of 128 a warp: 32 us for 21.)
+template <typename T, int ITERS, int WARPS>
+__global__ void __launch_bounds__(256) gated_part_rmsnorm_kernel(const float* y, const T* z, long long ld_z, const float* w, T* out, int n_tokens,
                                                                  int inner, int parts, float eps, int gate_after, int sigmoid_gate) {
     pb_grid_dep_launch();
-    const int lane = threadIdx.x & 31, width = inner / parts;
-    const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (item >= (long long)n_tokens * parts) return;
-    const int t = (int)(item / parts), part = (int)(item % parts);
+    __shared__ float red[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, width = inner / parts, side = warp % WARPS;
+    const unsigned item = (blockIdx.x * (blockDim.x >> 5) + warp) / WARPS;
+    const bool live = item < (unsigned)n_tokens * (unsigned)parts;
+    const unsigned t = live ? item / (unsigned)parts : 0u, part = live ? item - t * (unsigned)parts : 0u;
+    const float* yr = y + (size_t)t * inner + (size_t)part * width;
+    const T* zr = z + (size_t)t * ld_z + (size_t)part * width;
     float4 yv[ITERS];
     uint2 zv[ITERS];
     float4 zf[sizeof(T) == 4 ? ITERS : 1];
-    const float* wr = w + (size_t)part * width;
     pb_grid_dep_wait();
-    const float* yr = y + (size_t)t * inner + (size_t)part * width;
-    const T* zr = z + (size_t)t * ld_z + (size_t)part * width;
 #pragma unroll
     for (int i = 0; i < ITERS; ++i) {
-        const int c = (lane + 32 * i) * 4;
+        const int c = (lane + 32 * (side + WARPS * i)) * 4;
         yv[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         zv[i] = make_uint2(0, 0);
         if constexpr (sizeof(T) == 4) zf[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (c < width) {
+        if (c < width && live) {
             yv[i] = *reinterpret_cast<const float4*>(yr + c);
             if constexpr (sizeof(T) == 2) zv[i] = *reinterpret_cast<const uint2*>(zr + c);
             else zf[i] = *reinterpret_cast<const float4*>(zr + c);
@@ -504,23 +522,23 @@ __global__ void __launch_bounds__(256, ITERS >= 8 ? 3 : 4) gated_part_rmsnorm_ke
         ss += n.x * n.x + n.y * n.y + n.z * n.z + n.w * n.w;
         yv[i] = v;                                             // the same product either way
     }
-    const float inv = 1.0f / sqrtf(pb_warp_sum(ss) / (float)width + eps);
+    ss = pb_warp_sum(ss);
+    if constexpr (WARPS == 2) {
+        if (lane == 0) red[warp] = ss;
+        __syncthreads();
+        ss = red[warp & ~1] + red[warp | 1];
+    }
+    if (!live) return;
+    const float inv = 1.0f / sqrtf(ss / (float)width + eps);
     T* o = out + (size_t)t * inner + (size_t)part * width;
+    const float* wr = w + (size_t)part * width;
 #pragma unroll
     for (int i = 0; i < ITERS; ++i) {
-        const int c = (lane + 32 * i) * 4;
+        const int c = (lane + 32 * (side + WARPS * i)) * 4;
         if (c < width) {
             const float4 wv = *reinterpret_cast<const float4*>(wr + c);
             const float r[4] = {yv[i].x * inv * wv.x, yv[i].y * inv * wv.y, yv[i].z * inv * wv.z, yv[i].w * inv * wv.w};
-            if constexpr (sizeof(T) == 2) {
-                const __nv_bfloat162 a = __floats2bfloat162_rn(r[0], r[1]), b = __floats2bfloat162_rn(r[2], r[3]);
-                uint2 raw;
-                raw.x = *reinterpret_cast<const uint32_t*>(&a);
-                raw.y = *reinterpret_cast<const uint32_t*>(&b);
-                *reinterpret_cast<uint2*>(o + c) = raw;
-            } else {
-                *reinterpret_cast<float4*>(o + c) = make_float4(r[0], r[1], r[2], r[3]);
-            }
+            pb_st_vec(o + c, r);
         }
     }
 }
@@ -593,7 +611,7 @@ PB_API int pb_causal_conv_silu(const void* in, long long ld_in, const float* w, 
         (taps != 4 || pb_aligned(w, 16))) {
         // up to 64 tokens a thread has one: a run's threads would leave most of the chip idle
         const int run = n_tokens <= 64 || advance ? 1 : CONV_RUN, threads = run == 1 ? 64 : 128;
-        const dim3 grid((n_tokens + run - 1) / run, (channels / vn + threads - 1) / threads);
+        const dim3 grid((n_tokens + run - 1) / run, (channels / (run == 1 ? vn : 4) + threads - 1) / threads);
 #define CONV_LAUNCH(TAPS, RUN)                                                                                                \
     PB_DISPATCH_DTYPE(dtype, T, (pb_launch(causal_conv_silu_vec_kernel<T, TAPS, RUN>, grid, dim3(threads), 0, stream, (const T*)in, ld_in, w, bias, \
                                            (const T*)carried, (T*)out, token_seq, positions, q_start, slots, n_tokens, channels, advance ? (T*)carried : (T*)nullptr)))
@@ -723,16 +741,17 @@ PB_API int pb_gated_group_rmsnorm(const float* y, const void* z, long long ld_z,
     // for a block each); in 32-bit a row's sum keeps one order whatever the step holds
     if ((width <= 512 || (width <= 1024 && dtype == PB_BF16 && (long long)n_tokens * parts >= 4096)) && width % 4 == 0 && ld_z % 4 == 0 && pb_aligned(y, 16) && pb_aligned(w, 16) && pb_aligned(z, 4 * esz) && pb_aligned(out, 4 * esz)) {
         const long long items = (long long)n_tokens * parts;
-        const int warps = items >= 4096 ? 8 : 1;
-        const dim3 grid((unsigned)((items + warps - 1) / warps)), block(32 * warps);
-        PB_REQUIRE((items + warps - 1) / warps < (1ll << 31), "gated_group_rmsnorm: too many rows");
-#define PART_LAUNCH(IT)                                                                                                       \
-    PB_DISPATCH_DTYPE(dtype, T, (pb_launch(gated_part_rmsnorm_kernel<T, IT>, grid, block, 0, stream, y, (const T*)z, ld_z, w, (T*)out, n_tokens, inner, \
+        const int each = width > 512 ? 2 : 1, warps = items >= 4096 ? 8 : 1;
+        const long long units = items * each;
+        const dim3 grid((unsigned)((units + warps - 1) / warps)), block(32 * warps);
+        PB_REQUIRE(units < (1ll << 31), "gated_group_rmsnorm: too many rows");
+#define PART_LAUNCH(IT, WARPS)                                                                                                \
+    PB_DISPATCH_DTYPE(dtype, T, (pb_launch(gated_part_rmsnorm_kernel<T, IT, WARPS>, grid, block, 0, stream, y, (const T*)z, ld_z, w, (T*)out, n_tokens, inner, \
                                            parts, eps, gate_after, sigmoid_gate)))
-        if (width <= 128) PART_LAUNCH(1);
-        else if (width <= 256) PART_LAUNCH(2);
-        else if (width <= 512) PART_LAUNCH(4);
-        else PART_LAUNCH(8);
+        if (width <= 128) PART_LAUNCH(1, 1);
+        else if (width <= 256) PART_LAUNCH(2, 1);
+        else if (width <= 512) PART_LAUNCH(4, 1);
+        else PART_LAUNCH(4, 2);
 #undef PART_LAUNCH
         PB_CHECK_LAUNCH("gated_group_rmsnorm");
         return 0;
