@@ -9,23 +9,32 @@
 // Work of a block: 256 query rows = 256/G tokens of one request x the G query heads that share one
 // key/value head (G a power of two), as two row tiles of 128; row R is head R / (256/G), token R % (256/G),
 // so every head's tokens are one box of the query tensor for TMA.  The block walks the visible keys in
-// tiles of 128; both row tiles use every key and value tile, which is fetched once.
+// tiles of 64; both row tiles use every key and value tile, which is fetched once.
 //
-// Shared memory: the query rows and a ring of key and value tiles, each tile as 64-column slabs of 128 rows
-// x 128 bytes with 128-byte swizzle - what the tensor cores read directly.  The cache stores the 16-byte
+// Shared memory: the query rows and a ring of key and value tiles, each tile as 64-column slabs of rows
+// of 128 bytes with 128-byte swizzle - what the tensor cores read directly.  The cache stores the 16-byte
 // chunks of every token row already permuted that way (pb_kv_elem_offset), so a tensor map WITHOUT swizzle
 // over [page][kv head][token][half][64] brings one page's run of one head into a slab as it is; keys are the
 // K-major B operand of the first product, values the MN-major B operand of the second.  The query tensor is
 // dense and its map swizzles.
 //
-// Tensor memory (512 columns): S_0, S_1 (128 float32 columns each: scores of the two row tiles), O_0, O_1
-// (head_dim columns each).  The probabilities, rounded to bfloat16, overwrite the first 64 columns of their
-// scores and are the A operand of the second product straight from tensor memory.
+// Tensor memory (512 columns): S_0, S_1 (64 float32 columns each: scores of the two row tiles), P_0, P_1 (two buffers of 32
+// columns each: the probabilities, rounded to bfloat16, the A operand of the second product straight from tensor memory),
+// O_0, O_1 (columns of a value row each).  With places of their own for S and P, and P twice, the scores of tile j + 1 are
+// computed while tile j is in its softmax, and nothing waits for the product of tile j before tile j + 1's probabilities: the
+// barrier of S(j) stands behind P(j - 2) V in the issue order.
 //
-// Warps: 0-3 and 4-7 are the softmax groups of row tile 0 and 1 (thread = row = tensor-memory lane: the
-// maximum and the sum of a row need no exchange), warp 8 issues the TMA loads, warp 9 owns the tensor-memory
-// allocation and issues the products.  The products of one row tile run while the other group is in its
-// softmax:  S_0(0) S_1(0) | PV_0(j) S_0(j+1) PV_1(j) S_1(j+1) | ...
+// Warps: 0-3 and 4-7 are the softmax groups of row tile 0 and 1 (thread = row = tensor-memory lane: the maximum and the sum
+// of a row need no exchange), 8 loads queries and keys, 11 values (a TMA copy keeps the issuing warp for about 95 cycles per
+// lane, and a 64-key tile from pages of 16 is up to 16 of them: one warp for both was what a tile took), 9 and 10 issue the products of
+// row tile 0 and 1 (9 owns the tensor-memory allocation):  S(j + 1) | P(j) V | ...
+//
+// What bounds it: the softmax groups.  A tile of 64 keys is 1,024 cycles of the special-function unit for both row tiles; in
+// step with one another the two groups kept it busy for half of the time and idle for the other, so their exponentials take
+// turns.  2,640 cycles a tile in step and with P waiting for its product, 2,330 with turns, 2,185 with two buffers of P.
+// 2,500 tokens of three requests, 32 heads over 8 of 128: 70 us with tiles of 128 and one warp each for loads and products,
+// 63 so (the whole attention layer 189 -> 178); keys of 192 and values of 128, 1,500 tokens, 16 heads: 48 -> 41 us.
+// Taken back: blocks that stay and take several pieces of work (no faster: 179 us).
 // The running maximum is kept in scaled log2 units and the accumulator is rescaled (by the row's own
 // thread, in tensor memory) only when a maximum grew by more than 2^8; the sum and the accumulator stay
 // relative to that slightly stale maximum and the final division cancels it.  Softmax, maximum, sum and
@@ -35,21 +44,54 @@
 #include "attention_common.cuh"
 #include "tcgen05.cuh"
 
-#define PT_KEYS 128                 // keys per tile
-#define PT_THREADS 320
-#define PT_SLAB (128 * 128)         // bytes of a slab: 128 rows x 64 bfloat16
-#define PT_S_COLS 128
+#define PT_KEYS 64                  // keys per tile
+#define PT_THREADS 384
+#define PT_Q_SLAB (128 * 128)       // bytes of a slab of queries: 128 rows x 64 bfloat16
+#define PT_SLAB (PT_KEYS * 128)     // and of keys or values
+#define PT_S_COLS 64
+#define PT_E_LAG 4                  // pairs of exponentials ahead of the sums
+#define PT_ROW_BLOCK 128            // dense rows come in blocks of this many
+#define PT_P_COL 128                // P_m starts at PT_P_COL + m * PT_KEYS: two buffers of PT_KEYS / 2 columns
+
+// Two-wide multiply-add and sum and the three-input maximum: each lane rounds as the plain instruction does.  The exponentials, their
+// sums and their roundings are `volatile` so that they stay in the order in which they are written.
+__device__ __forceinline__ float pt_max3(float a, float b, float c) {
+    float d;
+    asm("max.f32 %0, %1, %2, %3;\n" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+__device__ __forceinline__ float2 pt_fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("{\n.reg .b64 a, b, c, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nmov.b64 c, {%6, %7};\nfma.rn.f32x2 d, a, b, c;\nmov.b64 {%0, %1}, d;\n}\n"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+__device__ __forceinline__ float2 pt_add2(float2 a, float2 b) {
+    float2 d;
+    asm volatile("{\n.reg .b64 a, b, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nadd.rn.f32x2 d, a, b;\nmov.b64 {%0, %1}, d;\n}\n"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+__device__ __forceinline__ float pt_ex2(float x) {
+    float y;
+    asm volatile("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ uint32_t pt_pack(float lo, float hi) {
+    uint32_t d;
+    asm volatile("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(d) : "f"(hi), "f"(lo));
+    return d;
+}
 
 // KH, VH: 64-column slabs of a query or key row and of a value row (the last slab of a row may be filled in part: its rest is
 // zeros).  Keys and values have rings of their own.
 template <int KH, int VH> struct PtTiling {
-    static constexpr int K_BYTES = KH * PT_SLAB, V_BYTES = VH * PT_SLAB;      // 128 rows of keys, of values
-    static constexpr int Q_BYTES = 2 * K_BYTES;
-    static constexpr int K_STAGES = KH == 1 && VH == 1 ? 4 : 2;
-    static constexpr int V_STAGES = KH == 1 && VH == 1 ? 4 : (KH == 3 && VH == 2 ? 1 : 2);   // what 227 KB hold
+    static constexpr int K_BYTES = KH * PT_SLAB, V_BYTES = VH * PT_SLAB;      // a tile of keys, of values
+    static constexpr int Q_TILE = KH * PT_Q_SLAB, Q_BYTES = 2 * Q_TILE;
+    static constexpr int K_STAGES = KH == 3 ? 3 : 4, V_STAGES = K_STAGES;     // what 227 KB hold
     static constexpr int SMEM_BYTES = Q_BYTES + K_STAGES * K_BYTES + V_STAGES * V_BYTES + 1024;
     static constexpr int VD = VH * 64;
-    static constexpr int O_COL = 2 * PT_S_COLS;                  // O_m starts at O_COL + m * VD
+    static constexpr int O_COL = 256;                            // O_m starts at O_COL + m * VD
     static constexpr int TMEM_COLS = 512;
 };
 
@@ -57,7 +99,7 @@ struct PtParams {
     AttnParams a;
     int tok;                        // tokens of a block: 256 / group
     int q_rows;                     // rows of a query box: min(tok, 128)
-    int kv_rows;                    // rows of a key/value box: min(page_size, 128)
+    int kv_rows;                    // rows of a key/value box: min(page_size, PT_KEYS)
     // options of the masked attention (all off for the plain entry point)
     int keep_first;                 // positions below it stay visible behind a window
     int chunk;                      // > 0: a query sees its own run of `chunk` positions only (counted from 0)
@@ -83,7 +125,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     unsigned char* sQ = smem;
     unsigned char* sKr = smem + T::Q_BYTES;                      // the ring of key tiles
     unsigned char* sVr = sKr + KS * T::K_BYTES;                  // the ring of value tiles
-    __shared__ __align__(8) uint64_t q_full, k_full[KS], v_full[VS], k_empty[KS], v_empty[VS], s_full[2], p_full[2], o_full[2];
+    __shared__ __align__(8) uint64_t q_full, k_full[KS], v_full[VS], k_empty[KS], v_empty[VS], s_full[2], s_free[2], p_full[2], pv_done[2], turn[2][4];
     __shared__ uint32_t tmem_holder;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -115,9 +157,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
 
     if (threadIdx.x == 0) {
         mbar_init(&q_full, 1);
-        for (int s = 0; s < KS; ++s) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); }
-        for (int s = 0; s < VS; ++s) { mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1); }
-        for (int m = 0; m < 2; ++m) { mbar_init(&s_full[m], 1); mbar_init(&p_full[m], 128); mbar_init(&o_full[m], 1); }
+        for (int s = 0; s < KS; ++s) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 2); }
+        for (int s = 0; s < VS; ++s) { mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 2); }
+        for (int m = 0; m < 2; ++m) { mbar_init(&s_full[m], 1); mbar_init(&s_free[m], 4); mbar_init(&p_full[m], 4); mbar_init(&pv_done[m], 1); }
+        for (int i = 0; i < 8; ++i) mbar_init(&turn[i >> 2][i & 3], 1);
         mbar_fence_init();
     }
     if (warp == 9) tc_tmem_alloc(&tmem_holder, T::TMEM_COLS);
@@ -127,11 +170,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     tc_fence_after();
     const uint32_t tmem_base = tmem_holder;
 
-    if (warp == 8) {
-        // ---------------- loads ----------------
-        // The whole warp walks the loop.  It keeps 32 consecutive entries
-        // of the request's block table in registers, one per lane, and the 32 after them: a page number is then a
-        // shuffle away, not a trip to memory per copy.
+    if (warp == 8 || warp == 11) {
+        // ---------------- loads: queries and keys by warp 8, values by warp 11 ----------------
+        const int kv = warp == 11;
+        // The whole warp walks the loop.  It keeps 32 consecutive entries of the request's block table in registers,
+        // one per lane, and the 32 after them: a page number is then a shuffle away, not a trip to memory per copy.
         const int32_t* table = p.block_table + (size_t)p.token_seq[q_base + tok0] * p.table_stride;
         const int runs = PT_KEYS / pp.kv_rows;
         const int last_pi = p_max / ps;                          // the last page the block reads; the request holds it for sure
@@ -150,7 +193,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             else j0 = min(j0 < keep ? j0 : max(j0, lo_run), hi_run);
             const int pi = j0 / ps;
             row = j0 - pi * ps;
-            const int idx = pi - win_pi;                         // 0 .. 47: the tile starts inside `cur` and spans at most 16 pages
+            const int idx = pi - win_pi;                         // 0 .. 39: the tile starts inside `cur` and spans at most 8 pages
             const int a = __shfl_sync(0xffffffffu, cur, idx & 31), b = __shfl_sync(0xffffffffu, nxt, idx & 31);
             page = idx < 32 ? a : b;
             if (page < 0 || page >= p.num_pages) {               // never read outside the pool; the step is reported as bad
@@ -160,14 +203,14 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         };
         // q and the newest keys and values are the output of the kernel before this one
         pb_grid_dep_wait();
-        if (tc_elect_one()) {
+        if (kv == 0 && tc_elect_one()) {
             mbar_arrive_expect_tx(&q_full, T::Q_BYTES);
             for (int i = 0; i < 256 / pp.q_rows; ++i) {
                 const int R0 = i * pp.q_rows, hg = R0 / TOK, tl0 = R0 - hg * TOK;
-                unsigned char* dst = sQ + (R0 >> 7) * T::K_BYTES + (R0 & 127) * 128;
+                unsigned char* dst = sQ + (R0 >> 7) * T::Q_TILE + (R0 & 127) * 128;
 #pragma unroll
                 for (int h = 0; h < KH; ++h)
-                    tc_tma_load_3d(dst + h * PT_SLAB, &map_q, h * 64, kvh * G + hg, q_base + tok0 + tl0, &q_full);
+                    tc_tma_load_3d(dst + h * PT_Q_SLAB, &map_q, h * 64, kvh * G + hg, q_base + tok0 + tl0, &q_full);
             }
         }
         __syncwarp();
@@ -185,95 +228,88 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 win_pi += 32;
                 nxt = table[min(win_pi + 32 + lane, last_pi)];
             }
-            // lane u brings the u-th run of the tile, its keys and then its values: the copies of a tile are issued
-            // side by side, not one after the other
+            // lane u brings the u-th run of the tile
             int page, row;
             locate(j, lane < runs ? lane : 0, page, row);
-#pragma unroll 1
-            for (int kv = 0; kv < 2 && ok; ++kv) {
-                const int stage = kv ? j % VS : j % KS;
-                const unsigned phase = (kv ? j / VS : j / KS) & 1;
-                uint64_t* full = kv ? &v_full[stage] : &k_full[stage];
-                ok = __all_sync(0xffffffffu, mbar_wait_bounded(kv ? &v_empty[stage] : &k_empty[stage], phase ^ 1));
-                if (!ok) break;
-                if (lane == 0) mbar_arrive_expect_tx(full, kv ? T::V_BYTES : T::K_BYTES);
-                __syncwarp();
-                if (lane < runs) {
-                    unsigned char* dst = (kv ? sVr + stage * T::V_BYTES : sKr + stage * T::K_BYTES) + lane * pp.kv_rows * 128;
-                    const CUtensorMap* map = kv ? &map_v : &map_k;
-                    const int slabs = kv ? VH : KH;
-#pragma unroll
-                    for (int h = 0; h < (KH > VH ? KH : VH); ++h)
-                        if (h < slabs) {
-                            if (pp.flat) tc_tma_load_4d(dst + h * PT_SLAB, map, h * 64, row, kvh, page, full);
-                            else tc_tma_load_5d(dst + h * PT_SLAB, map, 0, h, row, kvh, page, full);
-                        }
-                }
-                __syncwarp();
-            }
+            const int stage = kv ? j % VS : j % KS;
+            const unsigned phase = (kv ? j / VS : j / KS) & 1;
+            uint64_t* full = kv ? &v_full[stage] : &k_full[stage];
+            ok = __all_sync(0xffffffffu, mbar_wait_bounded(kv ? &v_empty[stage] : &k_empty[stage], phase ^ 1));
             if (!ok) break;
+            if (lane == 0) mbar_arrive_expect_tx(full, kv ? T::V_BYTES : T::K_BYTES);
+            __syncwarp();
+            if (lane < runs) {
+                unsigned char* dst = (kv ? sVr + stage * T::V_BYTES : sKr + stage * T::K_BYTES) + lane * pp.kv_rows * 128;
+                const CUtensorMap* map = kv ? &map_v : &map_k;
+                const int slabs = kv ? VH : KH;
+#pragma unroll
+                for (int h = 0; h < (KH > VH ? KH : VH); ++h)
+                    if (h < slabs) {
+                        if (pp.flat) tc_tma_load_4d(dst + h * PT_SLAB, map, h * 64, row, kvh, page, full);
+                        else tc_tma_load_5d(dst + h * PT_SLAB, map, 0, h, row, kvh, page, full);
+                    }
+            }
+            __syncwarp();
         }
         if (!ok && lane == 0 && p.status) atomicExch(p.status, 7);
-    } else if (warp == 9) {
-        // ---------------- products: reads shared and tensor memory only ----------------
+    } else if (warp >= 9) {
+        // ---------------- products of row tile warp - 9: reads shared and tensor memory only ----------------
         // The whole warp walks the loop and waits; one elected lane issues.  (Issued from a branch on the lane
         // number instead, every tcgen05.mma cost the thread about 100 cycles, more than the product itself takes;
         // under elect.sync the descriptors stay in uniform registers and a 128 x 128 x 16 product issues every 64.)
+        const int m = warp - 9;
         const uint32_t idesc_s = tc_instr_desc(PT_KEYS), idesc_o = tc_instr_desc(T::VD, true);
         bool ok = true;
         auto wait_all = [&](uint64_t* bar, unsigned parity) {
             ok = __all_sync(0xffffffffu, ok && mbar_wait_bounded(bar, parity));
             return ok;
         };
-        // S_m = Q_m K^T for the key tile in stage `stage` of the key ring; release_k: the key stage is free once these have finished
-        auto issue_s = [&](int m, int stage, bool release_k) {
+        // S_m = Q_m K^T for the key tile in stage `stage` of the key ring.  (One commit for each of the two: a commit keeps the warp for 150
+        // cycles and more, and what this warp does between two tiles is what a tile takes.  The softmax threads, who learn of both
+        // products' ends, say when a stage is free.)
+        auto issue_s = [&](int stage) {
             tc_fence_after();
             if (tc_elect_one()) {
-                const uint64_t dq = tc_smem_desc(sQ + m * T::K_BYTES), dk = tc_smem_desc(sKr + stage * T::K_BYTES);
+                const uint64_t dq = tc_smem_desc(sQ + m * T::Q_TILE), dk = tc_smem_desc(sKr + stage * T::K_BYTES);
 #pragma unroll
-                for (int ks = 0; ks < KH * 4; ++ks) {
-                    const unsigned off = ((ks >> 2) * PT_SLAB + (ks & 3) * 32) >> 4;
-                    tc_mma(tmem_base + m * PT_S_COLS, dq + off, dk + off, idesc_s, ks > 0 ? 1u : 0u);
-                }
+                for (int ks = 0; ks < KH * 4; ++ks)
+                    tc_mma(tmem_base + m * PT_S_COLS, dq + (((ks >> 2) * PT_Q_SLAB + (ks & 3) * 32) >> 4), dk + (((ks >> 2) * PT_SLAB + (ks & 3) * 32) >> 4),
+                           idesc_s, ks > 0 ? 1u : 0u);
                 tc_commit(&s_full[m]);
-                if (release_k) tc_commit(&k_empty[stage]);
             }
             __syncwarp();
         };
         // O_m (+)= P_m V for the value tile in stage `stage` of the value ring
-        auto issue_o = [&](int m, int stage, bool first, bool last, bool release_v) {
+        auto issue_o = [&](int stage, int buf, bool first) {
             tc_fence_after();
             if (tc_elect_one()) {
                 const uint64_t dv = tc_smem_desc_mn(sVr + stage * T::V_BYTES, PT_SLAB);
 #pragma unroll
                 for (int ks = 0; ks < PT_KEYS / 16; ++ks)
-                    tc_mma_ts(tmem_base + T::O_COL + m * T::VD, tmem_base + m * PT_S_COLS + ks * 8, dv + ((ks * 16 * 128) >> 4), idesc_o,
+                    tc_mma_ts(tmem_base + T::O_COL + m * T::VD, tmem_base + PT_P_COL + m * PT_KEYS + buf * (PT_KEYS / 2) + ks * 8, dv + ((ks * 16 * 128) >> 4), idesc_o,
                               (!first || ks > 0) ? 1u : 0u);
-                if (last) tc_commit(&o_full[m]);
-                if (release_v) tc_commit(&v_empty[stage]);
+                tc_commit(&pv_done[m]);
             }
             __syncwarp();
         };
-        const auto first_active = [&](int j) { return j < n_m[0] ? 0 : 1; };
-        const auto last_active = [&](int j) { return j < n_m[1] ? 1 : 0; };
-        if (wait_all(&q_full, 0) && wait_all(&k_full[0], 0)) {
-            for (int m = 0; m < 2; ++m)
-                if (n_m[m] > 0) issue_s(m, 0, m == last_active(0));
-        }
+        const int n = n_m[m];
+        if (n > 0 && wait_all(&q_full, 0) && wait_all(&k_full[0], 0)) issue_s(0);
 #pragma unroll 1
-        for (int j = 0; j < n_tiles && ok; ++j) {
-            const int stage = j % VS, nstage = (j + 1) % KS;
-            const unsigned phase = (j / VS) & 1, nphase = ((j + 1) / KS) & 1;
-            for (int m = 0; m < 2 && ok; ++m) {
-                if (j >= n_m[m]) continue;
-                if (!wait_all(&p_full[m], j & 1)) break;
-                if (m == first_active(j) && !wait_all(&v_full[stage], phase)) break;
-                issue_o(m, stage, j == 0, j == n_m[m] - 1, m == last_active(j));
-                if (j + 1 < n_m[m]) {
-                    if (m == first_active(j + 1) && !wait_all(&k_full[nstage], nphase)) break;
-                    issue_s(m, nstage, m == last_active(j + 1));
-                }
+        for (int j = 0; j < n && ok; ++j) {
+            // the next tile's scores, as soon as the softmax has this one's in its registers, then this tile's product with the values
+            if (j + 1 < n) {
+                if (!wait_all(&k_full[(j + 1) % KS], ((j + 1) / KS) & 1) || !wait_all(&s_free[m], j & 1)) break;
+                issue_s((j + 1) % KS);
             }
+            if (!wait_all(&p_full[m], j & 1) || !wait_all(&v_full[j % VS], (j / VS) & 1)) break;
+            issue_o(j % VS, j & 1, j == 0);
+        }
+        // tiles that only the other row tile's rows see: this one is done with them as they arrive
+        for (int j = n; j < n_tiles && ok; ++j) {
+            if (!wait_all(&k_full[j % KS], (j / KS) & 1)) break;
+            if (lane == 0) tc_mbar_arrive(&k_empty[j % KS]);
+            if (!wait_all(&v_full[j % VS], (j / VS) & 1)) break;
+            if (lane == 0) tc_mbar_arrive(&v_empty[j % VS]);
         }
         if (!ok && lane == 0 && p.status) atomicExch(p.status, 9);
     } else {
@@ -286,18 +322,33 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         const int row_lo = p.window > 0 ? row_pos - p.window + 1 : (pp.chunk > 0 ? row_pos - row_pos % pp.chunk : 0);
         const float cap2 = pp.cap_in * 2.8853900817779268f;       // 2 log2(e) / cap, in the units of q . k
         const uint32_t lane_base = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
-        const uint32_t s_addr = lane_base + m * PT_S_COLS, o_addr = lane_base + T::O_COL + m * T::VD;
+        const uint32_t s_addr = lane_base + m * PT_S_COLS, p_addr = lane_base + PT_P_COL + m * PT_KEYS, o_addr = lane_base + T::O_COL + m * T::VD;
         float m_ref = -INFINITY, l = 0.f;
         bool ok = true;
+        const int turns = min(n_m[0], n_m[1]);
+        if (m == 1 && turns > 0 && lane == 0) tc_mbar_arrive(&turn[0][warp & 3]);
+        // the product of tile j - 1 has finished
+        auto last_product = [&](int j) {
+            const bool done = mbar_wait_bounded(&pv_done[m], (j - 1) & 1);
+            tc_fence_after();
+            return done;
+        };
 #pragma unroll 1
         for (int j = 0; j < n_m[m]; ++j) {
             ok = mbar_wait_bounded(&s_full[m], j & 1);
             if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
             tc_fence_after();
+            if ((warp & 3) == 0 && lane == 0) {
+                tc_mbar_arrive(&k_empty[j % KS]);
+                if (j >= 2) tc_mbar_arrive(&v_empty[(j - 2) % VS]);        // the scores stand behind the product before the last
+            }
             uint32_t sr[PT_KEYS];
 #pragma unroll
             for (int c = 0; c < PT_KEYS; c += 32) tc_tmem_ld32(s_addr + c, sr + c);
             tc_tmem_ld_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) tc_mbar_arrive(&s_free[m]);                     // the next tile's scores may take their place
             const int key0 = key_tile(j) * PT_KEYS;
             if (pp.cap_in > 0.f) {                                 // capped scores, before the mask
                 float am[4] = {0.f, 0.f, 0.f, 0.f};
@@ -329,20 +380,21 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                     if (kj > row_pos || (kj < row_lo && kj >= keep)) sr[c] = __float_as_uint(-INFINITY);
                 }
             }
-            // eight chains side by side: one chain of 128 dependent operations would take their latency 128 times
-            float mx[8];
+            // four chains side by side, two scores an instruction
+            float mx[4];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) mx[i] = __uint_as_float(sr[i]);
+            for (int i = 0; i < 4; ++i) mx[i] = fmaxf(__uint_as_float(sr[i]), __uint_as_float(sr[i + 4]));
 #pragma unroll
-            for (int c = 8; c < PT_KEYS; ++c) mx[c & 7] = fmaxf(mx[c & 7], __uint_as_float(sr[c]));
-            const float rmax = fmaxf(fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])), fmaxf(fmaxf(mx[4], mx[5]), fmaxf(mx[6], mx[7])));
+            for (int c = 8; c < PT_KEYS; c += 2) mx[(c >> 1) & 3] = pt_max3(mx[(c >> 1) & 3], __uint_as_float(sr[c]), __uint_as_float(sr[c + 1]));
+            const float rmax = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
             const float cand = fmaxf(m_ref, rmax * p.scale_log2);  // scale > 0: the maximum commutes with it
             const bool grow = cand > m_ref + ATT_RESCALE_STEP;      // also true for -inf -> finite
             if (__any_sync(0xffffffffu, grow)) {
                 const float corr = (m_ref == -INFINITY) ? 0.f : ex2_approx(m_ref - cand);
                 m_ref = cand;
                 l *= corr;
-                if (j > 0) {                                       // the accumulator holds something: no product is writing it now
+                if (j > 0) {                                       // the accumulator holds something, behind the last product
+                    ok = last_product(j);
 #pragma unroll 1
                     for (int c = 0; c < T::VD; c += 32) {
                         uint32_t orr[32];
@@ -356,20 +408,35 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             }
             // exp2(s * scale - m); a row that has seen nothing yet has m = -inf and only -inf scores: exp2(-inf - 0) = 0
             const float mref = m_ref == -INFINITY ? 0.f : m_ref;
-            float ls[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-            for (int c = 0; c < PT_KEYS; c += 32) {
-                uint32_t pk[16];
-#pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    const float p0 = ex2_approx(fmaf(__uint_as_float(sr[c + 2 * i]), p.scale_log2, -mref));
-                    const float p1 = ex2_approx(fmaf(__uint_as_float(sr[c + 2 * i + 1]), p.scale_log2, -mref));
-                    ls[i & 3] += p0 + p1;
-                    pk[i] = pack_bf16(p0, p1);
-                }
-                tc_tmem_st16(s_addr + (c >> 1), pk);
+            float2 ls[4] = {};
+            uint32_t pk[PT_KEYS / 2];
+            // one row tile's exponentials at a time: see the head of the file
+            if (j < turns) {
+                ok = ok && mbar_wait_bounded(&turn[m][warp & 3], j & 1);
+                if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
             }
-            l += (ls[0] + ls[1]) + (ls[2] + ls[3]);
+            // the sum and the rounding of a pair stand behind the four pairs after it: nothing waits for the one before it
+            float2 e[PT_KEYS / 2];
+            const float2 sc2 = make_float2(p.scale_log2, p.scale_log2), mr2 = make_float2(-mref, -mref);
+#pragma unroll
+            for (int i = 0; i < PT_KEYS / 2 + PT_E_LAG; ++i) {
+                if (i < PT_KEYS / 2) {
+                    const float2 x = pt_fma2(make_float2(__uint_as_float(sr[2 * i]), __uint_as_float(sr[2 * i + 1])), sc2, mr2);
+                    e[i] = make_float2(pt_ex2(x.x), pt_ex2(x.y));
+                }
+                if (i >= PT_E_LAG) {
+                    const int k = i - PT_E_LAG;
+                    ls[k & 3] = pt_add2(ls[k & 3], e[k]);
+                    pk[k] = pt_pack(e[k].x, e[k].y);
+                }
+            }
+            ls[0] = pt_add2(pt_add2(ls[0], ls[1]), pt_add2(ls[2], ls[3]));
+            const float lsum = ls[0].x + ls[0].y;
+            // (a sum is never negative: asking keeps the arrival behind the exponentials)
+            if (j < turns && lane == 0 && !(lsum < 0.f) && (m == 0 || j + 1 < turns)) tc_mbar_arrive(&turn[1 - m][warp & 3]);
+            if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+            tc_tmem_st32(p_addr + (j & 1) * (PT_KEYS / 2), pk);
+            l += lsum;
             // Value rows of keys that nobody may see (before the first visible run, after the last key) hold whatever
             // their page holds, and 0 x NaN is NaN: this group clears them once the tile has landed and before it
             // lets its product start.  Only the first and the last tile of the block have such rows.
@@ -390,7 +457,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             }
             tc_tmem_st_wait();
             tc_fence_before();
-            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(&p_full[m])) : "memory");
+            __syncwarp();
+            if (lane == 0) tc_mbar_arrive(&p_full[m]);
         }
         if (n_m[m] > 0) {
             const int head = kvh * G + hg;
@@ -402,7 +470,14 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 for (int i = 0; i < T::VD / 8; ++i)
                     if (i * 8 < pp.vd) gates[i] = *reinterpret_cast<const uint4*>(src + i * 8);
             }
-            if (ok) ok = mbar_wait_bounded(&o_full[m], 0);
+            // the product before the last as well: the last scores stand behind the one before it, and a barrier two phases back
+            // would take the wait for the last one's parity as over
+            if (ok && n_m[m] > 1) ok = last_product(n_m[m] - 1);
+            if (ok) ok = last_product(n_m[m]);
+            if ((warp & 3) == 0 && lane == 0) {
+                if (n_m[m] > 1) tc_mbar_arrive(&v_empty[(n_m[m] - 2) % VS]);
+                tc_mbar_arrive(&v_empty[(n_m[m] - 1) % VS]);
+            }
             if (__all_sync(0xffffffffu, ok)) {
                 tc_fence_after();
                 if (pp.sink != nullptr && m_ref != -INFINITY) l += ex2_approx(fmaf(pp.sink[head], 1.4426950408889634f, -m_ref));
@@ -489,7 +564,7 @@ PB_API int pb_attention_prefill_tc_supported(int n_heads, int n_kv_heads, int he
     const int g = n_heads / n_kv_heads;
     if (!pt_pow2(g) || g > 32) return 0;
     if (head_dim != 64 && head_dim != 128) return 0;
-    if (!swizzle || page_size % 8 || !(PT_KEYS % page_size == 0 || page_size % PT_KEYS == 0)) return 0;
+    if (!swizzle || page_size % 8 || !(128 % page_size == 0 || page_size % 128 == 0)) return 0;
     return 1;
 }
 
@@ -610,7 +685,7 @@ PB_API int pb_attention_prefill_tc_rows_bf16(const void* q, const void* kv, void
     p.q = (const __nv_bfloat16*)q; p.k_pages = (const __nv_bfloat16*)kv; p.v_pages = (const __nv_bfloat16*)kv + kd;
     p.out = (__nv_bfloat16*)out; p.block_table = row_blocks; p.positions = positions; p.token_seq = token_seq;
     p.cu_q = cu_q; p.q_start = q_start; p.tile_seq = tile_seq; p.tile_tok0 = tile_tok0; p.n_splits = 1;
-    p.table_stride = table_stride; p.page_size = PT_KEYS; p.num_pages = n_blocks; p.n_tokens = n_tokens;
+    p.table_stride = table_stride; p.page_size = PT_ROW_BLOCK; p.num_pages = n_blocks; p.n_tokens = n_tokens;
     p.n_heads = n_heads; p.n_kv_heads = n_heads; p.head_dim = kd; p.window = window; p.group = 1;
     p.scale_log2 = scale * 1.4426950408889634f; p.status = status; p.swizzle = 0;
     if (int e = attn_check_common("attention_prefill_tc (rows)", p)) return e;
@@ -632,8 +707,8 @@ PB_API int pb_attention_prefill_tc_rows_bf16(const void* q, const void* kv, void
     }
     const cuuint64_t head = (cuuint64_t)(kd + vd) * 2, row = head * n_heads;
     for (int which = 0; which < 2; ++which) {
-        cuuint64_t dims[4] = {(cuuint64_t)(which ? vd : kd), PT_KEYS, (cuuint64_t)n_heads, (cuuint64_t)n_blocks};
-        cuuint64_t strides[3] = {row, head, row * PT_KEYS};
+        cuuint64_t dims[4] = {(cuuint64_t)(which ? vd : kd), PT_ROW_BLOCK, (cuuint64_t)n_heads, (cuuint64_t)n_blocks};
+        cuuint64_t strides[3] = {row, head, row * PT_ROW_BLOCK};
         cuuint32_t box[4] = {64, PT_KEYS, 1, 1};
         if (int e = pt_encode(which ? &mv : &mk, which ? (const void*)p.v_pages : (const void*)p.k_pages, 4, dims, strides, box,
                               CU_TENSOR_MAP_SWIZZLE_128B, which ? "the value rows" : "the key rows")) return e;

@@ -146,7 +146,7 @@ def attention_general(q: torch.Tensor, k_pages: torch.Tensor, v_pages: Optional[
 
 
 # -- keys and values of every query head's own in dense rows (made of a latent for a long prompt portion) -----------------
-ROW_BLOCK = 128                       # rows of a block of the dense rows, keys of a tile of the tcgen05 prompt kernel
+ROW_BLOCK = 128                       # rows of a block of the dense rows: two key tiles of the tcgen05 prompt kernel
 ROWS_MIN_PORTION = int(256 * TC_MIN_FILL)         # tokens from which a portion fills that kernel's blocks
 # most rows (cached tokens of all long portions of a step) for which keys and values are made per head
 ROWS_MAX = int(os.environ.get("PRELUDE_LATENT_ROWS_MAX", str(1 << 16)))
