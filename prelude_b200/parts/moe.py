@@ -45,7 +45,7 @@ ROUTE_FEW_TOKENS = int(os.environ.get("PRELUDE_MOE_ROUTE_FEW_TOKENS", "32"))
 # results throughout), and from which on the one with the weights as rows.  Against the 64- and 128-row tiles, both products and the
 # gather, us: 64 experts of 4,096 x 2,048 506 against 489 at 2 rows, 546 against 614 at 3, 584 against 751 at 4, 588 against 1,380
 # at 32, 598 against 1,135 at 64, 686 against 1,826 at 128; 32 experts of 2,048 x 2,048 163 against 154, 192 against 208, 190 against 253,
-# 182 against 390, 185 against 322, 195 against 485
+# 182 against 390, 185 against 322, 195 against 485 (its stages were 64 of K then; with 128, 504 us at 4 rows and 536 at 64 of the first)
 MOE_PAIR_MIN_ROWS = int(os.environ.get("PRELUDE_MOE_PAIR_MIN_ROWS", "192"))
 MOE_GROUPED_MIN_ROWS = int(os.environ.get("PRELUDE_MOE_GROUPED_MIN_ROWS", "3"))
 
