@@ -434,6 +434,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             const float lsum = ls[0].x + ls[0].y;
             // (a sum is never negative: asking keeps the arrival behind the exponentials)
             if (j < turns && lane == 0 && !(lsum < 0.f) && (m == 0 || j + 1 < turns)) tc_mbar_arrive(&turn[1 - m][warp & 3]);
+            // Before the last tile's weights are handed over, the product before theirs has ended: the wait for the last product names its
+            // phase by the parity, which a barrier two phases back has too, and the last scores stand behind no more than tile n - 3's product.
+            if (j > 0 && j + 1 == n_m[m]) ok = ok && last_product(j);
             if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
             tc_tmem_st32(p_addr + (j & 1) * (PT_KEYS / 2), pk);
             l += lsum;
@@ -470,9 +473,6 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 for (int i = 0; i < T::VD / 8; ++i)
                     if (i * 8 < pp.vd) gates[i] = *reinterpret_cast<const uint4*>(src + i * 8);
             }
-            // the product before the last as well: the last scores stand behind the one before it, and a barrier two phases back
-            // would take the wait for the last one's parity as over
-            if (ok && n_m[m] > 1) ok = last_product(n_m[m] - 1);
             if (ok) ok = last_product(n_m[m]);
             if ((warp & 3) == 0 && lane == 0) {
                 if (n_m[m] > 1) tc_mbar_arrive(&v_empty[(n_m[m] - 2) % VS]);
