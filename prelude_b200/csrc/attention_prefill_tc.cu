@@ -125,7 +125,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     unsigned char* sQ = smem;
     unsigned char* sKr = smem + T::Q_BYTES;                      // the ring of key tiles
     unsigned char* sVr = sKr + KS * T::K_BYTES;                  // the ring of value tiles
-    __shared__ __align__(8) uint64_t q_full, k_full[KS], v_full[VS], k_empty[KS], v_empty[VS], s_full[2], s_free[2], p_full[2], pv_done[2], turn[2][4];
+    __shared__ __align__(8) uint64_t q_full, k_full[KS], v_full[VS], k_empty[KS], v_empty[VS], s_full[2], s_free[2], p_full[2][2], pv_done[2], turn[2][4];
     __shared__ uint32_t tmem_holder;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -159,7 +159,15 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         mbar_init(&q_full, 1);
         for (int s = 0; s < KS; ++s) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 2); }
         for (int s = 0; s < VS; ++s) { mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 2); }
-        for (int m = 0; m < 2; ++m) { mbar_init(&s_full[m], 1); mbar_init(&s_free[m], 4); mbar_init(&p_full[m], 4); mbar_init(&pv_done[m], 1); }
+        for (int m = 0; m < 2; ++m) { mbar_init(&s_full[m], 1); mbar_init(&s_free[m], 4); mbar_init(&pv_done[m], 1); }
+        // The weights' barriers, one for each of a row tile's two buffers of P.  A warp's next tile is not held back by its group: S(j + 1) is
+        // there once all four warps have READ S(j), and a warp that is quick (no rescaling, no score near the cap) hands over P(j + 1) while
+        // another is still at P(j).  On one barrier its second arrival stood for the slow warp's first, and the product took weights that
+        // nobody had written.  Two arrivals of one warp on one of these are two tiles apart, and P(j + 2) is made behind S(j + 2), which stands
+        // behind every warp's `s_free` of tile j + 1, which each gives behind its arrival for tile j.  (The others, by the same question: an
+        // arrival on `s_free` for j + 1 stands behind S(j + 1), which waited for all four of j; one on `k_empty` or `v_empty` behind a refill of
+        // the stage, which waited for both row tiles; `turn` changes hands with every arrival; the rest are commits of one warp in order.)
+        for (int i = 0; i < 4; ++i) mbar_init(&p_full[i >> 1][i & 1], 4);
         for (int i = 0; i < 8; ++i) mbar_init(&turn[i >> 2][i & 3], 1);
         mbar_fence_init();
     }
@@ -301,7 +309,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 if (!wait_all(&k_full[(j + 1) % KS], ((j + 1) / KS) & 1) || !wait_all(&s_free[m], j & 1)) break;
                 issue_s((j + 1) % KS);
             }
-            if (!wait_all(&p_full[m], j & 1) || !wait_all(&v_full[j % VS], (j / VS) & 1)) break;
+            if (!wait_all(&p_full[m][j & 1], (j >> 1) & 1) || !wait_all(&v_full[j % VS], (j / VS) & 1)) break;
             issue_o(j % VS, j & 1, j == 0);
         }
         // tiles that only the other row tile's rows see: this one is done with them as they arrive
@@ -461,7 +469,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             tc_tmem_st_wait();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) tc_mbar_arrive(&p_full[m]);
+            if (lane == 0) tc_mbar_arrive(&p_full[m][j & 1]);
         }
         if (n_m[m] > 0) {
             const int head = kvh * G + hg;
