@@ -43,6 +43,12 @@ def decode_splits(n_tokens: int, n_kv_heads: int, max_context: int, device, most
     return max(1, min(tiles, want, most))
 
 
+def tcgen05_takes_options(spec, coef: float, out: torch.Tensor) -> bool:
+    """What the tcgen05 kernel asks for beside the shape, and the mma.sync kernel does not: it takes a row's maximum before the scale and the
+    temperature, which must not turn the order round, and stores 16 bytes at a time."""
+    return spec.softmax_scale > 0.0 and coef >= 0.0 and not (spec.window and spec.window < 0) and out.data_ptr() % 16 == 0
+
+
 def diff_attention(q: torch.Tensor, gate: Optional[torch.Tensor], k_pages: torch.Tensor, v_pages: torch.Tensor, batch,
                    group: int, spec, lam: float, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """q [T, heads * 2 * head_dim] and gate [T, heads * value_dim] (columns of the merged projection) of the batch's
@@ -88,7 +94,7 @@ def diff_attention(q: torch.Tensor, gate: Optional[torch.Tensor], k_pages: torch
         # every portion, single tokens among them, on the tcgen05 kernel where it takes the shape, else on the mma.sync kernel (16 heads over 4,
         # us there / here: 16 tokens 13.3 / 22.9, 1,024 tokens 34 / 106, 64 behind 2,000 57 / 90; 512 beside 16 single tokens behind 2,000 57 / 129)
         gate_at = (0, None) if gate is None else (gate.stride(0), gate.data_ptr())
-        if (coef >= 0.0 and KERNEL != "mma" and lib.pb_diff_attention_tcgen05_supported(
+        if (KERNEL != "mma" and tcgen05_takes_options(spec, coef, out) and lib.pb_diff_attention_tcgen05_supported(
                 spec.num_heads, spec.num_kv_heads, dim, vdim, page_size, q.stride(0), q.data_ptr(), *gate_at)):
             tile_seq, tile_tok0, n_tiles = _prefill_plan(
                 batch, lib.pb_diff_attention_tcgen05_tile_tokens(spec.num_heads, spec.num_kv_heads), 0, None)

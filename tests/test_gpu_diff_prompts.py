@@ -102,3 +102,21 @@ def test_calls_that_keep_the_other_kernel():
                 (16, 4, 64, 96, 16, 4096, 1 << 20, 0, None), (16, 4, 64, 128, 12, 4096, 1 << 20, 0, None), (16, 4, 64, 128, 48, 4096, 1 << 20, 0, None),
                 (16, 4, 64, 128, 16, 4100, 1 << 20, 0, None), (16, 4, 64, 128, 16, 4096, (1 << 20) + 8, 0, None), (16, 4, 64, 128, 16, 4096, 1 << 20, 4100, 1 << 20)):
         assert not takes(*bad)
+
+
+@pytest.mark.parametrize("scale,offset", [(-0.125, 0), (0.0, 0), (0.125, 4), (-0.125, 2)])
+def test_scales_and_results_that_keep_the_other_kernel(monkeypatch, scale, offset):
+    # a scale that is not positive, a result that is not 16-byte aligned: taken before there was a tcgen05 kernel, and still
+    from prelude_b200.ops import diff_attention as D
+    shape = [(40, 100), (0, 20)]
+    q, gate, keys, values, batch, mine, spec, _ = case(shape, 4, 2, 128, 16, None, seed=7)
+    spec.softmax_scale = scale
+    room = torch.zeros(q.shape[0] * 4 * 128 + offset, dtype=torch.bfloat16, device=DEV)
+    out = room[offset:].view(q.shape[0], 4, 128)
+    got = D.diff_attention(q, gate, mine.k_pages, mine.v_pages, batch, 0, spec, 0.3, out)
+    monkeypatch.setattr(D, "KERNEL", "mma")
+    assert got.data_ptr() == out.data_ptr() and torch.equal(got, D.diff_attention(q, gate, mine.k_pages, mine.v_pages, batch, 0, spec, 0.3))
+    want = plain(q * (scale / 0.125), gate, keys, values, shape, spec, 0.3)         # (exact: -1, 0 or 1, and 64 ** -0.5 is 0.125)
+    # weights rounded to bfloat16 once, 2^-9 each, and the difference of two maps is smaller than either: four times the rounding of the result
+    assert float((got.double() - want).norm() / want.norm()) < 4 * 2.2e-3
+    assert int(batch.status) == 0
