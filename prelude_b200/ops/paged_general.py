@@ -90,7 +90,8 @@ def attention_general(q: torch.Tensor, k_pages: torch.Tensor, v_pages: Optional[
                                                               keep_first, chunk, softcap, gate, below))
         return out
     seen = batch.max_kv_len if batch.max_kv_len else batch.block_tables[group].shape[1] * k_pages.shape[2]
-    if latent_takes(q, k_pages, v_pages, value_dim, batch, keep_first, chunk, softcap, min(seen, window) if window else seen):
+    # (the latent kernel stores eight bytes at a time, the general kernel four)
+    if out.data_ptr() % 8 == 0 and latent_takes(q, k_pages, v_pages, value_dim, batch, keep_first, chunk, softcap, min(seen, window) if window else seen):
         return attention_latent(q, k_pages, value_dim, batch, group, scale, window, sink, gate, out)
     lib = _l.library()
     table = batch.block_tables[group]

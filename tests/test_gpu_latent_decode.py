@@ -146,3 +146,18 @@ def test_both_sides_of_the_rule_agree(context, window, tokens):
     batch.workspace = lambda name, shape, dtype: torch.empty(shape, dtype=dtype, device=DEV)
     want, big = plain(q, pages, batch, 512, 0.05, window or 0, None, None)
     assert agrees(PG.attention_general(q, pages, None, 512, batch, 0, 0.05, window, None), want, big)
+
+
+def test_a_result_that_is_four_byte_aligned():
+    # the general kernel takes it, as it did before there was another one
+    from prelude_b200.ops import paged_general as PG
+    H, vd = 16, 512
+    q, pages, batch = make([1300, 1100, 40], H, 576, vd, 16, seed=9)
+    pages[torch.isnan(pages)] = 0
+    batch.cu_q, batch.max_q_len = torch.arange(4, dtype=torch.int32, device=DEV), 1
+    batch.workspace = lambda name, shape, dtype: torch.empty(shape, dtype=dtype, device=DEV)
+    want, big = plain(q, pages, batch, vd, 0.05, 0, None, None)
+    for offset in (2, 4, 8):
+        out = torch.zeros(3 * H * vd + offset, dtype=torch.bfloat16, device=DEV)[offset:].view(3, H, vd)
+        assert agrees(PG.attention_general(q, pages, None, vd, batch, 0, 0.05, None, None, out), want, big)
+    assert int(batch.status) == 0
