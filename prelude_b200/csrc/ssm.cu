@@ -739,12 +739,11 @@ PB_API int pb_gated_group_rmsnorm(const float* y, const void* z, long long ld_z,
     const size_t esz = dtype == PB_BF16 ? 2 : 4;
     // parts of up to 1,024 in bfloat16 too where there are rows enough that a warp each fills the chip (2 x 8,192: 13 us against 11
     // for a block each); in 32-bit a row's sum keeps one order whatever the step holds
-    if ((width <= 512 || (width <= 1024 && dtype == PB_BF16 && (long long)n_tokens * parts >= 4096)) && width % 4 == 0 && ld_z % 4 == 0 && pb_aligned(y, 16) && pb_aligned(w, 16) && pb_aligned(z, 4 * esz) && pb_aligned(out, 4 * esz)) {
-        const long long items = (long long)n_tokens * parts;
-        const int each = width > 512 ? 2 : 1, warps = items >= 4096 ? 8 : 1;
-        const long long units = items * each;
+    // (its places are counted in 32 bits: 2^31 and more go to the kernels below)
+    const long long items = (long long)n_tokens * parts, units = items * (width > 512 ? 2 : 1);
+    if ((width <= 512 || (width <= 1024 && dtype == PB_BF16 && items >= 4096)) && units < (1ll << 31) && width % 4 == 0 && ld_z % 4 == 0 && pb_aligned(y, 16) && pb_aligned(w, 16) && pb_aligned(z, 4 * esz) && pb_aligned(out, 4 * esz)) {
+        const int warps = items >= 4096 ? 8 : 1;
         const dim3 grid((unsigned)((units + warps - 1) / warps)), block(32 * warps);
-        PB_REQUIRE(units < (1ll << 31), "gated_group_rmsnorm: too many rows");
 #define PART_LAUNCH(IT, WARPS)                                                                                                \
     PB_DISPATCH_DTYPE(dtype, T, (pb_launch(gated_part_rmsnorm_kernel<T, IT, WARPS>, grid, block, 0, stream, y, (const T*)z, ld_z, w, (T*)out, n_tokens, inner, \
                                            parts, eps, gate_after, sigmoid_gate)))

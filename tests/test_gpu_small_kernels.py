@@ -302,3 +302,22 @@ def test_queries_turned_where_they_lie(dtype, adjacent, H, d, dims):
         mine = q.clone()
         got = turn(mine, mine)
         assert bool(((got.double() - want.double()).abs() <= 2 * UNIT[dtype] * want.double().abs() + 2 * 6 * 2.0 ** -23).all())
+
+
+def test_gated_norm_of_more_parts_than_32_bits_count():
+    # 2^31 parts of four: past what the kernel of a warp a part counts, and still taken
+    from prelude_b200.ops import kernels as K
+    if torch.cuda.mem_get_info()[0] < 90 << 30:
+        pytest.skip("needs 70 GB")
+    T, inner = 1 << 30, 8
+    y = torch.zeros(T, inner, device=DEV)
+    z = torch.zeros(T, inner, dtype=torch.bfloat16, device=DEV)
+    w = torch.rand(inner, device=DEV) + 0.5
+    where = [slice(0, 999), slice((1 << 29) - 500, (1 << 29) + 499), slice(T - 999, T)]
+    for s in where:
+        y[s], z[s] = torch.randn(999, inner, device=DEV), torch.randn(999, inner, device=DEV).bfloat16()
+    got = K.gated_group_rmsnorm(y, z, w, 2, 1e-6)
+    for s in where:
+        v = (y[s].double() * torch.nn.functional.silu(z[s].double())).view(-1, 2, 4)
+        want = (v * (v.pow(2).mean(-1, keepdim=True) + 1e-6).rsqrt()).view(-1, inner) * w.double()
+        assert bool(((got[s].double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all())        # rounded to bfloat16 once
