@@ -16,7 +16,7 @@ __global__ void silu_mul_kernel(const T* gu, T* out, long long n_tokens, int int
     int i = (int)(idx % inter);
     float g = pb_ld(gu + t * 2 * inter + i);
     float u = pb_ld(gu + t * 2 * inter + inter + i);
-    pb_st(out + idx, g / (1.0f + expf(-g)) * u);
+    pb_st(out + idx, pb_silu_for<T>(g) * u);
 }
 
 // bfloat16, 8 elements per thread; inter % 8 == 0.
@@ -181,7 +181,7 @@ __global__ void silu_cols_kernel(T* x, long long ld, long long n_tokens, int col
     if (idx >= n_tokens * cols) return;
     T* p = x + (idx / cols) * ld + idx % cols;
     const float v = pb_ld(p);
-    pb_st(p, v / (1.0f + expf(-v)));
+    pb_st(p, pb_silu_for<T>(v));
 }
 
 // bfloat16, 8 elements per thread; cols % 8 == 0, ld % 8 == 0, x 16-byte aligned.

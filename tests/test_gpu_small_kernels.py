@@ -321,3 +321,29 @@ def test_gated_norm_of_more_parts_than_32_bits_count():
         v = (y[s].double() * torch.nn.functional.silu(z[s].double())).view(-1, 2, 4)
         want = (v * (v.pow(2).mean(-1, keepdim=True) + 1e-6).rsqrt()).view(-1, inner) * w.double()
         assert bool(((got[s].double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all())        # rounded to bfloat16 once
+
+
+def _every_bfloat16():
+    return torch.arange(1 << 16, device=DEV, dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+
+
+@pytest.mark.parametrize("form", ["gated", "columns", "sigmoid"])
+def test_activations_give_the_same_bits_in_both_forms(form):
+    # a row of eight elements an access and an element an access, which an odd address takes; every gate there is
+    from prelude_b200.ops import kernels as K
+    g, u = _every_bfloat16().view(64, 1024), torch.randn(64, 1024, generator=_gen(), device=DEV).bfloat16()
+
+    def made(offset):
+        if form == "gated":
+            x = torch.empty(64 * 2048 + offset, dtype=torch.bfloat16, device=DEV)[offset:].view(64, 2048)
+            x[:, :1024], x[:, 1024:] = g, u
+            return K.silu_mul(x)
+        x = torch.empty(64 * 1024 + offset, dtype=torch.bfloat16, device=DEV)[offset:].view(64, 1024)
+        x.copy_(u if form == "sigmoid" else g)
+        if form == "sigmoid":
+            K.sigmoid_gate_(x, g)
+        else:
+            K.check(K._l.library().pb_silu_cols(x.data_ptr(), x.stride(0), K.dtype_code(x.dtype), 64, 1024, K._stream()), "silu_cols")
+        return x
+    a, b = made(0), made(1)
+    assert torch.equal(torch.isnan(a), torch.isnan(b)) and torch.equal(a.nan_to_num(), b.nan_to_num())
