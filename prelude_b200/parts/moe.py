@@ -24,7 +24,6 @@ first tensor.
 """
 from __future__ import annotations
 
-import math
 import os
 from typing import Dict
 
@@ -47,18 +46,27 @@ ROUTE_FEW_TOKENS = int(os.environ.get("PRELUDE_MOE_ROUTE_FEW_TOKENS", "32"))
 # at 32, 598 against 1,135 at 64, 686 against 1,826 at 128; 32 experts of 2,048 x 2,048 163 against 154, 192 against 208, 190 against 253,
 # 182 against 390, 185 against 322, 195 against 485 (its stages were 64 of K then; with 128, 504 us at 4 rows and 536 at 64 of the first)
 MOE_PAIR_MIN_ROWS = int(os.environ.get("PRELUDE_MOE_PAIR_MIN_ROWS", "192"))
-MOE_GROUPED_MIN_ROWS = int(os.environ.get("PRELUDE_MOE_GROUPED_MIN_ROWS", "3"))
+MOE_GROUPED_MIN_ROWS = 3
+# PRELUDE_MOE_GROUPED_MIN_ROWS: that many, whatever the rule below says, also for the steps that the streaming kernel takes
+MOE_GROUPED_ROWS_SET = os.environ.get("PRELUDE_MOE_GROUPED_MIN_ROWS")
+# where a step of few rows leaves the streaming kernel (``grouped_pays``): what a repeated read is counted as, and the bytes
+GROUPED_FIRST_READS, GROUPED_MIN_BYTES = 1.75, 150e6
 
 
-def grouped_min_rows(matrix: int, gated: bool) -> float:
-    """Average rows per expert from which the product with the weights as rows, its sort and its gather are ahead of the kernel that only streams
-    the weights, once for every (token, expert) pair; ``matrix``: elements of one of an expert's matrices.  The whole feed-forward, us, streamed
-    / there: gated, 4,096 x 2,048 1.1 rows 401 / 410, 1.5 457 / 442, 3 686 / 551, 6 1,131 / 565; 2,048 x 2,048 1.5 154 / 154, 2 180 / 172,
-    4 250 / 176; 2,048 x 768 0.5 139 / 149, 1.5 244 / 207, 4 440 / 260; without a gate, 4,096 x 2,048 0.2 135 / 137, 0.4 199 / 186, 1.5 420 / 340;
-    2,048 x 2,048 0.5 86 / 88, 1 117 / 115, 2 154 / 137; 2,048 x 768 0.25 90 / 96, 1 170 / 150; 1,024 x 512, either, 3 37 / 39, 5 41 / 39."""
-    if matrix < 3 << 19:
-        return math.inf
-    return min(1.5 if gated else 0.375 if matrix >= 8 << 20 else 1.0, MOE_GROUPED_MIN_ROWS)
+def grouped_pays(tokens: int, top_k: int, n_experts: int, expert_bytes: int) -> bool:
+    """Whether a step of few rows is faster on the product with the weights as rows, which reads every expert's matrices once and pays for a sort, a
+    gather and its own latencies, than on the kernel that streams them once for every (token, expert) pair; ``expert_bytes``: one
+    expert's matrices.  The experts hit are those that an even router hits, n (1 - (1 - k/n)^T).  A pair that repeats an expert costs the
+    streaming kernel about half of what a first one does (the matrices are in the L2 cache), and the other way's beginning what 150 MB
+    take; one token hits every expert once and always streams.
+
+    The whole feed-forward at 8 to 128 experts of 1,024 x 512 to 4,096 x 2,048, top 2 to 8, with and without a gate, 1 to 64 tokens, weights
+    from memory (2,768 steps): of the 795 that leave the streaming kernel 17 are slower for it by more than 2 %, and by 16 % at most; all of
+    them together take 0.78 of the time.  Left behind: 228 steps that would gain more than 5 %.  At both ends, us, streamed / there: 16
+    experts of 2,048 x 768, top 2, gated, 20 tokens 52 / 52, 28 tokens 63 / 53; 64 of 4,096 x 2,048, top 6, gated, 16 tokens 450 / 448, 20
+    tokens 509 / 484, 32 tokens 684 / 518; 32 of 2,048 x 2,048, top 4, no gate, 8 tokens 76 / 87, 16 tokens 110 / 110, 24 tokens 137 / 111."""
+    hit = n_experts * (1.0 - (1.0 - top_k / n_experts) ** tokens)
+    return (tokens * top_k - GROUPED_FIRST_READS * hit) * expert_bytes >= GROUPED_MIN_BYTES
 
 
 # an activation's name: (two matrices on the way up or one, its number in the products' epilogues)
@@ -152,6 +160,16 @@ class RoutedExperts:
         an expert's 256-row tiles are mostly full (PRELUDE_MOE_PAIR_MIN_ROWS rows per expert on average, default 192)."""
         return self._paired(x, MOE_PAIR_MIN_ROWS)
 
+    def _grouped(self, x: torch.Tensor, streamed: bool) -> bool:
+        """Whether a step's products run on the kernel with the weights as rows; ``streamed``: the streaming kernel would take them."""
+        s = self.spec
+        if MOE_GROUPED_ROWS_SET is not None:
+            return self._paired(x, float(MOE_GROUPED_ROWS_SET))
+        if not streamed:
+            return self._paired(x, MOE_GROUPED_MIN_ROWS)
+        expert_bytes = (3 if self.gated else 2) * s.hidden_size * s.expert_size * x.element_size()
+        return grouped_pays(x.shape[0], s.top_k, s.n_experts, expert_bytes) and self._paired(x, 0)
+
     def _router_args(self):
         s = self.spec
         return (s.top_k, s.n_groups, s.keep_groups, s.group_score_top, s.renormalize, self.correction, s.scoring == "softmax",
@@ -197,11 +215,12 @@ class RoutedExperts:
         small = x.dtype != torch.bfloat16 or s.hidden_size % 8 or s.expert_size % 8
         few = not small and x.shape[0] * s.top_k <= MOE_FEW_ROWS * s.n_experts       # a decode step: stream the weights
         streamed = few and K.moe_gemv_takes(x, self.w_gate_up, ids.numel())
-        if streamed and not self._paired(x, grouped_min_rows(s.hidden_size * s.expert_size, self.gated)):
+        grouped = self._grouped(x, streamed)
+        if streamed and not grouped:
             h = K.moe_gemv(x, self.w_gate_up, ids, False, x.dtype, gated=self.gated, **self.act)
             y = K.moe_gemv(h, self.w_down, ids, True, torch.float32)
             return self._sum(y, None, weights, shared, x.dtype)
-        if streamed or self._paired(x, MOE_GROUPED_MIN_ROWS):
+        if grouped:
             # fewer rows: the experts' weights are the rows of the paired-block products, the tokens their columns
             plan = K.moe_sort(ids, s.n_experts, 256)
             status = L.tc_status(x.device)
