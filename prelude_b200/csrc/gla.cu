@@ -60,10 +60,11 @@ __device__ __forceinline__ float gla_decay(float z, float inv_tau) {
 }
 
 // ---------------------------------------------------------------------------------------------------------
-// For ranks of 16 or 32 in bfloat16: a thread owns one channel, its row of the matrix in registers, and walks the block's tokens eight at a
-// time, two in one instruction; their narrow rows lie in shared memory turned, so that one access brings four tokens.  Sums over the rank
-// in ascending order, as below, and the same bits.  (2,048 tokens of 4,096 channels, rank 32: 58 us below, where a block has eight tokens and
-// a thread fetches its row of the matrix for them alone; 36 here.)
+// For ranks in multiples of 8 up to 64 in bfloat16: a thread owns one channel, its row of the matrix in registers (two for a number: more of
+// them do not fit), and walks the block's tokens eight at a time, two in one instruction; their narrow rows lie in shared memory turned, so
+// that one access brings four tokens.  Sums over the rank in ascending order, as below, and the same bits.  (2,048 tokens of 4,096 channels:
+// rank 32 56 us below, where a block has eight tokens and every block fetches the rows of the matrix for them alone, 31 here; rank 64 157
+// and 59; rank 8 25 and 19.)
 template <int RANK>
 __global__ void __launch_bounds__(128) channel_decay_rows_kernel(const __nv_bfloat16* x1, long long ld_x1, const __nv_bfloat16* w2, const float* bias,
                                                                  float inv_tau, float* out, int n_tokens, int channels, int block_tokens) {
@@ -555,15 +556,24 @@ PB_API int pb_channel_decay(const void* x1, long long ld_x1, const void* w2, con
     PB_REQUIRE(smem <= 48 * 1024, "channel_decay: a rank of %d (at most %d)", rank, 48 * 1024 / DECAY_TOKENS / 4);
     PB_REQUIRE((channels + 127) / 128 < 65536, "channel_decay: %d channels", channels);
     if (n_tokens == 0) return 0;
-    if (dtype == PB_BF16 && (rank == 16 || rank == 32) && n_tokens >= 64 && pb_aligned(w2, 16) && pb_aligned(x1, 16) && ld_x1 % 8 == 0) {
-        // as many tokens a block as leave the chip twice full
-        const int cols = (channels + 127) / 128, tokens = (long long)((n_tokens + 63) / 64) * cols >= 296 ? 64 : 16;
+    if (dtype == PB_BF16 && rank % 8 == 0 && rank <= 64 && n_tokens >= 64 && pb_aligned(w2, 16) && pb_aligned(x1, 16) && ld_x1 % 8 == 0) {
+        // A block's time grows with its tokens, and with the rank the registers, so that fewer blocks are on a multiprocessor: many tokens a
+        // block (the row of the matrix is fetched once) where there are several waves of such blocks.  us with 8 / 16 / 32 / 64 tokens a
+        // block, behind them a block of eight on the kernel below: rank 32, 500 tokens of 4,096 channels 13.1 / 9.8 / 10.0 / 24.7, 17.0;
+        // 2,048 of 2,048 27.6 / 20.3 / 17.4 / 18.9, 30.1; 2,048 of 4,096 52 / 40 / 33 / 31, 56; rank 16, 2,048 of 2,048 12.9 / 12.2 /
+        // 16.4 / 27.6, 16.8; 200 of 4,096 5.2 / 7.6 / 9.8 / 9.7, 6.4; 2,048 of 4,096 24.0 / 22.6 / 22.6 / 30.6, 30.9.
+        const int cols = (channels + 127) / 128;
+        const long long blocks = (long long)((n_tokens + 63) / 64) * cols;
+        const int tokens = rank >= 32 ? (blocks >= 960 ? 64 : blocks >= 256 ? 32 : 16) : (blocks >= 960 ? 16 : 8);
         const dim3 grid((n_tokens + tokens - 1) / tokens, cols);
         const size_t bytes = (size_t)rank * (tokens + 4) * sizeof(float);
-        if (rank == 16) pb_launch(channel_decay_rows_kernel<16>, grid, dim3(128), bytes, stream, (const __nv_bfloat16*)x1, ld_x1, (const __nv_bfloat16*)w2, bias, 1.0f / tau,
-                                  out, n_tokens, channels, tokens);
-        else pb_launch(channel_decay_rows_kernel<32>, grid, dim3(128), bytes, stream, (const __nv_bfloat16*)x1, ld_x1, (const __nv_bfloat16*)w2, bias, 1.0f / tau, out,
-                       n_tokens, channels, tokens);
+#define DECAY_ROWS(RANK)                                                                                                      \
+    case RANK:                                                                                                               \
+        pb_launch(channel_decay_rows_kernel<RANK>, grid, dim3(128), bytes, stream, (const __nv_bfloat16*)x1, ld_x1, (const __nv_bfloat16*)w2, bias, \
+                  1.0f / tau, out, n_tokens, channels, tokens);                                                              \
+        break;
+        switch (rank) { DECAY_ROWS(8) DECAY_ROWS(16) DECAY_ROWS(24) DECAY_ROWS(32) DECAY_ROWS(40) DECAY_ROWS(48) DECAY_ROWS(56) DECAY_ROWS(64) }
+#undef DECAY_ROWS
         PB_CHECK_LAUNCH("channel_decay");
         return 0;
     }

@@ -347,3 +347,22 @@ def test_activations_give_the_same_bits_in_both_forms(form):
         return x
     a, b = made(0), made(1)
     assert torch.equal(torch.isnan(a), torch.isnan(b)) and torch.equal(a.nan_to_num(), b.nan_to_num())
+
+
+@pytest.mark.parametrize("rank", [8, 16, 24, 32, 40, 64])
+@pytest.mark.parametrize("T,channels", [(64, 128), (65, 129), (79, 1000), (2048, 40), (4100, 1024), (700, 2900)])
+def test_channel_decays_by_rows_give_the_same_bits(rank, T, channels):
+    # every number of tokens a block takes, against the kernel of eight tokens a block, which a matrix at an odd address goes to
+    from prelude_b200.ops import kernels as K
+    g = _gen(rank)
+    x1 = torch.randn(T, rank + 8, generator=g, device=DEV).bfloat16()[:, 8:]
+    room = torch.empty(channels * rank + 1, dtype=torch.bfloat16, device=DEV)
+    w2 = (torch.randn(channels, rank, generator=g, device=DEV) / rank ** 0.5).bfloat16()
+    odd = room[1:].view(channels, rank).copy_(w2)
+    bias = torch.linspace(-60.0, 30.0, channels, device=DEV)
+    got, want = K.channel_decay(x1, w2, bias, 16.0), K.channel_decay(x1, odd, bias, 16.0)
+    assert torch.equal(got, want)
+    z = x1.double() @ w2.double().T + bias.double()
+    exact = torch.exp(torch.nn.functional.logsigmoid(z) / 16.0)
+    # z from `rank` float32 products and sums of size below 60, a 16th of it in the exponent
+    assert bool(((got.double() - exact).abs() <= (rank * 6e-8 * 8 + 60 * 6e-8 + 4e-7) * exact + 1e-12).all())
