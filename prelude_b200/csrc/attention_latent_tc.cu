@@ -4,7 +4,7 @@
 //   q [n_tokens, H, kd] bfloat16      pages [num_pages, G, page_size, kd] bfloat16, the values a row's first vd elements
 //   out[t, h] = sum_j softmax_j(scale q[t, h] . k_j) k_j[0 .. vd)      float32 scores, weights and sums
 //
-// What bounds it are the cached rows, read once: 16 requests behind 3,000 tokens of 576 elements are 47 MB.  A block has one token's
+// What bounds it are the cached rows, read once: 16 requests behind 3,000 tokens of 576 elements are 55 MB.  A block has one token's
 // heads, at most 32 of them, and walks 64 rows at a time.
 //   Scores: S = Q K^T with the queries in tensor memory, where each of the four groups of 32 lanes holds all heads' queries: a thread has
 // one head and a quarter of the tile's rows, and the products' idle 96 lanes serve to spread the softmax over four warps.
@@ -19,8 +19,8 @@
 // order, each for its share of the heads: no scratch memory and no second kernel.
 //
 // Measured against the form on mma.sync with its merge (attention_paged_tc.cu, 32-row tiles with four barriers each), 32 heads, rows of 576
-// from memory, us: 16 requests behind 3,000 tokens 42.7 -> 22.2, 64 of them 125 -> 49 (3.8 TB/s), one 20.5 -> 15.7; behind 512 tokens 16
-// requests 17.3 -> 13.7, but 2 requests 10.7 and 11.6; behind 64 the other is ahead, 9.5 and 12.2.  What is left besides the bytes:
+// from memory, us: 16 requests behind 3,000 tokens each 42.4 -> 22.5, 64 of them 130 -> 50 (4.4 TB/s), one 22.2 -> 15.8; behind 512 tokens 16
+// requests 17.5 -> 12.3, 2 requests 11.4 -> 9.3; behind 64 tokens 16 requests 10.7 and 10.8, 256 requests 18.5 and 25.  What is left besides the bytes:
 // 5,000 cycles until the first scores, and 9,000 from the last tile to the end (two cluster barriers around the parts' way to the block
 // that adds them up).  Copies into the L2 cache four tiles ahead were no faster alone and 0.9 us slower between a layer's other kernels.
 //

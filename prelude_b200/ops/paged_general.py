@@ -28,9 +28,14 @@ from .library import check
 KERNEL = os.environ.get("PRELUDE_GENERAL_ATTN", "auto")
 PROMPT_KERNEL = os.environ.get("PRELUDE_GENERAL_PROMPT_ATTN", "auto")
 MAX_SPLITS = 32
-# rows that a token sees, at most, from which a decode step over a latent goes to the tcgen05 kernel, of few tokens and of more (32
-# heads, us there / on the general kernel: 512 rows, 2 tokens 11.6 / 10.7, 8 tokens 11.8 / 12.2, 16 tokens 13.7 / 17.3; 3,000 rows, 1 token
-# 15.7 / 20.5, 16 tokens 22.2 / 42.7; 64 rows, 16 tokens 12.2 / 9.5)
+# Rows that a token sees, at most, from which a decode step over a latent goes to the tcgen05 kernel, of few tokens and of more.  A launched
+# step knows its longest context (32 heads, us there / on the general kernel: 64 rows, 1 token 10.5 / 9.0, 16 tokens 10.8 / 10.7, 64 tokens
+# 12.0 / 15.2, 256 tokens 25 / 18.5; 256 rows, 2 tokens 9.5 / 9.6, 16 tokens 10.6 / 13.4; 512 rows, 2 tokens 9.3 / 11.4, 16 tokens 12.3 / 17.5;
+# 3,000 rows, 1 token 15.8 / 22.2, 16 tokens 22.5 / 42.4).  A recorded step does not: what counts is how many rows its block tables have room
+# for.  There the general kernel cuts the keys by that room too, and puts the parts together, so that short contexts gain as well (64 rows
+# in tables of 4,096: 1 token 9.1 / 12.7, 16 tokens 10.0 / 15.0, 64 tokens 12.1 / 17.1; of 128 heads 16 tokens 11.8 / 16.3) - but for
+# recorded steps of more blocks than multiprocessors, whose keys it leaves whole: 64 rows, 256 tokens 25.6 / 19.1, of 128 heads 64 tokens
+# 24.3 / 17.1.  From 256 rows these are ahead too (35.8 / 47.4, 32.7 / 45.6).
 LATENT_MIN_ROWS, LATENT_FEW_TOKENS, LATENT_MIN_ROWS_FEW = 512, 8, 1024
 
 
