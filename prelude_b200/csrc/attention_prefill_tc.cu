@@ -31,12 +31,13 @@
 //
 // What bounds it: the softmax groups.  A tile of 64 keys is 1,024 cycles of the special-function unit for both row tiles; in
 // step with one another the two groups kept it busy for half of the time and idle for the other, so their exponentials take
-// turns (8,192 tokens, 32 heads over 8 of 128: 612 us in step, 520 in turns, 2,175 cycles a tile).
+// turns (8,192 tokens, 32 heads over 8 of 128: 612 us in step, 520 in turns; 508 and 2,115 cycles a tile since capped scores have a kernel
+// of their own).
 // Against tiles of 128 keys with one warp each for loads and products, us: 32 heads over 8 of 128, 2,500 tokens of three requests behind 180 to
-// 300 64 -> 58, 2,048 tokens 52 -> 48, 8,192 543 -> 521, capped scores 80 -> 64; keys of 192 and values of 128, 16 heads, 1,500 tokens
-// behind 700 52 -> 47.  Heads of 64 gain less or lose: 64 over 8, 2,048 tokens 88 -> 83, but 16 over 16, 4,096 tokens 73.5 -> 75 and 8,192
-// 251 -> 262, 32 over 1, 8,192 496 -> 513; dense rows of 64 and of 128 elements, 2,048 tokens, 16 heads 39.5 and 42.5 -> 40 and 41.5, in some
-// processes 47 (more stages of the rings change neither).
+// 300 64 -> 57, 2,048 tokens 53 -> 48, 8,192 544 -> 508, capped scores 80.5 -> 65; keys of 192 and values of 128, 16 heads, 1,500 tokens
+// behind 700 52.5 -> 46.5.  Heads of 64 gain least: 64 over 8, 2,048 tokens 89 -> 83, 16 over 16, 4,096 tokens 78.5 -> 77, but 8,192 260 -> 267,
+// 32 over 1, 8,192 502 -> 506; dense rows of 64 and of 128 elements, 2,048 tokens, 16 heads 39.5 and 42.5 -> 38 and 40 (with either in some
+// processes 45 to 48; more stages of the rings do not change that).
 // Taken back: blocks that stay and take several pieces of work (no faster); the turn handed on before the last exponentials of
 // a tile (2,048 tokens 47.8 -> 48.0 to 49.0); five stages for rows of 128 (48.7).
 // The running maximum is kept in scaled log2 units and the accumulator is rescaled (by the row's own
@@ -116,7 +117,10 @@ struct PtParams {
     int flat;                       // keys and values lie in rows of their own maps (4 dimensions: element, row, head, page)
 };
 
-template <int KH, int VH>
+// CAP: scores are capped.  A kernel of its own: with the caps' two ways to a tanh in it the softmax groups' loop is twice as long, and waits for
+// instructions without ever capping a score (uncapped, us: 8,192 tokens, 32 heads over 8 of 128 521 -> 508, 16 over 16 of 64 271 -> 267,
+// 32 over 1 517 -> 506; 4,096 tokens, 16 over 16 of 64 82 -> 77; 1,500 rows of 192 behind 700 48.0 -> 46.6; 166 registers -> 138).
+template <int KH, int VH, bool CAP>
 __global__ void __launch_bounds__(PT_THREADS, 1)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                        const __grid_constant__ CUtensorMap map_v, PtParams pp) {
@@ -332,7 +336,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         const bool valid = tl < n_tok;
         const int row_pos = pos0 + tok0 + min(tl, n_tok - 1);      // rows without a token behave like the last token
         const int row_lo = p.window > 0 ? row_pos - p.window + 1 : (pp.chunk > 0 ? row_pos - row_pos % pp.chunk : 0);
-        const float cap2 = pp.cap_in * 2.8853900817779268f;       // 2 log2(e) / cap, in the units of q . k
+        [[maybe_unused]] const float cap2 = pp.cap_in * 2.8853900817779268f;       // 2 log2(e) / cap, in the units of q . k
         const uint32_t lane_base = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
         const uint32_t s_addr = lane_base + m * PT_S_COLS, p_addr = lane_base + PT_P_COL + m * PT_KEYS, o_addr = lane_base + T::O_COL + m * T::VD;
         float m_ref = -INFINITY, l = 0.f;
@@ -362,7 +366,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             __syncwarp();
             if (lane == 0) tc_mbar_arrive(&s_free[m]);                     // the next tile's scores may take their place
             const int key0 = key_tile(j) * PT_KEYS;
-            if (pp.cap_in > 0.f) {                                 // capped scores, before the mask
+            if constexpr (CAP) {                                   // before the mask
                 float am[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
                 for (int c = 0; c < PT_KEYS; ++c) am[c & 3] = fmaxf(am[c & 3], fabsf(__uint_as_float(sr[c])));
@@ -551,20 +555,28 @@ static int pt_encode(CUtensorMap* map, const void* ptr, int rank, const cuuint64
     return 0;
 }
 
-template <int KH, int VH>
-static int pt_launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const PtParams& pp, int n_tiles,
-                     cudaStream_t stream) {
+template <int KH, int VH, bool CAP>
+static int pt_launch_form(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const PtParams& pp, int n_tiles,
+                          cudaStream_t stream) {
     using T = PtTiling<KH, VH>;
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<KH, VH>, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM_BYTES);
+        cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<KH, VH, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM_BYTES);
         if (e != cudaSuccess)
             return pb_fail("attention_prefill_tc: cannot get %d bytes of shared memory: %s", T::SMEM_BYTES, cudaGetErrorString(e));
         configured = true;
     }
-    pb_launch(attn_prefill_tc_kernel<KH, VH>, dim3((unsigned)n_tiles * pp.a.n_kv_heads), dim3(PT_THREADS), (size_t)T::SMEM_BYTES, stream,
+    pb_launch(attn_prefill_tc_kernel<KH, VH, CAP>, dim3((unsigned)n_tiles * pp.a.n_kv_heads), dim3(PT_THREADS), (size_t)T::SMEM_BYTES, stream,
               mq, mk, mv, pp);
     return 0;
+}
+
+template <int KH, int VH>
+static int pt_launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const PtParams& pp, int n_tiles,
+                     cudaStream_t stream) {
+    if constexpr (KH == VH)                                      // (the sizes of paged heads: dense rows have no cap)
+        if (pp.cap_in > 0.f) return pt_launch_form<KH, VH, true>(mq, mk, mv, pp, n_tiles, stream);
+    return pt_launch_form<KH, VH, false>(mq, mk, mv, pp, n_tiles, stream);
 }
 
 static bool pt_pow2(int v) { return v > 0 && (v & (v - 1)) == 0; }
