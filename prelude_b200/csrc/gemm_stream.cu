@@ -12,9 +12,11 @@
 //    shared-memory stages (8 rows x one chunk of K per stage, one bulk copy per
 //    row, full and empty barriers); the compute warps take the stages two at a
 //    time.  Issuing a bulk copy costs a warp about 60 cycles whatever its size,
-//    and warps issue side by side (measured), so every loader warp issues two of
-//    a stage's eight copies, and the chunks are as long as shared memory allows:
-//    a whole row where it fits.  Weights are written by no kernel, so the
+//    and as much goes into a stage's wait and its announcement; warps issue side
+//    by side, so they take the stages in turn (all four on every stage, two copies
+//    each: chunks of 512 elements 45 us for 150 MB instead of 34, of 1,024 30
+//    instead of 26.5), and the chunks are as long as leaves four stages (gs_plan).
+//    Weights are written by no kernel, so the
 //    loaders fill the ring before they wait for the kernel before this one on
 //    the stream: the stream is already flowing when x becomes available.
 //  * x (a few KB per row) is copied whole into shared memory by the compute warps
@@ -48,10 +50,10 @@
 PB_TIMELINE_UNIT(gemm_stream)
 
 #define GS_WARPS 8                              // compute warps
-#define GS_LOADERS 4                            // loader warps; each issues GS_ROWS / GS_LOADERS copies per stage
+#define GS_LOADERS 4                            // loader warps, which take the stages in turn
 #define GS_THREADS ((GS_WARPS + GS_LOADERS) * 32)
 #define GS_ROWS 8                               // features per stage; a tile of the product is two stages
-#define GS_MAX_STAGES 8
+#define GS_MAX_STAGES 16
 #define GS_CHAINS 4                             // independent accumulators per warp
 #define GS_SMEM_LIMIT (227 * 1024 - 2048)
 
@@ -65,6 +67,7 @@ struct GsParams {
     int ks;                 // elements of K per stage
     int n_chunks;           // chunks of K per row
     int stages;
+    int sets;               // of the warps' sums in shared memory: two, or one where a second does not fit
     int out_f32;
     long long split_stride; // elements between the partial outputs of the splits of K (gridDim.y of them)
     int gated;              // W holds N gate rows, then N up rows; the output is silu(gate) * up, N wide
@@ -108,14 +111,15 @@ __global__ void __launch_bounds__(GS_THREADS, 1) gemm_stream_kernel(GsParams p) 
     }
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(8) uint64_t full_bar[GS_MAX_STAGES], empty_bar[GS_MAX_STAGES], x_bar;
-    __shared__ int s_issued, s_dead;
+    __shared__ int s_dead;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int x_stride = p.K * 2 + 16;                         // bytes between rows of x in shared memory
     const int w_stride = p.ks * 2 + 16;                        // bytes between rows of a stage
     const int stage_bytes = GS_ROWS * w_stride;
     unsigned char* sX = smem;                                  // [M] rows
     unsigned char* ring = sX + (size_t)p.M * x_stride;
-    float* red = reinterpret_cast<float*>(ring + (size_t)p.stages * stage_bytes);   // [GS_WARPS][8 MT batch rows][16 features]
+    // sets of [GS_WARPS][8 MT batch rows][16 features], which tiles take in turn: of two, one is written again behind the next tile's barrier only
+    float* sums = reinterpret_cast<float*>(ring + (size_t)p.stages * stage_bytes);
 
     // This block's features, in tiles of 16 = two stages of 8 (the last tile may have one).  Loader and compute
     // warps walk the stages in the same order: tile, chunk of K, half.
@@ -124,42 +128,42 @@ __global__ void __launch_bounds__(GS_THREADS, 1) gemm_stream_kernel(GsParams p) 
     const int n_tiles = (r1 - r0 + span - 1) / span;
 
     if (threadIdx.x == 0) {
-        s_issued = 0;
         s_dead = 0;
-        for (int s = 0; s < p.stages; ++s) { mbar_init(&full_bar[s], GS_LOADERS); mbar_init(&empty_bar[s], GS_WARPS); }
+        for (int s = 0; s < p.stages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], GS_WARPS); }
         mbar_init(&x_bar, GS_LOADERS);
         mbar_fence_init();
     }
     __syncthreads();
 
     if (warp >= GS_WARPS) {
-        // ---------------- loaders: warp j copies rows 2 j and 2 j + 1 of every stage (lanes 0 and 1) ----------------
-        const int lw = warp - GS_WARPS;
-        constexpr int PER = GS_ROWS / GS_LOADERS;
+        // ---------------- loaders: the warps take the stages in turn, a lane copies a row ----------------
+        // No more warps than stages: a warp that waits for a stage's tenant of one lap ago then knows that the one of two laps ago has left (it
+        // has waited for that or a later one), and a parity tells only two laps apart
+        const int lw = warp - GS_WARPS, n_loaders = min(GS_LOADERS, p.stages);
         bool ok = true;
-        int stage = 0, phase = 0, i = 0;
+        int stage = 0, phase = 0, i = 0, turn = 0;
 #pragma unroll 1
         for (int tile = 0; tile < n_tiles && ok; ++tile) {
             const int halves = (p.gated || r1 - (r0 + tile * span) > GS_ROWS) ? 2 : 1;
 #pragma unroll 1
             for (int kc = 0; kc < p.n_chunks && ok; ++kc) {
                 for (int h = 0; h < halves; ++h, ++i) {
-                    if (i >= p.stages) {                       // the first ring-full finds every stage free
-                        ok = mbar_wait_bounded(&empty_bar[stage], phase ^ 1);
-                        if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+                    if (turn == lw) {
+                        if (i >= p.stages) {                   // the first ring-full finds every stage free
+                            ok = mbar_wait_bounded(&empty_bar[stage], phase ^ 1);
+                            if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+                        }
+                        const int feat0 = r0 + tile * span + (p.gated ? 0 : h * GS_ROWS);   // first feature of the stage
+                        const int row0 = feat0 + (p.gated ? h * p.N : 0);             // its row of W: up rows follow the gate rows
+                        const int k0 = kc * p.ks, len = min(p.ks, p.K - k0);
+                        const int n_rows = min(GS_ROWS, r1 - feat0);
+                        // the copies may land before the expected bytes are posted: the phase cannot end before this arrival
+                        if (lane == 0) mbar_arrive_expect_tx(&full_bar[stage], (unsigned)n_rows * len * 2);
+                        if (lane < n_rows)
+                            bulk_copy_g2s(ring + (size_t)stage * stage_bytes + (size_t)lane * w_stride, p.W + (size_t)(row0 + lane) * p.ldw + k0,
+                                          (unsigned)len * 2, &full_bar[stage]);
                     }
-                    if (lw == 0 && lane == 0) *(volatile int*)&s_issued = i + 1;   // the stage's previous tenant has been consumed
-                    const int feat0 = r0 + tile * span + (p.gated ? 0 : h * GS_ROWS);   // first feature of the stage
-                    const int row0 = feat0 + (p.gated ? h * p.N : 0);                 // its row of W: up rows follow the gate rows
-                    const int k0 = kc * p.ks, len = min(p.ks, p.K - k0);
-                    const int n_rows = min(GS_ROWS, r1 - feat0);
-                    const int mine = min(PER, max(0, n_rows - lw * PER));        // rows of this stage that this warp brings
-                    // the copies may land before the expected bytes are posted: the phase cannot end before this arrival
-                    if (lane == 0) mbar_arrive_expect_tx(&full_bar[stage], (unsigned)mine * len * 2);
-                    const int rr = lw * PER + lane;
-                    if (lane < mine)
-                        bulk_copy_g2s(ring + (size_t)stage * stage_bytes + (size_t)rr * w_stride,
-                                      p.W + (size_t)(row0 + rr) * p.ldw + k0, (unsigned)len * 2, &full_bar[stage]);
+                    if (++turn == n_loaders) turn = 0;
                     if (++stage == p.stages) { stage = 0; phase ^= 1; }
                 }
             }
@@ -196,7 +200,7 @@ __global__ void __launch_bounds__(GS_THREADS, 1) gemm_stream_kernel(GsParams p) 
     const bool upper = (lane & 8) != 0;                        // this lane addresses a row of the second stage
     const int x_row = (MT == 1) ? (lane & 7) : ((lane & 7) + (lane >> 4) * 8);
     const unsigned b_off = min(x_row, p.M - 1) * x_stride + ((lane >> 3) & 1) * 16;
-    int stage = 0, phase = 0, item = 0;
+    int stage = 0, phase = 0;
 #pragma unroll 1
     for (int tile = 0; tile < n_tiles; ++tile) {
         const int halves = (p.gated || r1 - (r0 + tile * span) > GS_ROWS) ? 2 : 1;
@@ -215,14 +219,7 @@ __global__ void __launch_bounds__(GS_THREADS, 1) gemm_stream_kernel(GsParams p) 
 #pragma unroll 1
         for (int kc = 0; kc < p.n_chunks; ++kc) {
             const int stage2 = (stage + 1 == p.stages) ? 0 : stage + 1, phase2 = (stage + 1 == p.stages) ? phase ^ 1 : phase;
-            const int last = item + halves - 1;
-            bool landed = true;
-            if (*(volatile int*)&s_issued <= last) {           // not announced yet: the barrier may still be in an older phase
-                const long long t0 = clock64();
-                while (*(volatile int*)&s_issued <= last)
-                    if (clock64() - t0 > (1ll << 31)) { landed = false; break; }
-            }
-            landed = landed && mbar_wait_bounded(&full_bar[stage], phase);
+            bool landed = mbar_wait_bounded(&full_bar[stage], phase);
             if (halves == 2) landed = landed && mbar_wait_bounded(&full_bar[stage2], phase2);
             if (!__all_sync(0xffffffffu, landed)) {
                 if (lane == 0) { *(volatile int*)&s_dead = 1; if (p.status) atomicExch(p.status, 12); }
@@ -257,11 +254,11 @@ __global__ void __launch_bounds__(GS_THREADS, 1) gemm_stream_kernel(GsParams p) 
                 gs_mbar_arrive(&empty_bar[stage]);
                 if (halves == 2) gs_mbar_arrive(&empty_bar[stage2]);
             }
-            item += halves;
             for (int h = 0; h < halves; ++h)
                 if (++stage == p.stages) { stage = 0; phase ^= 1; }
         }
         // add the eight warps' sums: acc[.][j][e] is feature g (+8 for e >= 2), batch row 8 j + 2 t4 + (e & 1)
+        float* red = sums + (p.sets == 2 ? tile & 1 : 0) * (GS_WARPS * 16 * 8 * MT);
         float* mine = red + (size_t)warp * 16 * 8 * MT;
 #pragma unroll
         for (int j = 0; j < MT; ++j)
@@ -321,7 +318,7 @@ __global__ void __launch_bounds__(GS_THREADS, 1) gemm_stream_kernel(GsParams p) 
                 }
             }
         }
-        gs_bar_compute();                                      // the sums are read before the next tile overwrites them
+        if (p.sets == 1) gs_bar_compute();                     // the sums are read before the next tile overwrites them
     }
     PB_TL(PB_TL_GEMM_STREAM, PB_TL_DONE);
 }
@@ -340,23 +337,28 @@ static int gs_sms() {
     return g_gs_sms;
 }
 
-// Chunk of K per stage and number of stages for a shape: the fewest chunks per row (the longest copies) that
-// leave room for three stages, or for two if three never fit; false when x and two stages do not fit.
-static bool gs_plan(int M, int K, int* ks, int* n_chunks, int* stages, size_t* smem) {
+// Chunk of K per stage and number of stages for a shape: the fewest equal chunks per row (the longest copies) that leave room for four
+// stages.  A tile takes its stages two by two: with three, one is on its way while it waits.  150 MB of weights, us, chunk x stages: K = 2,560,
+// 12 rows 2,560 x 3 33.8, 1,280 x 7 28.6; 4,096, 2 rows 4,096 x 3 29.3, 2,048 x 6 25.2; 4,096, 16 rows 1,408 x 3 43.8, 1,024 x 5 32.2; 8,192, 8
+// rows 1,664 x 3 37.9, 1,024 x 5 30.2; 5,120, 16 rows 1,024 x 3 50.7, 640 x 4 46.0.
+static bool gs_plan(int M, int K, int* ks, int* n_chunks, int* stages, int* sets, size_t* smem) {
     const size_t x_bytes = (size_t)M * ((size_t)K * 2 + 16);
-    const size_t red_bytes = (size_t)GS_WARPS * 16 * 16 * 4;
-    if (x_bytes + red_bytes >= GS_SMEM_LIMIT) return false;
-    const size_t room = GS_SMEM_LIMIT - x_bytes - red_bytes;
-    for (int want = 3; want >= 2; --want) {
+    const size_t set_bytes = (size_t)GS_WARPS * 16 * (M <= 8 ? 8 : 16) * 4;
+    // pieces of 1,024 elements at least, of 640 where those leave too few stages, and where neither gives four stages as many as there are
+    const int least[4] = {1024, 640, 512, 512}, want[4] = {4, 4, 2, 2};
+    for (int rule = 0; rule < 4; ++rule) {
+        *sets = rule < 3 ? 2 : 1;
+        const size_t sums = *sets * set_bytes < 8192 ? 8192 : *sets * set_bytes, taken = x_bytes + sums, room = GS_SMEM_LIMIT - taken;
+        if (taken >= GS_SMEM_LIMIT) continue;
         for (int n = 1; n <= K / 16; ++n) {
-            const int k_per = ((K + n - 1) / n + 15) / 16 * 16;
+            const int unit = rule < 2 ? 128 : 16, k_per = n == 1 ? K : ((K + n - 1) / n + unit - 1) / unit * unit;
             const size_t stage = (size_t)GS_ROWS * ((size_t)k_per * 2 + 16);
-            if (k_per * 2 < 1024 && n > 1) break;                 // copies this short are not worth having
-            if (stage * want <= room) {
+            if (k_per < least[rule] && n > 1) break;              // copies this short are not worth having
+            if (stage * want[rule] <= room) {
                 size_t s = room / stage;
                 if (s > GS_MAX_STAGES) s = GS_MAX_STAGES;
                 *ks = k_per; *n_chunks = (K + k_per - 1) / k_per; *stages = (int)s;
-                *smem = x_bytes + red_bytes + s * stage;
+                *smem = taken + s * stage;
                 return true;
             }
         }
@@ -367,9 +369,9 @@ static bool gs_plan(int M, int K, int* ks, int* n_chunks, int* stages, size_t* s
 // Whether the kernel takes the shape (else the caller uses another product).
 PB_API int pb_gemm_stream_supported(int M, int N, int K, long long ldw, long long ldx) {
     if (M < 1 || M > 16 || N < 1 || K < 16 || K % 16 || ldw % 8 || ldx % 8) return 0;
-    int ks, nc, st;
+    int ks, nc, st, sets;
     size_t smem;
-    return gs_plan(M, K, &ks, &nc, &st, &smem) ? 1 : 0;
+    return gs_plan(M, K, &ks, &nc, &st, &sets, &smem) ? 1 : 0;
 }
 
 // gated: W is [2 N, K], N gate rows then N up rows, and out [M, N] = silu(x Wg^T) * (x Wu^T); no bias, no splits.
@@ -399,7 +401,7 @@ static int gs_run(const void* X, const void* W, const float* bias, void* out, in
     p.act = act; p.limit = limit; p.alpha = alpha;
     p.res = residual.res; p.gain = residual.gain; p.shift = residual.shift; p.slope = residual.slope;
     size_t smem;
-    gs_plan(M, k_part, &p.ks, &p.n_chunks, &p.stages, &smem);
+    gs_plan(M, k_part, &p.ks, &p.n_chunks, &p.stages, &p.sets, &smem);
     int blocks = gs_sms() / splits;
     if (blocks < 1) blocks = 1;
     if (blocks > (N + 7) / 8) blocks = (N + 7) / 8;           // at least 8 features per block
