@@ -740,9 +740,10 @@ def moe_gemv_takes(a: torch.Tensor, w: torch.Tensor, n_slots: int) -> bool:
 
 
 def moe_gemv(a: torch.Tensor, w: torch.Tensor, ids: torch.Tensor, rows_are_slots: bool, out_dtype: torch.dtype, gated: bool = False,
-             act: int = ACT_NONE, limit: float = 0.0, alpha: float = 0.0) -> torch.Tensor:
+             act: int = ACT_NONE, limit: float = 0.0, alpha: float = 0.0, status: Optional[torch.Tensor] = None) -> torch.Tensor:
     """The experts' products for a few tokens without a plan: ids int32 [T, top]; a [T, K] (the tokens' rows) or, with
-    ``rows_are_slots``, [T * top, K]; the result's rows are the slots token * top + choice."""
+    ``rows_are_slots``, [T * top, K]; the result's rows are the slots token * top + choice.  ``status`` is raised where a
+    block gave up waiting."""
     _cols(a, "a")
     _need(w, "w", a.dtype)
     _need(ids, "ids", torch.int32)
@@ -752,6 +753,11 @@ def moe_gemv(a: torch.Tensor, w: torch.Tensor, ids: torch.Tensor, rows_are_slots
         raise KernelLibraryError(f"moe_gemv: a {tuple(a.shape)}, choices {tuple(ids.shape)}")
     N = rows_w // 2 if gated else rows_w
     out = torch.empty((T * top, N), dtype=out_dtype, device=a.device)
+    if _l.library().pb_moe_stream_supported(Kdim, T * top, E):
+        check(_l.library().pb_moe_stream(a.data_ptr(), a.stride(0), 1 if rows_are_slots else top, w.data_ptr(), w.stride(0), N, Kdim, 1 if gated else 0, act,
+                                         float(limit), float(alpha), ids.data_ptr(), T * top, E, out.data_ptr(), out.stride(0), dtype_code(out_dtype), _ptr(status),
+                                         _stream()), "moe_stream")
+        return out
     check(_l.library().pb_moe_gemv(a.data_ptr(), a.stride(0), None, 1 if rows_are_slots else top, w.data_ptr(), w.stride(0), N, Kdim,
                                    1 if gated else 0, act, float(limit), float(alpha), None, None, None, E, ids.data_ptr(), T * top, out.data_ptr(), out.stride(0),
                                    dtype_code(out_dtype), _stream()), "moe_gemv")

@@ -61,10 +61,11 @@ def grouped_pays(tokens: int, top_k: int, n_experts: int, expert_bytes: int) -> 
     take; one token hits every expert once and always streams.
 
     The whole feed-forward at 8 to 128 experts of 1,024 x 512 to 4,096 x 2,048, top 2 to 8, with and without a gate, 1 to 64 tokens, weights
-    from memory (2,768 steps): of the 795 that leave the streaming kernel 17 are slower for it by more than 2 %, and by 16 % at most; all of
-    them together take 0.78 of the time.  Left behind: 228 steps that would gain more than 5 %.  At both ends, us, streamed / there: 16
-    experts of 2,048 x 768, top 2, gated, 20 tokens 52 / 52, 28 tokens 63 / 53; 64 of 4,096 x 2,048, top 6, gated, 16 tokens 450 / 448, 20
-    tokens 509 / 484, 32 tokens 684 / 518; 32 of 2,048 x 2,048, top 4, no gate, 8 tokens 76 / 87, 16 tokens 110 / 110, 24 tokens 137 / 111."""
+    from memory (2,768 steps), against the streaming kernel of matrices with short rows: of the 795 that leave it 17 are slower for it by
+    more than 2 %, and by 16 % at most; all of them together take 0.78 of the time.  Left behind: 228 steps that would gain more than 5 %.
+    The kernel that streams rows of 768 elements and more (``moe_stream.cu``) reads an expert once for eight pairs, so for these the line
+    lies on the early side: us, streamed / there: 64 experts of 4,096 x 2,048, top 6, gated, 12 tokens 332 / 378, 16 tokens 391 / 450, 32 tokens
+    505 / 514, 48 tokens 756 / 537; 32 of 2,048 x 2,048, top 4, no gate, 8 tokens 66 / 86, 24 tokens 92 / 111, 32 tokens 130 / 112."""
     hit = n_experts * (1.0 - (1.0 - top_k / n_experts) ** tokens)
     return (tokens * top_k - GROUPED_FIRST_READS * hit) * expert_bytes >= GROUPED_MIN_BYTES
 
@@ -217,8 +218,9 @@ class RoutedExperts:
         streamed = few and K.moe_gemv_takes(x, self.w_gate_up, ids.numel())
         grouped = self._grouped(x, streamed)
         if streamed and not grouped:
-            h = K.moe_gemv(x, self.w_gate_up, ids, False, x.dtype, gated=self.gated, **self.act)
-            y = K.moe_gemv(h, self.w_down, ids, True, torch.float32)
+            status = L.tc_status(x.device)
+            h = K.moe_gemv(x, self.w_gate_up, ids, False, x.dtype, gated=self.gated, status=status, **self.act)
+            y = K.moe_gemv(h, self.w_down, ids, True, torch.float32, status=status)
             return self._sum(y, None, weights, shared, x.dtype)
         if grouped:
             # fewer rows: the experts' weights are the rows of the paired-block products, the tokens their columns

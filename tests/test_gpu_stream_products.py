@@ -23,3 +23,37 @@ def test_stream_plans(M, K_, N):
     # products exact in float32; a chain adds K / 512 steps of 16, each cut to 2^-23 of the sum so far, then 4 chains and 8 warps are added
     assert float((got.double() - want).norm() / want.norm()) < 2.0 ** -23 * (K_ / 512 + 16)
     assert torch.equal(gemm_stream(x, w, out_dtype=torch.float32), got) and int(tc_status(x.device)) == 0
+
+
+@pytest.mark.parametrize("gated,act", [(False, "NONE"), (False, "RELU2"), (True, "NONE"), (True, "CLAMPED")])
+@pytest.mark.parametrize("slots", [False, True])
+@pytest.mark.parametrize("T,top,E,N,K_", [(1, 1, 1, 8, 768), (1, 4, 32, 100, 1040), (2, 2, 4, 136, 2048), (8, 4, 32, 2048, 2048), (9, 2, 3, 24, 4096), (17, 1, 2, 40, 2416),
+                                          (16, 6, 64, 512, 4096), (40, 8, 256, 64, 768), (24, 2, 2, 300, 7168), (3, 8, 1024, 16, 784)])
+def test_experts_streamed(T, top, E, N, K_, gated, act, slots):
+    from prelude_b200.ops import kernels as K
+    from prelude_b200.ops import library
+    assert library.library().pb_moe_stream_supported(K_, T * top, E)
+    w = rnd(E, N * (2 if gated else 1), K_, scale=K_ ** -0.5)
+    a = rnd(T * top if slots else T, K_, seed=3)
+    g = torch.Generator(device=DEV).manual_seed(5)
+    ids = torch.stack([torch.randperm(E, generator=g, device=DEV)[:top] for _ in range(T)]).int()
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    kw = dict(gated=gated, act=getattr(K, "ACT_" + act), limit=2.0, alpha=1.7, status=status)
+    got = K.moe_gemv(a, w, ids, slots, torch.float32, **kw)
+    rows, want = (a if slots else a.repeat_interleave(top, 0)).double(), torch.empty(T * top, N, dtype=torch.float64, device=DEV)
+    for e in ids.unique().tolist():
+        m = (ids.flatten() == e).nonzero().flatten()
+        z = rows[m] @ w[e].double().T
+        if gated:
+            u = z[:, N:]
+            z = z[:, :N]
+            z = torch.nn.functional.silu(z) * u if act == "NONE" else z.clamp(max=2.0) * torch.sigmoid(1.7 * z.clamp(max=2.0)) * (u.clamp(-2, 2) + 1)
+        elif act == "RELU2":
+            z = torch.relu(z) ** 2
+        want[m] = z
+    assert float((got.double() - want).norm() / want.norm()) < 3e-6
+    assert int(status) == 0 and torch.equal(K.moe_gemv(a, w, ids, slots, torch.float32, **kw), got)
+    # one rounding to bfloat16
+    assert torch.equal(K.moe_gemv(a, w, ids, slots, torch.bfloat16, **kw), got.bfloat16())
+    if not slots and T > 1:                          # a token's result does not depend on who else chose its experts
+        assert torch.equal(K.moe_gemv(a[1:2], w, ids[1:2].contiguous(), False, torch.float32, **kw), got[top:2 * top])
