@@ -54,6 +54,12 @@ __device__ __forceinline__ void pb_unpack16(const uint4& raw, float (&out)[8]) {
 template <typename T, int N>
 __device__ __forceinline__ void pb_ld16(const T* p, float (&out)[N]) { pb_unpack16(*reinterpret_cast<const uint4*>(p), out); }
 
+__device__ __forceinline__ void moe_mma(float* c, const unsigned* a, unsigned b0, unsigned b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
 // Router logits in 32-bit: out[t, e] = sum_k x[t, k] * W[e, k], every product exact in float32 (the operands are
 // float32, or bfloat16 whose products fit), float32 sums.  A warp takes a token and four experts; a lane sums every
 // 32nd element in ascending order and the lanes meet in a fixed tree, so the order depends on K alone.
@@ -211,15 +217,13 @@ PB_API int pb_router_logits(const void* x, long long ldx, const void* W, float* 
 }
 
 // One warp per token.  Lane l holds the scores of experts l, l + 32, ...; a choice is a warp-wide argmax (larger
-// score, then smaller index), so a token costs (groups * gtop + top) rounds of five shuffles instead of as many
-// passes of one thread over all experts.
+// score, then smaller index) by two reductions of whole numbers: a score's bits in an order that whole numbers share, then the
+// smallest index that has it (five rounds of shuffles take as long as ten times one of them).
 __device__ __forceinline__ void moe_warp_argmax(float& val, int& idx) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float ov = __shfl_xor_sync(0xffffffffu, val, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-        if (ov > val || (ov == val && oi < idx)) { val = ov; idx = oi; }
-    }
+    const unsigned u = __float_as_uint(val + 0.f), key = idx == 0x7fffffff ? 0u : (u & 0x80000000u) ? ~u : u | 0x80000000u;   // + 0: one zero
+    const unsigned best = __reduce_max_sync(0xffffffffu, key);
+    idx = (int)__reduce_min_sync(0xffffffffu, key == best ? (unsigned)idx : 0x7fffffffu);
+    val = best == 0u ? -INFINITY : __uint_as_float((best & 0x80000000u) ? best & 0x7fffffffu : ~best);
 }
 
 enum MoeScoring : int { MOE_SIGMOID = 0, MOE_SOFTMAX = 1, MOE_SOFTMAX_CHOSEN = 2 };
@@ -254,10 +258,12 @@ __device__ __forceinline__ void moe_route_token(const float* z, const MoeRouteAr
         return a.scoring == MOE_SOFTMAX ? expf(v - zmax) * inv_sum : a.scoring == MOE_SOFTMAX_CHOSEN ? v : 1.0f / (1.0f + expf(-v));
     };
     float sc[SLOTS];                                         // what the choice goes by
+    int gid[SLOTS];                                          // its group
 #pragma unroll
     for (int i = 0; i < SLOTS; ++i) {
         const int e = lane + 32 * i;
         sc[i] = e < n_experts ? score(e) + (a.correction ? a.correction[e] : 0.f) : NONE;
+        gid[i] = e < n_experts ? e / per : 0;
     }
     unsigned long long allowed = groups >= 64 ? ~0ull : ((1ull << groups) - 1ull);
     if (a.keep < groups) {
@@ -272,7 +278,7 @@ __device__ __forceinline__ void moe_route_token(const float* z, const MoeRouteAr
 #pragma unroll
                 for (int i = 0; i < SLOTS; ++i) {
                     const int e = lane + 32 * i;
-                    if (e < n_experts && e / per == g && !((taken >> i) & 1u) && sc[i] > val) { val = sc[i]; idx = e; }
+                    if (e < n_experts && gid[i] == g && !((taken >> i) & 1u) && sc[i] > val) { val = sc[i]; idx = e; }
                 }
                 moe_warp_argmax(val, idx);
                 if (idx < n_experts) sum += val;
@@ -299,7 +305,7 @@ __device__ __forceinline__ void moe_route_token(const float* z, const MoeRouteAr
 #pragma unroll
         for (int i = 0; i < SLOTS; ++i) {
             const int e = lane + 32 * i;
-            if (e < n_experts && ((allowed >> (e / per)) & 1ull) && !((chosen >> i) & 1u) && sc[i] > val) { val = sc[i]; idx = e; }
+            if (e < n_experts && ((allowed >> gid[i]) & 1ull) && !((chosen >> i) & 1u) && sc[i] > val) { val = sc[i]; idx = e; }
         }
         moe_warp_argmax(val, idx);
         if (idx >= n_experts) {                              // scores that are no numbers: any allowed expert not yet chosen
@@ -454,55 +460,217 @@ PB_API int pb_moe_route_few(const void* x, long long ldx, const void* W, int dty
     return 0;
 }
 
-// One block.  ids [n_slots] in [0, n_experts); offsets [n_experts + 1]; order, place_of [n_slots];
+// Router logits and choice of a prompt step, on the tensor cores: a block takes 16 tokens and 64 experts, its sixteen warps a sixteenth of K
+// each, operands straight from global memory (a lane reads 16 bytes of a row, which serve two steps of 16: k is permuted alike in
+// both operands), products exact, float32 sums; the warps' sums meet in shared memory in a fixed tree.  With up to 64 experts the block
+// chooses too, a warp a token, else another kernel does.  The order of the sums depends on K alone.
+// What bounds it: trips to the L2 cache, where every block reads its share of the router's matrix.  Logits and choice, us, against the kernels above on
+// the float32 units: 64 experts, K 4,096: 64 tokens 13.3 (16.3), 300 13.7 (20.6), 2,048 14.2 (48); 256, K 7,168: 64 tokens 26 (63), 2,048 88 (277);
+// 32, K 2,048, 2,048 tokens 8.6 (23).  Error of the logits against 64 bits: 8.5e-8 (9.5e-8), 9.7e-8 (1.16e-7), 7.5e-8 (7.9e-8); with the tensor cores'
+// own running sums 4.8e-7.
+#define RT_TOKENS 16
+#define RT_WARPS 16
+#define RT_EXPERTS 64                                        // of one pass
+#define RT_MIN_TOKENS 64
+template <int SLOTS>
+__global__ void __launch_bounds__(32 * RT_WARPS, 1)
+moe_route_tokens_kernel(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* W, int n_tokens, int K, MoeRouteArgs args, int32_t* ids, float* weights,
+                        float* logits) {
+    extern __shared__ __align__(16) float rt_sm[];           // [warps][tokens][RT_EXPERTS] sums, then [tokens][n_experts] logits
+    float* z = rt_sm + RT_WARPS * RT_TOKENS * RT_EXPERTS;
+    pb_grid_dep_launch();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane >> 2, c = lane & 3;
+    const int t0 = blockIdx.x * RT_TOKENS, E = args.n_experts;
+    const int steps = K / 32, per = (steps + RT_WARPS - 1) / RT_WARPS, s0 = warp * per, s1 = min(s0 + per, steps);
+    const __nv_bfloat16* xa = x + (size_t)min(t0 + r, n_tokens - 1) * ldx + c * 8;
+    const __nv_bfloat16* xb = x + (size_t)min(t0 + r + 8, n_tokens - 1) * ldx + c * 8;
+    const int e0 = blockIdx.y * RT_EXPERTS;
+    {
+        float acc[8][4];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+        const __nv_bfloat16* wr = W + (size_t)c * 8;
+        uint4 w[8], a, b;
+        auto ask_w = [&](int s) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) w[j] = *reinterpret_cast<const uint4*>(wr + (size_t)min(e0 + 8 * j + r, E - 1) * K + s * 32);
+        };
+        auto ask_x = [&](int s) {
+            a = *reinterpret_cast<const uint4*>(xa + s * 32);
+            b = *reinterpret_cast<const uint4*>(xb + s * 32);
+        };
+        if (s0 < s1) ask_w(s0);                              // written by no kernel: before the wait
+        pb_grid_dep_wait();
+        if (s0 < s1) ask_x(s0);
+        for (int s = s0; s < s1; ++s) {
+            const uint4 ca = a, cb = b;
+            uint4 cw[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) cw[j] = w[j];
+            if (s + 1 < s1) { ask_w(s + 1); ask_x(s + 1); }
+            const unsigned a0[4] = {ca.x, cb.x, ca.y, cb.y}, a1[4] = {ca.z, cb.z, ca.w, cb.w};
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                // sixteen products at a time: what the tensor cores add to a running sum they cut off instead of rounding it
+                float p[4] = {0.f, 0.f, 0.f, 0.f}, q[4] = {0.f, 0.f, 0.f, 0.f};
+                moe_mma(p, a0, cw[j].x, cw[j].y);
+                moe_mma(q, a1, cw[j].z, cw[j].w);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) acc[j][u] += p[u] + q[u];
+            }
+        }
+        float* mine = rt_sm + warp * RT_TOKENS * RT_EXPERTS;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            *reinterpret_cast<float2*>(mine + r * RT_EXPERTS + 8 * j + 2 * c) = make_float2(acc[j][0], acc[j][1]);
+            *reinterpret_cast<float2*>(mine + (r + 8) * RT_EXPERTS + 8 * j + 2 * c) = make_float2(acc[j][2], acc[j][3]);
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < RT_TOKENS * RT_EXPERTS; i += 32 * RT_WARPS) {
+            const int t = i / RT_EXPERTS, e = e0 + i % RT_EXPERTS;
+            float v[RT_WARPS];
+#pragma unroll
+            for (int k = 0; k < RT_WARPS; ++k) v[k] = rt_sm[k * RT_TOKENS * RT_EXPERTS + i];
+#pragma unroll
+            for (int o = RT_WARPS / 2; o > 0; o >>= 1)
+#pragma unroll
+                for (int k = 0; k < o; ++k) v[k] += v[k + o];
+            if (e < E) {
+                if (SLOTS <= 2) z[t * E + e] = v[0];
+                if (logits && t0 + t < n_tokens) logits[(size_t)(t0 + t) * E + e] = v[0];
+            }
+        }
+        __syncthreads();
+    }
+    if (SLOTS > 2) return;                                   // more experts than a block sums: the choice is another kernel's
+    for (int t = warp; t < RT_TOKENS && t0 + t < n_tokens; t += RT_WARPS)
+        moe_route_token<SLOTS>(z + t * E, args, ids + (size_t)(t0 + t) * args.top, weights + (size_t)(t0 + t) * args.top);
+}
+
+// Whether pb_moe_route_tokens takes the sizes.  Fewer tokens than 64 take no longer on the kernels above, nor do eight experts once the blocks of 16
+// tokens make a second wave (K 1,024, 4,096 tokens: 9.6 us against 8.9).
+PB_API int pb_moe_route_tokens_supported(int n_tokens, int n_experts, int K) {
+    return n_tokens >= RT_MIN_TOKENS && K % 32 == 0 && (n_experts > 8 || n_tokens <= 148 * RT_TOKENS) ? 1 : 0;
+}
+
+// x [n_tokens, K] with row stride ldx, W [n_experts, K], both bfloat16; logits float32 [n_tokens, n_experts], null with up to 64 experts if
+// nobody wants them; the rest as pb_moe_route.
+PB_API int pb_moe_route_tokens(const void* x, long long ldx, const void* W, int K, const float* correction, const float* bias, int n_tokens, int n_experts,
+                               int top, int groups, int keep, int gtop, int scoring, int renorm, float renorm_eps, float scale, int32_t* ids, float* weights,
+                               float* logits, cudaStream_t stream) {
+    const MoeRouteArgs args{correction, bias, n_experts, top, groups, keep, gtop, renorm, scoring, renorm_eps, scale};
+    if (int e = moe_route_check(n_tokens, args)) return e;
+    PB_REQUIRE(K > 0 && K % 32 == 0 && ldx >= K && ldx % 8 == 0, "moe_route_tokens: K=%d ldx=%lld not taken", K, ldx);
+    PB_REQUIRE(x && W && ids && weights && pb_aligned(x, 16) && pb_aligned(W, 16) && (logits || n_experts <= RT_EXPERTS), "moe_route_tokens: null or unaligned pointer");
+    if (n_tokens == 0) return 0;
+    const size_t smem = ((size_t)RT_WARPS + 1) * RT_TOKENS * RT_EXPERTS * 4;
+    const dim3 grid((n_tokens + RT_TOKENS - 1) / RT_TOKENS, (n_experts + RT_EXPERTS - 1) / RT_EXPERTS);
+#define ROUTE_LAUNCH(S)                                                                                                                              \
+    do {                                                                                                                                             \
+        static const cudaError_t set_ = cudaFuncSetAttribute(moe_route_tokens_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);     \
+        PB_REQUIRE(set_ == cudaSuccess, "moe_route_tokens: %s", cudaGetErrorString(set_));                                                           \
+        pb_launch(moe_route_tokens_kernel<S>, grid, dim3(32 * RT_WARPS), smem, stream, (const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)W, n_tokens, K, args, \
+                  ids, weights, logits);                                                                                                             \
+    } while (0)
+    if (n_experts <= 32) ROUTE_LAUNCH(1);
+    else if (n_experts <= RT_EXPERTS) ROUTE_LAUNCH(2);
+    else ROUTE_LAUNCH(8);
+#undef ROUTE_LAUNCH
+    PB_CHECK_LAUNCH("moe_route_tokens");
+    if (n_experts <= RT_EXPERTS) return 0;
+    return pb_moe_route(logits, correction, bias, n_tokens, n_experts, top, groups, keep, gtop, scoring, renorm, renorm_eps, scale, ids, weights, stream);
+}
+
+// One cluster.  ids [n_slots] in [0, n_experts); offsets [n_experts + 1]; order, place_of [n_slots];
 // tile_expert, tile_row0 [max_tiles], max_tiles >= ceil(n_slots / MOE_BM) + n_experts.
+// What bounds it: trips to memory one behind the other, and a shared counter per choice.  So every block of the cluster takes an equal run
+// of the choices, asks for all of a thread's (up to MOE_SORT_HELD) at once, and counting them gives each its rank among its
+// expert's in the run; the blocks then read one another's counts.  12,288 choices of 64 experts 16 -> 4.8 us, 1,800 of them 4 by one block.
+#define MOE_SORT_HELD 8
+#define MOE_SORT_CLUSTER 8
 __global__ void __launch_bounds__(1024) moe_sort_kernel(const int32_t* ids, int n_slots, int n_experts,
                                                         int32_t* offsets, int32_t* order,
                                                         int32_t* place_of, int32_t* tile_expert,
                                                         int32_t* tile_row0, int max_tiles, int tile_rows) {
     pb_grid_dep_launch();
+    __shared__ int count[MOE_MAX_EXPERTS];                   // of this block's choices
+    __shared__ int cursor[MOE_MAX_EXPERTS];                  // of places handed out in chunks before
+    __shared__ int start[MOE_MAX_EXPERTS + 1], mine[MOE_MAX_EXPERTS], tile0[MOE_MAX_EXPERTS + 1];
+    cg::cluster_group cluster = cg::this_cluster();
+    const int rank_in = (int)cluster.block_rank(), blocks = (int)cluster.num_blocks(), tid = threadIdx.x, threads = blockDim.x;
+    for (int e = tid; e < n_experts; e += threads) count[e] = cursor[e] = 0;
+    __syncthreads();
     pb_grid_dep_wait();
-    __shared__ int count[MOE_MAX_EXPERTS], start[MOE_MAX_EXPERTS + 1], tile0[MOE_MAX_EXPERTS + 1];
-    for (int e = threadIdx.x; e < n_experts; e += blockDim.x) count[e] = 0;
-    __syncthreads();
-    for (int i = threadIdx.x; i < n_slots; i += blockDim.x) {
-        const int e = min(max(ids[i], 0), n_experts - 1);
-        atomicAdd(&count[e], 1);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int at = 0, tiles = 0;
-        for (int e = 0; e < n_experts; ++e) {
-            start[e] = at;
-            tile0[e] = tiles;
-            at += count[e];
-            tiles += (count[e] + tile_rows - 1) / tile_rows;
+    const int per = (n_slots + blocks - 1) / blocks, lo = min(rank_in * per, n_slots), hi = min(lo + per, n_slots);
+    const int chunk = MOE_SORT_HELD * threads;
+    int held[MOE_SORT_HELD], rank[MOE_SORT_HELD];
+    auto number = [&](int base, int* counter) {
+#pragma unroll
+        for (int j = 0; j < MOE_SORT_HELD; ++j) {
+            const int i = base + j * threads + tid;
+            held[j] = i < hi ? min(max(ids[i], 0), n_experts - 1) : -1;
         }
-        start[n_experts] = at;
-        tile0[n_experts] = tiles;
+#pragma unroll
+        for (int j = 0; j < MOE_SORT_HELD; ++j) rank[j] = held[j] >= 0 ? atomicAdd(&counter[held[j]], 1) : 0;
+    };
+    for (int base = lo; base < hi; base += chunk) number(base, count);
+    cluster.sync();                                          // every block's counts are there
+    for (int e = tid; e < n_experts; e += threads) {
+        int total = 0, before = 0;
+        for (int r = 0; r < blocks; ++r) {
+            const int c = cluster.map_shared_rank(count, r)[e];
+            before += r < rank_in ? c : 0;
+            total += c;
+        }
+        start[e] = total;
+        mine[e] = before;
     }
     __syncthreads();
-    for (int e = threadIdx.x; e <= n_experts; e += blockDim.x) offsets[e] = start[e];
-    for (int e = threadIdx.x; e < n_experts; e += blockDim.x) {
-        for (int k = 0, n = tile0[e + 1] - tile0[e]; k < n; ++k) {
-            if (tile0[e] + k < max_tiles) {
-                tile_expert[tile0[e] + k] = e;
-                tile_row0[tile0[e] + k] = start[e] + k * tile_rows;
+    if (tid < 32) {
+        int at = 0, tiles = 0;
+        for (int e0 = 0; e0 < n_experts; e0 += 32) {
+            const int e = e0 + tid, n = e < n_experts ? start[e] : 0, nt = (n + tile_rows - 1) / tile_rows;
+            int sn = n, st = nt;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int vn = __shfl_up_sync(0xffffffffu, sn, o), vt = __shfl_up_sync(0xffffffffu, st, o);
+                if (tid >= o) { sn += vn; st += vt; }
+            }
+            if (e < n_experts) { start[e] = at + sn - n; tile0[e] = tiles + st - nt; }
+            at += __shfl_sync(0xffffffffu, sn, 31);
+            tiles += __shfl_sync(0xffffffffu, st, 31);
+        }
+        if (tid == 0) { start[n_experts] = at; tile0[n_experts] = tiles; }
+    }
+    __syncthreads();
+    // a block of one chunk still holds its choices and their ranks; else they are numbered again
+    const bool again = hi - lo > chunk;
+    for (int base = lo; base < hi; base += chunk) {
+        if (again) number(base, cursor);
+#pragma unroll
+        for (int j = 0; j < MOE_SORT_HELD; ++j) {
+            if (held[j] < 0) continue;
+            const int i = base + j * threads + tid, place = start[held[j]] + mine[held[j]] + rank[j];
+            order[place] = i;
+            place_of[i] = place;
+        }
+    }
+    if (rank_in == 0) {
+        for (int e = tid; e <= n_experts; e += threads) offsets[e] = start[e];
+        for (int i = tile0[n_experts] + tid; i < max_tiles; i += threads) {
+            tile_expert[i] = -1;
+            tile_row0[i] = 0;
+        }
+        for (int e = tid; e < n_experts; e += threads) {
+            for (int k = 0, n = tile0[e + 1] - tile0[e]; k < n; ++k) {
+                if (tile0[e] + k < max_tiles) {
+                    tile_expert[tile0[e] + k] = e;
+                    tile_row0[tile0[e] + k] = start[e] + k * tile_rows;
+                }
             }
         }
-        count[e] = 0;                                       // now the cursor of the expert's places
     }
-    for (int i = tile0[n_experts] + threadIdx.x; i < max_tiles; i += blockDim.x) {
-        tile_expert[i] = -1;
-        tile_row0[i] = 0;
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < n_slots; i += blockDim.x) {
-        const int e = min(max(ids[i], 0), n_experts - 1);
-        const int place = start[e] + atomicAdd(&count[e], 1);
-        order[place] = i;
-        place_of[i] = place;
-    }
+    cluster.sync();                                          // nobody leaves while others read its counts
 }
 
 // Rows of a tile: 128 where the experts have many rows each (prompt steps: the large-tile kernel), else 64.
@@ -514,8 +682,20 @@ PB_API int pb_moe_sort(const int32_t* ids, int n_slots, int n_experts, int32_t* 
     PB_REQUIRE(tile_rows == MOE_BM || tile_rows == MOE_BM_LARGE || tile_rows == 256, "moe_sort: tiles have %d, %d or 256 rows", MOE_BM, MOE_BM_LARGE);
     PB_REQUIRE(max_tiles >= (n_slots + tile_rows - 1) / tile_rows + n_experts, "moe_sort: room for %d tiles is too little", max_tiles);
     PB_REQUIRE(ids && offsets && order && place_of && tile_expert && tile_row0, "moe_sort: null pointer");
-    pb_launch(moe_sort_kernel, dim3(1), dim3(1024), 0, stream, ids, n_slots, n_experts, offsets, order, place_of, tile_expert,
-              tile_row0, max_tiles, tile_rows);
+    // a cluster of one block, or of eight where one block would hold two choices a thread and more
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = n_slots >= 2048 ? MOE_SORT_CLUSTER : 1;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = dim3(attr[0].val.clusterDim.x);
+    cfg.blockDim = dim3(1024);
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = pb_pdl_enabled() ? 2 : 1;
+    cudaLaunchKernelEx(&cfg, moe_sort_kernel, ids, n_slots, n_experts, offsets, order, place_of, tile_expert, tile_row0, max_tiles, tile_rows);
     PB_CHECK_LAUNCH("moe_sort");
     return 0;
 }
@@ -721,11 +901,6 @@ __device__ __forceinline__ void moe_cp16(void* smem, const void* gmem, bool pred
 __device__ __forceinline__ void moe_ldsm4(unsigned (&r)[4], unsigned addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-__device__ __forceinline__ void moe_mma(float* c, const unsigned* a, unsigned b0, unsigned b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
 template <typename TC, bool GATED>
@@ -1064,7 +1239,15 @@ __global__ void moe_gather_rows_kernel(const T* x, long long ldx, const int32_t*
     if (width % (16 / sizeof(T)) == 0 && ldx % (16 / sizeof(T)) == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 &&
         reinterpret_cast<uintptr_t>(out) % 16 == 0) {
         const int n = width / (16 / (int)sizeof(T));
-        for (int i = threadIdx.x; i < n; i += blockDim.x) reinterpret_cast<uint4*>(dst)[i] = reinterpret_cast<const uint4*>(src)[i];
+        for (int i0 = threadIdx.x; i0 < n; i0 += 4 * blockDim.x) {      // four pieces on their way at a time
+            uint4 piece[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (i0 + u * (int)blockDim.x < n) piece[u] = reinterpret_cast<const uint4*>(src)[i0 + u * blockDim.x];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (i0 + u * (int)blockDim.x < n) reinterpret_cast<uint4*>(dst)[i0 + u * blockDim.x] = piece[u];
+        }
     } else {
         for (int i = threadIdx.x; i < width; i += blockDim.x) dst[i] = src[i];
     }
@@ -1161,6 +1344,31 @@ __device__ __forceinline__ void moe_stv(__nv_bfloat16* p, const float (&v)[V]) {
     }
 }
 
+// V elements of a row as they lie in memory
+template <typename T, int V>
+struct MoeRaw {
+    static constexpr int PIECES = sizeof(T) * V / 16;
+    uint4 raw[PIECES > 0 ? PIECES : 1];
+    __device__ __forceinline__ void load(const T* p) {
+        if constexpr (PIECES > 0) {
+#pragma unroll
+            for (int i = 0; i < PIECES; ++i) raw[i] = reinterpret_cast<const uint4*>(p)[i];
+        } else raw[0].x = __float_as_uint(pb_ld(p));
+    }
+    __device__ __forceinline__ void unpack(float (&o)[V]) const {
+        if constexpr (PIECES > 0) {
+            constexpr int N = 16 / sizeof(T);
+#pragma unroll
+            for (int i = 0; i < PIECES; ++i) {
+                float f[N];
+                pb_unpack16(raw[i], f);
+#pragma unroll
+                for (int e = 0; e < N; ++e) o[i * N + e] = f[e];
+            }
+        } else o[0] = __uint_as_float(raw[0].x);
+    }
+};
+
 struct MoeSumArgs {
     const int32_t* place_of;
     const float* weights;
@@ -1191,21 +1399,27 @@ __global__ void __launch_bounds__(256) moe_sum_kernel(const TY* y, const TS* sha
     float r[V];
     float* rp = a.res ? a.res + (size_t)t * a.width + col : nullptr;
     if (rp) moe_ldv<V>(rp, r);
-    for (int c0 = 0; c0 < a.top; c0 += 4) {                  // four choices' loads in flight
-        float yv[4][V], w[4];
+    // the choices' rows in flight, as they lie in memory: eight of 16 bytes, four of 32 (2,048 tokens of 4,096, six bfloat16 choices from memory, us:
+    // 45 -> 31; four at a time, unpacked, kept half the registers' worth in flight)
+    constexpr int AT = sizeof(TY) * V <= 16 ? 8 : 4;
+    for (int c0 = 0; c0 < a.top; c0 += AT) {
+        MoeRaw<TY, V> raw[AT];
+        float w[AT];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < AT; ++u) {
             if (c0 + u < a.top) {
                 const int slot = t * a.top + c0 + u;
                 w[u] = a.weights[slot];
-                moe_ldv<V>(y + (size_t)(a.place_of ? a.place_of[slot] : slot) * a.width + col, yv[u]);
+                raw[u].load(y + (size_t)(a.place_of ? a.place_of[slot] : slot) * a.width + col);
             }
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
+        for (int u = 0; u < AT; ++u)
             if (c0 + u < a.top) {
+                float yv[V];
+                raw[u].unpack(yv);
 #pragma unroll
-                for (int e = 0; e < V; ++e) v[e] = fmaf(w[u], yv[u][e], v[e]);
+                for (int e = 0; e < V; ++e) v[e] = fmaf(w[u], yv[e], v[e]);
             }
     }
     for (int p = 0; p < a.shared_parts; ++p) {

@@ -668,6 +668,35 @@ def moe_route_few(x: torch.Tensor, w: torch.Tensor, top: int, groups: int, keep:
     return ids, weights
 
 
+def moe_route_tokens_takes(x: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether the router of a prompt step's rows x [T, K] against w [E, K] runs on the tensor cores."""
+    return (x.dtype == torch.bfloat16 and w.dtype == x.dtype and x.stride(1) == 1 and w.is_contiguous() and x.data_ptr() % 16 == 0
+            and w.data_ptr() % 16 == 0 and x.stride(0) % 8 == 0 and bool(_l.library().pb_moe_route_tokens_supported(x.shape[0], w.shape[0], w.shape[1])))
+
+
+def moe_route_tokens(x: torch.Tensor, w: torch.Tensor, top: int, groups: int, keep: int, group_top: int, renormalize: bool,
+                     correction: Optional[torch.Tensor] = None, softmax: bool = False, renormalize_eps: float = 0.0, scale: float = 1.0,
+                     bias: Optional[torch.Tensor] = None, softmax_chosen: bool = False, logits: Optional[torch.Tensor] = None):
+    """``router_logits`` and ``moe_route`` for a prompt step's rows, in one kernel with up to 64 experts; the products of sixteen are summed by
+    the tensor cores, these sums in float32 (``logits`` float32 [T, E] gets them)."""
+    _cols(x, "x")
+    T, Kdim = x.shape
+    E = w.shape[0]
+    _route_vectors(correction, bias, E)
+    if logits is not None:
+        _need(logits, "logits", torch.float32)
+        if logits.shape != (T, E):
+            raise KernelLibraryError(f"moe_route_tokens: room for logits {tuple(logits.shape)}, not {(T, E)}")
+    elif E > 64:
+        logits = torch.empty((T, E), dtype=torch.float32, device=x.device)
+    ids = torch.empty((T, top), dtype=torch.int32, device=x.device)
+    weights = torch.empty((T, top), dtype=torch.float32, device=x.device)
+    check(_l.library().pb_moe_route_tokens(x.data_ptr(), x.stride(0), w.data_ptr(), Kdim, _ptr(correction), _ptr(bias), T, E, top, groups, keep, group_top,
+                                           _scoring(softmax, softmax_chosen), 1 if renormalize else 0, float(renormalize_eps), float(scale),
+                                           ids.data_ptr(), weights.data_ptr(), _ptr(logits), _stream()), "moe_route_tokens")
+    return ids, weights
+
+
 class MoePlan:
     """Where a step's (token, choice) slots sit once grouped by expert; all on the device."""
 

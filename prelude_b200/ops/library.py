@@ -85,6 +85,8 @@ _SIGNATURES = {
     "pb_moe_route": ([P, P, P, I, I, I, I, I, I, I, I, F, F, P, P, P], I),
     "pb_moe_route_few_supported": ([I, I, I], I),
     "pb_moe_route_few": ([P, L, P, I, I, P, P, I, I, I, I, I, I, I, I, F, F, P, P, P], I),
+    "pb_moe_route_tokens_supported": ([I, I, I], I),
+    "pb_moe_route_tokens": ([P, L, P, I, P, P, I, I, I, I, I, I, I, I, F, F, P, P, P, P], I),
     "pb_moe_sum": ([P, I, P, P, P, I, I, L, P, P, F, P, P, P, I, I, I, I, I, P], I),
     "pb_moe_sum_normed_supported": ([I, I], I),
     "pb_moe_sum_normed": ([P, I, P, P, P, I, I, L, P, F, P, P, P, P, F, P, I, I, I, I, I, P], I),

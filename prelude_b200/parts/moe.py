@@ -1,8 +1,8 @@
 """Routed experts: a mixture of feed-forwards (SiLU-gated, gated by the clamped unit, or plain with squared ReLU), a few per token.
 
 The router's logits are a 32-bit product of the feed-forward's input with the
-router matrix (float32 sums of exact products on the float32 units, whatever
-the run's type: ``kernels.router_logits``), plus a bias where the design has one.  Scores are their sigmoids or their softmax,
+router matrix (float32 sums of exact products, whatever the run's type: ``kernels.router_logits``,
+``kernels.moe_route_tokens``), plus a bias where the design has one.  Scores are their sigmoids or their softmax,
 or the logits themselves with the softmax over the chosen ones as weights; experts form equal groups of
 neighbours, a group scores the sum of its largest scores, and only experts of
 the best groups can be chosen; the chosen scores weigh the experts' outputs
@@ -180,6 +180,8 @@ class RoutedExperts:
         """(experts int32 [T, top_k], weights float32 [T, top_k]) for the rows of x."""
         if x.shape[0] <= ROUTE_FEW_TOKENS and K.moe_route_few_takes(x, self.w_router):
             return K.moe_route_few(x, self.w_router, *self._router_args())
+        if K.moe_route_tokens_takes(x, self.w_router):
+            return K.moe_route_tokens(x, self.w_router, *self._router_args())
         return K.moe_route(K.router_logits(x, self.w_router), *self._router_args())
 
     def shared(self, x: torch.Tensor):
