@@ -224,10 +224,11 @@ __global__ void qkv_prepare_staged_kernel(const T* q_in, long long ldq, const T*
 }
 
 // The same where the queries take no norm (attention through a latent): nothing of a query depends on more than its own 16 bytes and
-// those of its rotation partners, so every thread asks for its QP pieces at once and keeps them in registers; the key row, its norm
-// included, is the last warp's, which reads it twice.  One barrier, for the token's angles.  Heads, split points and the rotated span
-// in whole pieces.  (Through shared memory as float32: 1,500 tokens of 16 x 192 queries and rows of 576 24.6 us, here 15.5; 16
-// tokens of 32 x 192 11.4, here 8.1.)
+// those of its rotation partners, so every thread asks for its QP pieces and their partners at once and keeps them in registers; the
+// key row, its norm included, is a warp's of its own.  One barrier, for the token's angles.  Heads, split points and the rotated span in
+// whole pieces.  What bounds it is the chain of trips to memory, which was four long where the partners and the key row were asked for behind the
+// barrier.  (Through shared memory as float32: 1,500 tokens of 16 x 192 queries and rows of 576 24.6 us, 15.5 and 15.6 here;
+// 16 tokens of 32 x 192 11.4, 8.1, here 7.2.)
 #define QP_MOST 4                                          // pieces of queries a thread holds at most
 template <typename T>
 __device__ __forceinline__ void qp_turn(uint4& own, const uint4& other, int rel, const RotArgs& r, const float* cs) {
@@ -253,7 +254,7 @@ __device__ __forceinline__ void qp_turn(uint4& own, const uint4& other, int rel,
 }
 
 template <typename T, int QP>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(288)
 qkv_prepare_direct_kernel(const T* q_in, long long ldq, const T* k_in, long long ldk, const T* v_in, long long ldv, const float* k_w, int k_norm_cols,
                           float eps, RotArgs rot, int q_rot_off, int k_rot_off, const int32_t* positions, const int32_t* table_row, const int32_t* block_table,
                           int table_stride, int page_size, int num_pages, T* q_out, int q_split, T* q_out2, long long q2_head_stride, long long q2_off,
@@ -262,60 +263,83 @@ qkv_prepare_direct_kernel(const T* q_in, long long ldq, const T* k_in, long long
     extern __shared__ float cs[];                          // cosine and sine of the token's angles, times the amplitude
     pb_grid_dep_launch();
     pb_grid_dep_wait();
+    // everything that does not hang on something read here is asked for at once: the token's row, its position, the rates, and the queries and
+    // their partners in the rotation or, in a warp of its own, the key row
     const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
-    const int row = table_row[t];
-    if (row < 0) return;
-    const int p = positions[t], nq = H * qd, nk = k_pages ? G * kd : 0, half = rot.dims >> 1;
-    const bool keys = nk > 0 && tid >= (int)blockDim.x - 32;
-    const T* q = q_in + (size_t)t * ldq;
-    const T* k = k_in + (size_t)t * ldk;
+    const int row = table_row[t], p = positions[t], nq = H * qd, nk = k_pages ? G * kd : 0, half = rot.dims >> 1;
+    const int q_threads = (int)blockDim.x - (nk > 0 ? 32 : 0);
     // where a piece at element d of a head lies in the rotated span from `off` on, or -1
     auto in_span = [&](int d, int off) { return rot.dims > 0 && d >= off && d < off + rot.dims ? d - off : -1; };
     // the piece that the rotation pairs with the one at `at` (adjacent pairs lie in one piece)
-    auto partner = [&](const T* at, int rel) { return rot.adjacent ? make_uint4(0, 0, 0, 0) : *reinterpret_cast<const uint4*>(at + (rel < half ? half : -half)); };
-    uint4 mine[QP];
+    auto partner = [&](const T* at, int rel) { return rel < 0 || rot.adjacent ? make_uint4(0, 0, 0, 0) : *reinterpret_cast<const uint4*>(at + (rel < half ? half : -half)); };
+    auto angles = [&]() {
+        for (int i = tid; i < half; i += blockDim.x) {
+            float sn, c;
+            sincosf((float)p * rot.rates[i], &sn, &c);
+            cs[2 * i] = c * rot.amplitude;
+            cs[2 * i + 1] = sn * rot.amplitude;
+        }
+        __syncthreads();
+    };
+    if (tid < q_threads) {
+        const T* q = q_in + (size_t)t * ldq;
+        uint4 mine[QP], other[QP];
 #pragma unroll
-    for (int it = 0; it < QP; ++it) {
-        const int i = (tid + it * (int)blockDim.x) * VN;
-        mine[it] = i < nq ? *reinterpret_cast<const uint4*>(q + i) : make_uint4(0, 0, 0, 0);
-    }
-    int page = -1;
-    float ss = 0.f;
-    if (keys) {
-        page = block_table[(size_t)row * table_stride + p / page_size];
-        if (k_w != nullptr)
-            for (int i = lane * VN; i < k_norm_cols; i += 32 * VN) {
+        for (int it = 0; it < QP; ++it) {
+            const int i = (tid + it * q_threads) * VN;
+            mine[it] = other[it] = make_uint4(0, 0, 0, 0);
+            if (i < nq) {
+                mine[it] = *reinterpret_cast<const uint4*>(q + i);
+                other[it] = partner(q + i, in_span(i % qd, q_rot_off));
+            }
+        }
+        if (row < 0) return;                               // (the whole block)
+        angles();
+#pragma unroll
+        for (int it = 0; it < QP; ++it) {
+            const int i = (tid + it * q_threads) * VN;
+            if (i >= nq) break;
+            const int h = i / qd, d = i - h * qd, rel = in_span(d, q_rot_off);
+            if (rel >= 0) qp_turn<T>(mine[it], other[it], rel, rot, cs);
+            T* dst = d < q_split ? q_out + ((size_t)t * H + h) * q_split + d : q_out2 + ((size_t)t * H + h) * q2_head_stride + q2_off + (d - q_split);
+            *reinterpret_cast<uint4*>(dst) = mine[it];
+        }
+    } else {
+        const T* k = k_in + (size_t)t * ldk;
+        constexpr int KP = 3;                              // pieces a lane has before it looks at more
+        uint4 key[KP], key_other[KP];
+#pragma unroll
+        for (int j = 0; j < KP; ++j) {
+            const int i = (lane + 32 * j) * VN;
+            key[j] = key_other[j] = make_uint4(0, 0, 0, 0);
+            if (i < nk) {
+                key[j] = *reinterpret_cast<const uint4*>(k + i);
+                key_other[j] = partner(k + i, in_span(i % kd, k_rot_off));
+            }
+        }
+        if (row < 0) return;
+        const int page = block_table[(size_t)row * table_stride + p / page_size];
+        float ss = 0.f;
+        if (k_w != nullptr) {
+            auto add = [&](const T* at) {
                 float v[VN];
-                qp_ld_vec(k + i, v);
+                qp_ld_vec(at, v);
 #pragma unroll
                 for (int e = 0; e < VN; ++e) ss += v[e] * v[e];
-            }
-    }
-    for (int i = tid; i < half; i += blockDim.x) {
-        float sn, c;
-        sincosf((float)p * rot.rates[i], &sn, &c);
-        cs[2 * i] = c * rot.amplitude;
-        cs[2 * i + 1] = sn * rot.amplitude;
-    }
-    __syncthreads();
+            };
 #pragma unroll
-    for (int it = 0; it < QP; ++it) {
-        const int i = (tid + it * (int)blockDim.x) * VN;
-        if (i >= nq) break;
-        const int h = i / qd, d = i - h * qd, rel = in_span(d, q_rot_off);
-        if (rel >= 0) qp_turn<T>(mine[it], partner(q + i, rel), rel, rot, cs);
-        T* dst = d < q_split ? q_out + ((size_t)t * H + h) * q_split + d : q_out2 + ((size_t)t * H + h) * q2_head_stride + q2_off + (d - q_split);
-        *reinterpret_cast<uint4*>(dst) = mine[it];
-    }
-    if (keys) {
+            for (int j = 0; j < KP; ++j)
+                if ((lane + 32 * j) * VN < k_norm_cols) add(reinterpret_cast<const T*>(&key[j]));
+            for (int i = (lane + 32 * KP) * VN; i < k_norm_cols; i += 32 * VN) add(k + i);
+        }
+        angles();
         const float inv = k_w ? 1.0f / sqrtf(pb_warp_sum(ss) / (float)k_norm_cols + eps) : 1.0f;
         if (page < 0 || page >= num_pages) {
             if (lane == 0 && status) atomicExch(status, 2);
         } else {
             const int in_page = p % page_size;
-            for (int i = lane * VN; i < nk; i += 32 * VN) {
+            auto put = [&](int i, uint4 own, const uint4& with) {
                 const int g = i / kd, d = i - g * kd, rel = in_span(d, k_rot_off);
-                uint4 own = *reinterpret_cast<const uint4*>(k + i);
                 if (k_w != nullptr && i < k_norm_cols) {       // (a rotated span that is normed is the general kernels' case)
                     float v[VN];
                     qp_ld_vec(reinterpret_cast<const T*>(&own), v);
@@ -323,14 +347,18 @@ qkv_prepare_direct_kernel(const T* q_in, long long ldq, const T* k_in, long long
                     for (int e = 0; e < VN; ++e) v[e] = v[e] * inv * k_w[i + e];
                     qp_st_vec(reinterpret_cast<T*>(&own), v);
                 } else if (rel >= 0) {
-                    qp_turn<T>(own, partner(k + i, rel), rel, rot, cs);
+                    qp_turn<T>(own, with, rel, rot, cs);
                 }
                 *reinterpret_cast<uint4*>(k_pages + (((size_t)page * G + g) * page_size + in_page) * kd + pb_kv_elem_offset(d, in_page, swizzle_k)) = own;
-            }
+            };
+#pragma unroll
+            for (int j = 0; j < KP; ++j)
+                if ((lane + 32 * j) * VN < nk) put((lane + 32 * j) * VN, key[j], key_other[j]);
+            for (int i = (lane + 32 * KP) * VN; i < nk; i += 32 * VN) put(i, *reinterpret_cast<const uint4*>(k + i), partner(k + i, in_span(i % kd, k_rot_off)));
         }
     }
     if (nk == 0 || v_pages == nullptr || v_in == nullptr) return;
-    page = block_table[(size_t)row * table_stride + p / page_size];
+    const int page = block_table[(size_t)row * table_stride + p / page_size];
     if (page < 0 || page >= num_pages) return;                  // the key row's warp has raised the status
     const int in_page = p % page_size;
     for (int i = tid * VN; i < Gv * vd; i += blockDim.x * VN) {
@@ -406,6 +434,7 @@ PB_API int pb_qkv_prepare(const void* q_in, long long ldq, const void* k_in, lon
         int block = 64;
         while (block < 256 && block < pieces) block <<= 1;
         const int each = (pieces + block - 1) / block;
+        if (nk > 0) block += 32;                             // the key row's warp
 #define DIRECT_LAUNCH(QP)                                                                                                     \
     PB_DISPATCH_DTYPE(dtype, T,                                                                                               \
         (pb_launch(qkv_prepare_direct_kernel<T, QP>, dim3(n_tokens), dim3(block), (size_t)rot.dims * sizeof(float), stream, (const T*)q_in, ldq, \
