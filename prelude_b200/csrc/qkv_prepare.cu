@@ -227,7 +227,7 @@ __global__ void qkv_prepare_staged_kernel(const T* q_in, long long ldq, const T*
 // those of its rotation partners, so every thread asks for its QP pieces and their partners at once and keeps them in registers; the
 // key row, its norm included, is a warp's of its own.  One barrier, for the token's angles.  Heads, split points and the rotated span in
 // whole pieces.  What bounds it is the chain of trips to memory, which was four long where the partners and the key row were asked for behind the
-// barrier.  (Through shared memory as float32: 1,500 tokens of 16 x 192 queries and rows of 576 24.6 us, 15.5 and 15.6 here;
+// barrier.  (Through shared memory as float32: 1,500 tokens of 16 x 192 queries and rows of 576 24.6 us, 15.5, here 14.6;
 // 16 tokens of 32 x 192 11.4, 8.1, here 7.2.)
 #define QP_MOST 4                                          // pieces of queries a thread holds at most
 template <typename T>
@@ -431,10 +431,11 @@ PB_API int pb_qkv_prepare(const void* q_in, long long ldq, const void* k_in, lon
         for (int g = 0; g < G; ++g) direct = direct && g * kd + k_rot_off >= k_norm_cols;
     if (direct) {
         const int pieces = H * qd / vn;
-        int block = 64;
-        while (block < 256 && block < pieces) block <<= 1;
-        const int each = (pieces + block - 1) / block;
-        if (nk > 0) block += 32;                             // the key row's warp
+        // threads for the queries, and a warp for the key row: 256 together where the queries fit so (a block counts as a multiple of four warps)
+        const int most = pieces <= QP_MOST * 224 ? 224 : 256, each = (pieces + most - 1) / most;
+        int block = ((pieces + each - 1) / each + 31) / 32 * 32;
+        if (block < 64) block = 64;
+        if (nk > 0) block += 32;
 #define DIRECT_LAUNCH(QP)                                                                                                     \
     PB_DISPATCH_DTYPE(dtype, T,                                                                                               \
         (pb_launch(qkv_prepare_direct_kernel<T, QP>, dim3(n_tokens), dim3(block), (size_t)rot.dims * sizeof(float), stream, (const T*)q_in, ldq, \
