@@ -568,7 +568,7 @@ struct DcCall {
     float *state, *y;
     const int32_t *cu_q, *slots;
     void* scratch;
-    int n_chunks, n_long, counted, H, G, E;
+    int n_chunks, n_long, counted, longest, H, G, E;
     PbSequences all;
     cudaStream_t stream;
 };
@@ -592,7 +592,18 @@ int dc_run(const DcCall& c) {
     pb_launch(delta_prepare_kernel<D>, dim3(c.n_chunks, c.H), dim3(256), bytes, c.stream, (const bf16*)c.u, c.ld_u, (const bf16*)c.b, c.ld_b, (const bf16*)c.a,
               c.ld_a, c.a_log, c.dt_bias, c.cu_q, (unsigned char*)c.scratch, c.all.n_seqs, c.all.from, c.all.few, c.all.beside, c.H, c.G);
     PB_CHECK_LAUNCH("gated_delta_scan_chunked");
-    return pb_for_widths(c.H, c.E, 16, 32, c.all, c.n_long, c.counted, [&](int width, int rows, const PbSequences& which) {
+    // Where the lengths are at hand: the slices for which the longest chain, or all chains over the multiprocessors, takes less.  A chunk of 16 columns
+    // takes 0.6 of what one of 32 does.  us, slices of 16 / 32 columns: 16 heads, 592 and 1,185 tokens 74 / 86; 1,333 and 2,667 158 / 191; one of
+    // 1,000 41 / 72; 32 heads, 592 and 1,185 145 / 132, one of 1,000 80 / 73.
+    int narrowest = 16, widest = 32;
+    if (c.counted && c.longest > 0 && c.E % 32 == 0) {
+        auto takes = [&](int width) {
+            const double chain = (c.longest + DC_L - 1) / DC_L, all = (double)c.n_chunks * c.H * (c.E / width) / pb_multiprocessors();
+            return (width == 16 ? 0.62 : 1.0) * (chain > all ? chain : all);
+        };
+        narrowest = widest = takes(16) < takes(32) ? 16 : 32;
+    }
+    return pb_for_widths(c.H, c.E, narrowest, widest, c.all, c.n_long, c.counted, [&](int width, int rows, const PbSequences& which) {
         if (which.recorded) return width == 32 ? dc_walk<D, 32, true>(c, rows, which) : dc_walk<D, 16, true>(c, rows, which);
         return width == 32 ? dc_walk<D, 32, false>(c, rows, which) : dc_walk<D, 16, false>(c, rows, which);
     });
@@ -617,14 +628,15 @@ PB_API long long pb_gated_delta_chunk_bytes(int n_chunks, int H) { return (long 
 // most there can be, for a step that is being recorded (few, beside: sequences.cuh).
 PB_API int pb_gated_delta_scan_chunked(const void* u, long long ld_u, const void* b_in, long long ld_b, const void* a_in, long long ld_a, const float* a_log,
                                        const float* dt_bias, float* state, float* y, const int32_t* cu_q, const int32_t* slots, void* scratch, int n_chunks,
-                                       int n_seqs, int least, int few, int beside, int n_long, int counted, int H, int G, int D, int E, cudaStream_t stream) {
+                                       int n_seqs, int least, int few, int beside, int n_long, int counted, long long order, int longest, int H, int G, int D, int E,
+                                       cudaStream_t stream) {
     PB_REQUIRE(n_seqs >= 0 && n_chunks >= 0 && pb_gated_delta_chunked_takes(u, ld_u, state, y, H, G, D, E), "gated_delta_scan_chunked: %d over %d heads of %d, %d", H, G, D, E);
     PB_REQUIRE(u && b_in && a_in && a_log && dt_bias && state && y && cu_q && slots && scratch, "gated_delta_scan_chunked: null pointer");
     PB_REQUIRE(ld_u >= 2ll * G * D + (long long)H * E && ld_b >= H && ld_a >= H, "gated_delta_scan_chunked: rows too short");
     PB_REQUIRE(pb_aligned(scratch, 16), "gated_delta_scan_chunked: misaligned operands");
     PB_REQUIRE(least > 0 && n_long >= 0 && n_long <= n_seqs && n_long < 65536, "gated_delta_scan_chunked: %d of %d sequences in one launch", n_long, n_seqs);
     if (n_long == 0 || n_chunks == 0) return 0;
-    const DcCall c{u, b_in, a_in, ld_u, ld_b, ld_a, a_log, dt_bias, state, y, cu_q, slots, scratch, n_chunks, n_long, counted, H, G, E,
-                   PbSequences{n_seqs, least, INT_MAX, few, beside, 0, 0, 0, 0}, stream};
+    const DcCall c{u, b_in, a_in, ld_u, ld_b, ld_a, a_log, dt_bias, state, y, cu_q, slots, scratch, n_chunks, n_long, counted, longest, H, G, E,
+                   PbSequences{n_seqs, least, INT_MAX, few, beside, 0, 0, 0, 0, longest > 0, (unsigned long long)order}, stream};
     return D == 128 ? dc_run<128>(c) : dc_run<64>(c);
 }

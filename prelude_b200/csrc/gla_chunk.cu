@@ -440,7 +440,8 @@ struct GcCall {
     float *state, *y;
     const int32_t *cu_q, *slots;
     unsigned char* scratch;
-    int n_steps, n_seqs, most, counted, H, P;
+    int n_steps, n_seqs, most, counted, longest, H, P;
+    long long order;
     cudaStream_t stream;
 };
 
@@ -463,7 +464,7 @@ int gc_run(const GcCall& c) {
               c.scratch, c.n_steps, c.n_seqs, c.H);
     PB_CHECK_LAUNCH("gla_scan_chunked");
     // 64 channels: always two column groups of 16
-    const PbSequences all{c.n_seqs, 1, INT_MAX, 0, 0, 0, 0, 0, 0};
+    const PbSequences all{c.n_seqs, 1, INT_MAX, 0, 0, 0, 0, 0, 0, c.longest > 0, (unsigned long long)c.order};
     return pb_for_widths(c.H, c.P, N == 64 ? 32 : 16, 32, all, c.most, c.counted, [&](int width, int rows, const PbSequences& which) {
         if constexpr (N == 64) return which.recorded ? gc_walk<64, 32, true>(c, rows, which) : gc_walk<64, 32, false>(c, rows, which);
         else if (which.recorded) return width == 32 ? gc_walk<128, 32, true>(c, rows, which) : gc_walk<128, 16, true>(c, rows, which);
@@ -486,16 +487,16 @@ PB_API int pb_gla_chunks(int n_tokens, int n_seqs) { return n_tokens / GC_L + (n
 PB_API long long pb_gla_chunk_bytes(int n_steps, int H, int N) { return (long long)n_steps * H * (N == 64 ? GcBlob<64>::bytes : GcBlob<128>::bytes); }
 
 // Operands as for pb_gla_scan, bfloat16; n_steps and scratch as the two functions above say.  most: how many sequences there are
-// (`counted`), or can be, for a step that is being recorded.
+// (`counted`), or can be, for a step that is being recorded.  order, longest: PbSequences, and the longest sequence's tokens (0: no order).
 PB_API int pb_gla_scan_chunked(const void* q, const void* k, const void* v, long long ld, const float* decay, float scale, float* state, float* y,
-                               const int32_t* cu_q, const int32_t* slots, void* scratch, int n_steps, int n_seqs, int most, int counted, int H, int N, int P,
-                               cudaStream_t stream) {
+                               const int32_t* cu_q, const int32_t* slots, void* scratch, int n_steps, int n_seqs, int most, int counted, long long order, int longest, int H,
+                               int N, int P, cudaStream_t stream) {
     PB_REQUIRE(n_seqs >= 0 && n_steps >= 0 && pb_gla_chunked_takes(q, k, v, decay, y, ld, H, N, P), "gla_scan_chunked: %d heads of %d x %d", H, N, P);
     PB_REQUIRE(q && k && v && decay && state && y && cu_q && slots && scratch, "gla_scan_chunked: null pointer");
     PB_REQUIRE(pb_aligned(scratch, 16), "gla_scan_chunked: misaligned operands");
     PB_REQUIRE(most >= 0 && most <= n_seqs && most < 65536, "gla_scan_chunked: %d of %d sequences in one launch", most, n_seqs);
     if (most == 0 || n_steps == 0) return 0;
     const GcCall c{(const bf16*)q, (const bf16*)k, (const bf16*)v, ld, decay, scale, state, y, cu_q, slots, (unsigned char*)scratch, n_steps, n_seqs, most,
-                   counted, H, P, stream};
+                   counted, longest, H, P, order, stream};
     return N == 128 ? gc_run<128>(c) : gc_run<64>(c);
 }

@@ -14,8 +14,11 @@
 // `direct`: all of them, the rows of the launch are the step's (a lookup costs every block a trip to memory).  `recorded`: the launch is
 // replayed for other lengths.  Its rows are fewer than the sequences there may be, a block goes on from row to row, and it works only
 // where there are lo to hi such sequences (lo 0: however many).
+// `ordered`: the rows of such a launch are the sequences in this order, four bits each (at most sixteen), the longest first: what blocks there are
+// beyond the multiprocessors then begin behind short sequences' blocks, and the longest chain does not begin last.
 struct PbSequences {
-    int n_seqs, from, below, few, beside, direct, recorded, lo, hi;
+    int n_seqs, from, below, few, beside, direct, recorded, lo, hi, ordered;
+    unsigned long long order;
 };
 
 // The limit between short and long that holds for the step's lengths.
@@ -62,7 +65,7 @@ __device__ __forceinline__ void pb_for_sequences(const int32_t* cu_q, const PbSe
     const int lane = threadIdx.x & 31;
     int count;
     if constexpr (!RECORDED) {
-        const int seq = s.direct ? (int)blockIdx.y : pb_nth_sequence<4>(cu_q, s.n_seqs, s.from, s.below, blockIdx.y, lane, false, count);
+        const int seq = s.direct ? (s.ordered ? (int)(s.order >> (4 * blockIdx.y)) & 15 : (int)blockIdx.y) : pb_nth_sequence<4>(cu_q, s.n_seqs, s.from, s.below, blockIdx.y, lane, false, count);
         if (seq >= 0 && cu_q[seq + 1] > cu_q[seq]) work(seq, s.from);
     } else {
         int from = s.from, below = s.below;

@@ -384,11 +384,11 @@ PB_API int pb_ssm_scan_chunked_takes(const void* u, const float* state, const fl
 // there are (`counted`), or the most there can be, for a step that is being recorded (few, beside: sequences.cuh).
 PB_API int pb_ssm_scan_chunked(const void* u, const void* dt_in, long long ld_dt, const float* dt_bias, const float* a_log, const float* d_skip,
                                float* state, float* y, const int32_t* cu_q, const int32_t* slots, int n_seqs, int least, int few, int beside, int n_long, int counted,
-                               int heads, int P, int N, int groups, cudaStream_t stream) {
+                               long long order, int longest, int heads, int P, int N, int groups, cudaStream_t stream) {
     PB_REQUIRE(n_seqs >= 0 && pb_ssm_scan_chunked_takes(u, state, y, heads, P, N, groups), "ssm_scan_chunked: %d heads of %d, state %d, %d groups", heads, P, N, groups);
     PB_REQUIRE(u && dt_in && dt_bias && a_log && d_skip && state && y && cu_q && slots && ld_dt >= heads, "ssm_scan_chunked: null pointer");
     PB_REQUIRE(least > 0 && n_long >= 0 && n_long <= n_seqs && n_long < 65536, "ssm_scan_chunked: %d of %d sequences in one launch", n_long, n_seqs);
-    const PbSequences all{n_seqs, least, INT_MAX, few, beside, 0, 0, 0, 0};
+    const PbSequences all{n_seqs, least, INT_MAX, few, beside, 0, 0, 0, 0, longest > 0, (unsigned long long)order};
     return pb_for_widths(heads, P, 16, 64, all, n_long, counted, [&](int width, int rows, const PbSequences& which) {
 #define SC_ARGS u, dt_in, ld_dt, dt_bias, a_log, d_skip, state, y, cu_q, slots, which, rows, heads, P, groups, stream
 #define SC_CASE(NN, PP) if (N == NN && width == PP) return which.recorded ? sc_launch<NN, PP, true>(SC_ARGS) : sc_launch<NN, PP, false>(SC_ARGS)
@@ -407,7 +407,7 @@ PB_API int pb_ssm_scan_chunked(const void* u, const void* dt_in, long long ld_dt
 // For tests: the launches that pb_for_widths makes of a walk, four numbers each - width, rows, lo, hi; how many there are.
 PB_API int pb_walk_launches(int heads, int cols, int narrowest, int widest, int n_long, int counted, int* out) {
     int n = 0;
-    pb_for_widths(heads, cols, narrowest, widest, PbSequences{n_long, 1, INT_MAX, 0, 0, 0, 0, 0, 0}, n_long, counted, [&](int width, int rows, const PbSequences& which) {
+    pb_for_widths(heads, cols, narrowest, widest, PbSequences{n_long, 1, INT_MAX, 0, 0, 0, 0, 0, 0, 0, 0}, n_long, counted, [&](int width, int rows, const PbSequences& which) {
         int* o = out + 4 * n++;
         o[0] = width; o[1] = rows; o[2] = which.lo; o[3] = which.hi;
         return 0;

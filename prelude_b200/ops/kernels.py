@@ -7,7 +7,7 @@ is missing the call raises.
 """
 from __future__ import annotations
 
-from typing import NamedTuple, Optional
+from typing import NamedTuple, Optional, Tuple
 
 import torch
 
@@ -1128,6 +1128,17 @@ def _split(batch, T: int, min_tokens: int, length: int = 1, few: int = 0, beside
     return _Split(length, few, beside, min(n_seqs, T // length + few), min(n_seqs, T), False)
 
 
+def _longest_first(batch, part: _Split) -> Tuple[int, int]:
+    """(order, longest) of a launch with a row for each of the step's sequences, at most sixteen: their indices from the longest on, four
+    bits each, and the longest one's tokens.  (0, 0): no order, the lengths are not at hand or too many."""
+    n = batch.q_lens.shape[0]
+    if not part.counted or part.least != 1 or part.n_long != n or not 0 < n <= 16:
+        return 0, 0
+    lens = [int(v) for v in batch.q_lens]
+    order = sum(r << (4 * i) for i, r in enumerate(sorted(range(n), key=lambda r: -lens[r])))
+    return order - (1 << 64 if order >> 63 else 0), max(lens)
+
+
 def ssm_scan(u: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: torch.Tensor, d_skip: torch.Tensor,
              state: torch.Tensor, batch, groups: int, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """The recurrence over the step's tokens, sequence by sequence; u [T, heads * P + 2 * groups * N] dense, dt [T, heads] a
@@ -1153,7 +1164,7 @@ def ssm_scan(u: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: to
     if part is not None:
         check(lib.pb_ssm_scan_chunked(u.data_ptr(), dt.data_ptr(), dt.stride(0), dt_bias.data_ptr(), a_log.data_ptr(), d_skip.data_ptr(),
                                       state.data_ptr(), out.data_ptr(), batch.cu_q.data_ptr(), batch.state_slots.data_ptr(), n_seqs, part.least,
-                                      part.few, part.beside, part.n_long, part.counted, heads, P, N, groups, _stream()), "ssm_scan_chunked")
+                                      part.few, part.beside, part.n_long, part.counted, *_longest_first(batch, part), heads, P, N, groups, _stream()), "ssm_scan_chunked")
     if steps and (batch.decode_only or (part is not None and part.n_short)):
         which = (0, 0, 0, 0, 1) if part is None else (1, part.few, part.beside, part.n_short, part.counted)
         check(lib.pb_ssm_step(u.data_ptr(), dt.data_ptr(), dt.stride(0), dt_bias.data_ptr(), a_log.data_ptr(), d_skip.data_ptr(), state.data_ptr(),
@@ -1399,7 +1410,8 @@ def gated_delta_scan(u: torch.Tensor, beta: torch.Tensor, a: torch.Tensor, a_log
         check(lib.pb_gated_delta_scan_chunked(u.data_ptr(), u.stride(0), beta.data_ptr(), beta.stride(0), a.data_ptr(), a.stride(0),
                                               a_log.data_ptr(), dt_bias.data_ptr(), state.data_ptr(), out.data_ptr(), batch.cu_q.data_ptr(),
                                               batch.state_slots.data_ptr(), scratch.data_ptr(), n_chunks, n_seqs, part.least, part.few,
-                                              part.beside, part.n_long, part.counted, H, kv_heads, D, E, _stream()), "gated_delta_scan_chunked")
+                                              part.beside, part.n_long, part.counted, *_longest_first(batch, part), H, kv_heads, D, E, _stream()),
+              "gated_delta_scan_chunked")
         if not part.n_short:
             return out
     which = (0, 0, 0, 0, 1) if part is None else (part.least, part.few, part.beside, part.n_short, part.counted)
@@ -1501,7 +1513,7 @@ def gla_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Ten
         scratch = torch.empty((lib.pb_gla_chunk_bytes(n_steps, H, N),), dtype=torch.uint8, device=q.device)
         check(lib.pb_gla_scan_chunked(q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), decay.data_ptr(), float(scale), state.data_ptr(),
                                       out.data_ptr(), batch.cu_q.data_ptr(), batch.state_slots.data_ptr(), scratch.data_ptr(), n_steps, n_seqs,
-                                      part.n_long, part.counted, H, N, P, _stream()), "gla_scan_chunked")
+                                      part.n_long, part.counted, *_longest_first(batch, part), H, N, P, _stream()), "gla_scan_chunked")
         return out
     check(lib.pb_gla_scan(q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), dtype_code(q.dtype), decay.data_ptr(), float(scale),
                                    state.data_ptr(), out.data_ptr(), batch.cu_q.data_ptr(), batch.state_slots.data_ptr(), n_seqs,

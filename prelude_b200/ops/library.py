@@ -112,7 +112,7 @@ _SIGNATURES = {
     "pb_ssm_step_takes": ([P, P, I, I, I, I], I),
     "pb_ssm_step": ([P, P, L, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, P], I),
     "pb_ssm_scan_chunked_takes": ([P, P, P, I, I, I, I], I),
-    "pb_ssm_scan_chunked": ([P, P, L, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, P], I),
+    "pb_ssm_scan_chunked": ([P, P, L, P, P, P, P, P, P, P, I, I, I, I, I, I, L, I, I, I, I, I, P], I),
     "pb_walk_launches": ([I, I, I, I, I, I, P], I),
     "pb_gated_group_rmsnorm": ([P, P, L, P, P, I, I, I, I, F, I, I, P], I),
     "pb_decay_scan": ([P, L, I, P, P, P, P, P, I, I, I, I, I, P], I),
@@ -133,7 +133,7 @@ _SIGNATURES = {
     "pb_gla_chunked_takes": ([P, P, P, P, P, L, I, I, I], I),
     "pb_gla_chunks": ([I, I], I),
     "pb_gla_chunk_bytes": ([I, I, I], L),
-    "pb_gla_scan_chunked": ([P, P, P, L, P, F, P, P, P, P, P, I, I, I, I, I, I, I, P], I),
+    "pb_gla_scan_chunked": ([P, P, P, L, P, F, P, P, P, P, P, I, I, I, I, L, I, I, I, I, P], I),
     "pb_gla_step_supported": ([I, I], I),
     "pb_gla_step": ([P, P, P, P, P, L, I, P, P, F, F, P, F, P, P, P, P, I, I, I, I, I, P], I),
     "pb_scaled_add_rmsnorm": ([P, I, L, F, P, P, I, I, P, P, I, I, F, P], I),
@@ -145,7 +145,7 @@ _SIGNATURES = {
     "pb_gated_delta_chunked_takes": ([P, L, P, P, I, I, I, I], I),
     "pb_gated_delta_chunks": ([I, I], I),
     "pb_gated_delta_chunk_bytes": ([I, I], L),
-    "pb_gated_delta_scan_chunked": ([P, L, P, L, P, L, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, P], I),
+    "pb_gated_delta_scan_chunked": ([P, L, P, L, P, L, P, P, P, P, P, P, P, I, I, I, I, I, I, I, L, I, I, I, I, I, P], I),
     "pb_token_shift_mix": ([P, P, P, P, I, P, P, P, P, I, I, I, P], I),
     "pb_wkv_scan": ([P, L, P, L, P, L, P, L, I, P, P, P, P, P, P, I, I, I, P], I),
 }
