@@ -12,7 +12,10 @@
 //  * The column operand are up to eight rows of A, those that chose the expert at hand.  Where all rows of A fit they lie in shared
 //    memory from the start, else those of the next expert are asked for while one is worked on (two buffers where two fit).  An
 //    expert with more than eight rows is walked again for the next eight.
-//  * Which rows come first is known only when the router is done, so nothing is fetched ahead of the wait for the kernel before.
+//  * Which rows come first is known only when the router is done, so nothing is fetched ahead of the wait for the kernel before - but by
+//    the second of two such products in a row, which finds the choices settled: the first one lets the kernel behind it begin only when
+//    it has itself waited, so that a block fills its ring while other multiprocessors are still at the first product.  The experts of 8 rows,
+//    2,048 x 2,048, both products 79.0 -> 76.6 us.
 // Every sum is over k in an order that K alone decides (steps of 16 dealt to eight warps with four chains each, piece by piece), so a token's
 // result does not depend on who else chose the expert.
 //
@@ -40,7 +43,7 @@ struct MsParams {
     long long lda, w_expert_stride, ldo;
     int n_slots, n_src, a_div, n_experts, N, K;
     int ks, n_chunks, stages, bufs;
-    int gated, act, out_f32;
+    int gated, act, out_f32, settled;       // settled: see pb_moe_stream
     float limit, alpha;
     int* status;
 };
@@ -57,7 +60,6 @@ struct MsWalk {
 };
 
 __global__ void __launch_bounds__(MS_THREADS, 1) moe_stream_kernel(MsParams p) {
-    pb_grid_dep_launch();
     extern __shared__ __align__(128) unsigned char ms_sm[];
     __shared__ __align__(8) uint64_t full_bar[MS_MAX_STAGES], empty_bar[MS_MAX_STAGES], x_bar[2];
     __shared__ int s_dead, s_hits;
@@ -80,9 +82,11 @@ __global__ void __launch_bounds__(MS_THREADS, 1) moe_stream_kernel(MsParams p) {
         mbar_fence_init();
     }
     __syncthreads();
-    pb_grid_dep_wait();
+    if (!p.settled) pb_grid_dep_wait();
+    // Only now: a kernel whose blocks begin behind this finds done whatever was launched ahead of this one
+    if (!p.settled) pb_grid_dep_launch();
     for (int i = tid; i < p.n_slots; i += MS_THREADS) {
-        const int e = p.ids[i];
+        const int e = __ldcg(p.ids + i);                       // from L2: written a moment ago
         ids[i] = e;
         if (e >= 0 && e < p.n_experts) atomicAdd(&count[e], 1);
     }
@@ -101,7 +105,10 @@ __global__ void __launch_bounds__(MS_THREADS, 1) moe_stream_kernel(MsParams p) {
     const int units = (p.N + MS_ROWS - 1) / MS_ROWS;           // of one expert
     const long long all = (long long)s_hits * units;
     const long long u0 = blockIdx.x * all / gridDim.x, u1 = (blockIdx.x + 1) * all / gridDim.x;
-    if (u0 >= u1) return;
+    if (u0 >= u1) {
+        if (p.settled) pb_grid_dep_wait();                     // no block ends before the kernel ahead has
+        return;
+    }
     const int span = p.gated ? MS_ROWS : 16;                   // features of a tile
     auto open = [&](int hit) {
         MsWalk w;
@@ -162,6 +169,10 @@ __global__ void __launch_bounds__(MS_THREADS, 1) moe_stream_kernel(MsParams p) {
     }
 
     // ---------------- multiplying warps ----------------
+    if (p.settled) {                                           // the weights are on their way; the rows are the kernel's just ahead, and its readers' the results
+        pb_grid_dep_wait();
+        pb_grid_dep_launch();
+    }
     const bool resident = p.n_src <= p.bufs * MS_ROWS;
     // the slots of a segment, and its rows of A on their way (warp 0): segment n uses slot list n % 4 and, where the rows do not all stay, buffer
     // n % bufs, which nobody reads any more
@@ -312,9 +323,10 @@ PB_API int pb_moe_stream_supported(int K, int n_slots, int n_experts) {
 }
 
 // A [n_slots / a_div, K] with row stride lda; W [n_experts, (2) N, K], w_expert_stride elements from one expert to the next, gate rows
-// first; ids int32 [n_slots]; out [n_slots, N] with row stride ldo, float32 or bfloat16.  act, limit, alpha: as in pb_moe_gemv.
+// first; ids int32 [n_slots]; out [n_slots, N] with row stride ldo, float32 or bfloat16.  act, limit, alpha: as in pb_moe_gemv.  settled: ids and W were
+// there when the kernel launched before this one passed its own wait, and that one is a pb_moe_stream; they are read ahead of the wait.
 PB_API int pb_moe_stream(const void* A, long long lda, int a_div, const void* W, long long w_expert_stride, int N, int K, int gated, int act, float limit,
-                         float alpha, const int32_t* ids, int n_slots, int n_experts, void* out, long long ldo, int out_dtype, int* status, cudaStream_t stream) {
+                         float alpha, const int32_t* ids, int n_slots, int n_experts, int settled, void* out, long long ldo, int out_dtype, int* status, cudaStream_t stream) {
     PB_REQUIRE(pb_moe_stream_supported(K, n_slots, n_experts) && N > 0 && a_div > 0 && n_slots % a_div == 0, "moe_stream: K=%d, %d choices of %d experts", K, n_slots, n_experts);
     PB_REQUIRE(A && W && ids && out && pb_aligned(A, 16) && pb_aligned(W, 16) && lda % 8 == 0 && w_expert_stride % 8 == 0, "moe_stream: null or unaligned pointer");
     PB_REQUIRE(lda >= K && ldo >= N && w_expert_stride >= (long long)(gated ? 2 : 1) * N * K, "moe_stream: a stride is shorter than its row");
@@ -324,7 +336,7 @@ PB_API int pb_moe_stream(const void* A, long long lda, int a_div, const void* W,
     MsParams p{};
     p.A = (const __nv_bfloat16*)A; p.W = (const __nv_bfloat16*)W; p.ids = ids; p.out = out; p.lda = lda; p.w_expert_stride = w_expert_stride; p.ldo = ldo;
     p.n_slots = n_slots; p.n_src = n_slots / a_div; p.a_div = a_div; p.n_experts = n_experts; p.N = N; p.K = K; p.gated = gated ? 1 : 0; p.act = act;
-    p.out_f32 = out_dtype == PB_F32; p.limit = limit; p.alpha = alpha; p.status = status;
+    p.out_f32 = out_dtype == PB_F32; p.settled = settled ? 1 : 0; p.limit = limit; p.alpha = alpha; p.status = status;
     size_t smem;
     ms_plan(K, &p.ks, &p.n_chunks, &p.stages, &p.bufs, &smem);
     static const cudaError_t set = cudaFuncSetAttribute(moe_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MS_SMEM_LIMIT);

@@ -227,8 +227,8 @@ __global__ void qkv_prepare_staged_kernel(const T* q_in, long long ldq, const T*
 // those of its rotation partners, so every thread asks for its QP pieces and their partners at once and keeps them in registers; the
 // key row, its norm included, is a warp's of its own.  One barrier, for the token's angles.  Heads, split points and the rotated span in
 // whole pieces.  What bounds it is the chain of trips to memory, which was four long where the partners and the key row were asked for behind the
-// barrier.  (Through shared memory as float32: 1,500 tokens of 16 x 192 queries and rows of 576 24.6 us, 15.5, here 14.6;
-// 16 tokens of 32 x 192 11.4, 8.1, here 7.2.)
+// barrier.  (Through shared memory as float32: 1,500 tokens of 16 x 192 queries and rows of 576 24.6 us, with the partners behind the
+// barrier 15.5; 16 tokens of 32 x 192 11.4 and 8.1.  What the kernel adds to a layer's time, partners behind it / here: 13.2 / 12.3 and 5.8 / 4.9.)
 #define QP_MOST 4                                          // pieces of queries a thread holds at most
 template <typename T>
 __device__ __forceinline__ void qp_turn(uint4& own, const uint4& other, int rel, const RotArgs& r, const float* cs) {

@@ -768,11 +768,18 @@ def moe_gemv_takes(a: torch.Tensor, w: torch.Tensor, n_slots: int) -> bool:
             and a.stride(0) % 8 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and 0 < n_slots <= MOE_GEMV_MAX_SLOTS)
 
 
+def moe_streams(w: torch.Tensor, n_slots: int) -> bool:
+    """Whether ``moe_gemv`` runs on the streaming kernel (rows of 768 elements and more)."""
+    return bool(_l.library().pb_moe_stream_supported(w.shape[2], n_slots, w.shape[0]))
+
+
 def moe_gemv(a: torch.Tensor, w: torch.Tensor, ids: torch.Tensor, rows_are_slots: bool, out_dtype: torch.dtype, gated: bool = False,
-             act: int = ACT_NONE, limit: float = 0.0, alpha: float = 0.0, status: Optional[torch.Tensor] = None) -> torch.Tensor:
+             act: int = ACT_NONE, limit: float = 0.0, alpha: float = 0.0, status: Optional[torch.Tensor] = None,
+             settled: bool = False) -> torch.Tensor:
     """The experts' products for a few tokens without a plan: ids int32 [T, top]; a [T, K] (the tokens' rows) or, with
     ``rows_are_slots``, [T * top, K]; the result's rows are the slots token * top + choice.  ``status`` is raised where a
-    block gave up waiting."""
+    block gave up waiting.  ``settled``: the call just before this one on the stream was another of these, on the streaming kernel
+    (``moe_streams``), for the same choices."""
     _cols(a, "a")
     _need(w, "w", a.dtype)
     _need(ids, "ids", torch.int32)
@@ -782,9 +789,9 @@ def moe_gemv(a: torch.Tensor, w: torch.Tensor, ids: torch.Tensor, rows_are_slots
         raise KernelLibraryError(f"moe_gemv: a {tuple(a.shape)}, choices {tuple(ids.shape)}")
     N = rows_w // 2 if gated else rows_w
     out = torch.empty((T * top, N), dtype=out_dtype, device=a.device)
-    if _l.library().pb_moe_stream_supported(Kdim, T * top, E):
+    if moe_streams(w, T * top):
         check(_l.library().pb_moe_stream(a.data_ptr(), a.stride(0), 1 if rows_are_slots else top, w.data_ptr(), w.stride(0), N, Kdim, 1 if gated else 0, act,
-                                         float(limit), float(alpha), ids.data_ptr(), T * top, E, out.data_ptr(), out.stride(0), dtype_code(out_dtype), _ptr(status),
+                                         float(limit), float(alpha), ids.data_ptr(), T * top, E, 1 if settled else 0, out.data_ptr(), out.stride(0), dtype_code(out_dtype), _ptr(status),
                                          _stream()), "moe_stream")
         return out
     check(_l.library().pb_moe_gemv(a.data_ptr(), a.stride(0), None, 1 if rows_are_slots else top, w.data_ptr(), w.stride(0), N, Kdim,

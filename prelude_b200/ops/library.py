@@ -95,7 +95,7 @@ _SIGNATURES = {
     "pb_moe_gemm": ([P, L, P, I, P, L, I, I, I, I, F, F, P, P, P, I, I, P, L, I, I, P], I),
     "pb_moe_gemv": ([P, L, P, I, P, L, I, I, I, I, F, F, P, P, P, I, P, I, P, L, I, P], I),
     "pb_moe_stream_supported": ([I, I, I], I),
-    "pb_moe_stream": ([P, L, I, P, L, I, I, I, I, F, F, P, I, I, P, L, I, P, P], I),
+    "pb_moe_stream": ([P, L, I, P, L, I, I, I, I, F, F, P, I, I, I, P, L, I, P, P], I),
     "pb_moe_combine": ([P, I, P, P, P, I, I, I, I, P], I),
     "pb_moe_gather_rows": ([P, L, P, I, P, I, I, I, P], I),
     "pb_gemm_ref_batched": ([P, P, P, I, I, I, I, I, L, L, L, I, L, L, L, P], I),

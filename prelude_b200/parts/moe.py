@@ -222,7 +222,7 @@ class RoutedExperts:
         if streamed and not grouped:
             status = L.tc_status(x.device)
             h = K.moe_gemv(x, self.w_gate_up, ids, False, x.dtype, gated=self.gated, status=status, **self.act)
-            y = K.moe_gemv(h, self.w_down, ids, True, torch.float32, status=status)
+            y = K.moe_gemv(h, self.w_down, ids, True, torch.float32, status=status, settled=K.moe_streams(self.w_gate_up, ids.numel()))
             return self._sum(y, None, weights, shared, x.dtype)
         if grouped:
             # fewer rows: the experts' weights are the rows of the paired-block products, the tokens their columns

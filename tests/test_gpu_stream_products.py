@@ -57,3 +57,26 @@ def test_experts_streamed(T, top, E, N, K_, gated, act, slots):
     assert torch.equal(K.moe_gemv(a, w, ids, slots, torch.bfloat16, **kw), got.bfloat16())
     if not slots and T > 1:                          # a token's result does not depend on who else chose its experts
         assert torch.equal(K.moe_gemv(a[1:2], w, ids[1:2].contiguous(), False, torch.float32, **kw), got[top:2 * top])
+
+
+# a pair, the second of which reads the choices before the first has ended: resident rows, rows that move, blocks without a share
+@pytest.mark.parametrize("T,top,E,N,K_", [(1, 1, 2, 768, 784), (8, 4, 32, 2048, 2048), (40, 8, 64, 1024, 768), (3, 8, 1024, 800, 1040)])
+def test_second_product_begins_early(T, top, E, N, K_):
+    from prelude_b200.ops import kernels as K
+    up, down, x = rnd(E, N, K_, scale=K_ ** -0.5), rnd(E, K_, N, seed=2, scale=N ** -0.5), rnd(T, K_, seed=3)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+
+    def pair(n, settled):
+        ids = (torch.arange(T * top, device=DEV, dtype=torch.int32).view(T, top) * 7 + n) % E     # new choices just ahead
+        h = K.moe_gemv(x, up, ids, False, torch.bfloat16, act=K.ACT_RELU2, status=status)
+        return K.moe_gemv(h, down, ids, True, torch.float32, status=status, settled=settled)
+
+    want = [pair(n, False) for n in range(8)]
+    got = [pair(n, True) for n in range(8)]
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+    # ids that name no expert leave every block without a share
+    none = torch.full((T, top), -1, dtype=torch.int32, device=DEV)
+    h = K.moe_gemv(x, up, none, False, torch.bfloat16, act=K.ACT_RELU2, status=status)
+    K.moe_gemv(torch.zeros_like(h), down, none, True, torch.float32, status=status, settled=True)
+    assert int(status) == 0
