@@ -55,6 +55,46 @@ __global__ void kv_write_pages_kernel(const T* k, long long k_stride, const T* v
     }
 }
 
+// The same by 16-byte pieces, for heads, rows and pages in whole pieces (the permutation of a page moves whole ones).  It is bound by its chain of trips
+// to memory - the token's row, its page, keys and values - so what a thread copies is asked for before the page is looked up.
+// 1,024 tokens behind a product 5.6 -> 2.8 us; a layer of 3,001 tokens 209 -> 205.
+#define KW_HELD 2                                          // pieces a thread has asked for by then
+template <typename T>
+__global__ void __launch_bounds__(256) kv_write_pages_vec_kernel(const T* k, long long k_stride, const T* v, long long v_stride, T* k_pages, T* v_pages,
+                                                                 const int32_t* positions, const int32_t* token_row, const int32_t* block_table,
+                                                                 int table_stride, int page_size, int num_pages, int n_k_heads, int dk, int n_v_heads, int dv,
+                                                                 int k_swizzle, int v_swizzle, int* status) {
+    constexpr int VN = 16 / sizeof(T);
+    pb_grid_dep_launch();
+    pb_grid_dep_wait();
+    const int t = blockIdx.x, nk = n_k_heads * dk, all = nk + n_v_heads * dv, step = blockDim.x * VN;
+    const T* kr = k + (size_t)t * k_stride;
+    const T* vr = v + (size_t)t * v_stride - nk;
+    uint4 held[KW_HELD];
+    int i = threadIdx.x * VN;
+#pragma unroll
+    for (int j = 0; j < KW_HELD; ++j)
+        if (i + j * step < all) held[j] = *reinterpret_cast<const uint4*>((i + j * step < nk ? kr : vr) + i + j * step);
+    const int row = token_row[t], pos = positions[t];
+    if (row < 0) return;                                   // a padding row of a captured step
+    const int page = block_table[(size_t)row * table_stride + pos / page_size];
+    if (page < 0 || page >= num_pages) {
+        if (threadIdx.x == 0 && status) atomicExch(status, 2);
+        return;
+    }
+    const int in_page = pos % page_size;
+    auto put = [&](int at, const uint4& piece) {
+        const bool key = at < nk;
+        const int e = key ? at : at - nk, dim = key ? dk : dv, h = e / dim, d = e - h * dim;
+        T* head = (key ? k_pages : v_pages) + (((size_t)page * (key ? n_k_heads : n_v_heads) + h) * page_size + in_page) * dim;
+        *reinterpret_cast<uint4*>(head + pb_kv_elem_offset(d, in_page, key ? k_swizzle : v_swizzle)) = piece;
+    };
+#pragma unroll
+    for (int j = 0; j < KW_HELD; ++j, i += step)
+        if (i < all) put(i, held[j]);
+    for (; i < all; i += step) put(i, *reinterpret_cast<const uint4*>((i < nk ? kr : vr) + i));
+}
+
 // k [T, n_k_heads * dk] and v [T, n_v_heads * dv] with row strides in elements (columns of a merged projection);
 // pages as described above; token_row[t] is the row of block_table of token t's request (-1: no such token).
 PB_API int pb_kv_write_pages(const void* k, long long k_stride, const void* v, long long v_stride, void* k_pages, void* v_pages,
@@ -67,6 +107,19 @@ PB_API int pb_kv_write_pages(const void* k, long long k_stride, const void* v, l
     PB_REQUIRE(k_stride >= (long long)n_k_heads * dk && v_stride >= (long long)n_v_heads * dv, "kv_write_pages: a row stride is shorter than its row");
     PB_REQUIRE((!k_swizzle || dk % 8 == 0) && (!v_swizzle || dv % 8 == 0), "kv_write_pages: permuted pages need head sizes in multiples of 8");
     if (n_tokens == 0) return 0;
+    // whole pieces wherever they can be read and written, else by elements
+    const int vn = dtype == PB_BF16 ? 8 : 4;
+    if ((dtype == PB_BF16 || dtype == PB_F32) && dk % vn == 0 && dv % vn == 0 && k_stride % vn == 0 && v_stride % vn == 0 && pb_aligned(k, 16) && pb_aligned(v, 16) &&
+        pb_aligned(k_pages, 16) && pb_aligned(v_pages, 16)) {
+        const long long pieces = ((long long)n_k_heads * dk + (long long)n_v_heads * dv) / vn;
+        const int threads = pieces >= 256 ? 256 : (int)(pieces + 31) / 32 * 32;
+        PB_DISPATCH_DTYPE(dtype, T,
+            (pb_launch(kv_write_pages_vec_kernel<T>, dim3(n_tokens), dim3(threads), 0, stream, (const T*)k, k_stride, (const T*)v, v_stride,
+                       (T*)k_pages, (T*)v_pages, positions, token_row, block_table, table_stride, page_size, num_pages,
+                       n_k_heads, dk, n_v_heads, dv, k_swizzle, v_swizzle, status)));
+        PB_CHECK_LAUNCH("kv_write_pages");
+        return 0;
+    }
     PB_DISPATCH_DTYPE(dtype, T,
         (pb_launch(kv_write_pages_kernel<T>, dim3(n_tokens), dim3(128), 0, stream, (const T*)k, k_stride, (const T*)v, v_stride,
                    (T*)k_pages, (T*)v_pages, positions, token_row, block_table, table_stride, page_size, num_pages,
