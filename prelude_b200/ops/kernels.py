@@ -603,11 +603,8 @@ def diff_attention_ref(q: torch.Tensor, gate: Optional[torch.Tensor], k_pages: t
 
 def router_logits(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     """x [T, K] times w [E, K] transposed as float32 [T, E]: exact products, float32 sums in an order that depends on K alone."""
-    _cols(x, "x")
-    _need(w, "w", x.dtype)
+    _router_operands("router_logits", x, w)
     T, Kdim = x.shape
-    if w.dim() != 2 or w.shape[1] != Kdim:
-        raise KernelLibraryError(f"router_logits: x {tuple(x.shape)} against w {tuple(w.shape)}")
     out = torch.empty((T, w.shape[0]), dtype=torch.float32, device=x.device)
     check(_l.library().pb_router_logits(x.data_ptr(), x.stride(0), w.data_ptr(), out.data_ptr(), dtype_code(x.dtype), T, w.shape[0],
                                         Kdim, _stream()), "router_logits")
@@ -620,6 +617,14 @@ def _route_vectors(correction: Optional[torch.Tensor], bias: Optional[torch.Tens
             _need(v, name, torch.float32)
             if v.numel() != E:
                 raise KernelLibraryError(f"moe_route: a {name} of {v.numel()} numbers for {E} experts")
+
+
+def _router_operands(what: str, x: torch.Tensor, w: torch.Tensor) -> None:
+    """A kernel walks the rows of w with the width of x's: rows of another width, or of another type, would be read past their end."""
+    _cols(x, "x")
+    _need(w, "w", x.dtype)
+    if w.dim() != 2 or w.shape[1] != x.shape[1]:
+        raise KernelLibraryError(f"{what}: x {tuple(x.shape)} against w {tuple(w.shape)}")
 
 
 def _scoring(softmax: bool, softmax_chosen: bool) -> int:
@@ -647,7 +652,7 @@ def moe_route(logits: torch.Tensor, top: int, groups: int, keep: int, group_top:
 
 def moe_route_few_takes(x: torch.Tensor, w: torch.Tensor) -> bool:
     """Whether router logits and choice of x [T, K] against w [E, K] run in one kernel (meant for a decode step's few rows)."""
-    return (x.dtype == w.dtype and x.stride(1) == 1 and w.is_contiguous() and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
+    return (x.dtype == w.dtype and x.shape[1] == w.shape[1] and x.stride(1) == 1 and w.is_contiguous() and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
             and x.stride(0) % (8 if x.dtype == torch.bfloat16 else 4) == 0
             and bool(_l.library().pb_moe_route_few_supported(w.shape[0], w.shape[1], dtype_code(x.dtype))))
 
@@ -656,7 +661,7 @@ def moe_route_few(x: torch.Tensor, w: torch.Tensor, top: int, groups: int, keep:
                   correction: Optional[torch.Tensor] = None, softmax: bool = False, renormalize_eps: float = 0.0, scale: float = 1.0,
                   bias: Optional[torch.Tensor] = None, softmax_chosen: bool = False):
     """``router_logits`` and ``moe_route`` in one kernel for a few tokens; the same numbers."""
-    _cols(x, "x")
+    _router_operands("moe_route_few", x, w)
     T, Kdim = x.shape
     E = w.shape[0]
     _route_vectors(correction, bias, E)
@@ -670,8 +675,8 @@ def moe_route_few(x: torch.Tensor, w: torch.Tensor, top: int, groups: int, keep:
 
 def moe_route_tokens_takes(x: torch.Tensor, w: torch.Tensor) -> bool:
     """Whether the router of a prompt step's rows x [T, K] against w [E, K] runs on the tensor cores."""
-    return (x.dtype == torch.bfloat16 and w.dtype == x.dtype and x.stride(1) == 1 and w.is_contiguous() and x.data_ptr() % 16 == 0
-            and w.data_ptr() % 16 == 0 and x.stride(0) % 8 == 0 and bool(_l.library().pb_moe_route_tokens_supported(x.shape[0], w.shape[0], w.shape[1])))
+    return (x.dtype == torch.bfloat16 and w.dtype == x.dtype and x.shape[1] == w.shape[1] and x.stride(1) == 1 and w.is_contiguous()
+            and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and x.stride(0) % 8 == 0 and bool(_l.library().pb_moe_route_tokens_supported(x.shape[0], w.shape[0], w.shape[1])))
 
 
 def moe_route_tokens(x: torch.Tensor, w: torch.Tensor, top: int, groups: int, keep: int, group_top: int, renormalize: bool,
@@ -679,7 +684,9 @@ def moe_route_tokens(x: torch.Tensor, w: torch.Tensor, top: int, groups: int, ke
                      bias: Optional[torch.Tensor] = None, softmax_chosen: bool = False, logits: Optional[torch.Tensor] = None):
     """``router_logits`` and ``moe_route`` for a prompt step's rows, in one kernel with up to 64 experts; the products of sixteen are summed by
     the tensor cores, these sums in float32 (``logits`` float32 [T, E] gets them)."""
-    _cols(x, "x")
+    _router_operands("moe_route_tokens", x, w)
+    if x.dtype != torch.bfloat16:
+        raise KernelLibraryError(f"moe_route_tokens: rows of {x.dtype}, not of {torch.bfloat16}")
     T, Kdim = x.shape
     E = w.shape[0]
     _route_vectors(correction, bias, E)
