@@ -16,6 +16,8 @@
 //    by side, so they take the stages in turn (all four on every stage, two copies
 //    each: chunks of 512 elements 45 us for 150 MB instead of 34, of 1,024 30
 //    instead of 26.5), and the chunks are as long as leaves four stages (gs_plan).
+//    How K is cut into chunks changes no sum: a step is dealt to its warp and
+//    chain by its place in K, or in a part of K that the rows' number sets.
 //    Weights are written by no kernel, so the
 //    loaders fill the ring before they wait for the kernel before this one on
 //    the stream: the stream is already flowing when x becomes available.
@@ -65,7 +67,7 @@ struct GsParams {
     long long ldw, ldx, ldo;
     int M, N, K;
     int ks;                 // elements of K per stage
-    int n_chunks;           // chunks of K per row
+    int part;               // elements of K whose steps are dealt to the warps' chains from the first on; stages do not go across parts
     int stages;
     int sets;               // of the warps' sums in shared memory: two, or one where a second does not fit
     int out_f32;
@@ -146,7 +148,9 @@ __global__ void __launch_bounds__(GS_THREADS, 1) gemm_stream_kernel(GsParams p) 
         for (int tile = 0; tile < n_tiles && ok; ++tile) {
             const int halves = (p.gated || r1 - (r0 + tile * span) > GS_ROWS) ? 2 : 1;
 #pragma unroll 1
-            for (int kc = 0; kc < p.n_chunks && ok; ++kc) {
+            for (int k0 = 0, end = 0, len; k0 < p.K && ok; k0 += len) {
+                if (k0 == end) end = min(end + p.part, p.K);
+                len = min(p.ks, end - k0);
                 for (int h = 0; h < halves; ++h, ++i) {
                     if (turn == lw) {
                         if (i >= p.stages) {                   // the first ring-full finds every stage free
@@ -155,7 +159,6 @@ __global__ void __launch_bounds__(GS_THREADS, 1) gemm_stream_kernel(GsParams p) 
                         }
                         const int feat0 = r0 + tile * span + (p.gated ? 0 : h * GS_ROWS);   // first feature of the stage
                         const int row0 = feat0 + (p.gated ? h * p.N : 0);             // its row of W: up rows follow the gate rows
-                        const int k0 = kc * p.ks, len = min(p.ks, p.K - k0);
                         const int n_rows = min(GS_ROWS, r1 - feat0);
                         // the copies may land before the expected bytes are posted: the phase cannot end before this arrival
                         if (lane == 0) mbar_arrive_expect_tx(&full_bar[stage], (unsigned)n_rows * len * 2);
@@ -217,7 +220,9 @@ __global__ void __launch_bounds__(GS_THREADS, 1) gemm_stream_kernel(GsParams p) 
 #pragma unroll
             for (int j = 0; j < MT; ++j) acc[c][j][0] = acc[c][j][1] = acc[c][j][2] = acc[c][j][3] = 0.f;
 #pragma unroll 1
-        for (int kc = 0; kc < p.n_chunks; ++kc) {
+        for (int k0 = 0, end = 0, first = 0, len; k0 < p.K; k0 += len) {
+            if (k0 == end) { first = end; end = min(end + p.part, p.K); }
+            len = min(p.ks, end - k0);
             const int stage2 = (stage + 1 == p.stages) ? 0 : stage + 1, phase2 = (stage + 1 == p.stages) ? phase ^ 1 : phase;
             bool landed = mbar_wait_bounded(&full_bar[stage], phase);
             if (halves == 2) landed = landed && mbar_wait_bounded(&full_bar[stage2], phase2);
@@ -225,17 +230,18 @@ __global__ void __launch_bounds__(GS_THREADS, 1) gemm_stream_kernel(GsParams p) 
                 if (lane == 0) { *(volatile int*)&s_dead = 1; if (p.status) atomicExch(p.status, 12); }
                 break;
             }
-            const int k0 = kc * p.ks, steps = min(p.ks, p.K - k0) >> 4;
+            // the stage's steps go on where the part's last stage stopped: step i of a part is warp i % 8's, chain i / 8 % 4, however it is cut
+            const int steps = len >> 4, at = ((k0 - first) >> 4) & (GS_WARPS * GS_CHAINS - 1);
             // with one stage only, the upper eight rows read the lower ones again (their sums are not stored)
             const unsigned a_base = ring_a + ((upper && halves == 2) ? stage2 : stage) * stage_bytes + a_off;
             const unsigned b_base = sX_a + b_off + k0 * 2;
 #pragma unroll 1
-            for (int s0 = warp; s0 < steps; s0 += GS_WARPS * GS_CHAINS) {
+            for (int s0 = warp - at; s0 < steps; s0 += GS_WARPS * GS_CHAINS) {
                 unsigned a[GS_CHAINS][4], b[GS_CHAINS][4];
 #pragma unroll
                 for (int c = 0; c < GS_CHAINS; ++c) {
                     const int s = s0 + c * GS_WARPS;
-                    if (s < steps) {
+                    if ((unsigned)s < (unsigned)steps) {
                         ldmatrix_x4_a(a[c], a_base + s * 32);
                         if (MT == 1) ldmatrix_x2(b[c][0], b[c][1], b_base + s * 32);
                         else ldmatrix_x4_a(b[c], b_base + s * 32);
@@ -243,7 +249,7 @@ __global__ void __launch_bounds__(GS_THREADS, 1) gemm_stream_kernel(GsParams p) 
                 }
 #pragma unroll
                 for (int c = 0; c < GS_CHAINS; ++c) {
-                    if (s0 + c * GS_WARPS < steps) {
+                    if ((unsigned)(s0 + c * GS_WARPS) < (unsigned)steps) {
                         mma_bf16_free(acc[c][0], a[c], b[c][0], b[c][1]);
                         if (MT == 2) mma_bf16_free(acc[c][MT - 1], a[c], b[c][2], b[c][3]);
                     }
@@ -337,41 +343,51 @@ static int gs_sms() {
     return g_gs_sms;
 }
 
-// Chunk of K per stage and number of stages for a shape: the fewest equal chunks per row (the longest copies) that leave room for four
-// stages.  A tile takes its stages two by two: with three, one is on its way while it waits.  150 MB of weights, us, chunk x stages: K = 2,560,
-// 12 rows 2,560 x 3 33.8, 1,280 x 7 28.6; 4,096, 2 rows 4,096 x 3 29.3, 2,048 x 6 25.2; 4,096, 16 rows 1,408 x 3 43.8, 1,024 x 5 32.2; 8,192, 8
-// rows 1,664 x 3 37.9, 1,024 x 5 30.2; 5,120, 16 rows 1,024 x 3 50.7, 640 x 4 46.0.
-static bool gs_plan(int M, int K, int* ks, int* n_chunks, int* stages, int* sets, size_t* smem) {
-    const size_t x_bytes = (size_t)M * ((size_t)K * 2 + 16);
-    const size_t set_bytes = (size_t)GS_WARPS * 16 * (M <= 8 ? 8 : 16) * 4;
-    // pieces of 1,024 elements at least, of 640 where those leave too few stages, and where neither gives four stages as many as there are
-    const int least[4] = {1024, 640, 512, 512}, want[4] = {4, 4, 2, 2};
-    for (int rule = 0; rule < 4; ++rule) {
-        *sets = rule < 3 ? 2 : 1;
-        const size_t sums = *sets * set_bytes < 8192 ? 8192 : *sets * set_bytes, taken = x_bytes + sums, room = GS_SMEM_LIMIT - taken;
-        if (taken >= GS_SMEM_LIMIT) continue;
+// The parts of K whose steps are dealt out together, the piece of a part that goes into a stage, and the number of stages.
+// The parts decide the order of the sums and nothing else does: the fewest equal ones, in steps of 16, of which three fit beside the rows of x and
+// one set of sums, or two.  Pieces: the longest equal cut of a part of which four stages fit (a tile takes its stages two by two: with three, one is on
+// its way while it waits), else the longest of which two do.
+// 64 MB of weights, us, piece x stages: K = 2,560, 12 rows 2,560 x 3 16.1, 1,280 x 7 14.7; 4,096, 2 rows 4,096 x 3 13.9, 2,048 x 6 13.2; 8,192, 8 rows 1,648 x 3
+// 18.4, 832 x 6 15.9; 6,144, 16 rows 512 x 2 40.5, 512 x 3 37.4, 768 x 2 31.9; 8,192, 12 rows 512 x 2 43.7, 512 x 3 39.9, 768 x 2 34.7.
+static bool gs_plan(int M, int K, int* ks, int* part, int* stages, int* sets, size_t* smem) {
+    const size_t x_bytes = (size_t)M * ((size_t)K * 2 + 16), set_bytes = (size_t)GS_WARPS * 16 * (M <= 8 ? 8 : 16) * 4, least = 8192;
+    if (x_bytes + least >= GS_SMEM_LIMIT) return false;
+    auto stage_of = [](int k) { return (size_t)GS_ROWS * ((size_t)k * 2 + 16); };
+    auto fit = [&](int k, int sums) { return (GS_SMEM_LIMIT - x_bytes - (sums * set_bytes < least ? least : sums * set_bytes)) / stage_of(k); };
+    *part = 0;
+    for (int want = 3; want >= 2 && *part == 0; --want)
         for (int n = 1; n <= K / 16; ++n) {
-            const int unit = rule < 2 ? 128 : 16, k_per = n == 1 ? K : ((K + n - 1) / n + unit - 1) / unit * unit;
-            const size_t stage = (size_t)GS_ROWS * ((size_t)k_per * 2 + 16);
-            if (k_per < least[rule] && n > 1) break;              // copies this short are not worth having
-            if (stage * want[rule] <= room) {
-                size_t s = room / stage;
-                if (s > GS_MAX_STAGES) s = GS_MAX_STAGES;
-                *ks = k_per; *n_chunks = (K + k_per - 1) / k_per; *stages = (int)s;
-                *smem = taken + s * stage;
-                return true;
-            }
+            const int k_per = ((K + n - 1) / n + 15) / 16 * 16;
+            if (k_per < 512 && n > 1) break;
+            if ((int)fit(k_per, 1) >= want) { *part = k_per; break; }
         }
-    }
+    if (*part == 0) return false;
+    // whole turns over the warps and chains: dealt as K in one part is
+    if (*part % (16 * GS_WARPS * GS_CHAINS) == 0) *part = K;
+    // In turns over the eight warps where the deal is K's own
+    const int unit = *part == K ? 16 * GS_WARPS : 16;
+    for (int want = 4; want >= 2; want -= 2)
+        for (int n = 1; n <= *part / 16; ++n) {
+            *ks = n == 1 ? *part : ((*part + n - 1) / n + unit - 1) / unit * unit;
+            if (*ks < 512 && n > 1) break;                        // copies this short are not worth having
+            const int one = (int)fit(*ks, 1);
+            if (one < want) continue;
+            const int two = x_bytes + 2 * set_bytes < GS_SMEM_LIMIT ? (int)fit(*ks, 2) : 0;
+            *sets = two >= 4 || two == one ? 2 : 1;
+            const int n_stages = *sets == 2 ? two : one;
+            *stages = n_stages > GS_MAX_STAGES ? GS_MAX_STAGES : n_stages;
+            *smem = x_bytes + (*sets * set_bytes < least ? least : *sets * set_bytes) + *stages * stage_of(*ks);
+            return true;
+        }
     return false;
 }
 
 // Whether the kernel takes the shape (else the caller uses another product).
 PB_API int pb_gemm_stream_supported(int M, int N, int K, long long ldw, long long ldx) {
     if (M < 1 || M > 16 || N < 1 || K < 16 || K % 16 || ldw % 8 || ldx % 8) return 0;
-    int ks, nc, st, sets;
+    int ks, part, st, sets;
     size_t smem;
-    return gs_plan(M, K, &ks, &nc, &st, &sets, &smem) ? 1 : 0;
+    return gs_plan(M, K, &ks, &part, &st, &sets, &smem) ? 1 : 0;
 }
 
 // gated: W is [2 N, K], N gate rows then N up rows, and out [M, N] = silu(x Wg^T) * (x Wu^T); no bias, no splits.
@@ -401,7 +417,7 @@ static int gs_run(const void* X, const void* W, const float* bias, void* out, in
     p.act = act; p.limit = limit; p.alpha = alpha;
     p.res = residual.res; p.gain = residual.gain; p.shift = residual.shift; p.slope = residual.slope;
     size_t smem;
-    gs_plan(M, k_part, &p.ks, &p.n_chunks, &p.stages, &p.sets, &smem);
+    gs_plan(M, k_part, &p.ks, &p.part, &p.stages, &p.sets, &smem);
     int blocks = gs_sms() / splits;
     if (blocks < 1) blocks = 1;
     if (blocks > (N + 7) / 8) blocks = (N + 7) / 8;           // at least 8 features per block

@@ -25,6 +25,17 @@ def test_stream_plans(M, K_, N):
     assert torch.equal(gemm_stream(x, w, out_dtype=torch.float32), got) and int(tc_status(x.device)) == 0
 
 
+# steps whose rows are fetched whole beside few rows of x, and in pieces beside many; pieces in whole turns over the chains and not
+@pytest.mark.parametrize("few,many,K_", [(2, 12, 2432), (2, 16, 2432), (8, 12, 2560), (1, 16, 2560), (2, 8, 3072), (1, 14, 3072), (2, 11, 4096), (8, 14, 4096), (1, 9, 5120),
+                                         (2, 14, 6144), (1, 6, 8192), (1, 2, 12288)])
+def test_sums_do_not_depend_on_how_k_is_fetched(few, many, K_):
+    from prelude_b200.ops.linear import gemm_stream
+    x, w = rnd(many, K_), rnd(3000, K_, seed=2, scale=K_ ** -0.5)
+    got = gemm_stream(x, w, out_dtype=torch.float32)
+    assert torch.equal(gemm_stream(x[:few], w, out_dtype=torch.float32), got[:few])
+    assert torch.equal(gemm_stream(x, w[:9], out_dtype=torch.float32), got[:, :9])
+
+
 @pytest.mark.parametrize("gated,act", [(False, "NONE"), (False, "RELU2"), (True, "NONE"), (True, "CLAMPED")])
 @pytest.mark.parametrize("slots", [False, True])
 @pytest.mark.parametrize("T,top,E,N,K_", [(1, 1, 1, 8, 768), (1, 4, 32, 100, 1040), (2, 2, 4, 136, 2048), (8, 4, 32, 2048, 2048), (9, 2, 3, 24, 4096), (17, 1, 2, 40, 2416),
