@@ -13,9 +13,9 @@
 //    row, full and empty barriers); the compute warps take the stages two at a
 //    time.  Issuing a bulk copy costs a warp about 60 cycles whatever its size,
 //    and as much goes into a stage's wait and its announcement; warps issue side
-//    by side, so they take the stages in turn (all four on every stage, two copies
-//    each: chunks of 512 elements 45 us for 150 MB instead of 34, of 1,024 30
-//    instead of 26.5), and the chunks are as long as leaves four stages (gs_plan).
+//    by side, so they share a stage only as far as its copies are waited for
+//    (GsPlan) and take the stages in turn, and the chunks are as long as leaves
+//    four stages.
 //    How K is cut into chunks changes no sum: a step is dealt to its warp and
 //    chain by its place in K, or in a part of K that the rows' number sets.
 //    Weights are written by no kernel, so the
@@ -52,7 +52,7 @@
 PB_TIMELINE_UNIT(gemm_stream)
 
 #define GS_WARPS 8                              // compute warps
-#define GS_LOADERS 4                            // loader warps, which take the stages in turn
+#define GS_LOADERS 4                            // loader warps
 #define GS_THREADS ((GS_WARPS + GS_LOADERS) * 32)
 #define GS_ROWS 8                               // features per stage; a tile of the product is two stages
 #define GS_MAX_STAGES 16
@@ -69,6 +69,7 @@ struct GsParams {
     int ks;                 // elements of K per stage
     int part;               // elements of K whose steps are dealt to the warps' chains from the first on; stages do not go across parts
     int stages;
+    int share;              // loader warps that bring a stage together
     int sets;               // of the warps' sums in shared memory: two, or one where a second does not fit
     int out_f32;
     long long split_stride; // elements between the partial outputs of the splits of K (gridDim.y of them)
@@ -131,17 +132,18 @@ __global__ void __launch_bounds__(GS_THREADS, 1) gemm_stream_kernel(GsParams p) 
 
     if (threadIdx.x == 0) {
         s_dead = 0;
-        for (int s = 0; s < p.stages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], GS_WARPS); }
+        for (int s = 0; s < p.stages; ++s) { mbar_init(&full_bar[s], p.share); mbar_init(&empty_bar[s], GS_WARPS); }
         mbar_init(&x_bar, GS_LOADERS);
         mbar_fence_init();
     }
     __syncthreads();
 
     if (warp >= GS_WARPS) {
-        // ---------------- loaders: the warps take the stages in turn, a lane copies a row ----------------
-        // No more warps than stages: a warp that waits for a stage's tenant of one lap ago then knows that the one of two laps ago has left (it
+        // ---------------- loaders: `share` warps at a time take the stages in turn, a lane copies a row ----------------
+        // No more turns than stages: a warp that waits for a stage's tenant of one lap ago then knows that the one of two laps ago has left (it
         // has waited for that or a later one), and a parity tells only two laps apart
-        const int lw = warp - GS_WARPS, n_loaders = min(GS_LOADERS, p.stages);
+        const int lw = (warp - GS_WARPS) / p.share, n_loaders = min(GS_LOADERS / p.share, p.stages);
+        const int per = GS_ROWS / p.share, row = (warp - GS_WARPS) % p.share * per + lane;   // this lane's, of the first `per` lanes
         bool ok = true;
         int stage = 0, phase = 0, i = 0, turn = 0;
 #pragma unroll 1
@@ -161,9 +163,9 @@ __global__ void __launch_bounds__(GS_THREADS, 1) gemm_stream_kernel(GsParams p) 
                         const int row0 = feat0 + (p.gated ? h * p.N : 0);             // its row of W: up rows follow the gate rows
                         const int n_rows = min(GS_ROWS, r1 - feat0);
                         // the copies may land before the expected bytes are posted: the phase cannot end before this arrival
-                        if (lane == 0) mbar_arrive_expect_tx(&full_bar[stage], (unsigned)n_rows * len * 2);
-                        if (lane < n_rows)
-                            bulk_copy_g2s(ring + (size_t)stage * stage_bytes + (size_t)lane * w_stride, p.W + (size_t)(row0 + lane) * p.ldw + k0,
+                        if (lane == 0) mbar_arrive_expect_tx(&full_bar[stage], (unsigned)min(per, max(0, n_rows - row)) * len * 2);
+                        if (lane < per && row < n_rows)
+                            bulk_copy_g2s(ring + (size_t)stage * stage_bytes + (size_t)row * w_stride, p.W + (size_t)(row0 + row) * p.ldw + k0,
                                           (unsigned)len * 2, &full_bar[stage]);
                     }
                     if (++turn == n_loaders) turn = 0;
@@ -343,40 +345,52 @@ static int gs_sms() {
     return g_gs_sms;
 }
 
-// The parts of K whose steps are dealt out together, the piece of a part that goes into a stage, and the number of stages.
-// The parts decide the order of the sums and nothing else does: the fewest equal ones, in steps of 16, of which three fit beside the rows of x and
-// one set of sums, or two.  Pieces: the longest equal cut of a part of which four stages fit (a tile takes its stages two by two: with three, one is on
-// its way while it waits), else the longest of which two do.
-// 64 MB of weights, us, piece x stages: K = 2,560, 12 rows 2,560 x 3 16.1, 1,280 x 7 14.7; 4,096, 2 rows 4,096 x 3 13.9, 2,048 x 6 13.2; 8,192, 8 rows 1,648 x 3
-// 18.4, 832 x 6 15.9; 6,144, 16 rows 512 x 2 40.5, 512 x 3 37.4, 768 x 2 31.9; 8,192, 12 rows 512 x 2 43.7, 512 x 3 39.9, 768 x 2 34.7.
-static bool gs_plan(int M, int K, int* ks, int* part, int* stages, int* sets, size_t* smem) {
+// How a product's rows of W pass through shared memory.
+// Parts: they decide the order of the sums and nothing else does: the fewest equal ones, in steps of 16, of which three fit beside the rows of x and one
+// set of sums, or two.
+// Pieces of a part: all of it where the block's rows then lie in the ring at once, as copies are few and nothing waits; else the longest equal cut of
+// which four stages fit (a tile takes its stages two by two: with three, one is on its way while it waits); else the longest of which two do.
+// Two sets of the warps' sums unless the second costs a pair of stages.
+// Warps a stage: two; all four where there are three stages, which the tiles wait for whatever is done; one where pieces are short, as what a warp spends
+// on a stage besides its copies then counts.
+// us, piece x stages, 64 MB of weights: K = 2,560, 12 rows 2,560 x 3 16.1, 1,280 x 7 14.6; 4,096, 2 rows 4,096 x 3 13.8, 2,048 x 6 13.2; 16 MB: 2,560, 12
+// rows 2,560 x 3 6.2, 1,280 x 7 6.7; 4,096, 2 rows 4.8 and 5.1.  One, two and four warps a stage: 67 MB, 4,096, 16 rows, 1,376 x 4 13.5, 13.2, 13.5 (134 MB
+// 27.3, 26.6, 27.8); 67 to 80 MB, 6,912, 10 rows, 864 x 6 14.4, 14.1, 15.6; 9,728, 8 rows, 608 x 6 21.0, 21.7, 27.0; 8,192, 11 rows, 832 x 3 30.4, 29.7, 28.5;
+// 8,192, 12 rows, 768 x 2 34.6, 32.8, 36.8 (512 x 3 40.4, 39.0, 37.7).
+struct GsPlan {
+    int part, ks, stages, sets, share;      // as in GsParams
+    size_t smem;
+};
+
+// `rows`: of W, of one block (0: any number).  False: not even two stages fit.
+static bool gs_plan(int M, int K, int rows, GsPlan* p) {
     const size_t x_bytes = (size_t)M * ((size_t)K * 2 + 16), set_bytes = (size_t)GS_WARPS * 16 * (M <= 8 ? 8 : 16) * 4, least = 8192;
-    if (x_bytes + least >= GS_SMEM_LIMIT) return false;
+    auto taken = [&](int sets) { return x_bytes + (sets * set_bytes < least ? least : sets * set_bytes); };
     auto stage_of = [](int k) { return (size_t)GS_ROWS * ((size_t)k * 2 + 16); };
-    auto fit = [&](int k, int sums) { return (GS_SMEM_LIMIT - x_bytes - (sums * set_bytes < least ? least : sums * set_bytes)) / stage_of(k); };
-    *part = 0;
-    for (int want = 3; want >= 2 && *part == 0; --want)
+    auto fit = [&](int k, int sets) { return taken(sets) < GS_SMEM_LIMIT ? (int)((GS_SMEM_LIMIT - taken(sets)) / stage_of(k)) : 0; };
+    p->part = 0;
+    for (int want = 3; want >= 2 && p->part == 0; --want)
         for (int n = 1; n <= K / 16; ++n) {
             const int k_per = ((K + n - 1) / n + 15) / 16 * 16;
             if (k_per < 512 && n > 1) break;
-            if ((int)fit(k_per, 1) >= want) { *part = k_per; break; }
+            if (fit(k_per, 1) >= want) { p->part = k_per; break; }
         }
-    if (*part == 0) return false;
-    // whole turns over the warps and chains: dealt as K in one part is
-    if (*part % (16 * GS_WARPS * GS_CHAINS) == 0) *part = K;
-    // In turns over the eight warps where the deal is K's own
-    const int unit = *part == K ? 16 * GS_WARPS : 16;
-    for (int want = 4; want >= 2; want -= 2)
-        for (int n = 1; n <= *part / 16; ++n) {
-            *ks = n == 1 ? *part : ((*part + n - 1) / n + unit - 1) / unit * unit;
-            if (*ks < 512 && n > 1) break;                        // copies this short are not worth having
-            const int one = (int)fit(*ks, 1);
+    if (p->part == 0) return false;
+    if (p->part % (16 * GS_WARPS * GS_CHAINS) == 0) p->part = K;          // whole turns over the chains: dealt as K in one part is
+    const int unit = p->part == K ? 16 * GS_WARPS : 16, all = (rows + GS_ROWS - 1) / GS_ROWS * ((K + p->part - 1) / p->part);
+    const int whole = fit(p->part, 1);
+    for (int rule = all > 0 && whole >= all && whole >= 2 ? 0 : 1; rule < 3; ++rule)
+        for (int n = 1; n <= p->part / 16; ++n) {
+            const int want = rule == 0 && all > 2 ? all : rule == 1 ? 4 : 2, ks = n == 1 ? p->part : ((p->part + n - 1) / n + unit - 1) / unit * unit;
+            if (ks < 512 && n > 1) break;                                   // copies this short are not worth having
+            const int one = fit(ks, 1), two = fit(ks, 2);
             if (one < want) continue;
-            const int two = x_bytes + 2 * set_bytes < GS_SMEM_LIMIT ? (int)fit(*ks, 2) : 0;
-            *sets = two >= 4 || two == one ? 2 : 1;
-            const int n_stages = *sets == 2 ? two : one;
-            *stages = n_stages > GS_MAX_STAGES ? GS_MAX_STAGES : n_stages;
-            *smem = x_bytes + (*sets * set_bytes < least ? least : *sets * set_bytes) + *stages * stage_of(*ks);
+            p->sets = two == one || two >= 6 || (two >= 4 && two / 2 == one / 2) || (rule == 0 && two >= want) ? 2 : 1;
+            const int stages = p->sets == 2 ? two : one;
+            p->ks = ks;
+            p->stages = stages > GS_MAX_STAGES ? GS_MAX_STAGES : stages;
+            p->share = p->stages == 3 ? 4 : ks <= 704 && p->stages > 3 ? 1 : 2;
+            p->smem = taken(p->sets) + p->stages * stage_of(ks);
             return true;
         }
     return false;
@@ -385,9 +399,8 @@ static bool gs_plan(int M, int K, int* ks, int* part, int* stages, int* sets, si
 // Whether the kernel takes the shape (else the caller uses another product).
 PB_API int pb_gemm_stream_supported(int M, int N, int K, long long ldw, long long ldx) {
     if (M < 1 || M > 16 || N < 1 || K < 16 || K % 16 || ldw % 8 || ldx % 8) return 0;
-    int ks, part, st, sets;
-    size_t smem;
-    return gs_plan(M, K, &ks, &part, &st, &sets, &smem) ? 1 : 0;
+    GsPlan plan;
+    return gs_plan(M, K, 0, &plan) ? 1 : 0;
 }
 
 // gated: W is [2 N, K], N gate rows then N up rows, and out [M, N] = silu(x Wg^T) * (x Wu^T); no bias, no splits.
@@ -416,11 +429,13 @@ static int gs_run(const void* X, const void* W, const float* bias, void* out, in
     p.gated = gated ? 1 : 0;
     p.act = act; p.limit = limit; p.alpha = alpha;
     p.res = residual.res; p.gain = residual.gain; p.shift = residual.shift; p.slope = residual.slope;
-    size_t smem;
-    gs_plan(M, k_part, &p.ks, &p.part, &p.stages, &p.sets, &smem);
     int blocks = gs_sms() / splits;
     if (blocks < 1) blocks = 1;
     if (blocks > (N + 7) / 8) blocks = (N + 7) / 8;           // at least 8 features per block
+    const int features = (N + blocks - 1) / blocks;
+    GsPlan plan;
+    gs_plan(M, k_part, gated ? (features + GS_ROWS - 1) / GS_ROWS * 2 * GS_ROWS : features, &plan);
+    p.part = plan.part; p.ks = plan.ks; p.stages = plan.stages; p.sets = plan.sets; p.share = plan.share;
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(gemm_stream_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, GS_SMEM_LIMIT);
@@ -431,11 +446,11 @@ static int gs_run(const void* X, const void* W, const float* bias, void* out, in
         configured = true;
     }
     if (p.res) {
-        if (M <= 8) pb_launch(gemm_stream_kernel<1, true>, dim3(blocks, splits), dim3(GS_THREADS), smem, stream, p);
-        else pb_launch(gemm_stream_kernel<2, true>, dim3(blocks, splits), dim3(GS_THREADS), smem, stream, p);
+        if (M <= 8) pb_launch(gemm_stream_kernel<1, true>, dim3(blocks, splits), dim3(GS_THREADS), plan.smem, stream, p);
+        else pb_launch(gemm_stream_kernel<2, true>, dim3(blocks, splits), dim3(GS_THREADS), plan.smem, stream, p);
     } else {
-        if (M <= 8) pb_launch(gemm_stream_kernel<1, false>, dim3(blocks, splits), dim3(GS_THREADS), smem, stream, p);
-        else pb_launch(gemm_stream_kernel<2, false>, dim3(blocks, splits), dim3(GS_THREADS), smem, stream, p);
+        if (M <= 8) pb_launch(gemm_stream_kernel<1, false>, dim3(blocks, splits), dim3(GS_THREADS), plan.smem, stream, p);
+        else pb_launch(gemm_stream_kernel<2, false>, dim3(blocks, splits), dim3(GS_THREADS), plan.smem, stream, p);
     }
     PB_CHECK_LAUNCH("gemm_stream");
     return 0;

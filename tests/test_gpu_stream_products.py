@@ -10,9 +10,10 @@ def rnd(*shape, seed=1, scale=1.0):
     return (torch.randn(*shape, generator=torch.Generator(device=DEV).manual_seed(seed), device=DEV) * scale).bfloat16()
 
 
-# rows x K: one chunk with many stages, four; two chunks; 1,024-element chunks beside 16 rows; 640; three stages; two; one set of sums
+# rows x K: one chunk with many stages, four; two chunks; 1,024-element chunks beside 16 rows; 640; three stages; two; one set of sums; three stages of
+# parts, short pieces of parts; N: all of a block's rows in the ring at once, and not
 @pytest.mark.parametrize("M,K_", [(1, 48), (8, 1024), (8, 2560), (16, 2560), (2, 4096), (8, 4096), (16, 4096), (12, 5120), (16, 5120), (8, 8192), (2, 12288), (16, 6160),
-                                  (16, 6144), (1, 20000), (2, 49600)])
+                                  (16, 6144), (1, 20000), (2, 49600), (11, 8192), (8, 9728), (14, 6912)])
 @pytest.mark.parametrize("N", [9, 700, 3000])
 def test_stream_plans(M, K_, N):
     from prelude_b200.ops.linear import gemm_stream, stream_takes, tc_status
