@@ -17,12 +17,16 @@
 //    it has itself waited, so that a block fills its ring while other multiprocessors are still at the first product.  The experts of 8 rows,
 //    2,048 x 2,048, both products 79.0 -> 76.6 us.
 // Every sum is over k in an order that K alone decides (steps of 16 dealt to eight warps with four chains each, piece by piece), so a token's
-// result does not depend on who else chose the expert.
+// result does not depend on who else chose the expert.  No sum runs on in the tensor cores, which cut what they add up: a step's sixteen products
+// are added to a chain in float32, and the eight warps' sums meet in 64 bits.  Error against 64 bits, with running sums / with chains in float32 and the
+// warps in 32 bits / here / the kernel in moe.cu: K = 768 7.4e-8, 6.7e-8, 5.4e-8, 6.6e-8; 2,048 9.4e-8, 7.5e-8, 6.3e-8, 7.9e-8; 4,096, gated 2.6e-7, 1.3e-7,
+// 1.2e-7, 1.5e-7; 7,168, gated 4.2e-7, 1.5e-7, 1.4e-7, 1.8e-7.  It costs nothing with rows of 2,048 and more, of 768 up to 4 %.
 //
-// What bounds it: the weights' bytes.  A product alone, 26 experts hit by 32 choices, us against the kernel in moe.cu, whose warps keep four rows of
-// 2 KB in flight and spend half their lives on beginnings and ends: 4,096 x 4,096 gated 122 against 133 (6.8 TB/s), 4,096 x 2,048 66 against 77,
-// 2,048 x 2,048 36 against 41, eight experts hit 14 against 19.  Short rows leave it bound by the copies and by each tile's sums (1,000 and 1,300 cycles
-// a tile of 16 rows): rows of 768 elements take the same time either way, of 512 a fifth more, and keep the kernel in moe.cu.
+// What bounds it: the weights' bytes.  A product alone, us against the kernel in moe.cu, whose warps keep four rows of 2 KB in flight and spend half
+// their lives on beginnings and ends: 21 experts hit by 32 choices, 4,096 x 4,096 gated 106 against 115 (6.7 TB/s); 26 hit, 4,096 x 2,048 68 against 77,
+// 2,048 x 2,048 37 against 42, eight hit 14 against 19.  Short rows leave it bound by the copies and by each tile's sums (1,000 and 1,300 cycles a tile
+// of 16 rows): 2,048 rows of 768, one token 7.4 against 11.6, eight 26 against 24, sixteen 36 against 37; rows of 512 take a fifth more and keep the
+// kernel in moe.cu.
 #include "attention_common.cuh"
 
 #define MS_WARPS 8                              // multiplying warps
@@ -257,7 +261,13 @@ __global__ void __launch_bounds__(MS_THREADS, 1) moe_stream_kernel(MsParams p) {
                     }
 #pragma unroll
                     for (int c = 0; c < MS_CHAINS; ++c)
-                        if (s0 + c * MS_WARPS < steps) mma_bf16_free(acc[c], a[c], b[c][0], b[c][1]);
+                        if (s0 + c * MS_WARPS < steps) {
+                            // sixteen products at a time: what the tensor cores add to a running sum they cut off instead of rounding it
+                            float q[4] = {0.f, 0.f, 0.f, 0.f};
+                            mma_bf16_free(q, a[c], b[c][0], b[c][1]);
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) acc[c][e] += q[e];
+                        }
                 }
                 __syncwarp();
                 if (lane == 0) {
@@ -278,12 +288,14 @@ __global__ void __launch_bounds__(MS_THREADS, 1) moe_stream_kernel(MsParams p) {
             for (int idx = tid; idx < rows * per; idx += MS_WARPS * 32) {
                 const int m = idx / per, rr = idx % per, feat = f + rr;
                 if (feat >= w.f1) continue;
-                float v = 0.f, u = 0.f;
+                auto sum = [&](int at) {                       // of the warps, in 64 bits: rounded once (in 32 bits these sums alone are half of the error)
+                    double w8[MS_WARPS];
 #pragma unroll
-                for (int k = 0; k < MS_WARPS; ++k) {
-                    v += set[k * 128 + m * 16 + rr];
-                    if (p.gated) u += set[k * 128 + m * 16 + rr + 8];
-                }
+                    for (int k = 0; k < MS_WARPS; ++k) w8[k] = set[k * 128 + m * 16 + at];
+                    return (float)(((w8[0] + w8[1]) + (w8[2] + w8[3])) + ((w8[4] + w8[5]) + (w8[6] + w8[7])));
+                };
+                float v = sum(rr);
+                const float u = p.gated ? sum(rr + 8) : 0.f;
                 if (p.gated) v = p.act == PB_ACT_CLAMPED ? pb_clamped_unit(v, u, p.limit, p.alpha) : v / (1.0f + expf(-v)) * u;
                 else if (p.act == PB_ACT_RELU2) v = pb_relu2(v);
                 const size_t at = (size_t)mine_slots[m] * p.ldo + feat;

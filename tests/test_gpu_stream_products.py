@@ -63,7 +63,10 @@ def test_experts_streamed(T, top, E, N, K_, gated, act, slots):
         elif act == "RELU2":
             z = torch.relu(z) ** 2
         want[m] = z
-    assert float((got.double() - want).norm() / want.norm()) < 3e-6
+    # Steps of sixteen products cut to 2^-23 of the largest (2^-24 in the root mean square); a chain adds K / 512 of them, four chains meet, the warps'
+    # sums are added in 64 bits: that many sums rounded by 2^-25 of themselves, a chain's early ones of less.  Activations: a product of two such sums, or more
+    most = 2.0 ** -25 * (4 + (K_ / 512 + 1) / 2 + 3) ** 0.5
+    assert float((got.double() - want).norm() / want.norm()) < (most if act == "NONE" and not gated else 4 * most)
     assert int(status) == 0 and torch.equal(K.moe_gemv(a, w, ids, slots, torch.float32, **kw), got)
     # one rounding to bfloat16
     assert torch.equal(K.moe_gemv(a, w, ids, slots, torch.bfloat16, **kw), got.bfloat16())
