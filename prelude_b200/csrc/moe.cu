@@ -462,16 +462,18 @@ PB_API int pb_moe_route_few(const void* x, long long ldx, const void* W, int dty
 
 // Router logits and choice of a prompt step, on the tensor cores: a block takes 16 tokens and 64 experts, its sixteen warps a sixteenth of K
 // each, operands straight from global memory (a lane reads 16 bytes of a row, which serve two steps of 16: k is permuted alike in
-// both operands), products exact, float32 sums; the warps' sums meet in shared memory in a fixed tree.  With up to 64 experts the block
+// both operands), products exact, float32 sums; the warps' sums meet in shared memory in 64 bits.  With up to 64 experts the block
 // chooses too, a warp a token, else another kernel does.  The order of the sums depends on K alone.
 // What bounds it: trips to the L2 cache, where every block reads its share of the router's matrix.  Logits and choice, us, against the kernels above on
-// the float32 units: 64 experts, K 4,096: 64 tokens 13.3 (16.3), 300 13.7 (20.6), 2,048 14.2 (48); 256, K 7,168: 64 tokens 26 (63), 2,048 88 (277);
-// 32, K 2,048, 2,048 tokens 8.6 (23).  Error of the logits against 64 bits: 8.5e-8 (9.5e-8), 9.7e-8 (1.16e-7), 7.5e-8 (7.9e-8); with the tensor cores'
-// own running sums 4.8e-7.
+// the float32 units: 64 experts, K 4,096: 64 tokens 13.7 (16.0), 300 14.0 (20.5), 2,048 14.5 (48); K 512, 2,048 tokens 6.2 (11.6); 256, K 7,168: 64 tokens
+// 26 (60), 2,048 89 (275); 32, K 2,048, 2,048 tokens 9.2 (24).  Error of the logits against 64 bits: K 128 4.3e-8 (4.8e-8), 512 4.2e-8 (6.2e-8), 2,048 5.8e-8
+// (7.9e-8), 4,096 7.0e-8 (9.5e-8), 7,168 8.4e-8 (1.17e-7); with the warps' sums in 32 bits 5.0e-8, 6.4e-8, 7.6e-8, 8.5e-8, 9.7e-8, with the tensor cores'
+// own running sums 4.8e-7 at 4,096.
 #define RT_TOKENS 16
 #define RT_WARPS 16
 #define RT_EXPERTS 64                                        // of one pass
 #define RT_MIN_TOKENS 64
+#define RT_MIN_K 128
 template <int SLOTS>
 __global__ void __launch_bounds__(32 * RT_WARPS, 1)
 moe_route_tokens_kernel(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* W, int n_tokens, int K, MoeRouteArgs args, int32_t* ids, float* weights,
@@ -528,7 +530,7 @@ moe_route_tokens_kernel(const __nv_bfloat16* x, long long ldx, const __nv_bfloat
         __syncthreads();
         for (int i = threadIdx.x; i < RT_TOKENS * RT_EXPERTS; i += 32 * RT_WARPS) {
             const int t = i / RT_EXPERTS, e = e0 + i % RT_EXPERTS;
-            float v[RT_WARPS];
+            double v[RT_WARPS];                              // in 64 bits: rounded once (in 32 bits these sums are most of the error)
 #pragma unroll
             for (int k = 0; k < RT_WARPS; ++k) v[k] = rt_sm[k * RT_TOKENS * RT_EXPERTS + i];
 #pragma unroll
@@ -536,8 +538,8 @@ moe_route_tokens_kernel(const __nv_bfloat16* x, long long ldx, const __nv_bfloat
 #pragma unroll
                 for (int k = 0; k < o; ++k) v[k] += v[k + o];
             if (e < E) {
-                if (SLOTS <= 2) z[t * E + e] = v[0];
-                if (logits && t0 + t < n_tokens) logits[(size_t)(t0 + t) * E + e] = v[0];
+                if (SLOTS <= 2) z[t * E + e] = (float)v[0];
+                if (logits && t0 + t < n_tokens) logits[(size_t)(t0 + t) * E + e] = (float)v[0];
             }
         }
         __syncthreads();
@@ -547,10 +549,11 @@ moe_route_tokens_kernel(const __nv_bfloat16* x, long long ldx, const __nv_bfloat
         moe_route_token<SLOTS>(z + t * E, args, ids + (size_t)(t0 + t) * args.top, weights + (size_t)(t0 + t) * args.top);
 }
 
-// Whether pb_moe_route_tokens takes the sizes.  Fewer tokens than 64 take no longer on the kernels above, nor do eight experts once the blocks of 16
+// Whether pb_moe_route_tokens takes the sizes.  Rows of 64 would be less exact here (4.3e-8 against 4.0e-8); fewer tokens than 64 take no longer on
+// the kernels above, nor do eight experts once the blocks of 16
 // tokens make a second wave (K 1,024, 4,096 tokens: 9.6 us against 8.9).
 PB_API int pb_moe_route_tokens_supported(int n_tokens, int n_experts, int K) {
-    return n_tokens >= RT_MIN_TOKENS && K % 32 == 0 && (n_experts > 8 || n_tokens <= 148 * RT_TOKENS) ? 1 : 0;
+    return n_tokens >= RT_MIN_TOKENS && K % 32 == 0 && K >= RT_MIN_K && (n_experts > 8 || n_tokens <= 148 * RT_TOKENS) ? 1 : 0;
 }
 
 // x [n_tokens, K] with row stride ldx, W [n_experts, K], both bfloat16; logits float32 [n_tokens, n_experts], null with up to 64 experts if

@@ -22,12 +22,24 @@ def test_router_of_a_prompt(T, K_, E, groups, keep, top):
     ids, p = K.moe_route_tokens(x, w, *args, logits=logits)
     want = x.double() @ w.double().T
     ok = torch.arange(T, device=DEV) != 3
-    # sums of sixteen cut to 2^-23 of the largest product, then rounded K / 512 + 5 times to 2^-24 of a partial sum
-    assert float((logits[ok].double() - want[ok]).norm() / want[ok].norm()) < 2.0 ** -24 * (K_ / 512 + 9)
+    # sums of sixteen cut to 2^-23 of the largest product (2^-24 in the root mean square); a warp adds them in twos, K / 512 of these, and the warps' sums
+    # are added in 64 bits: that many sums rounded by 2^-25 of themselves, a warp's early ones of less
+    assert float((logits[ok].double() - want[ok]).norm() / want[ok].norm()) < 2.0 ** -25 * (4 + 1 + (K_ / 512 + 1) / 2 + 1) ** 0.5
     assert bool(logits[3].isnan().all())
     ids2, p2 = K.moe_route(logits, *args)            # the choice is that of the logits alone
     assert torch.equal(ids, ids2) and torch.equal(p[ok], p2[ok])
-    assert K.moe_route_tokens_takes(x, w) == (E > 8 or T <= 2368)
+    assert K.moe_route_tokens_takes(x, w) == (K_ >= 128 and (E > 8 or T <= 2368))
+
+
+@pytest.mark.parametrize("K_", [128, 256, 512, 768, 1024, 4096])
+def test_logits_are_no_less_exact_than_those_of_fewer_rows(K_):
+    from prelude_b200.ops import kernels as K
+    g = torch.Generator(device=DEV).manual_seed(K_)
+    x, w = torch.randn(4096, K_, generator=g, device=DEV).bfloat16(), (torch.randn(64, K_, generator=g, device=DEV) * K_ ** -0.5).bfloat16()
+    assert K.moe_route_tokens_takes(x, w)
+    logits, want = torch.empty(4096, 64, device=DEV), x.double() @ w.double().T
+    K.moe_route_tokens(x, w, 4, 1, 1, 1, False, logits=logits)
+    assert float((logits.double() - want).norm()) <= float((K.router_logits(x, w).double() - want).norm())
 
 
 def test_choices_by_a_plain_sort():

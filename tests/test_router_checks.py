@@ -7,7 +7,7 @@ from prelude_b200.ops import kernels as K
 from prelude_b200.parts import model as _registers_the_parts  # noqa: F401
 from prelude_b200.parts.registry import RunContext, make_part
 
-WIDTH, E = 64, 8
+WIDTH, E = 128, 8
 
 
 @pytest.fixture
