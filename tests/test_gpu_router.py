@@ -83,3 +83,21 @@ def test_weighted_sum(T, top, width, y32):
     # `top` roundings of the running sum, whose size the terms bound, and one to bfloat16
     size = (y[place.long()].double().abs().view(T, top, width) * w.double().unsqueeze(-1)).sum(1)
     assert bool(((got - want).abs() <= 2.0 ** -8 * want.abs() + top * 2.0 ** -24 * size).all())
+
+
+@pytest.mark.parametrize("T,E,K_", [(64, 64, 4096), (100, 8, 1024), (64, 200, 2048)])
+def test_both_routers_choose_alike_away_from_ties(T, E, K_):
+    """A token's logits come from another order of sums from 64 rows on: they differ by roundings, and its experts only where two tie within them."""
+    from prelude_b200.ops import kernels as K
+    g = torch.Generator(device=DEV).manual_seed(E)
+    x, w = torch.randn(T, K_, generator=g, device=DEV).bfloat16(), (torch.randn(E, K_, generator=g, device=DEV) * K_ ** -0.5).bfloat16()
+    logits, args = torch.empty(T, E, device=DEV), (4, 1, 1, 1, False)
+    ids, _ = K.moe_route_tokens(x, w, *args, softmax_chosen=True, logits=logits)
+    few = K.router_logits(x, w)
+    ids_few, _ = K.moe_route(few, *args, softmax_chosen=True)
+    # K / 32 sums a lane and five between lanes; sums of sixteen cut in sixteen places, K / 512 pairs of them and one rounding at the end
+    most = 2.0 ** -24 * ((K_ / 32 + 5) + (32 + K_ / 512 + 2)) * (x.double().abs() @ w.double().abs().T)
+    assert bool(((logits.double() - few.double()).abs() <= most).all())
+    order = few.double().sort(1, descending=True).values[:, :5]
+    apart = (order[:, :4] - order[:, 1:]).min(1).values > 2 * most.max()
+    assert int(apart.sum()) > T // 2 and torch.equal(ids[apart], ids_few[apart])
