@@ -279,7 +279,8 @@ qkv_prepare_direct_kernel(const T* q_in, long long ldq, const T* k_in, long long
             cs[2 * i] = c * rot.amplitude;
             cs[2 * i + 1] = sn * rot.amplitude;
         }
-        __syncthreads();
+        // a barrier with its number and its count, all threads': the warps of either role come to it in their own branch
+        asm volatile("bar.sync 1, %0;\n" ::"r"((int)blockDim.x) : "memory");
     };
     if (tid < q_threads) {
         const T* q = q_in + (size_t)t * ldq;
@@ -415,8 +416,8 @@ PB_API int pb_qkv_prepare(const void* q_in, long long ldq, const void* k_in, lon
     auto whole = [&](int off) { return rates == nullptr || (off % vn == 0 && rot_dims % vn == 0 && (adjacent || (rot_dims / 2) % vn == 0)); };
     const int nk = k_pages ? G * kd : 0;
     bool direct = staged && q_w == nullptr && whole(q_rot_off) && H * qd <= QP_MOST * vn * 256 && (nk == 0 || whole(k_rot_off));
-    // queries written over what is read: a thread reads its pieces' rotation partners, and the last warp its key row, after others have
-    // stored; the staged kernel has read both rows by then
+    // queries written over what is read: the rotation partners, and of the key row three pieces a lane, are read ahead of the block's barrier, the
+    // pieces of a longer key row after others have stored; the staged kernel has read both rows by then
     const size_t esz = dtype == PB_BF16 ? 2 : 4;
     auto meets = [&](const void* a, size_t a_elems, const void* b, size_t b_elems) {
         const char *p = (const char*)a, *q = (const char*)b;
