@@ -550,10 +550,10 @@ moe_route_tokens_kernel(const __nv_bfloat16* x, long long ldx, const __nv_bfloat
 }
 
 // Whether pb_moe_route_tokens takes the sizes.  Rows of 64 would be less exact here (4.3e-8 against 4.0e-8); fewer tokens than 64 take no longer on
-// the kernels above, nor do eight experts once the blocks of 16
-// tokens make a second wave (K 1,024, 4,096 tokens: 9.6 us against 8.9).
+// the kernels above, nor do eight experts once the blocks of 16 tokens make a second wave over the multiprocessors (K 1,024, 4,096 tokens: 9.6 us
+// against 8.9).
 PB_API int pb_moe_route_tokens_supported(int n_tokens, int n_experts, int K) {
-    return n_tokens >= RT_MIN_TOKENS && K % 32 == 0 && K >= RT_MIN_K && (n_experts > 8 || n_tokens <= 148 * RT_TOKENS) ? 1 : 0;
+    return n_tokens >= RT_MIN_TOKENS && K % 32 == 0 && K >= RT_MIN_K && (n_experts > 8 || n_tokens <= pb_multiprocessors() * RT_TOKENS) ? 1 : 0;
 }
 
 // x [n_tokens, K] with row stride ldx, W [n_experts, K], both bfloat16; logits float32 [n_tokens, n_experts], null with up to 64 experts if

@@ -353,7 +353,7 @@ PB_API int pb_moe_stream(const void* A, long long lda, int a_div, const void* W,
     ms_plan(K, &p.ks, &p.n_chunks, &p.stages, &p.bufs, &smem);
     static const cudaError_t set = cudaFuncSetAttribute(moe_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MS_SMEM_LIMIT);
     PB_REQUIRE(set == cudaSuccess, "moe_stream: %s", cudaGetErrorString(set));
-    static const int sms = [] { int dev = 0, n = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev); return n > 0 ? n : 148; }();
+    static const int sms = pb_multiprocessors();
     pb_launch(moe_stream_kernel, dim3(sms), dim3(MS_THREADS), smem, stream, p);
     PB_CHECK_LAUNCH("moe_stream");
     return 0;

@@ -135,12 +135,6 @@ __device__ __forceinline__ int pb_find_chunk(const int32_t* cu_q, int n_seqs, in
     return 0;
 }
 
-static inline int pb_multiprocessors() {
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
-    return sms;
-}
-
 // Rows of a recorded launch of `each` blocks a row: twice `blocks` a multiprocessor, no more than the sequences there may be.  (256 rows
 // of a step with room for 256 requests, nearly all of them empty, took 30 to 90 us; with few rows a block's sequences wait for one
 // another: 60 single tokens of the gated delta rule, 32 heads, 264 us at two blocks, 244 at six.)
