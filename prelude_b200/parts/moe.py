@@ -24,6 +24,8 @@ first tensor.
 """
 from __future__ import annotations
 
+import functools
+import math
 import os
 from typing import Dict
 
@@ -51,23 +53,47 @@ MOE_GROUPED_MIN_ROWS = 3
 MOE_GROUPED_ROWS_SET = os.environ.get("PRELUDE_MOE_GROUPED_MIN_ROWS")
 # where a step of few rows leaves the streaming kernel (``grouped_pays``): what a repeated read is counted as, and the bytes
 GROUPED_FIRST_READS, GROUPED_MIN_BYTES = 1.75, 150e6
+# rows of an expert that one walk over its matrices serves in the kernel with a ring, and experts with more than these from which it is left
+STREAM_ROWS, RING_MOST_READ_TWICE = 8, 0.003
 
 
 def grouped_pays(tokens: int, top_k: int, n_experts: int, expert_bytes: int) -> bool:
     """Whether a step of few rows is faster on the product with the weights as rows, which reads every expert's matrices once and pays for a sort, a
-    gather and its own latencies, than on the kernel that streams them once for every (token, expert) pair; ``expert_bytes``: one
-    expert's matrices.  The experts hit are those that an even router hits, n (1 - (1 - k/n)^T).  A pair that repeats an expert costs the
-    streaming kernel about half of what a first one does (the matrices are in the L2 cache), and the other way's beginning what 150 MB
+    gather and its own latencies, than on the kernel of short rows, which streams them once for every (token, expert) pair; ``expert_bytes``: one
+    expert's matrices.  The experts hit are those that an even router hits, n (1 - (1 - k/n)^T).  A pair that repeats an expert costs that
+    kernel about half of what a first one does (the matrices are in the L2 cache), and the other way's beginning what 150 MB
     take; one token hits every expert once and always streams.
 
     The whole feed-forward at 8 to 128 experts of 1,024 x 512 to 4,096 x 2,048, top 2 to 8, with and without a gate, 1 to 64 tokens, weights
-    from memory (2,768 steps), against the streaming kernel of matrices with short rows: of the 795 that leave it 17 are slower for it by
-    more than 2 %, and by 16 % at most; all of them together take 0.78 of the time.  Left behind: 228 steps that would gain more than 5 %.
-    The kernel that streams rows of 768 elements and more (``moe_stream.cu``) reads an expert once for eight pairs, so for these the line
-    lies on the early side: us, streamed / there: 64 experts of 4,096 x 2,048, top 6, gated, 12 tokens 332 / 378, 16 tokens 391 / 450, 32 tokens
-    505 / 514, 48 tokens 756 / 537; 32 of 2,048 x 2,048, top 4, no gate, 8 tokens 66 / 86, 24 tokens 92 / 111, 32 tokens 130 / 112."""
+    from memory (2,768 steps): of the 795 that leave it 17 are slower for it by more than 2 %, and by 16 % at most; all of them
+    together take 0.78 of the time.  Left behind: 228 steps that would gain more than 5 %."""
     hit = n_experts * (1.0 - (1.0 - top_k / n_experts) ** tokens)
     return (tokens * top_k - GROUPED_FIRST_READS * hit) * expert_bytes >= GROUPED_MIN_BYTES
+
+
+@functools.lru_cache(maxsize=1024)
+def read_twice(tokens: int, top_k: int, n_experts: int) -> float:
+    """How many experts an even router is expected to give more than eight of a step's tokens."""
+    p = top_k / n_experts
+    if tokens <= STREAM_ROWS or p >= 1.0:
+        return 0.0 if tokens <= STREAM_ROWS else float(n_experts)
+    return n_experts * max(0.0, 1.0 - sum(math.comb(tokens, i) * p ** i * (1.0 - p) ** (tokens - i) for i in range(STREAM_ROWS + 1)))
+
+
+def ring_pays(tokens: int, top_k: int, n_experts: int) -> bool:
+    """Whether a step that ``grouped_pays`` would send to the grouped products stays on the kernel that streams rows of 768 elements and more through
+    a ring (``moe_stream.cu``).  That one reads an expert once for eight tokens; where one has more, the block that walks it again takes
+    twice as long and the others wait, so the line is where an expert with nine tokens is still an exception.
+
+    The whole feed-forward at 8 to 128 experts of 1,024 x 1,024 to 7,168 x 2,048, top 2 to 8, with and without a gate, 2 to 64 tokens, weights from memory
+    (2,868 steps), us, streamed / grouped: 64 experts of 4,096 x 2,048, top 6, gated, 16 tokens 383 / 438; 64 of 3,072 x 1,536, top 8, gated, 10 tokens
+    206 / 247; 32 of 2,048 x 2,048, top 4, no gate, 16 tokens 80 / 96; beyond the line 64 of 3,072 x 1,536, 24 tokens 266 / 306, 32 tokens 439 / 321.  Of
+    the 2,580 steps with more than eight experts 211 stay for it and take 0.86 of the time; 3 of them take up to 3 % more.  The better side of
+    every step would take 0.96 of the time of all, this rule takes 0.985: a later line gains more on the whole but loses up to 28 % where an
+    expert does get nine.
+    With up to eight experts the line stays where it was, held by tests of both of its sides, though streaming gains most there (8 of 3,072 x 1,536, top 2,
+    12 tokens 47 / 76)."""
+    return n_experts > 8 and read_twice(tokens, top_k, n_experts) < RING_MOST_READ_TWICE
 
 
 # an activation's name: (two matrices on the way up or one, its number in the products' epilogues)
@@ -169,6 +195,9 @@ class RoutedExperts:
         if not streamed:
             return self._paired(x, MOE_GROUPED_MIN_ROWS)
         expert_bytes = (3 if self.gated else 2) * s.hidden_size * s.expert_size * x.element_size()
+        pairs = x.shape[0] * s.top_k
+        if K.moe_streams(self.w_gate_up, pairs) and K.moe_streams(self.w_down, pairs) and ring_pays(x.shape[0], s.top_k, s.n_experts):
+            return False
         return grouped_pays(x.shape[0], s.top_k, s.n_experts, expert_bytes) and self._paired(x, 0)
 
     def _router_args(self):
