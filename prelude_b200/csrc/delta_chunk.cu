@@ -593,7 +593,7 @@ int dc_run(const DcCall& c) {
               c.ld_a, c.a_log, c.dt_bias, c.cu_q, (unsigned char*)c.scratch, c.all.n_seqs, c.all.from, c.all.few, c.all.beside, c.H, c.G);
     PB_CHECK_LAUNCH("gated_delta_scan_chunked");
     // Where the lengths are at hand: the slices for which the longest chain, or all chains over the multiprocessors, takes less.  A chunk of 16 columns
-    // takes 0.6 of what one of 32 does.  us, slices of 16 / 32 columns: 16 heads, 592 and 1,185 tokens 74 / 86; 1,333 and 2,667 158 / 191; one of
+    // takes 0.62 of what one of 32 does.  us, slices of 16 / 32 columns: 16 heads, 592 and 1,185 tokens 74 / 86; 1,333 and 2,667 158 / 191; one of
     // 1,000 41 / 72; 32 heads, 592 and 1,185 145 / 132, one of 1,000 80 / 73.
     int narrowest = 16, widest = 32;
     if (c.counted && c.longest > 0 && c.E % 32 == 0) {
