@@ -195,10 +195,12 @@ class RoutedExperts:
         if not streamed:
             return self._paired(x, MOE_GROUPED_MIN_ROWS)
         expert_bytes = (3 if self.gated else 2) * s.hidden_size * s.expert_size * x.element_size()
-        pairs = x.shape[0] * s.top_k
-        if K.moe_streams(self.w_gate_up, pairs) and K.moe_streams(self.w_down, pairs) and ring_pays(x.shape[0], s.top_k, s.n_experts):
+        if not grouped_pays(x.shape[0], s.top_k, s.n_experts, expert_bytes):
             return False
-        return grouped_pays(x.shape[0], s.top_k, s.n_experts, expert_bytes) and self._paired(x, 0)
+        pairs = x.shape[0] * s.top_k
+        if ring_pays(x.shape[0], s.top_k, s.n_experts) and K.moe_streams(self.w_gate_up, pairs) and K.moe_streams(self.w_down, pairs):
+            return False
+        return self._paired(x, 0)
 
     def _router_args(self):
         s = self.spec
