@@ -53,8 +53,9 @@ MOE_GROUPED_MIN_ROWS = 3
 MOE_GROUPED_ROWS_SET = os.environ.get("PRELUDE_MOE_GROUPED_MIN_ROWS")
 # where a step of few rows leaves the streaming kernel (``grouped_pays``): what a repeated read is counted as, and the bytes
 GROUPED_FIRST_READS, GROUPED_MIN_BYTES = 1.75, 150e6
-# rows of an expert that one walk over its matrices serves in the kernel with a ring, and experts with more than these from which it is left
-STREAM_ROWS, RING_MOST_READ_TWICE = 8, 0.003
+# rows of an expert that one walk over its matrices serves in the kernel with a ring; how many experts with more than these an even router may be
+# expected to make of a step, and how likely an expert of three times the average may get them, before the ring is left
+STREAM_ROWS, RING_EVEN_LIMIT, RING_HOT_LIMIT = 8, 0.003, 0.1
 
 
 def grouped_pays(tokens: int, top_k: int, n_experts: int, expert_bytes: int) -> bool:
@@ -72,28 +73,28 @@ def grouped_pays(tokens: int, top_k: int, n_experts: int, expert_bytes: int) -> 
 
 
 @functools.lru_cache(maxsize=1024)
-def read_twice(tokens: int, top_k: int, n_experts: int) -> float:
-    """How many experts an even router is expected to give more than eight of a step's tokens."""
-    p = top_k / n_experts
-    if tokens <= STREAM_ROWS or p >= 1.0:
-        return 0.0 if tokens <= STREAM_ROWS else float(n_experts)
-    return n_experts * max(0.0, 1.0 - sum(math.comb(tokens, i) * p ** i * (1.0 - p) ** (tokens - i) for i in range(STREAM_ROWS + 1)))
+def nine_or_more(tokens: int, chance: float) -> float:
+    """How likely an expert that a token chooses with this chance gets more than eight of the tokens."""
+    if tokens <= STREAM_ROWS or chance >= 1.0:
+        return 0.0 if tokens <= STREAM_ROWS else 1.0
+    return max(0.0, 1.0 - sum(math.comb(tokens, i) * chance ** i * (1.0 - chance) ** (tokens - i) for i in range(STREAM_ROWS + 1)))
 
 
 def ring_pays(tokens: int, top_k: int, n_experts: int) -> bool:
     """Whether a step that ``grouped_pays`` would send to the grouped products stays on the kernel that streams rows of 768 elements and more through
-    a ring (``moe_stream.cu``).  That one reads an expert once for eight tokens; where one has more, the block that walks it again takes
-    twice as long and the others wait, so the line is where an expert with nine tokens is still an exception.
+    a ring (``moe_stream.cu``).  That one reads an expert once for eight tokens; where one has more, the blocks that walk it again take
+    twice as long and the others wait.  So it is where an even router makes an expert with nine tokens an exception, and where an
+    expert that three times as many tokens as the average choose seldom gets them either.
 
     The whole feed-forward at 8 to 128 experts of 1,024 x 1,024 to 7,168 x 2,048, top 2 to 8, with and without a gate, 2 to 64 tokens, weights from memory
     (2,868 steps), us, streamed / grouped: 64 experts of 4,096 x 2,048, top 6, gated, 16 tokens 383 / 438; 64 of 3,072 x 1,536, top 8, gated, 10 tokens
     206 / 247; 32 of 2,048 x 2,048, top 4, no gate, 16 tokens 80 / 96; beyond the line 64 of 3,072 x 1,536, 24 tokens 266 / 306, 32 tokens 439 / 321.  Of
-    the 2,580 steps with more than eight experts 211 stay for it and take 0.86 of the time; 3 of them take up to 3 % more.  The better side of
-    every step would take 0.96 of the time of all, this rule takes 0.985: a later line gains more on the whole but loses up to 28 % where an
-    expert does get nine.
+    the 2,580 steps with more than eight experts 184 stay for it and take 0.87 of the time, 3 of them up to 1.03.  What a hot expert costs, the first and
+    the third of these without their routers: eight tokens at one expert 468 / 413 and 99 / 86, nine 591 / 414 and 125 / 90.
     With up to eight experts the line stays where it was, held by tests of both of its sides, though streaming gains most there (8 of 3,072 x 1,536, top 2,
     12 tokens 47 / 76)."""
-    return n_experts > 8 and read_twice(tokens, top_k, n_experts) < RING_MOST_READ_TWICE
+    even = top_k / n_experts
+    return n_experts > 8 and n_experts * nine_or_more(tokens, even) < RING_EVEN_LIMIT and nine_or_more(tokens, 3.0 * even) < RING_HOT_LIMIT
 
 
 # an activation's name: (two matrices on the way up or one, its number in the products' epilogues)
