@@ -8,10 +8,11 @@
 // bulk copy a row), eight warps multiply on the tensor cores with the weights as the row operand, their sums meet in shared memory.
 // What differs:
 //  * The rows to stream are those of the chosen experts: every block counts the choices for itself, lists the experts that were hit in
-//    ascending order and takes its equal share of all their rows, in units of 8 features; a share may span experts.
+//    ascending order, one with more than eight rows of A once for every eight, and takes its equal share of all their rows, in units of 8
+//    features; a share may span experts.  (With the eights of an expert walked by the blocks that have its share, those take twice as long and all wait:
+//    a feed-forward of 64 experts of 4,096 x 2,048, top 6, 12 tokens, nine of them at one expert, 522 us; here 309, the kernel in moe.cu 377.)
 //  * The column operand are up to eight rows of A, those that chose the expert at hand.  Where all rows of A fit they lie in shared
-//    memory from the start, else those of the next expert are asked for while one is worked on (two buffers where two fit).  An
-//    expert with more than eight rows is walked again for the next eight.
+//    memory from the start, else those of the next expert are asked for while one is worked on (two buffers where two fit).
 //  * Which rows come first is known only when the router is done, so nothing is fetched ahead of the wait for the kernel before - but by
 //    the second of two such products in a row, which finds the choices settled: the first one lets the kernel behind it begin only when
 //    it has itself waited, so that a block fills its ring while other multiprocessors are still at the first product.  The experts of 8 rows,
@@ -58,10 +59,11 @@ struct MsLayout {
                          slots = hits + MS_SLOTS * 4, x = slots + 4 * MS_ROWS * 4;
 };
 
-// One block's share: which experts, which of their features, how many passes over them; the loaders and the others walk it alike.
+// One block's share: which entries of the list (an expert, the eight of its rows), which of their features; the loaders and the others walk it alike.
 struct MsWalk {
-    int hit, pass, passes, f0, f1;
+    int hit, f0, f1;
 };
+#define MS_EIGHT 16                             // an entry: the expert, and from this bit on which eight of its rows
 
 __global__ void __launch_bounds__(MS_THREADS, 1) moe_stream_kernel(MsParams p) {
     extern __shared__ __align__(128) unsigned char ms_sm[];
@@ -98,15 +100,26 @@ __global__ void __launch_bounds__(MS_THREADS, 1) moe_stream_kernel(MsParams p) {
     if (warp == 0) {
         int n = 0;
         for (int e0 = 0; e0 < p.n_experts; e0 += 32) {
-            const bool hit = e0 + lane < p.n_experts && count[e0 + lane] > 0;
-            const unsigned who = __ballot_sync(0xffffffffu, hit);
-            if (hit) hits[n + __popc(who & ((1u << lane) - 1u))] = e0 + lane;
-            n += __popc(who);
+            const int eights = e0 + lane < p.n_experts ? (count[e0 + lane] + MS_ROWS - 1) / MS_ROWS : 0;
+            if (!__any_sync(0xffffffffu, eights > 1)) {
+                const unsigned who = __ballot_sync(0xffffffffu, eights > 0);
+                if (eights) hits[n + __popc(who & ((1u << lane) - 1u))] = e0 + lane;
+                n += __popc(who);
+            } else {
+                int upto = eights;                             // of this lane's expert and those before it
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int v = __shfl_up_sync(0xffffffffu, upto, o);
+                    if (lane >= o) upto += v;
+                }
+                for (int i = 0; i < eights; ++i) hits[n + upto - eights + i] = (e0 + lane) | (i << MS_EIGHT);
+                n += __shfl_sync(0xffffffffu, upto, 31);
+            }
         }
         if (lane == 0) s_hits = n;
     }
     __syncthreads();
-    const int units = (p.N + MS_ROWS - 1) / MS_ROWS;           // of one expert
+    const int units = (p.N + MS_ROWS - 1) / MS_ROWS;           // of one entry
     const long long all = (long long)s_hits * units;
     const long long u0 = blockIdx.x * all / gridDim.x, u1 = (blockIdx.x + 1) * all / gridDim.x;
     if (u0 >= u1) {
@@ -118,20 +131,19 @@ __global__ void __launch_bounds__(MS_THREADS, 1) moe_stream_kernel(MsParams p) {
         MsWalk w;
         const long long base = (long long)hit * units;
         w.hit = hit;
-        w.pass = 0;
-        w.passes = (count[hits[hit]] + MS_ROWS - 1) / MS_ROWS;
         w.f0 = (int)(max(u0 - base, 0ll)) * MS_ROWS;
         w.f1 = min((int)min(u1 - base, (long long)units) * MS_ROWS, p.N);
         return w;
     };
     const int first_hit = (int)(u0 / units), last_hit = (int)((u1 - 1) / units);
-    // to the next pass or the next expert; false: there is none
+    // to the next entry; false: there is none
     auto next = [&](MsWalk& w) {
-        if (++w.pass < w.passes) return true;
-        if (w.hit == last_hit) { w.pass = w.passes; return false; }
+        if (w.hit == last_hit) return false;
         w = open(w.hit + 1);
         return true;
     };
+    auto expert_of = [&](const MsWalk& w) { return hits[w.hit] & ((1 << MS_EIGHT) - 1); };
+    auto first_row = [&](const MsWalk& w) { return (hits[w.hit] >> MS_EIGHT) * MS_ROWS; };
 
     if (warp >= MS_WARPS) {
         // ---------------- loaders: the warps take the stages in turn, a lane copies a row ----------------
@@ -142,7 +154,7 @@ __global__ void __launch_bounds__(MS_THREADS, 1) moe_stream_kernel(MsParams p) {
         int stage = 0, phase = 0, i = 0, turn = 0;
         MsWalk w = open(first_hit);
         do {
-            const __nv_bfloat16* We = p.W + (size_t)hits[w.hit] * p.w_expert_stride;
+            const __nv_bfloat16* We = p.W + (size_t)expert_of(w) * p.w_expert_stride;
 #pragma unroll 1
             for (int f = w.f0; f < w.f1 && ok; f += span) {
                 const int halves = (p.gated || w.f1 - f > MS_ROWS) ? 2 : 1;
@@ -181,17 +193,17 @@ __global__ void __launch_bounds__(MS_THREADS, 1) moe_stream_kernel(MsParams p) {
     // the slots of a segment, and its rows of A on their way (warp 0): segment n uses slot list n % 4 and, where the rows do not all stay, buffer
     // n % bufs, which nobody reads any more
     auto stage_rows = [&](const MsWalk& w, int n) {
-        const int e = hits[w.hit];
+        const int e = expert_of(w), first = first_row(w);
         int found = 0;
         for (int s0 = 0; s0 < p.n_slots; s0 += 32) {
             const bool mine = s0 + lane < p.n_slots && ids[s0 + lane] == e;
             const unsigned who = __ballot_sync(0xffffffffu, mine);
-            const int at = found + __popc(who & ((1u << lane) - 1u)) - w.pass * MS_ROWS;
+            const int at = found + __popc(who & ((1u << lane) - 1u)) - first;
             if (mine && at >= 0 && at < MS_ROWS) slots[(n & 3) * MS_ROWS + at] = s0 + lane;
             found += __popc(who);
         }
         __syncwarp();
-        const int rows = min(MS_ROWS, found - w.pass * MS_ROWS), buf = resident ? 0 : n % p.bufs;
+        const int rows = min(MS_ROWS, found - first), buf = resident ? 0 : n % p.bufs;
         if (resident && n > 0) return;
         const int bring = resident ? p.n_src : rows;
         if (lane == 0) mbar_arrive_expect_tx(&x_bar[buf], (unsigned)bring * p.K * 2);
@@ -225,7 +237,7 @@ __global__ void __launch_bounds__(MS_THREADS, 1) moe_stream_kernel(MsParams p) {
                 if (lane == 0) { *(volatile int*)&s_dead = 1; if (p.status) atomicExch(p.status, 13); }
             }
         }
-        const int rows = min(MS_ROWS, count[hits[w.hit]] - w.pass * MS_ROWS);
+        const int rows = min(MS_ROWS, count[expert_of(w)] - first_row(w));
         const int* mine_slots = slots + (n & 3) * MS_ROWS;
         // warp 0 wrote the list before it arrived at the barrier just waited for, or before those of the tiles of the segment before
         const int m_row = min(lane & 7, rows - 1);

@@ -74,6 +74,23 @@ def test_experts_streamed(T, top, E, N, K_, gated, act, slots):
         assert torch.equal(K.moe_gemv(a[1:2], w, ids[1:2].contiguous(), False, torch.float32, **kw), got[top:2 * top])
 
 
+# one expert with many rows beside others with few: its eights are dealt like experts
+@pytest.mark.parametrize("T,top,E,N,K_", [(9, 1, 3, 40, 768), (40, 8, 33, 264, 1040), (64, 8, 64, 136, 2048), (128, 4, 1024, 24, 784), (100, 2, 2, 700, 4096)])
+def test_experts_with_many_rows(T, top, E, N, K_):
+    from prelude_b200.ops import kernels as K
+    w, a = rnd(E, N, K_, scale=K_ ** -0.5), rnd(T, K_, seed=3)
+    g = torch.Generator(device=DEV).manual_seed(7)
+    ids = torch.stack([torch.randperm(E, generator=g, device=DEV)[:top] for _ in range(T)]).int()
+    hot = E // 2
+    ids[: T - 3, 0] = torch.where((ids[: T - 3] == hot).any(1), ids[: T - 3, 0], hot)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    got = K.moe_gemv(a, w, ids, False, torch.float32, status=status)
+    for t in range(T):                               # each token's result is what it is alone
+        assert torch.equal(K.moe_gemv(a[t:t + 1], w, ids[t:t + 1].contiguous(), False, torch.float32), got[t * top:t * top + top])
+    want = torch.stack([w[e].double() @ a[i // top].double() for i, e in enumerate(ids.flatten().tolist())])
+    assert float((got.double() - want).norm() / want.norm()) < 2.0 ** -25 * (4 + (K_ / 512 + 1) / 2 + 3) ** 0.5 and int(status) == 0
+
+
 # a pair, the second of which reads the choices before the first has ended: resident rows, rows that move, blocks without a share
 @pytest.mark.parametrize("T,top,E,N,K_", [(1, 1, 2, 768, 784), (8, 4, 32, 2048, 2048), (40, 8, 64, 1024, 768), (3, 8, 1024, 800, 1040)])
 def test_second_product_begins_early(T, top, E, N, K_):
