@@ -24,8 +24,6 @@ first tensor.
 """
 from __future__ import annotations
 
-import functools
-import math
 import os
 from typing import Dict
 
@@ -53,9 +51,8 @@ MOE_GROUPED_MIN_ROWS = 3
 MOE_GROUPED_ROWS_SET = os.environ.get("PRELUDE_MOE_GROUPED_MIN_ROWS")
 # where a step of few rows leaves the streaming kernel (``grouped_pays``): what a repeated read is counted as, and the bytes
 GROUPED_FIRST_READS, GROUPED_MIN_BYTES = 1.75, 150e6
-# rows of an expert that one walk over its matrices serves in the kernel with a ring; how many experts with more than these an even router may be
-# expected to make of a step, and how likely an expert of three times the average may get them, before the ring is left
-STREAM_ROWS, RING_EVEN_LIMIT, RING_HOT_LIMIT = 8, 0.003, 0.1
+# experts above which ``ring_pays`` decides
+RING_MORE_EXPERTS = 16
 
 
 def grouped_pays(tokens: int, top_k: int, n_experts: int, expert_bytes: int) -> bool:
@@ -72,29 +69,19 @@ def grouped_pays(tokens: int, top_k: int, n_experts: int, expert_bytes: int) -> 
     return (tokens * top_k - GROUPED_FIRST_READS * hit) * expert_bytes >= GROUPED_MIN_BYTES
 
 
-@functools.lru_cache(maxsize=1024)
-def nine_or_more(tokens: int, chance: float) -> float:
-    """How likely an expert that a token chooses with this chance gets more than eight of the tokens."""
-    if tokens <= STREAM_ROWS or chance >= 1.0:
-        return 0.0 if tokens <= STREAM_ROWS else 1.0
-    return max(0.0, 1.0 - sum(math.comb(tokens, i) * chance ** i * (1.0 - chance) ** (tokens - i) for i in range(STREAM_ROWS + 1)))
-
-
-def ring_pays(tokens: int, top_k: int, n_experts: int) -> bool:
+def ring_pays(tokens: int, top_k: int, n_experts: int, shortest_row: int) -> bool:
     """Whether a step that ``grouped_pays`` would send to the grouped products stays on the kernel that streams rows of 768 elements and more through
-    a ring (``moe_stream.cu``).  That one reads an expert once for eight tokens; where one has more, the blocks that walk it again take
-    twice as long and the others wait.  So it is where an even router makes an expert with nine tokens an exception, and where an
-    expert that three times as many tokens as the average choose seldom gets them either.
+    a ring (``moe_stream.cu``; ``shortest_row``: of the two matrices).  That one reads an expert once for eight tokens, whatever the router does, and has
+    neither sort nor gather nor their latencies, so it stays ahead over all steps of few rows (six an expert) - but for short rows, where the ends of
+    its tiles and not the bytes bound it, once so many pairs hit so many experts that the other way's beginning is paid for.
 
     The whole feed-forward at 8 to 128 experts of 1,024 x 1,024 to 7,168 x 2,048, top 2 to 8, with and without a gate, 2 to 64 tokens, weights from memory
-    (2,868 steps), us, streamed / grouped: 64 experts of 4,096 x 2,048, top 6, gated, 16 tokens 383 / 438; 64 of 3,072 x 1,536, top 8, gated, 10 tokens
-    206 / 247; 32 of 2,048 x 2,048, top 4, no gate, 16 tokens 80 / 96; beyond the line 64 of 3,072 x 1,536, 24 tokens 266 / 306, 32 tokens 439 / 321.  Of
-    the 2,580 steps with more than eight experts 184 stay for it and take 0.87 of the time, 3 of them up to 1.03.  What a hot expert costs, the first and
-    the third of these without their routers: eight tokens at one expert 468 / 413 and 99 / 86, nine 591 / 414 and 125 / 90.
-    With up to eight experts the line stays where it was, held by tests of both of its sides, though streaming gains most there (8 of 3,072 x 1,536, top 2,
-    12 tokens 47 / 76)."""
-    even = top_k / n_experts
-    return n_experts > 8 and n_experts * nine_or_more(tokens, even) < RING_EVEN_LIMIT and nine_or_more(tokens, 3.0 * even) < RING_HOT_LIMIT
+    (2,868 steps), us, streamed / grouped: 64 experts of 4,096 x 2,048, top 6, gated, 16 tokens 381 / 437, 32 tokens 457 / 525; 32 of 2,048 x 2,048, top 4, no
+    gate, 24 tokens 90 / 115, 40 tokens 104 / 121; 64 of 2,048 x 768, top 8, no gate, 16 tokens 89 / 88, 48 tokens 116 / 100; 128 of them, gated, 64 tokens
+    247 / 228.  With more than 16 experts 630 of 2,004 steps stay for it and take 0.91 of the time; 12 of them take up to 1.07.  The better side of every
+    step would take 0.953 of the time, this rule takes 0.956.  With up to 16 experts the line stays where it was, held by tests of both of its
+    sides, though streaming gains most there (8 of 3,072 x 1,536, top 2, 12 tokens 48 / 76; 434 steps would take 0.82 of the time)."""
+    return n_experts > RING_MORE_EXPERTS and (shortest_row > 1024 or n_experts < 64 or tokens * top_k < 192)
 
 
 # an activation's name: (two matrices on the way up or one, its number in the products' epilogues)
@@ -199,7 +186,7 @@ class RoutedExperts:
         if not grouped_pays(x.shape[0], s.top_k, s.n_experts, expert_bytes):
             return False
         pairs = x.shape[0] * s.top_k
-        if ring_pays(x.shape[0], s.top_k, s.n_experts) and K.moe_streams(self.w_gate_up, pairs) and K.moe_streams(self.w_down, pairs):
+        if ring_pays(x.shape[0], s.top_k, s.n_experts, min(s.hidden_size, s.expert_size)) and K.moe_streams(self.w_gate_up, pairs) and K.moe_streams(self.w_down, pairs):
             return False
         return self._paired(x, 0)
 
