@@ -1385,7 +1385,8 @@ struct MoeSumArgs {
     int n_out, n_tokens, top, width;
 };
 
-template <typename TY, typename TS, typename TO, int V>
+// AT: choices' rows in flight, as they lie in memory
+template <typename TY, typename TS, typename TO, int V, int AT>
 __global__ void __launch_bounds__(256) moe_sum_kernel(const TY* y, const TS* shared, TO* out, MoeSumArgs a) {
     pb_grid_dep_launch();
     const int i = blockIdx.x, col = (blockIdx.y * blockDim.x + threadIdx.x) * V;
@@ -1402,9 +1403,6 @@ __global__ void __launch_bounds__(256) moe_sum_kernel(const TY* y, const TS* sha
     float r[V];
     float* rp = a.res ? a.res + (size_t)t * a.width + col : nullptr;
     if (rp) moe_ldv<V>(rp, r);
-    // the choices' rows in flight, as they lie in memory: eight of 16 bytes, four of 32 (2,048 tokens of 4,096, six bfloat16 choices from memory, us:
-    // 45 -> 31; four at a time, unpacked, kept half the registers' worth in flight)
-    constexpr int AT = sizeof(TY) * V <= 16 ? 8 : 4;
     for (int c0 = 0; c0 < a.top; c0 += AT) {
         MoeRaw<TY, V> raw[AT];
         float w[AT];
@@ -1463,10 +1461,18 @@ PB_API int pb_moe_sum(const void* y, int y_dtype, const int32_t* place_of, const
     PB_REQUIRE((pieces + threads - 1) / threads < 65536, "moe_sum: rows of %d", width);
     const dim3 grid(n_out, (pieces + threads - 1) / threads);
     const MoeSumArgs a{place_of, weights, shared_parts, (size_t)shared_stride, res, rows, gain, shift, slope, n_out, n_tokens, top, width};
-#define MOE_SUM(TY, TS, TO)                                                                                                        \
-    do {                                                                                                                           \
-        if (vec) pb_launch(moe_sum_kernel<TY, TS, TO, (sizeof(TO) == 2 ? 8 : 4)>, grid, dim3(threads), 0, stream, (const TY*)y, (const TS*)shared, (TO*)out, a); \
-        else pb_launch(moe_sum_kernel<TY, TS, TO, 1>, grid, dim3(threads), 0, stream, (const TY*)y, (const TS*)shared, (TO*)out, a);     \
+    // As many rows in flight as there are choices, up to eight of 16 bytes or four of 32: more than there are only cost registers, and by them warps.
+    // bfloat16 choices from memory, us, four at a time and unpacked / eight at a time whatever their number / as now: 2,048 tokens of 4,096, six choices
+    // 45 / 31 / 31; 4,096 tokens of 2,880, one choice 16.6 / 31.6 / 15.7, two 22.1 / 32.6 / 17.4; 1,000 tokens, four 8.6 / 9.8 / 6.8.
+#define MOE_SUM_AT(TY, TS, TO, VV, AT) \
+    pb_launch(moe_sum_kernel<TY, TS, TO, VV, AT>, grid, dim3(threads), 0, stream, (const TY*)y, (const TS*)shared, (TO*)out, a)
+#define MOE_SUM(TY, TS, TO)                                                                             \
+    do {                                                                                                \
+        constexpr int VV = sizeof(TO) == 2 ? 8 : 4, MOST = sizeof(TY) * VV <= 16 ? 8 : 4;               \
+        if (!vec) MOE_SUM_AT(TY, TS, TO, 1, 4);                                                         \
+        else if (top <= 2) MOE_SUM_AT(TY, TS, TO, VV, 2);                                               \
+        else if (top <= 4) MOE_SUM_AT(TY, TS, TO, VV, 4);                                               \
+        else MOE_SUM_AT(TY, TS, TO, VV, MOST);                                                          \
     } while (0)
     if (dtype == PB_F32) MOE_SUM(float, float, float);
     else if (dtype == PB_BF16) {
@@ -1477,6 +1483,7 @@ PB_API int pb_moe_sum(const void* y, int y_dtype, const int32_t* place_of, const
         return pb_fail("moe_sum: unknown element type code %d", dtype);
     }
 #undef MOE_SUM
+#undef MOE_SUM_AT
     PB_CHECK_LAUNCH("moe_sum");
     return 0;
 }

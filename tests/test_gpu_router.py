@@ -70,7 +70,8 @@ def test_grouping(T, top, E):
     assert got[:len(tiles)] == tiles and all(e == -1 for e, _ in got[len(tiles):])
 
 
-@pytest.mark.parametrize("T,top,width,y32", [(5, 3, 64, True), (9, 6, 4096, False), (70, 8, 520, False), (70, 9, 520, True), (3, 17, 100, False)])
+@pytest.mark.parametrize("T,top,width,y32", [(5, 3, 64, True), (9, 6, 4096, False), (70, 8, 520, False), (70, 9, 520, True), (3, 17, 100, False),
+                                             (300, 1, 2880, False), (40, 2, 512, False), (5, 1, 512, True), (33, 4, 2048, False), (7, 5, 2048, False)])
 def test_weighted_sum(T, top, width, y32):
     from prelude_b200.ops import kernels as K
     g = torch.Generator(device=DEV).manual_seed(top)
