@@ -588,9 +588,11 @@ PB_API int pb_moe_route_tokens(const void* x, long long ldx, const void* W, int 
 // tile_expert, tile_row0 [max_tiles], max_tiles >= ceil(n_slots / MOE_BM) + n_experts.
 // What bounds it: trips to memory one behind the other, and a shared counter per choice.  So every block of the cluster takes an equal run
 // of the choices, asks for all of a thread's (up to MOE_SORT_HELD) at once, and counting them gives each its rank among its
-// expert's in the run; the blocks then read one another's counts.  12,288 choices of 64 experts 16 -> 4.8 us, 1,800 of them 4 by one block.
+// expert's in the run; the blocks then read one another's counts.  12,288 choices of 64 experts 16 -> 4.8 us; by one block 2,000 of 64
+// experts 6.9 -> 3.7, 128 of 8 2.3 either way.
 #define MOE_SORT_HELD 8
 #define MOE_SORT_CLUSTER 8
+template <bool CLUSTER>
 __global__ void __launch_bounds__(1024) moe_sort_kernel(const int32_t* ids, int n_slots, int n_experts,
                                                         int32_t* offsets, int32_t* order,
                                                         int32_t* place_of, int32_t* tile_expert,
@@ -599,8 +601,7 @@ __global__ void __launch_bounds__(1024) moe_sort_kernel(const int32_t* ids, int 
     __shared__ int count[MOE_MAX_EXPERTS];                   // of this block's choices
     __shared__ int cursor[MOE_MAX_EXPERTS];                  // of places handed out in chunks before
     __shared__ int start[MOE_MAX_EXPERTS + 1], mine[MOE_MAX_EXPERTS], tile0[MOE_MAX_EXPERTS + 1];
-    cg::cluster_group cluster = cg::this_cluster();
-    const int rank_in = (int)cluster.block_rank(), blocks = (int)cluster.num_blocks(), tid = threadIdx.x, threads = blockDim.x;
+    const int rank_in = CLUSTER ? (int)cg::this_cluster().block_rank() : 0, blocks = CLUSTER ? MOE_SORT_CLUSTER : 1, tid = threadIdx.x, threads = blockDim.x;
     for (int e = tid; e < n_experts; e += threads) count[e] = cursor[e] = 0;
     __syncthreads();
     pb_grid_dep_wait();
@@ -617,22 +618,25 @@ __global__ void __launch_bounds__(1024) moe_sort_kernel(const int32_t* ids, int 
         for (int j = 0; j < MOE_SORT_HELD; ++j) rank[j] = held[j] >= 0 ? atomicAdd(&counter[held[j]], 1) : 0;
     };
     for (int base = lo; base < hi; base += chunk) number(base, count);
-    cluster.sync();                                          // every block's counts are there
-    for (int e = tid; e < n_experts; e += threads) {
-        int total = 0, before = 0;
-        for (int r = 0; r < blocks; ++r) {
-            const int c = cluster.map_shared_rank(count, r)[e];
-            before += r < rank_in ? c : 0;
-            total += c;
+    if constexpr (CLUSTER) {
+        cg::cluster_group cluster = cg::this_cluster();
+        cluster.sync();                                      // every block's counts are there
+        for (int e = tid; e < n_experts; e += threads) {
+            int total = 0, before = 0;
+            for (int r = 0; r < blocks; ++r) {
+                const int c = cluster.map_shared_rank(count, r)[e];
+                before += r < rank_in ? c : 0;
+                total += c;
+            }
+            start[e] = total;
+            mine[e] = before;
         }
-        start[e] = total;
-        mine[e] = before;
     }
     __syncthreads();
     if (tid < 32) {
         int at = 0, tiles = 0;
         for (int e0 = 0; e0 < n_experts; e0 += 32) {
-            const int e = e0 + tid, n = e < n_experts ? start[e] : 0, nt = (n + tile_rows - 1) / tile_rows;
+            const int e = e0 + tid, n = e < n_experts ? (CLUSTER ? start[e] : count[e]) : 0, nt = (n + tile_rows - 1) / tile_rows;
             int sn = n, st = nt;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -653,7 +657,7 @@ __global__ void __launch_bounds__(1024) moe_sort_kernel(const int32_t* ids, int 
 #pragma unroll
         for (int j = 0; j < MOE_SORT_HELD; ++j) {
             if (held[j] < 0) continue;
-            const int i = base + j * threads + tid, place = start[held[j]] + mine[held[j]] + rank[j];
+            const int i = base + j * threads + tid, place = start[held[j]] + (CLUSTER ? mine[held[j]] : 0) + rank[j];
             order[place] = i;
             place_of[i] = place;
         }
@@ -673,7 +677,7 @@ __global__ void __launch_bounds__(1024) moe_sort_kernel(const int32_t* ids, int 
             }
         }
     }
-    cluster.sync();                                          // nobody leaves while others read its counts
+    if constexpr (CLUSTER) cg::this_cluster().sync();        // nobody leaves while others read its counts
 }
 
 // Rows of a tile: 128 where the experts have many rows each (prompt steps: the large-tile kernel), else 64.
@@ -685,20 +689,26 @@ PB_API int pb_moe_sort(const int32_t* ids, int n_slots, int n_experts, int32_t* 
     PB_REQUIRE(tile_rows == MOE_BM || tile_rows == MOE_BM_LARGE || tile_rows == 256, "moe_sort: tiles have %d, %d or 256 rows", MOE_BM, MOE_BM_LARGE);
     PB_REQUIRE(max_tiles >= (n_slots + tile_rows - 1) / tile_rows + n_experts, "moe_sort: room for %d tiles is too little", max_tiles);
     PB_REQUIRE(ids && offsets && order && place_of && tile_expert && tile_row0, "moe_sort: null pointer");
-    // a cluster of one block, or of eight where one block would hold two choices a thread and more
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = n_slots >= 2048 ? MOE_SORT_CLUSTER : 1;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.gridDim = dim3(attr[0].val.clusterDim.x);
-    cfg.blockDim = dim3(1024);
-    cfg.stream = stream;
-    cfg.attrs = attr;
-    cfg.numAttrs = pb_pdl_enabled() ? 2 : 1;
-    cudaLaunchKernelEx(&cfg, moe_sort_kernel, ids, n_slots, n_experts, offsets, order, place_of, tile_expert, tile_row0, max_tiles, tile_rows);
+    // one block, or a cluster of eight where one would hold two choices a thread and more
+    if (n_slots < 2048) {
+        // a thread a choice: with 1,024 threads the barriers alone are half a microsecond (128 choices of 8 experts 2.9 us, 2.3 with 128 threads)
+        const int threads = n_slots > 512 ? 512 : n_slots > 128 ? (n_slots + 31) / 32 * 32 : 128;
+        pb_launch(moe_sort_kernel<false>, dim3(1), dim3(threads), 0, stream, ids, n_slots, n_experts, offsets, order, place_of, tile_expert, tile_row0, max_tiles, tile_rows);
+    } else {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = MOE_SORT_CLUSTER;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.gridDim = dim3(MOE_SORT_CLUSTER);
+        cfg.blockDim = dim3(1024);
+        cfg.stream = stream;
+        cfg.attrs = attr;
+        cfg.numAttrs = pb_pdl_enabled() ? 2 : 1;
+        cudaLaunchKernelEx(&cfg, moe_sort_kernel<true>, ids, n_slots, n_experts, offsets, order, place_of, tile_expert, tile_row0, max_tiles, tile_rows);
+    }
     PB_CHECK_LAUNCH("moe_sort");
     return 0;
 }

@@ -55,7 +55,8 @@ def test_choices_by_a_plain_sort():
         assert ids[t].tolist() == order[:6]
 
 
-@pytest.mark.parametrize("T,top,E", [(1, 1, 1), (7, 6, 64), (341, 6, 64), (342, 6, 64), (2048, 6, 64), (1000, 8, 1024), (12000, 6, 40)])
+@pytest.mark.parametrize("T,top,E", [(1, 1, 1), (7, 6, 64), (341, 6, 64), (342, 6, 64), (2048, 6, 64), (1000, 8, 1024), (12000, 6, 40), (64, 2, 4), (129, 1, 8),
+                                      (256, 2, 9), (513, 1, 300), (2047, 1, 5), (2048, 1, 5)])
 def test_grouping(T, top, E):
     from prelude_b200.ops import kernels as K
     ids = torch.randint(0, E, (T, top), generator=torch.Generator(device=DEV).manual_seed(T), device=DEV).int()
