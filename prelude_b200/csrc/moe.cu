@@ -549,11 +549,19 @@ moe_route_tokens_kernel(const __nv_bfloat16* x, long long ldx, const __nv_bfloat
         moe_route_token<SLOTS>(z + t * E, args, ids + (size_t)(t0 + t) * args.top, weights + (size_t)(t0 + t) * args.top);
 }
 
-// Whether pb_moe_route_tokens takes the sizes.  Rows of 64 would be less exact here (4.3e-8 against 4.0e-8); fewer tokens than 64 take no longer on
-// the kernels above, nor do eight experts once the blocks of 16 tokens make a second wave over the multiprocessors (K 1,024, 4,096 tokens: 9.6 us
-// against 8.9).
+// Whether pb_moe_route_tokens takes the sizes: where it is the faster way, and no less exact (rows of 64: 4.3e-8 against 4.0e-8).  A wave of its blocks, one
+// of 16 tokens a multiprocessor, takes as long for one expert as for 64, 3.9 us and 1.5 for every 1,024 of K; the kernels above take as long as
+// there are products.  us, above / here: 16 experts, K 1,024: 400 tokens 5.4 / 5.7, 800 6.1 / 5.7, 2,368 9.6 / 5.8, 2,400 (two waves) 10.1 / 10.4, 16,384
+// 27.5 / 36.7; K 2,048: 64 tokens 6.9 / 6.7, 16,384 46.4 / 46.4; 32 experts, K 1,024: 400 tokens 5.7 / 5.6, 16,384 47.4 / 36.9; 8 experts, K 4,096: 2,368 tokens
+// 12.6 / 10.0, 4,736 15.0 / 19.3; 64 experts, K 128: 16,384 tokens 37 / 30.  Over 1,248 steps of 64 to 16,384 tokens, 2 to 64 experts, K 128 to 4,096: 1.01 of
+// what the faster way of each would take.
+#define RT_WAVE_PRODUCTS 15000000                            // of a single wave of short rows
 PB_API int pb_moe_route_tokens_supported(int n_tokens, int n_experts, int K) {
-    return n_tokens >= RT_MIN_TOKENS && K % 32 == 0 && K >= RT_MIN_K && (n_experts > 8 || n_tokens <= pb_multiprocessors() * RT_TOKENS) ? 1 : 0;
+    if (n_tokens < RT_MIN_TOKENS || K % 32 != 0 || K < RT_MIN_K) return 0;
+    if (n_experts > RT_EXPERTS) return 1;
+    if (n_tokens <= pb_multiprocessors() * RT_TOKENS)
+        return K >= 2048 || (long long)n_tokens * (n_experts > 8 ? n_experts : 8) * K >= RT_WAVE_PRODUCTS ? 1 : 0;
+    return n_experts == RT_EXPERTS || (n_experts > 8 && n_experts * K >= 32768) ? 1 : 0;
 }
 
 // x [n_tokens, K] with row stride ldx, W [n_experts, K], both bfloat16; logits float32 [n_tokens, n_experts], null with up to 64 experts if

@@ -196,8 +196,8 @@ class RoutedExperts:
                 s.renormalize_eps, s.weight_scale, self.router_bias, s.scoring == "softmax_chosen")
 
     def route(self, x: torch.Tensor):
-        """(experts int32 [T, top_k], weights float32 [T, top_k]) for the rows of x.  From 64 rows of bfloat16 on the logits are summed in another
-        order, so a token's choice may depend on the step's size where two experts' scores tie within roundings."""
+        """(experts int32 [T, top_k], weights float32 [T, top_k]) for the rows of x.  From 64 rows of bfloat16 on the logits may be summed in another
+        order (``kernels.moe_route_tokens_takes``), so a token's choice may depend on the step's size where two experts' scores tie within roundings."""
         if x.shape[0] <= ROUTE_FEW_TOKENS and K.moe_route_few_takes(x, self.w_router):
             return K.moe_route_few(x, self.w_router, *self._router_args())
         if K.moe_route_tokens_takes(x, self.w_router):

@@ -7,7 +7,7 @@ from prelude_b200.ops import kernels as K
 from prelude_b200.parts import model as _registers_the_parts  # noqa: F401
 from prelude_b200.parts.registry import RunContext, make_part
 
-WIDTH, E = 128, 8
+WIDTH, E = 2048, 8
 
 
 @pytest.fixture
@@ -62,3 +62,13 @@ def test_routed_experts_refuse_rows_of_another_width(rows, width, launched):
     assert launched == []
     part.route(torch.zeros(rows, WIDTH, dtype=torch.bfloat16))
     assert launched[0] == {8: "pb_moe_route_few", 40: "pb_router_logits", 64: "pb_moe_route_tokens"}[rows]
+
+
+# one wave of blocks: long rows, or products enough; more waves: many experts with long rows, or a whole block's worth of experts
+@pytest.mark.parametrize("tokens,experts,width,taken", [
+    (63, 64, 4096, False), (64, 2, 2048, True), (64, 8, 1024, False), (1600, 16, 1024, True), (800, 16, 512, False), (1600, 24, 512, True), (64, 65, 128, True), (64, 64, 96, False),
+    (2368, 8, 4096, True), (2369, 8, 4096, False), (2369, 9, 4096, True), (16384, 16, 1024, False), (16384, 32, 1024, True), (16384, 64, 128, True)])
+def test_where_the_tensor_cores_router_pays(tokens, experts, width, taken):
+    if torch.cuda.is_available() and torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the waves are those of 148 multiprocessors")
+    assert bool(K._l.library().pb_moe_route_tokens_supported(tokens, experts, width)) == taken
