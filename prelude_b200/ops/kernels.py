@@ -1148,8 +1148,11 @@ def _longest_first(batch, part: _Split) -> Tuple[int, int]:
     n = batch.q_lens.shape[0]
     if not part.counted or part.least != 1 or part.n_long != n or not 0 < n <= 16:
         return 0, 0
-    lens = [int(v) for v in batch.q_lens]
-    order = sum(r << (4 * i) for i, r in enumerate(sorted(range(n), key=lambda r: -lens[r])))
+    if n == 1:
+        return 0, int(batch.q_lens[0])
+    lens, order = batch.q_lens.tolist(), 0
+    for r in sorted(range(n), key=lens.__getitem__):         # the shortest ends up in the highest bits
+        order = order << 4 | r
     return order - (1 << 64 if order >> 63 else 0), max(lens)
 
 
