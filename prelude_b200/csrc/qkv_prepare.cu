@@ -228,7 +228,10 @@ __global__ void qkv_prepare_staged_kernel(const T* q_in, long long ldq, const T*
 // key row, its norm included, is a warp's of its own.  One barrier, for the token's angles.  Heads, split points and the rotated span in
 // whole pieces.  What bounds it is the chain of trips to memory, which was four long where the partners and the key row were asked for behind the
 // barrier.  (Through shared memory as float32: 1,500 tokens of 16 x 192 queries and rows of 576 24.6 us, with the partners behind the
-// barrier 15.5; 16 tokens of 32 x 192 11.4 and 8.1.  What the kernel adds to a layer's time, partners behind it / here: 13.2 / 12.3 and 5.8 / 4.9.)
+// barrier 15.5; 16 tokens of 32 x 192 11.4 and 8.1.  What the kernel adds to a layer's time, partners behind it / here: 13.2 / 12.3 and 5.8 / 4.9.
+// In a row of its kind, rows of 576 with their norm, partners behind the barrier / ahead of it with divisions as they are and three pieces of the
+// key row a lane / here: 8 x 192, 1 token 3.1 / 3.3 / 3.0, 4,000 tokens 17.0 / 18.7 / 16.3; 16 x 192, 3.7 / 3.3 / 3.2 and 20.9 / 20.1 / 18.0; 32 x 192,
+// 4.7 / 3.5 / 3.9 and 38.3 / 32.6 / 31.1.)
 #define QP_MOST 4                                          // pieces of queries a thread holds at most
 template <typename T>
 __device__ __forceinline__ void qp_turn(uint4& own, const uint4& other, int rel, const RotArgs& r, const float* cs) {
@@ -253,13 +256,22 @@ __device__ __forceinline__ void qp_turn(uint4& own, const uint4& other, int rel,
     qp_st_vec(reinterpret_cast<T*>(&own), a);
 }
 
+// i / n by a product with 2^32 / n rounded up, which is less than n / 2^32 too much for every i: exact where i n < 2^32 (rows of queries and keys that
+// take this kernel are below 2^14 elements; values: pb_qkv_prepare).  Divisions are most of what the loads ahead of the barrier add to a long step.
+struct QpDiv {
+    unsigned n, inv;
+    __host__ explicit QpDiv(int of) : n(of > 0 ? of : 1), inv(of > 1 ? (unsigned)((0x100000000ull + of - 1) / of) : 0) {}
+    __device__ __forceinline__ int quotient(int i) const { return n > 1 ? (int)__umulhi((unsigned)i, inv) : i; }
+};
+
 template <typename T, int QP>
-__global__ void __launch_bounds__(288)
+__global__ void __launch_bounds__(288, 4)
 qkv_prepare_direct_kernel(const T* q_in, long long ldq, const T* k_in, long long ldk, const T* v_in, long long ldv, const float* k_w, int k_norm_cols,
                           float eps, RotArgs rot, int q_rot_off, int k_rot_off, const int32_t* positions, const int32_t* table_row, const int32_t* block_table,
                           int table_stride, int page_size, int num_pages, T* q_out, int q_split, T* q_out2, long long q2_head_stride, long long q2_off,
-                          T* k_pages, T* v_pages, int H, int qd, int G, int kd, int Gv, int vd, int swizzle_k, int swizzle_v, int* status) {
+                          T* k_pages, T* v_pages, int H, QpDiv q_div, int G, QpDiv k_div, int Gv, QpDiv v_div, int swizzle_k, int swizzle_v, int* status) {
     constexpr int VN = 16 / sizeof(T);
+    const int qd = (int)q_div.n, kd = (int)k_div.n, vd = (int)v_div.n;
     extern __shared__ float cs[];                          // cosine and sine of the token's angles, times the amplitude
     pb_grid_dep_launch();
     pb_grid_dep_wait();
@@ -291,7 +303,7 @@ qkv_prepare_direct_kernel(const T* q_in, long long ldq, const T* k_in, long long
             mine[it] = other[it] = make_uint4(0, 0, 0, 0);
             if (i < nq) {
                 mine[it] = *reinterpret_cast<const uint4*>(q + i);
-                other[it] = partner(q + i, in_span(i % qd, q_rot_off));
+                other[it] = partner(q + i, in_span(i - q_div.quotient(i) * qd, q_rot_off));
             }
         }
         if (row < 0) return;                               // (the whole block)
@@ -300,14 +312,14 @@ qkv_prepare_direct_kernel(const T* q_in, long long ldq, const T* k_in, long long
         for (int it = 0; it < QP; ++it) {
             const int i = (tid + it * q_threads) * VN;
             if (i >= nq) break;
-            const int h = i / qd, d = i - h * qd, rel = in_span(d, q_rot_off);
+            const int h = q_div.quotient(i), d = i - h * qd, rel = in_span(d, q_rot_off);
             if (rel >= 0) qp_turn<T>(mine[it], other[it], rel, rot, cs);
             T* dst = d < q_split ? q_out + ((size_t)t * H + h) * q_split + d : q_out2 + ((size_t)t * H + h) * q2_head_stride + q2_off + (d - q_split);
             *reinterpret_cast<uint4*>(dst) = mine[it];
         }
     } else {
         const T* k = k_in + (size_t)t * ldk;
-        constexpr int KP = 3;                              // pieces a lane has before it looks at more
+        constexpr int KP = 2;                              // pieces a lane has before it looks at more
         uint4 key[KP], key_other[KP];
 #pragma unroll
         for (int j = 0; j < KP; ++j) {
@@ -315,7 +327,7 @@ qkv_prepare_direct_kernel(const T* q_in, long long ldq, const T* k_in, long long
             key[j] = key_other[j] = make_uint4(0, 0, 0, 0);
             if (i < nk) {
                 key[j] = *reinterpret_cast<const uint4*>(k + i);
-                key_other[j] = partner(k + i, in_span(i % kd, k_rot_off));
+                key_other[j] = partner(k + i, in_span(i - k_div.quotient(i) * kd, k_rot_off));
             }
         }
         if (row < 0) return;
@@ -340,7 +352,7 @@ qkv_prepare_direct_kernel(const T* q_in, long long ldq, const T* k_in, long long
         } else {
             const int in_page = p % page_size;
             auto put = [&](int i, uint4 own, const uint4& with) {
-                const int g = i / kd, d = i - g * kd, rel = in_span(d, k_rot_off);
+                const int g = k_div.quotient(i), d = i - g * kd, rel = in_span(d, k_rot_off);
                 if (k_w != nullptr && i < k_norm_cols) {       // (a rotated span that is normed is the general kernels' case)
                     float v[VN];
                     qp_ld_vec(reinterpret_cast<const T*>(&own), v);
@@ -355,7 +367,7 @@ qkv_prepare_direct_kernel(const T* q_in, long long ldq, const T* k_in, long long
 #pragma unroll
             for (int j = 0; j < KP; ++j)
                 if ((lane + 32 * j) * VN < nk) put((lane + 32 * j) * VN, key[j], key_other[j]);
-            for (int i = (lane + 32 * KP) * VN; i < nk; i += 32 * VN) put(i, *reinterpret_cast<const uint4*>(k + i), partner(k + i, in_span(i % kd, k_rot_off)));
+            for (int i = (lane + 32 * KP) * VN; i < nk; i += 32 * VN) put(i, *reinterpret_cast<const uint4*>(k + i), partner(k + i, in_span(i - k_div.quotient(i) * kd, k_rot_off)));
         }
     }
     if (nk == 0 || v_pages == nullptr || v_in == nullptr) return;
@@ -363,7 +375,7 @@ qkv_prepare_direct_kernel(const T* q_in, long long ldq, const T* k_in, long long
     if (page < 0 || page >= num_pages) return;                  // the key row's warp has raised the status
     const int in_page = p % page_size;
     for (int i = tid * VN; i < Gv * vd; i += blockDim.x * VN) {
-        const int g = i / vd, d0 = i - g * vd;
+        const int g = v_div.quotient(i), d0 = i - g * vd;
         T* dst = v_pages + (((size_t)page * Gv + g) * page_size + in_page) * vd;
         *reinterpret_cast<uint4*>(dst + pb_kv_elem_offset(d0, in_page, swizzle_v)) = *reinterpret_cast<const uint4*>(v_in + (size_t)t * ldv + i);
     }
@@ -416,7 +428,7 @@ PB_API int pb_qkv_prepare(const void* q_in, long long ldq, const void* k_in, lon
     auto whole = [&](int off) { return rates == nullptr || (off % vn == 0 && rot_dims % vn == 0 && (adjacent || (rot_dims / 2) % vn == 0)); };
     const int nk = k_pages ? G * kd : 0;
     bool direct = staged && q_w == nullptr && whole(q_rot_off) && H * qd <= QP_MOST * vn * 256 && (nk == 0 || whole(k_rot_off));
-    // queries written over what is read: the rotation partners, and of the key row three pieces a lane, are read ahead of the block's barrier, the
+    // queries written over what is read: the rotation partners, and of the key row two pieces a lane, are read ahead of the block's barrier, the
     // pieces of a longer key row after others have stored; the staged kernel has read both rows by then
     const size_t esz = dtype == PB_BF16 ? 2 : 4;
     auto meets = [&](const void* a, size_t a_elems, const void* b, size_t b_elems) {
@@ -428,6 +440,7 @@ PB_API int pb_qkv_prepare(const void* q_in, long long ldq, const void* k_in, lon
     const size_t out_elems[2] = {(size_t)n_tokens * H * q_split, (size_t)n_tokens * H * q2_head_stride};
     for (int i = 0; i < 2; ++i)
         direct = direct && !meets(q_in, q_elems, outs[i], out_elems[i]) && !(k_elems && meets(k_in, k_elems, outs[i], out_elems[i]));
+    direct = direct && (v_pages == nullptr || (long long)Gv * vd * vd < (1ll << 32));          // QpDiv
     if (direct && nk > 0 && k_w != nullptr && rates != nullptr)
         for (int g = 0; g < G; ++g) direct = direct && g * kd + k_rot_off >= k_norm_cols;
     if (direct) {
@@ -441,7 +454,7 @@ PB_API int pb_qkv_prepare(const void* q_in, long long ldq, const void* k_in, lon
     PB_DISPATCH_DTYPE(dtype, T,                                                                                               \
         (pb_launch(qkv_prepare_direct_kernel<T, QP>, dim3(n_tokens), dim3(block), (size_t)rot.dims * sizeof(float), stream, (const T*)q_in, ldq, \
                    (const T*)k_in, ldk, (const T*)v_in, ldv, k_w, k_norm_cols, eps, rot, q_rot_off, k_rot_off, positions, table_row, block_table, table_stride, \
-                   page_size, num_pages, (T*)q_out, q_split, (T*)q_out2, q2_head_stride, q2_off, (T*)k_pages, (T*)v_pages, H, qd, G, kd, Gv, vd, swizzle_k, \
+                   page_size, num_pages, (T*)q_out, q_split, (T*)q_out2, q2_head_stride, q2_off, (T*)k_pages, (T*)v_pages, H, QpDiv(qd), G, QpDiv(kd), Gv, QpDiv(vd), swizzle_k, \
                    swizzle_v, status)))
         if (each <= 1) DIRECT_LAUNCH(1);
         else if (each <= 2) DIRECT_LAUNCH(2);
