@@ -130,10 +130,13 @@ __global__ void __launch_bounds__(GS_THREADS, 1) gemm_stream_kernel(GsParams p) 
     const int span = p.gated ? GS_ROWS : 16;                   // features per tile
     const int n_tiles = (r1 - r0 + span - 1) / span;
 
-    if (threadIdx.x == 0) {
-        s_dead = 0;
-        for (int s = 0; s < p.stages; ++s) { mbar_init(&full_bar[s], p.share); mbar_init(&empty_bar[s], GS_WARPS); }
-        mbar_init(&x_bar, GS_LOADERS);
+    // a thread a stage: all 33 barriers by one thread make a product of 2.5 us 0.15 longer
+    if (threadIdx.x < 32) {
+        if (lane == 0) {
+            s_dead = 0;
+            mbar_init(&x_bar, GS_LOADERS);
+        }
+        if (lane < p.stages) { mbar_init(&full_bar[lane], p.share); mbar_init(&empty_bar[lane], GS_WARPS); }
         mbar_fence_init();
     }
     __syncthreads();
@@ -348,11 +351,14 @@ static int gs_sms() {
 // How a product's rows of W pass through shared memory.
 // Parts: they decide the order of the sums and nothing else does: the fewest equal ones, in steps of 16, of which three fit beside the rows of x and one
 // set of sums, or two.
-// Pieces of a part: all of it where the block's rows then lie in the ring at once, as copies are few and nothing waits; else the longest equal cut of
-// which four stages fit (a tile takes its stages two by two: with three, one is on its way while it waits); else the longest of which two do.
+// Pieces of a part: all of it where the block's rows then lie in the ring at once, as copies are few and nothing waits, and no more stages than these
+// rows, so that the next kernel's blocks find room beside these ones (512 x 2,112, 1 row: with sixteen stages 2.55, here at most 2.1; but blocks of
+// eight rows leave no more room than eight stages do: 2,560 x 576 with two 3.0, here at most 2.7); else the longest equal cut of which
+// four stages fit (a tile takes its stages two by two: with three, one is on its way while it waits); else, and for blocks of eight rows, which take
+// single stages and wait for each, the longest of which two do.
 // Two sets of the warps' sums unless the second costs a pair of stages.
-// Warps a stage: two; all four where there are three stages, which the tiles wait for whatever is done; one where pieces are short, as what a warp spends
-// on a stage besides its copies then counts.
+// Warps a stage: two; all four where there are three stages, which the tiles wait for whatever is done, and for blocks of eight rows; one where
+// pieces are short, as what a warp spends on a stage besides its copies then counts.
 // us, piece x stages, 64 MB of weights: K = 2,560, 12 rows 2,560 x 3 16.1, 1,280 x 7 14.6; 4,096, 2 rows 4,096 x 3 13.8, 2,048 x 6 13.2; 16 MB: 2,560, 12
 // rows 2,560 x 3 6.2, 1,280 x 7 6.7; 4,096, 2 rows 4.8 and 5.1.  One, two and four warps a stage: 67 MB, 4,096, 16 rows, 1,376 x 4 13.5, 13.2, 13.5 (134 MB
 // 27.3, 26.6, 27.8); 67 to 80 MB, 6,912, 10 rows, 864 x 6 14.4, 14.1, 15.6; 9,728, 8 rows, 608 x 6 21.0, 21.7, 27.0; 8,192, 11 rows, 832 x 3 30.4, 29.7, 28.5;
@@ -379,17 +385,18 @@ static bool gs_plan(int M, int K, int rows, GsPlan* p) {
     if (p->part % (16 * GS_WARPS * GS_CHAINS) == 0) p->part = K;          // whole turns over the chains: dealt as K in one part is
     const int unit = p->part == K ? 16 * GS_WARPS : 16, all = (rows + GS_ROWS - 1) / GS_ROWS * ((K + p->part - 1) / p->part);
     const int whole = fit(p->part, 1);
-    for (int rule = all > 0 && whole >= all && whole >= 2 ? 0 : 1; rule < 3; ++rule)
+    const bool few = rows > 0 && rows <= GS_ROWS;
+    for (int rule = all > 0 && all <= GS_MAX_STAGES && whole >= all && whole >= 2 ? 0 : few ? 2 : 1; rule < 3; ++rule)
         for (int n = 1; n <= p->part / 16; ++n) {
             const int want = rule == 0 && all > 2 ? all : rule == 1 ? 4 : 2, ks = n == 1 ? p->part : ((p->part + n - 1) / n + unit - 1) / unit * unit;
             if (ks < 512 && n > 1) break;                                   // copies this short are not worth having
             const int one = fit(ks, 1), two = fit(ks, 2);
             if (one < want) continue;
-            p->sets = two == one || two >= 6 || (two >= 4 && two / 2 == one / 2) || (rule == 0 && two >= want) ? 2 : 1;
-            const int stages = p->sets == 2 ? two : one;
+            p->sets = rule == 0 ? (two >= want ? 2 : 1) : two == one || two >= 6 || (two >= 4 && two / 2 == one / 2) ? 2 : 1;
+            const int fits = p->sets == 2 ? two : one, stages = rule != 0 ? fits : few ? (fits < 8 ? fits : 8) : want;
             p->ks = ks;
             p->stages = stages > GS_MAX_STAGES ? GS_MAX_STAGES : stages;
-            p->share = p->stages == 3 ? 4 : ks <= 704 && p->stages > 3 ? 1 : 2;
+            p->share = few || p->stages == 3 ? 4 : ks <= 704 && p->stages > 3 ? 1 : 2;
             p->smem = taken(p->sets) + p->stages * stage_of(ks);
             return true;
         }

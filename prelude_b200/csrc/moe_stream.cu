@@ -80,11 +80,13 @@ __global__ void __launch_bounds__(MS_THREADS, 1) moe_stream_kernel(MsParams p) {
     unsigned char* ring = sx + (size_t)p.bufs * MS_ROWS * x_stride;
 
     for (int e = tid; e < p.n_experts; e += MS_THREADS) count[e] = 0;
-    if (tid == 0) {
-        s_dead = 0;
-        for (int s = 0; s < p.stages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], MS_WARPS); }
-        mbar_init(&x_bar[0], 1);
-        mbar_init(&x_bar[1], 1);
+    if (tid < 32) {                                            // a thread a stage, as in gemm_stream.cu
+        if (lane == 0) {
+            s_dead = 0;
+            mbar_init(&x_bar[0], 1);
+            mbar_init(&x_bar[1], 1);
+        }
+        if (lane < p.stages) { mbar_init(&full_bar[lane], 1); mbar_init(&empty_bar[lane], MS_WARPS); }
         mbar_fence_init();
     }
     __syncthreads();
