@@ -351,11 +351,12 @@ static int gs_sms() {
 // How a product's rows of W pass through shared memory.
 // Parts: they decide the order of the sums and nothing else does: the fewest equal ones, in steps of 16, of which three fit beside the rows of x and one
 // set of sums, or two.
-// Pieces of a part: all of it where the block's rows then lie in the ring at once, as copies are few and nothing waits, and no more stages than these
-// rows, so that the next kernel's blocks find room beside these ones (512 x 2,112, 1 row: with sixteen stages 2.55, here at most 2.1; but blocks of
-// eight rows leave no more room than eight stages do: 2,560 x 576 with two 3.0, here at most 2.7); else the longest equal cut of which
-// four stages fit (a tile takes its stages two by two: with three, one is on its way while it waits); else, and for blocks of eight rows, which take
-// single stages and wait for each, the longest of which two do.
+// Pieces of a part: all of it where the block's rows then lie in the ring at once, as copies are few and nothing waits; else the longest equal cut of which
+// four stages fit (a tile takes its stages two by two: with three, one is on its way while it waits); else, and for blocks of eight rows, which
+// take single stages and wait for each, the longest of which two do.
+// Stages: all that fit; where all rows do, no more than eight, so that short rows leave the next kernel's blocks room (512 x 2,112, 1 row: with sixteen
+// 2.55, with eight 2.1), but no fewer: a block that leaves room where the kernel before it ran one to a multiprocessor meets a second of its own
+// there while others have none (2,048 x 2,048, 8 rows, behind a linear-attention step: with the two stages that its rows fill 0.9 us more).
 // Two sets of the warps' sums unless the second costs a pair of stages.
 // Warps a stage: two; all four where there are three stages, which the tiles wait for whatever is done, and for blocks of eight rows; one where
 // pieces are short, as what a warp spends on a stage besides its copies then counts.
@@ -393,7 +394,7 @@ static bool gs_plan(int M, int K, int rows, GsPlan* p) {
             const int one = fit(ks, 1), two = fit(ks, 2);
             if (one < want) continue;
             p->sets = rule == 0 ? (two >= want ? 2 : 1) : two == one || two >= 6 || (two >= 4 && two / 2 == one / 2) ? 2 : 1;
-            const int fits = p->sets == 2 ? two : one, stages = rule != 0 ? fits : few ? (fits < 8 ? fits : 8) : want;
+            const int fits = p->sets == 2 ? two : one, stages = rule == 0 && fits > 8 ? (want > 8 ? want : 8) : fits;
             p->ks = ks;
             p->stages = stages > GS_MAX_STAGES ? GS_MAX_STAGES : stages;
             p->share = few || p->stages == 3 ? 4 : ks <= 704 && p->stages > 3 ? 1 : 2;
