@@ -596,8 +596,7 @@ int dc_run(const DcCall& c) {
     // takes 0.62 of what one of 32 does.  us, slices of 16 / 32 columns: 16 heads, 592 and 1,185 tokens 74 / 86; 1,333 and 2,667 158 / 191; one of
     // 1,000 41 / 72; 32 heads, 592 and 1,185 145 / 132, one of 1,000 80 / 73.
     int narrowest = 16, widest = 32;
-    // (a single chunk has no chain: one of 64, 32 heads, 32 / 30)
-    if (c.counted && c.longest > DC_L && c.E % 32 == 0) {
+    if (c.counted && c.longest > 0 && c.E % 32 == 0) {
         auto takes = [&](int width) {
             const double chain = (c.longest + DC_L - 1) / DC_L, all = (double)c.n_chunks * c.H * (c.E / width) / pb_multiprocessors();
             return (width == 16 ? 0.62 : 1.0) * (chain > all ? chain : all);
